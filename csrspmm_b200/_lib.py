@@ -6,6 +6,8 @@ Loading fails loudly when the shared object has not been built.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 from pathlib import Path
 
 import os
@@ -13,6 +15,9 @@ import os
 PKG = Path(__file__).resolve().parent
 # CSRSPMM_B200_LIBRARY points at another build of the same library (kernel tuning experiments)
 LIB_PATH = Path(os.environ.get("CSRSPMM_B200_LIBRARY") or PKG / "lib" / "libcsrspmm_b200.so")
+
+# the CPython/torch binding of the same library (csrc/torch/binding.cpp), used where a call's host time counts
+BINDING_PATH = PKG / "lib" / "_torch_binding.so"
 
 ABI_VERSION = 2
 OK = 0
@@ -182,6 +187,29 @@ def lib() -> C.CDLL:
         raise LibraryMissing(f"{LIB_PATH} has ABI version {L.csrspmm_b200_abi_version()}, expected {ABI_VERSION}")
     _lib = L
     return L
+
+
+_binding = None
+
+
+def binding():
+    """The CPython/torch binding, bound to the library ``lib()`` loaded."""
+    global _binding
+    if _binding is not None:
+        return _binding
+    L = lib()
+    if not BINDING_PATH.exists():
+        raise LibraryMissing(
+            f"{BINDING_PATH} is missing: build it with `python -m csrspmm_b200.build` "
+            "(there is no fallback path)")
+    loader = importlib.machinery.ExtensionFileLoader("_torch_binding", str(BINDING_PATH))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_torch_binding", BINDING_PATH, loader=loader))
+    loader.exec_module(mod)
+    address = lambda name: C.cast(getattr(L, name), C.c_void_p).value
+    mod.init(*(address(f"csrspmm_b200_{f}") for f in ("spmm", "spmm_sync", "select_kernel", "workspace_bytes", "row_stats_device")),
+             SpmmError)
+    _binding = mod
+    return mod
 
 
 def make_args(M, Kd, Nd, nnz, row_ptr=0, col_idx=0, values=0, B=0, Cptr=0, *, ldb=None, ldc=None,

@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -41,8 +42,9 @@ CMP_LIB = LIB_DIR / "libcsrspmm_b200_cusparse_cmp.so"
 
 
 def sources() -> list[Path]:
-    """Sources of the SpMM library itself (the cuSPARSE comparator under cmp/ is a separate object)."""
-    return sorted(p for p in list(CSRC.rglob("*.cu")) + list(CSRC.rglob("*.cpp")) if p.parent.name != "cmp")
+    """Sources of the SpMM library itself (the cuSPARSE comparator under cmp/ and the
+    torch binding under torch/ are separate objects)."""
+    return sorted(p for p in list(CSRC.rglob("*.cu")) + list(CSRC.rglob("*.cpp")) if p.parent.name not in ("cmp", "torch"))
 
 
 def build_comparator() -> Path:
@@ -56,6 +58,29 @@ def build_comparator() -> Path:
     if res.returncode != 0:
         raise RuntimeError(f"nvcc failed for {CMP_SRC}:\n{res.stdout}\n{res.stderr}")
     return CMP_LIB
+
+
+BINDING_SRC = CSRC / "torch" / "binding.cpp"
+BINDING = LIB_DIR / "_torch_binding.so"
+
+
+def build_binding() -> Path:
+    """lib/_torch_binding.so: the CPython/torch binding (host code only, links torch, gets the SpMM library's
+    functions by address)."""
+    LIB_DIR.mkdir(exist_ok=True)
+    newest = max(p.stat().st_mtime for p in (BINDING_SRC, ROOT / "include" / "csrspmm_b200.h"))
+    if BINDING.exists() and BINDING.stat().st_mtime >= newest:
+        return BINDING
+    from torch.utils import cpp_extension
+    cuda = Path(nvcc()).resolve().parent.parent
+    dirs = [str(ROOT / "include"), *cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{d}" for d in dirs), str(BINDING_SRC),
+           "-o", str(BINDING), *(f"-L{d}" for d in cpp_extension.library_paths()),
+           "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {BINDING_SRC}:\n{res.stdout}\n{res.stderr}")
+    return BINDING
 
 
 def headers() -> list[Path]:
@@ -99,6 +124,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    build_binding()
     return LIB
 
 

@@ -1,0 +1,358 @@
+// CPython/torch binding of the C ABI: what csrspmm_b200/ops.py calls on its per-product path.
+//
+// A small product is over in 3 to 10 us on the GPU, so what a call costs on the host is what the caller
+// waits for.  Reading a tensor's address, sizes and device through Python attributes, filling a ctypes
+// structure field by field and allocating C through torch.empty took 17 us per call; the same work here takes
+// about 4 us, most of it the kernel launch and the allocation of C (1024 x 1024 matrix, 10 entries per row,
+// 64 columns).  Plays the part of the reference's pybind wrappers (torch_csrspmm/binding.cpp:26-32,
+// torch_csrspmm/torch_csrspmm_naive.cpp:11-58) with its argument checks and messages, on the current stream.
+//
+// The library's functions arrive as addresses (init), so that the library itself stays free of torch and the
+// one ctypes loaded is the one used here.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "csrspmm_b200.h"
+
+namespace {
+
+struct Library {
+    int (*spmm)(const csrspmm_b200_args*, csrspmm_b200_stream_t);
+    int (*spmm_sync)(const csrspmm_b200_args*, csrspmm_b200_stream_t);
+    int (*select_kernel)(const csrspmm_b200_args*);
+    size_t (*workspace_bytes)(const csrspmm_b200_args*);
+    int (*row_stats)(int32_t, const int32_t*, int64_t*, csrspmm_b200_stream_t);
+};
+Library g_lib = {};
+PyObject* g_error = nullptr;  // _lib.SpmmError(status, where)
+
+// A failed library call, turned into SpmmError at the Python boundary.
+struct LibraryError {
+    int status;
+    const char* where;
+};
+
+void raise_library_error(const LibraryError& e)
+{
+    PyObject* exc = PyObject_CallFunction(g_error, "is", e.status, e.where);
+    if (exc == nullptr) return;
+    PyErr_SetObject(g_error, exc);
+    Py_DECREF(exc);
+}
+
+void want(bool ok, const char* message)
+{
+    if (!ok) throw std::runtime_error(message);
+}
+
+const at::Tensor& tensor_of(PyObject* o, const char* name)
+{
+    if (!THPVariable_Check(o)) throw c10::TypeError({__func__, __FILE__, static_cast<uint32_t>(__LINE__)}, std::string(name) + " must be a tensor");
+    return THPVariable_Unpack(o);
+}
+
+// The checks of the reference's wrappers, with its wording (torch_csrspmm/torch_csrspmm_naive.cpp:19-26).
+void check_csr(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, bool packed)
+{
+    want(rp.is_cuda(), "A_row_ptr must be a CUDA tensor");
+    want(ci.is_cuda(), "A_col_idx must be a CUDA tensor");
+    want(va.is_cuda(), "A_values must be a CUDA tensor");
+    want(B.is_cuda(), "B must be a CUDA tensor");
+    want(rp.scalar_type() == at::kInt, "A_row_ptr must be int32");
+    want(ci.scalar_type() == at::kInt, "A_col_idx must be int32");
+    if (packed) want(va.scalar_type() == at::kByte, "packed A_values must be uint8");
+    else want(va.scalar_type() == at::kFloat, "A_values must be float32");
+    want(B.scalar_type() == at::kFloat, "B must be float32");
+    want(B.dim() == 2 && rp.dim() == 1 && ci.dim() == 1 && va.dim() == 1 && rp.size(0) >= 1,
+         "expected 1-D row_ptr/col_idx/values and 2-D B");
+    want(rp.is_contiguous() && ci.is_contiguous() && va.is_contiguous(), "row_ptr, col_idx and values must be contiguous");
+    want(B.stride(1) == 1 || B.size(1) <= 1, "B must be row-major (unit stride along its columns)");
+    const auto dev = B.device();
+    want(rp.device() == dev && ci.device() == dev && va.device() == dev, "all tensors must be on the same device");
+}
+
+template <class T>
+T* address(const at::Tensor& t)
+{
+    return static_cast<T*>(t.data_ptr());
+}
+
+// Scratch of one call from torch's caching allocator, handed back when the call has been enqueued (the
+// allocator keeps the block for the stream's next request).
+class Scratch {
+public:
+    Scratch() = default;
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch()
+    {
+        if (ptr_) c10::cuda::CUDACachingAllocator::raw_delete(ptr_);
+    }
+    void* get(size_t bytes, cudaStream_t stream)
+    {
+        ptr_ = c10::cuda::CUDACachingAllocator::raw_alloc_with_stream(std::max<size_t>(bytes, 256), stream);
+        return ptr_;
+    }
+
+private:
+    void* ptr_ = nullptr;
+};
+
+struct Product {
+    at::Tensor rp, ci, va, B, C;  // C undefined: allocate it
+    at::Tensor workspace;         // undefined: take it from the allocator
+    double alpha = 1.0, beta = 0.0;
+    int entry = 0, kernel = 0;
+    int max_row_nnz = 0;
+    bool packed = false;
+    double scale = 1.0;
+    int64_t nnz = -1;  // -1: col_idx's length
+    int32_t* status_word = nullptr;
+    const csrspmm_b200_schedule* schedule = nullptr;
+    bool sync = false;
+};
+
+at::Tensor run_product(Product& q)
+{
+    check_csr(q.rp, q.ci, q.va, q.B, q.packed);
+    const int64_t M = q.rp.size(0) - 1, Kd = q.B.size(0), Nd = q.B.size(1);
+    const int64_t n = q.nnz < 0 ? q.ci.size(0) : q.nnz;
+    if (q.packed) want(q.va.size(0) >= (n + 1) / 2, "packed values too short");
+    else want(q.va.size(0) == n, "values and col_idx differ in length");
+    const c10::cuda::CUDAGuard guard(q.B.device());
+    if (!q.C.defined()) {
+        want(q.beta == 0.0, "beta != 0 needs C_out");
+        q.C = at::detail::empty_cuda({M, Nd}, at::kFloat, q.B.device(), std::nullopt);
+    } else {
+        want(q.C.is_cuda() && q.C.scalar_type() == at::kFloat && q.C.dim() == 2 && q.C.size(0) == M && q.C.size(1) == Nd &&
+                 q.C.device() == q.B.device(),
+             "C_out must be a float32 CUDA tensor of shape (M, Nd) on B's device");
+        want(q.C.stride(1) == 1 || Nd <= 1, "C_out must be row-major");
+    }
+    csrspmm_b200_args a = {};
+    a.struct_size = sizeof(a);
+    a.M = static_cast<int32_t>(M);
+    a.Kd = static_cast<int32_t>(Kd);
+    a.Nd = static_cast<int32_t>(Nd);
+    a.nnz = n;
+    a.row_ptr = address<int32_t>(q.rp);
+    a.col_idx = address<int32_t>(q.ci);
+    a.values = q.va.data_ptr();
+    a.value_format = q.packed ? CSRSPMM_B200_VALUES_E2M1 : CSRSPMM_B200_VALUES_F32;
+    a.value_scale = q.packed ? static_cast<float>(q.scale) : 1.0f;
+    a.B = address<float>(q.B);
+    a.ldb = std::max(Kd > 1 ? q.B.stride(0) : Nd, Nd);
+    a.C = address<float>(q.C);
+    a.ldc = std::max(M > 1 ? q.C.stride(0) : Nd, Nd);
+    a.alpha = static_cast<float>(q.alpha);
+    a.beta = static_cast<float>(q.beta);
+    a.entry = q.entry;
+    a.kernel = q.kernel;
+    a.max_row_nnz = q.max_row_nnz;
+    a.status_word = q.status_word;
+    a.schedule = q.schedule;
+
+    const auto stream = c10::cuda::getCurrentCUDAStream(q.B.device().index());
+    Scratch scratch;
+    if (M > 0 && Nd > 0) {
+        const int chosen = g_lib.select_kernel(&a);
+        if (chosen < 0) throw LibraryError{-chosen, "csrspmm_b200_select_kernel"};
+        if (chosen != CSRSPMM_B200_KERNEL_ROW) {
+            const size_t need = g_lib.workspace_bytes(&a);
+            if (q.workspace.defined() && q.workspace.nbytes() >= need) {
+                a.workspace = q.workspace.data_ptr();
+                a.workspace_bytes = q.workspace.nbytes();
+                if (q.workspace.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(q.workspace.storage().data_ptr(), stream);
+            } else {
+                a.workspace = scratch.get(need, stream);
+                a.workspace_bytes = std::max<size_t>(need, 256);
+            }
+        }
+    }
+    int status;
+    {
+        // as under ctypes: a launch may wait for room in the stream's queue, and sync waits for the GPU
+        pybind11::gil_scoped_release nogil;
+        status = (q.sync ? g_lib.spmm_sync : g_lib.spmm)(&a, reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
+    }
+    if (status != CSRSPMM_B200_OK) throw LibraryError{status, "csrspmm_b200_spmm"};
+    return q.C;
+}
+
+// ---- the longest row behind a row_ptr tensor, measured once ----------------------------------------------
+// One small kernel and a host read, remembered per (address, length, version, device) for the last 64
+// matrices.  It only steers the kernel choice, so a stale entry -- another matrix later placed at the same
+// address -- costs speed, never correctness.  The GIL guards the table.
+struct LongestRow {
+    const void* row_ptr;
+    int64_t length;
+    int64_t version;
+    int device;
+    int longest;
+};
+constexpr int kLongestRows = 64;
+LongestRow g_longest[kLongestRows];
+int g_longest_count = 0, g_longest_next = 0;
+
+int longest_row(const at::Tensor& rp)
+{
+    if (!rp.is_cuda() || rp.scalar_type() != at::kInt || rp.dim() != 1 || rp.size(0) < 2 || !rp.is_contiguous()) return 0;
+    const LongestRow key = {rp.data_ptr(), rp.size(0), rp.is_inference() ? 0 : (int64_t)rp._version(), rp.device().index(), 0};
+    for (int k = 0; k < g_longest_count; ++k) {
+        const LongestRow& e = g_longest[k];
+        if (e.row_ptr == key.row_ptr && e.length == key.length && e.version == key.version && e.device == key.device) return e.longest;
+    }
+    const c10::cuda::CUDAGuard guard(rp.device());
+    int64_t stats[4] = {0, 0, 0, 0};
+    int status;
+    {
+        const auto stream = c10::cuda::getCurrentCUDAStream(rp.device().index());
+        pybind11::gil_scoped_release nogil;
+        status = g_lib.row_stats(static_cast<int32_t>(rp.size(0) - 1), address<int32_t>(rp), stats,
+                                 reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
+    }
+    if (status != CSRSPMM_B200_OK) throw LibraryError{status, "csrspmm_b200_row_stats_device"};
+    LongestRow& e = g_longest[g_longest_next];
+    e = key;
+    e.longest = static_cast<int>(std::min<int64_t>(stats[0], INT32_MAX));
+    g_longest_next = (g_longest_next + 1) % kLongestRows;
+    g_longest_count = std::min(g_longest_count + 1, kLongestRows);
+    return e.longest;
+}
+
+// ---- Python functions -----------------------------------------------------------------------------------
+
+#define BEGIN_BINDING HANDLE_TH_ERRORS try {
+#define END_BINDING                   \
+    }                                 \
+    catch (const LibraryError& e)     \
+    {                                 \
+        raise_library_error(e);       \
+        return nullptr;               \
+    }                                 \
+    END_HANDLE_TH_ERRORS
+
+double as_double(PyObject* o)
+{
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw python_error();
+    return v;
+}
+
+long long as_integer(PyObject* o)
+{
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw python_error();
+    return v;
+}
+
+void expect_args(Py_ssize_t got, Py_ssize_t wanted)
+{
+    if (got != wanted) throw std::runtime_error("csrspmm_b200 binding: wrong number of arguments");
+}
+
+// init(spmm, spmm_sync, select_kernel, workspace_bytes, row_stats, SpmmError): addresses of the C functions
+PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 6);
+    auto fn = [&](int k) { return reinterpret_cast<void*>(static_cast<uintptr_t>(as_integer(args[k]))); };
+    g_lib.spmm = reinterpret_cast<decltype(g_lib.spmm)>(fn(0));
+    g_lib.spmm_sync = reinterpret_cast<decltype(g_lib.spmm_sync)>(fn(1));
+    g_lib.select_kernel = reinterpret_cast<decltype(g_lib.select_kernel)>(fn(2));
+    g_lib.workspace_bytes = reinterpret_cast<decltype(g_lib.workspace_bytes)>(fn(3));
+    g_lib.row_stats = reinterpret_cast<decltype(g_lib.row_stats)>(fn(4));
+    Py_INCREF(args[5]);
+    Py_XSETREF(g_error, args[5]);
+    Py_RETURN_NONE;
+    END_BINDING
+}
+
+// spmm(row_ptr, col_idx, values, B, C|None, alpha, beta, entry, kernel, max_row_nnz, e2m1_scale|None, nnz|None,
+//      workspace|None, status_word|None, sync, schedule handle) -> C
+PyObject* py_spmm(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 16);
+    Product q;
+    q.rp = tensor_of(args[0], "A_row_ptr");
+    q.ci = tensor_of(args[1], "A_col_idx");
+    q.va = tensor_of(args[2], "A_values");
+    q.B = tensor_of(args[3], "B");
+    if (args[4] != Py_None) q.C = tensor_of(args[4], "C_out");
+    q.alpha = as_double(args[5]);
+    q.beta = as_double(args[6]);
+    q.entry = static_cast<int>(as_integer(args[7]));
+    q.kernel = static_cast<int>(as_integer(args[8]));
+    q.max_row_nnz = static_cast<int>(as_integer(args[9]));
+    q.packed = args[10] != Py_None;
+    if (q.packed) q.scale = as_double(args[10]);
+    if (args[11] != Py_None) q.nnz = as_integer(args[11]);
+    if (args[12] != Py_None) q.workspace = tensor_of(args[12], "workspace");
+    if (args[13] != Py_None) q.status_word = address<int32_t>(tensor_of(args[13], "status_word"));
+    q.sync = PyObject_IsTrue(args[14]) == 1;
+    q.schedule = reinterpret_cast<const csrspmm_b200_schedule*>(static_cast<uintptr_t>(as_integer(args[15])));
+    return THPVariable_Wrap(run_product(q));
+    END_BINDING
+}
+
+// op(entry, row_ptr, col_idx, values, B, alpha) -> new C: the reference's ops.  The longest row is measured, not
+// believed: three of the reference's five ops carry no such argument, and a stale value passed to the other
+// two would send a skewed matrix to the whole-row kernel.
+PyObject* py_op(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 6);
+    Product q;
+    q.entry = static_cast<int>(as_integer(args[0]));
+    q.rp = tensor_of(args[1], "A_row_ptr");
+    q.ci = tensor_of(args[2], "A_col_idx");
+    q.va = tensor_of(args[3], "A_values");
+    q.B = tensor_of(args[4], "B");
+    q.alpha = as_double(args[5]);
+    q.max_row_nnz = longest_row(q.rp);
+    return THPVariable_Wrap(run_product(q));
+    END_BINDING
+}
+
+// enqueue(address of a csrspmm_b200_args, device index): a prepared product, on the device's current stream
+PyObject* py_enqueue(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 2);
+    const auto* a = reinterpret_cast<const csrspmm_b200_args*>(static_cast<uintptr_t>(as_integer(args[0])));
+    const auto stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(as_integer(args[1])));
+    int status;
+    {
+        pybind11::gil_scoped_release nogil;
+        status = g_lib.spmm(a, reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
+    }
+    if (status != CSRSPMM_B200_OK) throw LibraryError{status, "csrspmm_b200_spmm"};
+    Py_RETURN_NONE;
+    END_BINDING
+}
+
+#define FASTCALL(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL
+PyMethodDef g_methods[] = {
+    {"init", FASTCALL(py_init), nullptr},
+    {"spmm", FASTCALL(py_spmm), nullptr},
+    {"op", FASTCALL(py_op), nullptr},
+    {"enqueue", FASTCALL(py_enqueue), nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__torch_binding() { return PyModule_Create(&g_module); }

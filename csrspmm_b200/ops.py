@@ -5,7 +5,9 @@ The reference's ops are pybind wrappers that fill the two POD views from ``data_
 ``csrspmm::launch_*`` on the legacy default stream without a device guard
 (torch_csrspmm/torch_csrspmm_naive.cpp:11-58 and its four siblings).  Here the same arguments go
 through ``csrspmm_b200_spmm`` on torch's *current* stream of the tensors' device, and a failed
-call raises instead of returning an unwritten C.
+call raises instead of returning an unwritten C.  ``spmm``, the five ops and ``SpmmCall`` reach the library
+through the CPython binding (csrc/torch/binding.cpp), which also makes the argument checks; everything that is
+called once per matrix goes through ctypes.
 """
 from __future__ import annotations
 
@@ -121,53 +123,11 @@ def spmm(row_ptr, col_idx, values, B, C_out=None, alpha=1.0, beta=0.0, *, entry=
     from torch's caching allocator.  ``sync=True`` waits and raises on device-side errors.
     ``schedule`` is an optional ``Schedule`` built for this matrix.
     """
-    packed = e2m1_scale is not None
-    _check_csr(row_ptr, col_idx, values, B, packed)
-    M = row_ptr.numel() - 1
-    Kd, Nd = B.size(0), B.size(1)
-    n = int(col_idx.numel() if nnz is None else nnz)
-    if not packed and values.numel() != n:
-        raise RuntimeError("values and col_idx differ in length")
-    if packed and values.numel() < (n + 1) // 2:
-        raise RuntimeError("packed values too short")
-    if C_out is None:
-        if beta != 0.0:
-            raise RuntimeError("beta != 0 needs C_out")
-        C_out = torch.empty((M, Nd), dtype=torch.float32, device=B.device)
-    else:
-        if not C_out.is_cuda or C_out.dtype != torch.float32 or C_out.shape != (M, Nd) or C_out.device != B.device:
-            raise RuntimeError("C_out must be a float32 CUDA tensor of shape (M, Nd) on B's device")
-        if C_out.stride(1) != 1 and Nd > 1:
-            raise RuntimeError("C_out must be row-major")
-    L = _lib.lib()
-    ldb = B.stride(0) if Kd > 1 else Nd
-    ldc = C_out.stride(0) if M > 1 else Nd
-    a = _lib.make_args(M, Kd, Nd, n, row_ptr.data_ptr(), col_idx.data_ptr(), values.data_ptr(), B.data_ptr(),
-                       C_out.data_ptr(), ldb=max(ldb, Nd), ldc=max(ldc, Nd), alpha=alpha, beta=beta,
-                       entry=_ENTRY[entry] if isinstance(entry, str) else int(entry),
-                       kernel=_lib.KERNEL_IDS[kernel] if isinstance(kernel, str) else int(kernel),
-                       max_row_nnz=max_row_nnz,
-                       value_format=_lib.VALUES_E2M1 if packed else _lib.VALUES_F32,
-                       value_scale=float(e2m1_scale) if packed else 1.0,
-                       status_word=status_word.data_ptr() if status_word is not None else 0,
-                       schedule=schedule.handle if schedule is not None else 0)
-    with torch.cuda.device(B.device):
-        if M > 0 and Nd > 0:
-            chosen = L.csrspmm_b200_select_kernel(C.byref(a))
-            if chosen < 0:
-                raise _lib.SpmmError(-chosen, "csrspmm_b200_select_kernel")
-            if chosen != _lib.KERNEL_ROW:
-                need = int(L.csrspmm_b200_workspace_bytes(C.byref(a)))
-                if workspace is None or workspace.numel() * workspace.element_size() < need:
-                    workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=B.device)
-                a.workspace = workspace.data_ptr()
-                a.workspace_bytes = workspace.numel() * workspace.element_size()
-        stream = torch.cuda.current_stream(B.device).cuda_stream
-        fn = L.csrspmm_b200_spmm_sync if sync else L.csrspmm_b200_spmm
-        _lib.check(fn(C.byref(a), C.c_void_p(stream)), "csrspmm_b200_spmm")
-        if workspace is not None:
-            workspace.record_stream(torch.cuda.current_stream(B.device))
-    return C_out
+    return _lib.binding().spmm(row_ptr, col_idx, values, B, C_out, alpha, beta,
+                               _ENTRY[entry] if isinstance(entry, str) else entry,
+                               _lib.KERNEL_IDS[kernel] if isinstance(kernel, str) else kernel,
+                               max_row_nnz, e2m1_scale, nnz, workspace, status_word, sync,
+                               schedule.handle if schedule is not None else 0)
 
 
 def spmm_tiled(row_ptr, col_idx, values, B, C_out=None, alpha=1.0, beta=0.0, *, panel_rows=0, e2m1_scale=None,
@@ -251,14 +211,13 @@ class SpmmCall:
                 self.args.workspace_bytes = workspace.numel() * workspace.element_size()
         self.workspace = workspace  # scratch of the split kernels (None for the row kernel); may be shared
         self._keep = (row_ptr, col_idx, values, B, C_out, workspace, status_word, schedule)
-        self._ref = C.byref(self.args)
+        self._enqueue = _lib.binding().enqueue
+        self._where = (C.addressof(self.args), B.device.index)
         self.out = C_out
 
     def __call__(self):
         """Enqueue on the current stream of the operands' device (which must be the current device)."""
-        st = self.L.csrspmm_b200_spmm(self._ref, C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream))
-        if st != _lib.OK:
-            raise _lib.SpmmError(st, "csrspmm_b200_spmm")
+        self._enqueue(*self._where)
         return self.out
 
 
@@ -277,51 +236,28 @@ def selected_kernel(M, Kd, Nd, nnz, *, entry="naive", max_row_nnz=0, kernel="aut
 # (torch_csrspmm/torch_csrspmm_naive.cpp:32-34); the product with zero is skipped here, which
 # changes nothing but the sign of an exact zero.
 
-_ROW_STATS_CACHE: dict = {}
-
-
-def _longest_row_hint(row_ptr) -> int:
-    """Longest row of the matrix behind this row_ptr tensor, measured once (one small kernel and a
-    host read) and remembered per (address, length, version).  It only steers the kernel choice, so
-    a stale entry -- another matrix later placed at the same address -- costs speed, never
-    correctness."""
-    key = (row_ptr.data_ptr(), row_ptr.numel(), row_ptr._version, row_ptr.device.index)
-    hit = _ROW_STATS_CACHE.get(key)
-    if hit is None:
-        if len(_ROW_STATS_CACHE) >= 64:
-            _ROW_STATS_CACHE.pop(next(iter(_ROW_STATS_CACHE)))
-        hit = row_stats(row_ptr)["max_row_nnz"] if row_ptr.numel() > 1 else 0
-        _ROW_STATS_CACHE[key] = hit
-    return hit
-
-
-def _op(entry, row_ptr, col_idx, values, B, alpha, beta, max_row_nnz=0):
-    del beta
-    if row_ptr.is_cuda and row_ptr.dtype == torch.int32:
-        # measured, not believed: three of the reference's five ops carry no such argument, and a stale value
-        # passed to the other two would send a skewed matrix to the whole-row kernel
-        max_row_nnz = _longest_row_hint(row_ptr)
-    return spmm(row_ptr, col_idx, values, B, None, float(alpha), 0.0, entry=entry, max_row_nnz=int(max_row_nnz))
+def _op(entry, row_ptr, col_idx, values, B, alpha):
+    return _lib.binding().op(_ENTRY[entry], row_ptr, col_idx, values, B, alpha)
 
 
 def csrspmm_naive(A_rowptr, A_colidx, A_values, B, alpha, beta):
-    return _op("naive", A_rowptr, A_colidx, A_values, B, alpha, beta)
+    return _op("naive", A_rowptr, A_colidx, A_values, B, alpha)
 
 
 def csrspmm_warp_per_row(A_rowptr, A_colidx, A_values, B, alpha, beta):
-    return _op("warp_per_row", A_rowptr, A_colidx, A_values, B, alpha, beta)
+    return _op("warp_per_row", A_rowptr, A_colidx, A_values, B, alpha)
 
 
 def csrspmm_warp_per_row_smem(A_rowptr, A_colidx, A_values, A_max_row_nnz, B, alpha, beta):
-    return _op("warp_per_row_smem", A_rowptr, A_colidx, A_values, B, alpha, beta, A_max_row_nnz)
+    return _op("warp_per_row_smem", A_rowptr, A_colidx, A_values, B, alpha)
 
 
 def csrspmm_warp_per_row_fp4(A_rowptr, A_colidx, A_values, B, alpha, beta):
-    return _op("warp_per_row_fp4", A_rowptr, A_colidx, A_values, B, alpha, beta)
+    return _op("warp_per_row_fp4", A_rowptr, A_colidx, A_values, B, alpha)
 
 
 def csrspmm_warp_per_row_smem_fp4(A_rowptr, A_colidx, A_values, A_max_row_nnz, B, alpha, beta):
-    return _op("warp_per_row_smem_fp4", A_rowptr, A_colidx, A_values, B, alpha, beta, A_max_row_nnz)
+    return _op("warp_per_row_smem_fp4", A_rowptr, A_colidx, A_values, B, alpha)
 
 
 # ---- helpers over the host-only / utility entry points -----------------------------------------------
