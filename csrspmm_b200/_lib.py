@@ -43,6 +43,7 @@ EXPORTED_SYMBOLS = (
     "csrspmm_b200_e2m1_encode", "csrspmm_b200_e2m1_decode", "csrspmm_b200_dense2csr_count",
     "csrspmm_b200_dense2csr_fill", "csrspmm_b200_csr2dense", "csrspmm_b200_copy_rows", "csrspmm_b200_column_panels",
     "csrspmm_b200_e2m1_scale_device", "csrspmm_b200_e2m1_encode_device", "csrspmm_b200_e2m1_decode_device",
+    "csrspmm_b200_e2m1_quantize_device",
     "csrspmm_b200_spmm_tiled", "csrspmm_b200_tiled_workspace_bytes", "csrspmm_b200_tiled_panel_rows",
     "csrspmm_b200_schedule_create", "csrspmm_b200_schedule_destroy", "csrspmm_b200_schedule_info_get",
 )
@@ -205,9 +206,7 @@ def binding():
     loader = importlib.machinery.ExtensionFileLoader("_torch_binding", str(BINDING_PATH))
     mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_torch_binding", BINDING_PATH, loader=loader))
     loader.exec_module(mod)
-    address = lambda name: C.cast(getattr(L, name), C.c_void_p).value
-    mod.init(*(address(f"csrspmm_b200_{f}") for f in ("spmm", "spmm_sync", "select_kernel", "workspace_bytes", "row_stats_device")),
-             SpmmError)
+    mod.init(SpmmError, {n[len("csrspmm_b200_"):]: C.cast(getattr(L, n), C.c_void_p).value for n in EXPORTED_SYMBOLS})
     _binding = mod
     return mod
 

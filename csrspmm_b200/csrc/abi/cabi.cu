@@ -17,6 +17,7 @@
 #include "csrspmm_b200.h"
 #include "launch.h"
 #include "plan.h"
+#include "scratch.h"
 
 using namespace csrspmm_b200;
 
@@ -691,8 +692,9 @@ int csrspmm_b200_validate_csr_device(int32_t M, int32_t Kd, int64_t nnz, const i
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    unsigned* d_flags = nullptr;
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_flags), sizeof(unsigned), st));
+    Scratch scratch(st);
+    CUDA_TRY(scratch.alloc(sizeof(unsigned)));
+    unsigned* d_flags = scratch.as<unsigned>();
     CUDA_TRY(cudaMemsetAsync(d_flags, 0, sizeof(unsigned), st));
     const int threads = 256;
     long long blocks = ((long long)M + threads - 1) / threads;
@@ -702,7 +704,6 @@ int csrspmm_b200_validate_csr_device(int32_t M, int32_t Kd, int64_t nnz, const i
     CUDA_TRY(cudaGetLastError());
     unsigned flags = 0;
     CUDA_TRY(cudaMemcpyAsync(&flags, d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaFreeAsync(d_flags, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     *problems = flags;
     if (flags & 15u) {
@@ -720,25 +721,20 @@ int csrspmm_b200_row_stats_device(int32_t M, const int32_t* row_ptr, int64_t sta
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    int first = 0, last = 0;
-    CUDA_TRY(cudaMemcpyAsync(&first, row_ptr, 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(&last, row_ptr + M, 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    const long long nnz = (long long)last - first;
-    const long long mean = M > 0 ? nnz / M : 0;
-    unsigned long long* d_stats = nullptr;
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_stats), 4 * sizeof(unsigned long long), st));
-    CUDA_TRY(cudaMemsetAsync(d_stats, 0, 4 * sizeof(unsigned long long), st));
-    const int threads = 256;
-    long long blocks = ((long long)M + threads - 1) / threads;
+    // every CTA leaves its share of the four numbers, one more CTA adds them up and writes them where the host
+    // reads them: no zeroed counters, one wait
+    long long blocks = ((long long)M + kStatsThreads - 1) / kStatsThreads;
     if (blocks < 1) blocks = 1;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    row_stats_kernel<<<(unsigned)blocks, threads, 0, st>>>(M, row_ptr, 32 * (mean + 1), d_stats);
+    if (blocks > kStatsMaxCtas) blocks = kStatsMaxCtas;
+    Scratch scratch(st);
+    CUDA_TRY(scratch.alloc(4 * sizeof(long long) * (size_t)blocks));
+    Results results(st);
+    CUDA_TRY(results.init());
+    row_stats_kernel<<<(unsigned)blocks, kStatsThreads, 0, st>>>(M, row_ptr, scratch.as<long long>());
+    row_stats_sum_kernel<<<1, kStatsThreads, 0, st>>>((int)blocks, scratch.as<long long>(), results.ptr());
     CUDA_TRY(cudaGetLastError());
-    unsigned long long h[4] = {0, 0, 0, 0};
-    CUDA_TRY(cudaMemcpyAsync(h, d_stats, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaFreeAsync(d_stats, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    long long h[4] = {0, 0, 0, 0};
+    CUDA_TRY(results.wait(h, 4));
     for (int k = 0; k < 4; ++k) stats[k] = (int64_t)h[k];
     return CSRSPMM_B200_OK;
 }

@@ -9,6 +9,8 @@
 #include "../kernels/convert_kernels.cuh"
 #include "csrspmm_b200.h"
 #include "plan.h"
+#include "scan.h"
+#include "scratch.h"
 
 using namespace csrspmm_b200;
 
@@ -22,6 +24,27 @@ using namespace csrspmm_b200;
         }                                                                                     \
     } while (0)
 
+namespace {
+
+bool rows_on_16_bytes(const float* dense, int64_t ld) { return ld % 4 == 0 && (reinterpret_cast<uintptr_t>(dense) & 15u) == 0; }
+
+unsigned convert_grid(int32_t H, int wpr)
+{
+    const int rows = (kConvertThreads / 32) / wpr;
+    return (unsigned)(((long long)H + rows - 1) / rows);
+}
+
+// CTAs of the e2m1 kernels: enough to fill the chip, each with several 16-byte loads per thread
+unsigned codec_grid(int64_t n)
+{
+    const long long want = (n + kCodecThreads * kCodecPer - 1) / (kCodecThreads * kCodecPer);
+    return (unsigned)(want < kCodecMaxCtas ? want : kCodecMaxCtas);
+}
+
+float scale_from(float absmax) { return absmax > 0.0f ? absmax / 6.0f : 1.0f; }
+
+}  // namespace
+
 extern "C" {
 
 int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, int32_t* row_ptr,
@@ -32,31 +55,33 @@ int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const long long n = H;  // row_ptr[1..H] is scanned
-    const int nblocks = (int)((n + kScanBlock - 1) / kScanBlock);
-    int* scratch = nullptr;  // [0] = max row, [1..] = block sums
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&scratch), sizeof(int) * (size_t)(nblocks + 2), st));
-    CUDA_TRY(cudaMemsetAsync(scratch, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(row_ptr, 0, sizeof(int), st));
-    int last = 0, mx = 0;
-    if (H > 0) {
-        const unsigned grid = (unsigned)((n + 7) / 8);
-        dense_count_kernel<<<grid, 256, 0, st>>>(H, W, dense, ld, tol, row_ptr, scratch);
-        scan_blocks_kernel<<<nblocks, kScanBlock, 0, st>>>(row_ptr + 1, n, scratch + 1);
-        scan_block_sums_kernel<<<1, kScanBlock, 0, st>>>(scratch + 1, nblocks);
-        add_block_offsets_kernel<<<nblocks, kScanBlock, 0, st>>>(row_ptr + 1, n, scratch + 1);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemcpyAsync(&last, row_ptr + H, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(&mx, scratch, sizeof(int), cudaMemcpyDeviceToHost, st));
+    *nnz_out = 0;
+    if (max_row_nnz_out) *max_row_nnz_out = 0;
+    if (H == 0) {
+        CUDA_TRY(cudaMemsetAsync(row_ptr, 0, sizeof(int), st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        return CSRSPMM_B200_OK;
     }
-    CUDA_TRY(cudaFreeAsync(scratch, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    *nnz_out = last;
-    if (max_row_nnz_out) *max_row_nnz_out = mx;
-    if (last < 0) {  // more than 2^31 - 1 kept entries: the int32 offsets wrapped
+    const size_t scan_bytes = (scan_scratch_bytes(H) + 255) / 256 * 256;
+    Scratch scratch(st);  // the scan's, then one count per row
+    CUDA_TRY(scratch.alloc(scan_bytes + sizeof(int) * (size_t)H));
+    int* counts = reinterpret_cast<int*>(scratch.as<char>() + scan_bytes);
+    Results results(st);
+    CUDA_TRY(results.init());
+    const int wpr = convert_warps_per_row(W);
+    const unsigned grid = convert_grid(H, wpr);
+    if (rows_on_16_bytes(dense, ld)) dense_count_kernel<true><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, counts);
+    else dense_count_kernel<false><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, counts);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(exclusive_scan(counts, H, row_ptr, scratch.as<void>(), results.ptr(), st));
+    long long out[2] = {0, 0};
+    CUDA_TRY(results.wait(out, 2));
+    if (out[0] > 0x7fffffffLL) {  // the int32 offsets wrapped
         set_last_error("dense2csr_count: more than 2^31-1 non-zeros");
         return CSRSPMM_B200_ERR_UNSUPPORTED;
     }
+    *nnz_out = out[0];
+    if (max_row_nnz_out) *max_row_nnz_out = (int32_t)out[1];
     return CSRSPMM_B200_OK;
 }
 
@@ -73,7 +98,12 @@ int csrspmm_b200_dense2csr_fill(int32_t H, int32_t W, const float* dense, int64_
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    dense_fill_kernel<<<(unsigned)(((long long)H + 7) / 8), 256, 0, st>>>(H, W, dense, ld, tol, row_ptr, col_idx, values);
+    const int wpr = convert_warps_per_row(W);
+    const unsigned grid = convert_grid(H, wpr);
+    if (rows_on_16_bytes(dense, ld))
+        dense_fill_kernel<true><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, row_ptr, col_idx, values);
+    else
+        dense_fill_kernel<false><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, row_ptr, col_idx, values);
     CUDA_TRY(cudaGetLastError());
     return CSRSPMM_B200_OK;
 }
@@ -104,21 +134,17 @@ int csrspmm_b200_e2m1_scale_device(int64_t n, const float* values, float* scale_
     *scale_out = 1.0f;
     if (n == 0) return CSRSPMM_B200_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    unsigned* d_bits = nullptr;
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_bits), sizeof(unsigned), st));
-    CUDA_TRY(cudaMemsetAsync(d_bits, 0, sizeof(unsigned), st));
-    const long long want = (n + 255) / 256;
-    const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
-    e2m1_absmax_kernel<<<grid, 256, 0, st>>>(n, values, d_bits);
+    Scratch partial(st);
+    CUDA_TRY(partial.alloc(sizeof(float) * kCodecMaxCtas));
+    const unsigned grid = codec_grid(n);
+    e2m1_absmax_kernel<<<grid, kCodecThreads, 0, st>>>(n, values, partial.as<float>());
     CUDA_TRY(cudaGetLastError());
-    unsigned bits = 0;
-    CUDA_TRY(cudaMemcpyAsync(&bits, d_bits, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaFreeAsync(d_bits, st));
+    float h[kCodecMaxCtas];
+    CUDA_TRY(cudaMemcpyAsync(h, partial.as<float>(), sizeof(float) * grid, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
-    float mx;
-    static_assert(sizeof(mx) == sizeof(bits), "float is 32 bits");
-    memcpy(&mx, &bits, sizeof(mx));
-    *scale_out = mx > 0.0f ? mx / 6.0f : 1.0f;
+    float mx = 0.0f;
+    for (unsigned k = 0; k < grid; ++k) mx = h[k] > mx ? h[k] : mx;
+    *scale_out = scale_from(mx);
     return CSRSPMM_B200_OK;
 }
 
@@ -130,10 +156,37 @@ int csrspmm_b200_e2m1_encode_device(int64_t n, const float* values, float scale,
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
     if (n == 0) return CSRSPMM_B200_OK;
-    const long long want = ((n + 1) / 2 + 255) / 256;
-    const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
-    e2m1_encode_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, values, scale, packed);
+    e2m1_encode_kernel<<<codec_grid(n), kCodecThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, values, scale, nullptr, 0, packed, nullptr);
     CUDA_TRY(cudaGetLastError());
+    return CSRSPMM_B200_OK;
+}
+
+int csrspmm_b200_e2m1_quantize_device(int64_t n, const float* values, float* scale_out, uint8_t* packed,
+                                      csrspmm_b200_stream_t stream)
+{
+    if (n < 0 || scale_out == nullptr || (n > 0 && (values == nullptr || packed == nullptr))) {
+        set_last_error("e2m1_quantize_device: bad argument");
+        return CSRSPMM_B200_ERR_BAD_ARG;
+    }
+    *scale_out = 1.0f;
+    if (n == 0) return CSRSPMM_B200_OK;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    Scratch partial(st);
+    CUDA_TRY(partial.alloc(sizeof(float) * kCodecMaxCtas));
+    Results results(st);
+    CUDA_TRY(results.init());
+    const unsigned grid = codec_grid(n);
+    e2m1_absmax_kernel<<<grid, kCodecThreads, 0, st>>>(n, values, partial.as<float>());
+    e2m1_encode_kernel<<<grid, kCodecThreads, 0, st>>>(n, values, 1.0f, partial.as<float>(), (int)grid, packed, results.ptr());
+    CUDA_TRY(cudaGetLastError());
+    long long bits = 0;
+    CUDA_TRY(results.wait(&bits, 1));
+    const unsigned word = (unsigned)bits;
+    memcpy(scale_out, &word, sizeof(word));
+    if (!(*scale_out > 0.0f)) {  // the largest magnitude is under 6 times the smallest denormal: no scale to divide by
+        set_last_error("e2m1_quantize_device: the scale underflows");
+        return CSRSPMM_B200_ERR_BAD_ARG;
+    }
     return CSRSPMM_B200_OK;
 }
 

@@ -37,34 +37,60 @@ __global__ void validate_csr_kernel(int M, int Kd, long long nnz, const int* __r
     if (bad) atomicOr(problems, bad);
 }
 
-// stats[0] = longest row, [1] = empty rows, [2] = rows longer than `long_threshold`,
-// [3] = nnz in those rows.
-__global__ void row_stats_kernel(int M, const int* __restrict__ row_ptr, long long long_threshold,
-                                 unsigned long long* stats)
+// Four numbers over all threads of a CTA: v[0] maximum, v[1..3] sums; valid in thread 0.
+constexpr int kStatsThreads = 256;
+constexpr int kStatsMaxCtas = 148 * 4;
+
+__device__ __forceinline__ void stats_of_cta(long long (&v)[4])
 {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    unsigned long long mx = 0, empty = 0, nlong = 0, nnz_long = 0;
-    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += stride) {
-        const long long len = (long long)row_ptr[r + 1] - row_ptr[r];
-        if (len <= 0) ++empty;
-        if (len > (long long)mx) mx = (unsigned long long)len;
-        if (len > long_threshold) {
-            ++nlong;
-            nnz_long += (unsigned long long)len;
+    __shared__ long long part[kStatsThreads / 32][4];
+    for (int o = 16; o > 0; o >>= 1) {
+        v[0] = max(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+#pragma unroll
+        for (int k = 1; k < 4; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 4; ++k) part[threadIdx.x >> 5][k] = v[k];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kStatsThreads / 32; ++w) {
+            v[0] = max(v[0], part[w][0]);
+            for (int k = 1; k < 4; ++k) v[k] += part[w][k];
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        empty += __shfl_xor_sync(0xffffffffu, empty, o);
-        nlong += __shfl_xor_sync(0xffffffffu, nlong, o);
-        nnz_long += __shfl_xor_sync(0xffffffffu, nnz_long, o);
+}
+
+// Per CTA: longest row, empty rows, rows longer than 32 * (mean + 1), entries in those rows.
+__global__ void __launch_bounds__(kStatsThreads) row_stats_kernel(int M, const int* __restrict__ row_ptr, long long* __restrict__ part)
+{
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long nnz = (long long)row_ptr[M] - row_ptr[0];
+    const long long threshold = 32 * ((M > 0 ? nnz / M : 0) + 1);
+    long long v[4] = {0, 0, 0, 0};
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += stride) {
+        const long long len = (long long)row_ptr[r + 1] - row_ptr[r];
+        if (len <= 0) ++v[1];
+        v[0] = max(v[0], len);
+        if (len > threshold) {
+            ++v[2];
+            v[3] += len;
+        }
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(stats + 0, mx);
-        if (empty) atomicAdd(stats + 1, empty);
-        if (nlong) atomicAdd(stats + 2, nlong);
-        if (nnz_long) atomicAdd(stats + 3, nnz_long);
+    stats_of_cta(v);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 4; ++k) part[4 * blockIdx.x + k] = v[k];
+}
+
+__global__ void __launch_bounds__(kStatsThreads) row_stats_sum_kernel(int num, const long long* __restrict__ part, long long* stats)
+{
+    long long v[4] = {0, 0, 0, 0};
+    for (int b = threadIdx.x; b < num; b += kStatsThreads) {
+        v[0] = max(v[0], part[4 * b]);
+        for (int k = 1; k < 4; ++k) v[k] += part[4 * b + k];
     }
+    stats_of_cta(v);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 4; ++k) stats[k] = v[k];
 }
 
 }  // namespace csrspmm_b200

@@ -8,20 +8,56 @@
 
 namespace csrspmm_b200 {
 
-// max |v| over the array, NaNs ignored, as the bits of a non-negative float in *out_bits
-// (non-negative floats order like their unsigned bit patterns, so atomicMax on the bits works)
-__global__ void __launch_bounds__(256) e2m1_absmax_kernel(long long n, const float* __restrict__ values,
-                                                          unsigned* out_bits)
+// One CTA takes chunks of kCodecThreads * kCodecPer elements, every thread 16 of them, four 16-byte loads in
+// flight (arrays that do not start on 16 bytes: plain loads).
+constexpr int kCodecThreads = 256;
+constexpr int kCodecPer = 16;
+constexpr int kCodecMaxCtas = 148 * 4;
+
+// 16 values from position i0 on (0 beyond n)
+__device__ __forceinline__ void load_codec(long long n, const float* __restrict__ values, long long i0, float (&v)[kCodecPer])
+{
+    if (i0 + kCodecPer <= n && (reinterpret_cast<uintptr_t>(values) & 15u) == 0) {
+#pragma unroll
+        for (int q = 0; q < kCodecPer / 4; ++q) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(values + i0) + q);
+            v[4 * q] = x.x, v[4 * q + 1] = x.y, v[4 * q + 2] = x.z, v[4 * q + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < kCodecPer; ++q) v[q] = i0 + q < n ? __ldg(values + i0 + q) : 0.0f;
+    }
+}
+
+__device__ __forceinline__ float codec_block_max(float mx)
+{
+    __shared__ float warp_max[kCodecThreads / 32];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kCodecThreads / 32; ++w) mx = fmaxf(mx, warp_max[w]);
+    return mx;
+}
+
+// max |v| of each CTA's share, NaNs ignored
+__global__ void __launch_bounds__(kCodecThreads) e2m1_absmax_kernel(long long n, const float* __restrict__ values,
+                                                                    float* __restrict__ cta_max)
 {
     float mx = 0.0f;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float a = fabsf(__ldg(values + i));
-        if (a > mx) mx = a;  // false for NaN
-    }
-    unsigned bits = __float_as_uint(mx);
+    const long long stride = (long long)gridDim.x * (kCodecThreads * kCodecPer);
+    for (long long i = ((long long)blockIdx.x * kCodecThreads + threadIdx.x) * kCodecPer; i < n; i += stride) {
+        float v[kCodecPer];
+        load_codec(n, values, i, v);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, off));
-    if ((threadIdx.x & 31) == 0 && bits != 0) atomicMax(out_bits, bits);
+        for (int q = 0; q < kCodecPer; ++q) {
+            const float a = fabsf(v[q]);
+            if (a > mx) mx = a;  // false for NaN
+        }
+    }
+    mx = codec_block_max(mx);
+    if (threadIdx.x == 0) cta_max[blockIdx.x] = mx;
 }
 
 // nearest code point, ties to the even code, saturating at 6, sign kept, NaN -> +0
@@ -43,15 +79,34 @@ __device__ __forceinline__ unsigned e2m1_encode_one(float v, float scale)
     return s | code;
 }
 
-// one thread per output byte (elements 2k and 2k+1)
-__global__ void __launch_bounds__(256) e2m1_encode_kernel(long long n, const float* __restrict__ values, float scale,
-                                                          unsigned char* __restrict__ packed)
+// The codes of 16 elements per thread and step, 8 bytes at a time.  The scale is the argument, or
+// (cta_max given) follows from the maxima a previous kernel left, in which case CTA 0 reports its bits.
+__global__ void __launch_bounds__(kCodecThreads) e2m1_encode_kernel(long long n, const float* __restrict__ values, float scale,
+                                                                    const float* __restrict__ cta_max, int num_max,
+                                                                    unsigned char* __restrict__ packed, long long* scale_bits)
 {
-    const long long nbytes = (n + 1) / 2;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nbytes; k += (long long)gridDim.x * blockDim.x) {
-        const unsigned lo = e2m1_encode_one(__ldg(values + 2 * k), scale);
-        const unsigned hi = (2 * k + 1 < n) ? e2m1_encode_one(__ldg(values + 2 * k + 1), scale) : 0u;
-        packed[k] = (unsigned char)(lo | (hi << 4));
+    if (cta_max != nullptr) {
+        float mx = 0.0f;
+        for (int k = threadIdx.x; k < num_max; k += kCodecThreads) mx = fmaxf(mx, cta_max[k]);
+        mx = codec_block_max(mx);
+        scale = mx > 0.0f ? __fdiv_rn(mx, 6.0f) : 1.0f;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *scale_bits = (long long)__float_as_uint(scale);
+    }
+    const long long stride = (long long)gridDim.x * (kCodecThreads * kCodecPer);
+    const bool wide = (reinterpret_cast<uintptr_t>(packed) & 7u) == 0;
+    for (long long i = ((long long)blockIdx.x * kCodecThreads + threadIdx.x) * kCodecPer; i < n; i += stride) {
+        float v[kCodecPer];
+        load_codec(n, values, i, v);
+        unsigned word[2] = {0u, 0u};  // elements beyond n are 0: code 0
+#pragma unroll
+        for (int q = 0; q < kCodecPer; ++q) word[q >> 3] |= (i + q < n ? e2m1_encode_one(v[q], scale) : 0u) << (4 * (q & 7));
+        if (wide && i + kCodecPer <= n) {
+            *reinterpret_cast<uint2*>(packed + (i >> 1)) = make_uint2(word[0], word[1]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < kCodecPer; q += 2)
+                if (i + q < n) packed[(i + q) >> 1] = (unsigned char)(word[q >> 3] >> (4 * (q & 7)));
+        }
     }
 }
 

@@ -58,6 +58,16 @@ __device__ __forceinline__ void report_status(const SpmmParams& p, int bit)
     if (p.status_word != nullptr) atomicOr(p.status_word, bit);
 }
 
+// ---- launches that overlap (abi/pdl.h) ------------------------------------------------------------
+
+// Waits until the grid before this one in the stream has completed; first thing in every kernel started by
+// launch_overlapped (a kernel started plainly passes at once).
+__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the grid after this one be launched as soon as every CTA of this one has got here; it still waits for
+// this grid's end before it reads or writes anything.
+__device__ __forceinline__ void release_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- value formats ------------------------------------------------------------------------------
 
 // e2m1 code (s eem) -> fp32: magnitude in {0, .5, 1, 1.5, 2, 3, 4, 6} built directly as IEEE

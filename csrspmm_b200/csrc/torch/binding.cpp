@@ -19,6 +19,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -33,6 +34,9 @@ struct Library {
     int (*select_kernel)(const csrspmm_b200_args*);
     size_t (*workspace_bytes)(const csrspmm_b200_args*);
     int (*row_stats)(int32_t, const int32_t*, int64_t*, csrspmm_b200_stream_t);
+    int (*dense2csr_count)(int32_t, int32_t, const float*, int64_t, float, int32_t*, int64_t*, int32_t*, csrspmm_b200_stream_t);
+    int (*dense2csr_fill)(int32_t, int32_t, const float*, int64_t, float, const int32_t*, int32_t*, float*, csrspmm_b200_stream_t);
+    int (*quantize)(int64_t, const float*, float*, uint8_t*, csrspmm_b200_stream_t);
 };
 Library g_lib = {};
 PyObject* g_error = nullptr;  // _lib.SpmmError(status, where)
@@ -81,6 +85,21 @@ void check_csr(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va,
     const auto dev = B.device();
     want(rp.device() == dev && ci.device() == dev && va.device() == dev, "all tensors must be on the same device");
 }
+
+// Releases the GIL if this thread holds it (the registered operators run without it).
+class WithoutGil {
+public:
+    WithoutGil() : state_(PyGILState_Check() ? PyEval_SaveThread() : nullptr) {}
+    ~WithoutGil()
+    {
+        if (state_) PyEval_RestoreThread(state_);
+    }
+    WithoutGil(const WithoutGil&) = delete;
+    WithoutGil& operator=(const WithoutGil&) = delete;
+
+private:
+    PyThreadState* state_;
+};
 
 template <class T>
 T* address(const at::Tensor& t)
@@ -183,7 +202,7 @@ at::Tensor run_product(Product& q)
     int status;
     {
         // as under ctypes: a launch may wait for room in the stream's queue, and sync waits for the GPU
-        pybind11::gil_scoped_release nogil;
+        const WithoutGil nogil;
         status = (q.sync ? g_lib.spmm_sync : g_lib.spmm)(&a, reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
     }
     if (status != CSRSPMM_B200_OK) throw LibraryError{status, "csrspmm_b200_spmm"};
@@ -218,7 +237,7 @@ int longest_row(const at::Tensor& rp)
     int status;
     {
         const auto stream = c10::cuda::getCurrentCUDAStream(rp.device().index());
-        pybind11::gil_scoped_release nogil;
+        const WithoutGil nogil;
         status = g_lib.row_stats(static_cast<int32_t>(rp.size(0) - 1), address<int32_t>(rp), stats,
                                  reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
     }
@@ -262,19 +281,26 @@ void expect_args(Py_ssize_t got, Py_ssize_t wanted)
     if (got != wanted) throw std::runtime_error("csrspmm_b200 binding: wrong number of arguments");
 }
 
-// init(spmm, spmm_sync, select_kernel, workspace_bytes, row_stats, SpmmError): addresses of the C functions
+// init(SpmmError, {name: address of csrspmm_b200_<name>})
 PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
 {
     BEGIN_BINDING
-    expect_args(nargs, 6);
-    auto fn = [&](int k) { return reinterpret_cast<void*>(static_cast<uintptr_t>(as_integer(args[k]))); };
-    g_lib.spmm = reinterpret_cast<decltype(g_lib.spmm)>(fn(0));
-    g_lib.spmm_sync = reinterpret_cast<decltype(g_lib.spmm_sync)>(fn(1));
-    g_lib.select_kernel = reinterpret_cast<decltype(g_lib.select_kernel)>(fn(2));
-    g_lib.workspace_bytes = reinterpret_cast<decltype(g_lib.workspace_bytes)>(fn(3));
-    g_lib.row_stats = reinterpret_cast<decltype(g_lib.row_stats)>(fn(4));
-    Py_INCREF(args[5]);
-    Py_XSETREF(g_error, args[5]);
+    expect_args(nargs, 2);
+    auto fill = [&](auto& fn, const char* name) {
+        PyObject* o = PyDict_GetItemString(args[1], name);
+        if (o == nullptr) throw std::runtime_error(std::string("csrspmm_b200 binding: no address for ") + name);
+        fn = reinterpret_cast<std::decay_t<decltype(fn)>>(static_cast<uintptr_t>(as_integer(o)));
+    };
+    fill(g_lib.spmm, "spmm");
+    fill(g_lib.spmm_sync, "spmm_sync");
+    fill(g_lib.select_kernel, "select_kernel");
+    fill(g_lib.workspace_bytes, "workspace_bytes");
+    fill(g_lib.row_stats, "row_stats_device");
+    fill(g_lib.dense2csr_count, "dense2csr_count");
+    fill(g_lib.dense2csr_fill, "dense2csr_fill");
+    fill(g_lib.quantize, "e2m1_quantize_device");
+    Py_INCREF(args[0]);
+    Py_XSETREF(g_error, args[0]);
     Py_RETURN_NONE;
     END_BINDING
 }
@@ -335,11 +361,79 @@ PyObject* py_enqueue(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     const auto stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(as_integer(args[1])));
     int status;
     {
-        pybind11::gil_scoped_release nogil;
+        const WithoutGil nogil;
         status = g_lib.spmm(a, reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
     }
     if (status != CSRSPMM_B200_OK) throw LibraryError{status, "csrspmm_b200_spmm"};
     Py_RETURN_NONE;
+    END_BINDING
+}
+
+at::Tensor new_array(int64_t n, at::ScalarType type, at::Device device)
+{
+    return at::detail::empty_cuda({n}, type, device, std::nullopt);
+}
+
+csrspmm_b200_stream_t current_stream(at::Device device)
+{
+    return reinterpret_cast<csrspmm_b200_stream_t>(c10::cuda::getCurrentCUDAStream(device.index()).stream());
+}
+
+void check(int status, const char* where)
+{
+    if (status != CSRSPMM_B200_OK) throw LibraryError{status, where};
+}
+
+// dense2csr(dense, tol) -> (row_ptr, col_idx, values, longest row)
+PyObject* py_dense2csr(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 2);
+    const at::Tensor dense = tensor_of(args[0], "dense");
+    const float tol = static_cast<float>(as_double(args[1]));
+    want(dense.is_cuda() && dense.scalar_type() == at::kFloat && dense.dim() == 2 && (dense.stride(1) == 1 || dense.size(1) <= 1),
+         "dense must be a row-major float32 CUDA matrix");
+    const int64_t H = dense.size(0), W = dense.size(1);
+    const int64_t ld = std::max(H > 1 ? dense.stride(0) : W, W);
+    const auto device = dense.device();
+    const c10::cuda::CUDAGuard guard(device);
+    at::Tensor rp = new_array(H + 1, at::kInt, device), ci, va;
+    int64_t nnz = 0;
+    int32_t longest = 0;
+    {
+        const WithoutGil nogil;
+        const auto stream = current_stream(device);
+        const float* data = address<float>(dense);
+        check(g_lib.dense2csr_count((int32_t)H, (int32_t)W, data, ld, tol, address<int32_t>(rp), &nnz, &longest, stream),
+              "csrspmm_b200_dense2csr_count");
+        ci = new_array(nnz, at::kInt, device);
+        va = new_array(nnz, at::kFloat, device);
+        if (nnz > 0)
+            check(g_lib.dense2csr_fill((int32_t)H, (int32_t)W, data, ld, tol, address<int32_t>(rp), address<int32_t>(ci),
+                                       address<float>(va), stream),
+                  "csrspmm_b200_dense2csr_fill");
+    }
+    return Py_BuildValue("(NNNi)", THPVariable_Wrap(rp), THPVariable_Wrap(ci), THPVariable_Wrap(va), (int)longest);
+    END_BINDING
+}
+
+// quantize(values: contiguous float32 on the GPU) -> (packed, scale)
+PyObject* py_quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 1);
+    const at::Tensor v = tensor_of(args[0], "values");
+    want(v.is_cuda() && v.scalar_type() == at::kFloat && v.is_contiguous(), "values must be a contiguous float32 CUDA tensor");
+    const int64_t n = v.numel();
+    const c10::cuda::CUDAGuard guard(v.device());
+    at::Tensor packed = new_array((n + 1) / 2, at::kByte, v.device());
+    float scale = 1.0f;
+    {
+        const WithoutGil nogil;
+        check(g_lib.quantize(n, address<float>(v), &scale, address<uint8_t>(packed), current_stream(v.device())),
+              "csrspmm_b200_e2m1_quantize_device");
+    }
+    return Py_BuildValue("(Nd)", THPVariable_Wrap(packed), (double)scale);
     END_BINDING
 }
 
@@ -349,6 +443,8 @@ PyMethodDef g_methods[] = {
     {"spmm", FASTCALL(py_spmm), nullptr},
     {"op", FASTCALL(py_op), nullptr},
     {"enqueue", FASTCALL(py_enqueue), nullptr},
+    {"dense2csr", FASTCALL(py_dense2csr), nullptr},
+    {"quantize", FASTCALL(py_quantize), nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};

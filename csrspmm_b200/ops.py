@@ -267,17 +267,7 @@ def e2m1_quantize(values_f32):
     encoded on its device and the packed tensor stays there; anything else is encoded on the host."""
     import numpy as np
     if isinstance(values_f32, torch.Tensor) and values_f32.is_cuda:
-        v = values_f32.detach().to(torch.float32).contiguous()
-        n = v.numel()
-        L = _lib.lib()
-        scale = C.c_float(1.0)
-        packed = torch.empty((n + 1) // 2, dtype=torch.uint8, device=v.device)
-        with torch.cuda.device(v.device):
-            st = C.c_void_p(torch.cuda.current_stream(v.device).cuda_stream)
-            _lib.check(L.csrspmm_b200_e2m1_scale_device(n, v.data_ptr(), C.byref(scale), st), "e2m1_scale_device")
-            _lib.check(L.csrspmm_b200_e2m1_encode_device(n, v.data_ptr(), scale.value, packed.data_ptr(), st),
-                       "e2m1_encode_device")
-        return packed, float(scale.value)
+        return _lib.binding().quantize(values_f32.detach().to(torch.float32).contiguous())
     v = np.ascontiguousarray(values_f32.detach().cpu().numpy() if isinstance(values_f32, torch.Tensor)
                              else values_f32, dtype=np.float32)
     L = _lib.lib()
@@ -385,24 +375,7 @@ def host_arena_bytes(M, Kd, Nd, nnz) -> int:
 def dense2csr(dense: torch.Tensor, tol: float = 0.0):
     """CUDA float32 matrix -> (row_ptr, col_idx, values, max_row_nnz), the arrays the reference's host
     ``dense2csr`` would produce (entries with |v| > tol, ascending columns), built on the device."""
-    if not dense.is_cuda or dense.dtype != torch.float32 or dense.dim() != 2 or (dense.stride(1) != 1 and dense.size(1) > 1):
-        raise RuntimeError("dense must be a row-major float32 CUDA matrix")
-    H, W = dense.shape
-    ld = dense.stride(0) if H > 1 else max(W, 1)
-    L = _lib.lib()
-    row_ptr = torch.empty(H + 1, dtype=torch.int32, device=dense.device)
-    nnz, mx = C.c_int64(0), C.c_int32(0)
-    with torch.cuda.device(dense.device):
-        stream = C.c_void_p(torch.cuda.current_stream(dense.device).cuda_stream)
-        _lib.check(L.csrspmm_b200_dense2csr_count(H, W, dense.data_ptr(), max(ld, W), float(tol), row_ptr.data_ptr(),
-                                                  C.byref(nnz), C.byref(mx), stream), "csrspmm_b200_dense2csr_count")
-        col_idx = torch.empty(nnz.value, dtype=torch.int32, device=dense.device)
-        values = torch.empty(nnz.value, dtype=torch.float32, device=dense.device)
-        if nnz.value > 0:
-            _lib.check(L.csrspmm_b200_dense2csr_fill(H, W, dense.data_ptr(), max(ld, W), float(tol), row_ptr.data_ptr(),
-                                                     col_idx.data_ptr(), values.data_ptr(), stream),
-                       "csrspmm_b200_dense2csr_fill")
-    return row_ptr, col_idx, values, int(mx.value)
+    return _lib.binding().dense2csr(dense, tol)
 
 
 def csr2dense(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: torch.Tensor, shape) -> torch.Tensor:

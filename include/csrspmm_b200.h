@@ -318,6 +318,10 @@ int csrspmm_b200_e2m1_decode(int64_t n, const uint8_t* packed, float scale, floa
 int csrspmm_b200_e2m1_scale_device(int64_t n, const float* values, float* scale_out, csrspmm_b200_stream_t stream);
 int csrspmm_b200_e2m1_encode_device(int64_t n, const float* values, float scale, uint8_t* packed,
                                     csrspmm_b200_stream_t stream);
+/* Scale and codes in one call (what _scale_device followed by _encode_device gives, with one wait instead of a
+ * wait between them). */
+int csrspmm_b200_e2m1_quantize_device(int64_t n, const float* values, float* scale_out, uint8_t* packed,
+                                      csrspmm_b200_stream_t stream);
 int csrspmm_b200_e2m1_decode_device(int64_t n, const uint8_t* packed, float scale, float* values,
                                     csrspmm_b200_stream_t stream);
 
