@@ -43,7 +43,7 @@ EXPORTED_SYMBOLS = (
     "csrspmm_b200_e2m1_encode", "csrspmm_b200_e2m1_decode", "csrspmm_b200_dense2csr_count",
     "csrspmm_b200_dense2csr_fill", "csrspmm_b200_csr2dense", "csrspmm_b200_copy_rows", "csrspmm_b200_column_panels",
     "csrspmm_b200_e2m1_scale_device", "csrspmm_b200_e2m1_encode_device", "csrspmm_b200_e2m1_decode_device",
-    "csrspmm_b200_e2m1_quantize_device",
+    "csrspmm_b200_e2m1_quantize_device", "csrspmm_b200_transpose", "csrspmm_b200_transpose_workspace_bytes",
     "csrspmm_b200_spmm_tiled", "csrspmm_b200_tiled_workspace_bytes", "csrspmm_b200_tiled_panel_rows",
     "csrspmm_b200_schedule_create", "csrspmm_b200_schedule_destroy", "csrspmm_b200_schedule_info_get",
 )

@@ -18,8 +18,10 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
+#include <torch/library.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -36,6 +38,9 @@ struct Library {
     int (*row_stats)(int32_t, const int32_t*, int64_t*, csrspmm_b200_stream_t);
     int (*dense2csr_count)(int32_t, int32_t, const float*, int64_t, float, int32_t*, int64_t*, int32_t*, csrspmm_b200_stream_t);
     int (*dense2csr_fill)(int32_t, int32_t, const float*, int64_t, float, const int32_t*, int32_t*, float*, csrspmm_b200_stream_t);
+    size_t (*transpose_workspace_bytes)(int32_t, int64_t);
+    int (*transpose)(int32_t, int32_t, int64_t, const int32_t*, const int32_t*, const float*, int32_t*, int32_t*, float*, void*, size_t,
+                     csrspmm_b200_stream_t);
     int (*quantize)(int64_t, const float*, float*, uint8_t*, csrspmm_b200_stream_t);
 };
 Library g_lib = {};
@@ -299,6 +304,8 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     fill(g_lib.dense2csr_count, "dense2csr_count");
     fill(g_lib.dense2csr_fill, "dense2csr_fill");
     fill(g_lib.quantize, "e2m1_quantize_device");
+    fill(g_lib.transpose_workspace_bytes, "transpose_workspace_bytes");
+    fill(g_lib.transpose, "transpose");
     Py_INCREF(args[0]);
     Py_XSETREF(g_error, args[0]);
     Py_RETURN_NONE;
@@ -437,6 +444,154 @@ PyObject* py_quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     END_BINDING
 }
 
+// (row_ptr, col_idx, values) of A^T
+std::tuple<at::Tensor, at::Tensor, at::Tensor> transpose(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, int64_t Kd)
+{
+    want(rp.is_cuda() && ci.is_cuda() && va.is_cuda() && ci.device() == rp.device() && va.device() == rp.device(),
+         "row_ptr, col_idx and values must be CUDA tensors on one device");
+    want(rp.scalar_type() == at::kInt && ci.scalar_type() == at::kInt && va.scalar_type() == at::kFloat,
+         "row_ptr and col_idx must be int32, values float32");
+    want(rp.dim() == 1 && ci.dim() == 1 && va.dim() == 1 && rp.size(0) >= 1 && ci.size(0) == va.size(0) && rp.is_contiguous() &&
+             ci.is_contiguous() && va.is_contiguous(),
+         "expected contiguous 1-D row_ptr, col_idx and values");
+    const auto device = rp.device();
+    const c10::cuda::CUDAGuard guard(device);
+    const int64_t nnz = ci.size(0);
+    at::Tensor t_rp = new_array(Kd + 1, at::kInt, device), t_ci = new_array(nnz, at::kInt, device), t_va = new_array(nnz, at::kFloat, device);
+    const auto stream = c10::cuda::getCurrentCUDAStream(device.index());
+    const size_t need = g_lib.transpose_workspace_bytes((int32_t)Kd, nnz);
+    Scratch scratch;
+    void* ws = scratch.get(need, stream);
+    int status;
+    {
+        const WithoutGil nogil;
+        status = g_lib.transpose((int32_t)(rp.size(0) - 1), (int32_t)Kd, nnz, address<int32_t>(rp), address<int32_t>(ci), address<float>(va),
+                                 address<int32_t>(t_rp), address<int32_t>(t_ci), address<float>(t_va), ws, std::max<size_t>(need, 256),
+                                 reinterpret_cast<csrspmm_b200_stream_t>(stream.stream()));
+    }
+    check(status, "csrspmm_b200_transpose");
+    return {t_rp, t_ci, t_va};
+}
+
+// transpose(row_ptr, col_idx, values, Kd) -> (row_ptr, col_idx, values) of A^T
+PyObject* py_transpose(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    BEGIN_BINDING
+    expect_args(nargs, 4);
+    const auto t = transpose(tensor_of(args[0], "row_ptr"), tensor_of(args[1], "col_idx"), tensor_of(args[2], "values"), as_integer(args[3]));
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(std::get<0>(t)), THPVariable_Wrap(std::get<1>(t)), THPVariable_Wrap(std::get<2>(t)));
+    END_BINDING
+}
+
+// ---- torch.ops.csrspmm_b200 (schemas and fake implementations: csrspmm_b200/torch_library.py) ---------------
+// Registered here and not through torch.library.custom_op, whose Python layers cost more per call than a
+// product of a sampled subgraph takes on the GPU.
+
+// A failed library call leaves an operator as SpmmError too.
+template <class F>
+auto as_operator(F&& body)
+{
+    try {
+        return body();
+    } catch (const LibraryError& e) {
+        pybind11::gil_scoped_acquire gil;
+        raise_library_error(e);
+        throw pybind11::error_already_set();
+    }
+}
+
+int kernel_id(c10::string_view name)
+{
+    if (name == "auto") return CSRSPMM_B200_KERNEL_AUTO;
+    if (name == "row") return CSRSPMM_B200_KERNEL_ROW;
+    if (name == "merge") return CSRSPMM_B200_KERNEL_MERGE;
+    if (name == "tma") return CSRSPMM_B200_KERNEL_TMA;
+    throw std::runtime_error("unknown kernel '" + std::string(name) + "' (auto, row, merge or tma)");
+}
+
+at::Tensor op_spmm(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, double alpha, c10::string_view kernel)
+{
+    return as_operator([&] {
+        Product q;
+        q.rp = rp, q.ci = ci, q.va = va, q.B = B.contiguous();
+        q.alpha = alpha;
+        q.kernel = kernel_id(kernel);
+        return run_product(q);
+    });
+}
+
+void op_spmm_inplace(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, const at::Tensor& C, double alpha,
+                     double beta, c10::string_view kernel)
+{
+    as_operator([&] {
+        Product q;
+        q.rp = rp, q.ci = ci, q.va = va, q.B = B, q.C = C;
+        q.alpha = alpha, q.beta = beta;
+        q.kernel = kernel_id(kernel);
+        return run_product(q);
+    });
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> op_transpose(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, c10::SymInt Kd)
+{
+    return as_operator([&] { return transpose(rp, ci, va, Kd.expect_int()); });
+}
+
+at::Tensor call_spmm(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, double alpha, c10::string_view kernel)
+{
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("csrspmm_b200::spmm", "").typed<decltype(op_spmm)>();
+    return op.call(rp, ci, va, B, alpha, kernel);
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> call_transpose(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, c10::SymInt Kd)
+{
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("csrspmm_b200::transpose", "").typed<decltype(op_transpose)>();
+    return op.call(rp, ci, va, Kd);
+}
+
+// dB = alpha * A^T dC
+struct SpmmWithGradient : torch::autograd::Function<SpmmWithGradient> {
+    static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va,
+                              const at::Tensor& B, double alpha, std::string kernel)
+    {
+        ctx->save_for_backward({rp, ci, va});
+        ctx->saved_data["Kd"] = B.sym_size(0);
+        ctx->saved_data["alpha"] = alpha;
+        ctx->saved_data["kernel"] = kernel;
+        ctx->saved_data["values_need_grad"] = va.requires_grad();
+        at::AutoDispatchBelowADInplaceOrView below;
+        return call_spmm(rp, ci, va, B, alpha, kernel);
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads)
+    {
+        if (ctx->saved_data["values_need_grad"].toBool())
+            throw std::runtime_error("csrspmm_b200::spmm has no gradient for the stored values of A");
+        torch::autograd::variable_list out(6);
+        if (ctx->needs_input_grad(3) && grads[0].defined()) {
+            const auto saved = ctx->get_saved_variables();
+            const auto t = call_transpose(saved[0], saved[1], saved[2], ctx->saved_data["Kd"].toSymInt());
+            out[3] = call_spmm(std::get<0>(t), std::get<1>(t), std::get<2>(t), grads[0].contiguous(), ctx->saved_data["alpha"].toDouble(),
+                               ctx->saved_data["kernel"].toStringRef());
+        }
+        return out;
+    }
+};
+
+at::Tensor autograd_spmm(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, double alpha,
+                         c10::string_view kernel)
+{
+    return SpmmWithGradient::apply(rp, ci, va, B, alpha, std::string(kernel));
+}
+
+TORCH_LIBRARY_IMPL(csrspmm_b200, CUDA, m)
+{
+    m.impl("spmm", op_spmm);
+    m.impl("spmm_", op_spmm_inplace);
+    m.impl("transpose", op_transpose);
+}
+
+TORCH_LIBRARY_IMPL(csrspmm_b200, Autograd, m) { m.impl("spmm", autograd_spmm); }
+
 #define FASTCALL(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL
 PyMethodDef g_methods[] = {
     {"init", FASTCALL(py_init), nullptr},
@@ -445,6 +600,7 @@ PyMethodDef g_methods[] = {
     {"enqueue", FASTCALL(py_enqueue), nullptr},
     {"dense2csr", FASTCALL(py_dense2csr), nullptr},
     {"quantize", FASTCALL(py_quantize), nullptr},
+    {"transpose", FASTCALL(py_transpose), nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};

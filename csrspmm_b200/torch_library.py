@@ -18,13 +18,18 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 
 def transpose_csr(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: torch.Tensor, Kd: int):
     """CSR of A^T (Kd x M) from the CSR of A (M x Kd), on the arrays' device.  Entries of a column
     keep their row order (stable sort), so the result has ascending, distinct column indices
     whenever A has no repeated entry."""
+    if (row_ptr.is_cuda and col_idx.is_cuda and values.is_cuda and row_ptr.dtype == col_idx.dtype == torch.int32
+            and values.dtype == torch.float32 and not (values.requires_grad and torch.is_grad_enabled())
+            and row_ptr.is_contiguous() and col_idx.is_contiguous() and values.is_contiguous()):
+        return _lib.binding().transpose(row_ptr, col_idx, values, int(Kd))
+    # host arrays and other types
     M = row_ptr.numel() - 1
     lens = (row_ptr[1:] - row_ptr[:-1]).long()
     rows = torch.repeat_interleave(torch.arange(M, device=row_ptr.device, dtype=torch.int32), lens)
@@ -37,40 +42,39 @@ def transpose_csr(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: torch.Te
     return t_rp, t_col, t_val
 
 
-@torch.library.custom_op("csrspmm_b200::spmm", mutates_args=(), device_types="cuda")
-def spmm_op(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: torch.Tensor, B: torch.Tensor, alpha: float,
-            kernel: str) -> torch.Tensor:
-    return ops.spmm(row_ptr, col_idx, values, B.contiguous(), None, alpha, 0.0, kernel=kernel)
+# The operators' schemas and fake implementations; their CUDA kernels and the gradient are registered by the
+# binding (csrc/torch/binding.cpp), which is loaded here when it has been built.
+_library = torch.library.Library("csrspmm_b200", "DEF")
+_library.define("spmm(Tensor row_ptr, Tensor col_idx, Tensor values, Tensor B, float alpha, str kernel) -> Tensor",
+                tags=(torch.Tag.pt2_compliant_tag,))
+_library.define("spmm_(Tensor row_ptr, Tensor col_idx, Tensor values, Tensor B, Tensor(a!) C, float alpha, float beta, "
+                "str kernel) -> ()", tags=(torch.Tag.pt2_compliant_tag,))
+_library.define("transpose(Tensor row_ptr, Tensor col_idx, Tensor values, SymInt Kd) -> (Tensor, Tensor, Tensor)",
+                tags=(torch.Tag.pt2_compliant_tag,))
 
 
-@spmm_op.register_fake
+@torch.library.register_fake("csrspmm_b200::spmm")
 def _spmm_fake(row_ptr, col_idx, values, B, alpha, kernel):
     return B.new_empty((row_ptr.shape[0] - 1, B.shape[1]))
 
 
-@torch.library.custom_op("csrspmm_b200::spmm_", mutates_args=("C",), device_types="cuda")
-def spmm_inplace_op(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: torch.Tensor, B: torch.Tensor,
-                    C: torch.Tensor, alpha: float, beta: float, kernel: str) -> None:
-    ops.spmm(row_ptr, col_idx, values, B, C, alpha, beta, kernel=kernel)
+@torch.library.register_fake("csrspmm_b200::spmm_")
+def _spmm_inplace_fake(row_ptr, col_idx, values, B, C, alpha, beta, kernel):
+    return None
 
 
-def _setup_context(ctx, inputs, output):
-    row_ptr, col_idx, values, B, alpha, kernel = inputs
-    ctx.save_for_backward(row_ptr, col_idx, values)
-    ctx.Kd, ctx.alpha, ctx.kernel = B.shape[0], alpha, kernel
-    ctx.values_need_grad = values.requires_grad
+@torch.library.register_fake("csrspmm_b200::transpose")
+def _transpose_fake(row_ptr, col_idx, values, Kd):
+    return row_ptr.new_empty((Kd + 1,)), torch.empty_like(col_idx), torch.empty_like(values)
 
 
-def _backward(ctx, grad_C):
-    if ctx.values_need_grad:
-        raise RuntimeError("csrspmm_b200::spmm has no gradient for the stored values of A")
-    row_ptr, col_idx, values = ctx.saved_tensors
-    t_rp, t_ci, t_va = transpose_csr(row_ptr, col_idx, values, ctx.Kd)
-    dB = spmm_op(t_rp, t_ci, t_va, grad_C.contiguous(), ctx.alpha, ctx.kernel)
-    return None, None, None, dB, None, None
+try:
+    _lib.binding()
+except _lib.LibraryMissing:  # not built: the operators trace, and calling one on a GPU says there is no kernel
+    pass
 
-
-spmm_op.register_autograd(_backward, setup_context=_setup_context)
+spmm_op = torch.ops.csrspmm_b200.spmm
+spmm_inplace_op = torch.ops.csrspmm_b200.spmm_
 
 
 class CsrMatrix:

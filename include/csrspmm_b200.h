@@ -300,6 +300,15 @@ int csrspmm_b200_dense2csr_fill(int32_t H, int32_t W, const float* dense, int64_
 int csrspmm_b200_csr2dense(int32_t H, int32_t W, const int32_t* row_ptr, const int32_t* col_idx,
                            const float* values, float* dense, int64_t ld, csrspmm_b200_stream_t stream);
 
+/* CSR of A^T (Kd x M) from the CSR of A (M x Kd), device arrays, on `stream`, asynchronous: entries of a column keep
+ * their stored order, so rows ascend in each column.  t_row_ptr has Kd + 1 entries, t_col_idx and t_values nnz.
+ * workspace: csrspmm_b200_transpose_workspace_bytes(Kd, nnz) bytes, 256-byte aligned.  No counterpart in the
+ * reference. */
+size_t csrspmm_b200_transpose_workspace_bytes(int32_t Kd, int64_t nnz);
+int csrspmm_b200_transpose(int32_t M, int32_t Kd, int64_t nnz, const int32_t* row_ptr, const int32_t* col_idx,
+                           const float* values, int32_t* t_row_ptr, int32_t* t_col_idx, float* t_values, void* workspace,
+                           size_t workspace_bytes, csrspmm_b200_stream_t stream);
+
 /* ---- multi-GPU row partition (new) ------------------------------------------------------------
  * Contiguous row blocks [bounds[g], bounds[g+1]) for g < parts with near-equal cost, where the
  * cost of a row is its nnz + row_weight (row_weight = 1 balances B-row reads against C-row

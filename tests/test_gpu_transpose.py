@@ -1,0 +1,36 @@
+"""The device transposition against the host one: tile edges, one to three digit passes, repeats, hub columns."""
+import numpy as np
+import pytest
+import torch
+
+from csrspmm_b200 import _lib, torch_library as TL
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,Kd,nnz,hub", [(1, 1, 1, False), (5, 1, 1023, False), (300, 2, 1024, False), (300, 1024, 1025, False),
+                                          (70, 1025, 5000, True), (4000, 70001, 30000, False), (17, (1 << 20) + 1, 2000, False),
+                                          (50000, 2048, 1300000, True), (60000, (1 << 22) + 3, 1250000, False)])
+def test_transpose(cuda_lib, M, Kd, nnz, hub):
+    rng = np.random.default_rng(nnz)
+    rows = np.sort(rng.integers(0, M, nnz))  # many rows stay empty
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=M))]).astype(np.int32)
+    ci = rng.integers(0, Kd, nnz).astype(np.int32)  # unsorted, with repeats
+    if hub:
+        ci[rng.random(nnz) < 0.4] = Kd - 1
+    t = [torch.from_numpy(x) for x in (rp, ci, rng.standard_normal(nnz, dtype=np.float32))]
+    want = TL.transpose_csr(*t, Kd)
+    got = TL.transpose_csr(*(x.cuda() for x in t), Kd)
+    assert all(torch.equal(g.cpu(), w) for g, w in zip(got, want))
+
+
+def test_transpose_of_nothing(cuda_lib):
+    rp, ci, va = torch.zeros(4, dtype=torch.int32).cuda(), torch.zeros(0, dtype=torch.int32).cuda(), torch.zeros(0).cuda()
+    t_rp, t_ci, t_va = TL.transpose_csr(rp, ci, va, 9)
+    assert t_rp.tolist() == [0] * 10 and t_ci.numel() == t_va.numel() == 0
+
+
+def test_operator_errors_keep_their_type(cuda_lib):
+    rp, ci, va = torch.tensor([0, 1], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), torch.ones(1).cuda()
+    with pytest.raises(_lib.SpmmError):  # the bulk-copy kernel needs whole vectors
+        torch.ops.csrspmm_b200.spmm(rp, ci, va, torch.ones(1, 3).cuda(), 1.0, "tma")
