@@ -16,6 +16,7 @@
 #include "../kernels/tma_kernel.cuh"
 #include "csrspmm_b200.h"
 #include "launch.h"
+#include "pdl.h"
 #include "plan.h"
 #include "scratch.h"
 
@@ -33,6 +34,7 @@ void fill_params(const csrspmm_b200_args* a, const Plan& plan, SpmmParams* out)
     p.nnz = (int)a->nnz;
     p.ncolv = plan.ncolv;
     p.num_items = plan.num_items;
+    p.release_early = plan.fills_chip;
     p.row_ptr = a->row_ptr;
     p.rp_base = a->row_ptr_base;
     p.col_idx = a->col_idx;
@@ -76,24 +78,19 @@ namespace {
     } while (0)
 
 template <int S, int VW, int FMT>
-void launch_row(const SpmmParams& p, const Plan& plan, cudaStream_t st)
+cudaError_t launch_row(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
     constexpr int G = kShapes[S].G, NV = kShapes[S].NV;
     constexpr int U = VW == 1 ? 8 : row_unroll(NV);
     constexpr int ULOW = VW == 1 ? 8 : row_unroll_low(NV);
     constexpr int MINB = row_min_blocks(NV);
     const unsigned grid = (unsigned)plan.grid;
-    if (VW == 4 && plan.full) {
-        if (plan.low_occupancy && ULOW != U)
-            spmm_row_kernel<G, NV, VW, ULOW, FMT, (VW == 4), 2><<<grid, kRowThreads, 0, st>>>(p);
-        else
-            spmm_row_kernel<G, NV, VW, U, FMT, (VW == 4), MINB><<<grid, kRowThreads, 0, st>>>(p);
-    } else {
-        if (plan.low_occupancy && ULOW != U)
-            spmm_row_kernel<G, NV, VW, ULOW, FMT, false, 2><<<grid, kRowThreads, 0, st>>>(p);
-        else
-            spmm_row_kernel<G, NV, VW, U, FMT, false, MINB><<<grid, kRowThreads, 0, st>>>(p);
-    }
+    const bool low = plan.low_occupancy && ULOW != U;
+    if (VW == 4 && plan.full)
+        return low ? launch_overlapped(spmm_row_kernel<G, NV, VW, ULOW, FMT, (VW == 4), 2>, grid, kRowThreads, 0, st, p)
+                   : launch_overlapped(spmm_row_kernel<G, NV, VW, U, FMT, (VW == 4), MINB>, grid, kRowThreads, 0, st, p);
+    return low ? launch_overlapped(spmm_row_kernel<G, NV, VW, ULOW, FMT, false, 2>, grid, kRowThreads, 0, st, p)
+               : launch_overlapped(spmm_row_kernel<G, NV, VW, U, FMT, false, MINB>, grid, kRowThreads, 0, st, p);
 }
 
 template <int NV, int FMT>
@@ -115,20 +112,19 @@ cudaError_t launch_tma(const SpmmParams& p, const Plan& plan, cudaStream_t st)
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kern<<<(unsigned)plan.grid, kMergeThreads, plan.dynamic_smem, st>>>(p, (unsigned)plan.tma_slot_bytes,
-                                                                        (unsigned)(plan.dynamic_smem / (CSRSPMM_TUNE_MERGE_THREADS / 32)));
-    return cudaSuccess;
+    return launch_overlapped(kern, (unsigned)plan.grid, kMergeThreads, plan.dynamic_smem, st, p, (unsigned)plan.tma_slot_bytes,
+                             (unsigned)(plan.dynamic_smem / (CSRSPMM_TUNE_MERGE_THREADS / 32)));
 }
 
 template <int VW, int FMT>
-void dispatch_row(const SpmmParams& p, const Plan& plan, cudaStream_t st)
+cudaError_t dispatch_row(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
     switch (plan.shape) {
-        case 0: launch_row<0, VW, FMT>(p, plan, st); break;
-        case 1: launch_row<1, VW, FMT>(p, plan, st); break;
-        case 2: launch_row<2, VW, FMT>(p, plan, st); break;
-        case 3: launch_row<3, VW, FMT>(p, plan, st); break;
-        default: launch_row<4, VW, FMT>(p, plan, st); break;
+        case 0: return launch_row<0, VW, FMT>(p, plan, st);
+        case 1: return launch_row<1, VW, FMT>(p, plan, st);
+        case 2: return launch_row<2, VW, FMT>(p, plan, st);
+        case 3: return launch_row<3, VW, FMT>(p, plan, st);
+        default: return launch_row<4, VW, FMT>(p, plan, st);
     }
 }
 
@@ -194,16 +190,14 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
     }
 
     const bool e2m1 = a->value_format == CSRSPMM_B200_VALUES_E2M1;
-    cudaError_t attr_err = cudaSuccess;
+    cudaError_t err = cudaSuccess;
     if (plan.kernel == CSRSPMM_B200_KERNEL_ROW) {
-        attr_err = launch_row_kernel(p, plan, e2m1, st);
+        err = launch_row_kernel(p, plan, e2m1, st);
     } else if (plan.kernel == CSRSPMM_B200_KERNEL_MERGE) {
-        attr_err = launch_merge_kernel(p, plan, e2m1, st);
+        err = launch_merge_kernel(p, plan, e2m1, st);
     } else {
-        attr_err = e2m1 ? dispatch_tma<kValuesE2M1>(p, plan, st) : dispatch_tma<kValuesF32>(p, plan, st);
+        err = e2m1 ? dispatch_tma<kValuesE2M1>(p, plan, st) : dispatch_tma<kValuesF32>(p, plan, st);
     }
-    cudaError_t err = attr_err != cudaSuccess ? attr_err : cudaGetLastError();
-
     if (err == cudaSuccess && split) err = launch_fixup_kernel(p, plan, st);
     if (ws_owned) {
         cudaError_t ferr = cudaFreeAsync(ws, st);
@@ -379,14 +373,8 @@ namespace csrspmm_b200 {
 
 cudaError_t launch_row_kernel(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st)
 {
-    if (plan.VW == 4) {
-        if (e2m1) dispatch_row<4, kValuesE2M1>(p, plan, st);
-        else dispatch_row<4, kValuesF32>(p, plan, st);
-    } else {
-        if (e2m1) dispatch_row<1, kValuesE2M1>(p, plan, st);
-        else dispatch_row<1, kValuesF32>(p, plan, st);
-    }
-    return cudaGetLastError();
+    if (plan.VW == 4) return e2m1 ? dispatch_row<4, kValuesE2M1>(p, plan, st) : dispatch_row<4, kValuesF32>(p, plan, st);
+    return e2m1 ? dispatch_row<1, kValuesE2M1>(p, plan, st) : dispatch_row<1, kValuesF32>(p, plan, st);
 }
 
 }  // namespace csrspmm_b200

@@ -219,6 +219,12 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow)
 #endif
         }
     }
+    // A next grid placed early goes where slots are free.  Behind a grid that fills the chip those are the slots
+    // its CTAs leave, one by one and evenly; behind a smaller one they crowd on the SMs that had room, and the
+    // crowded SMs finish late (4096 rows of 410 entries, 128 columns: 46.2 us per product against 43.4).
+    plan->fills_chip = plan->grid >= 148LL * (kernel == CSRSPMM_B200_KERNEL_ROW     ? (plan->low_occupancy ? 2 : row_min_blocks(plan->NV))
+                                              : kernel == CSRSPMM_B200_KERNEL_MERGE ? merge_min_blocks(plan->NV)
+                                                                                    : CSRSPMM_TUNE_TMA_MINB);
     if (plan->grid > 0x7fffffffLL) {
         set_last_error("grid of %lld CTAs exceeds the launch limit", plan->grid);
         return CSRSPMM_B200_ERR_UNSUPPORTED;

@@ -21,6 +21,7 @@ struct Plan {
     bool small_tile = false;               // merge kernel: the small-problem tile (fewer items per lane group)
     int narrow = 0;                        // merge kernel: 1 + index into kNarrowShapes when the dense operand has at
                                            // most four column vectors (lane groups of 1, 2 or 4 lanes), else 0
+    bool fills_chip = false;               // the grid takes every CTA slot of the chip at least once
     int G = 8, NV = 1, VW = 4;             // lanes per group, vectors per lane, vector width
     int ncolv = 0;                         // ceil(Nd / VW)
     int tile = 0;                          // merge-path items per CTA (split kernels)

@@ -49,6 +49,7 @@ struct SpmmParams {
     long long carry_ld;  // multiple of 4
     int* status_word;    // may be null
     unsigned wait_limit; // bulk-copy kernel: attempts a wait on a row copy makes before it gives up
+    int release_early;   // let the next grid of the stream be placed while this one runs (Plan::fills_chip)
     int skip_len;        // merge kernel with SKIP: rows of this many entries or more are left to the
                          // scheduled pieces (neither summed nor written); 0 = every row is mine
 };

@@ -369,6 +369,10 @@ __device__ __forceinline__ void merge_tile_finish(const SpmmParams& p, Smem& s, 
 template <int G, int NV, int VW, int TG, int U, int FMT, bool FULL, bool SKIP = false>
 __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merge_kernel(const SpmmParams p)
 {
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
     using Smem = MergeSmem<G, NV, VW, TG>;
     __shared__ Smem s;
 
@@ -540,6 +544,10 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
 template <int VW>
 __global__ void __launch_bounds__(256) spmm_fixup_kernel(const SpmmParams p, int num_tiles)
 {
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (t >= num_tiles) return;

@@ -26,6 +26,10 @@ constexpr int kRowThreads = CSRSPMM_TUNE_ROW_THREADS;
 template <int G, int NV, int VW, int U, int FMT, bool FULL, int MINB>
 __global__ void __launch_bounds__(kRowThreads, MINB) spmm_row_kernel(const SpmmParams p)
 {
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
     constexpr int GROUPS = kRowThreads / G;
     const cg::thread_block_tile<G> tile = cg::tiled_partition<G>(cg::this_thread_block());
     const int lane = tile.thread_rank();

@@ -117,6 +117,8 @@ __global__ void __launch_bounds__(kMergeThreads, CSRSPMM_TUNE_TMA_MINB) spmm_tma
         fence_mbar_init();
         fence_proxy_async_smem();
     }
+    wait_for_previous_grid();
+    if (p.release_early) release_next_grid();
     // the __syncthreads inside merge_tile_setup make the initialised barriers visible
 
     TileRange r;
