@@ -9,6 +9,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <new>
+#include <vector>
 
 #include "../kernels/aux_kernels.cuh"
 #include "../kernels/merge_kernel.cuh"
@@ -281,6 +284,106 @@ int column_panel_layout(int32_t Kd, int32_t Nd, int requested, int32_t* first, i
     return count;
 }
 
+// Two streams and the events of one host round trip.  Making and destroying them took 60 to 100 us of every call; up to
+// kPipesKept sets per device wait for the next call instead (what is above is destroyed at once).
+class HostPipe {
+public:
+    static constexpr int kEvents = 2 * kMaxPanels;
+    ~HostPipe()
+    {
+        if (set_ == nullptr) return;
+        std::lock_guard<std::mutex> lock(mutex());
+        auto& kept = pool();
+        int same = 0;
+        for (const Set* k : kept) same += k->device == set_->device;
+        if (same < kPipesKept) kept.push_back(set_);
+        else destroy(set_);
+    }
+    cudaError_t init()
+    {
+        int device = -1;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return e;
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            auto& kept = pool();
+            for (size_t k = 0; k < kept.size(); ++k)
+                if (kept[k]->device == device) {
+                    set_ = kept[k];
+                    kept.erase(kept.begin() + (long)k);
+                    return cudaSuccess;
+                }
+        }
+        Set* s = new (std::nothrow) Set();
+        if (s == nullptr) return cudaErrorMemoryAllocation;
+        s->device = device;
+        e = cudaStreamCreateWithFlags(&s->compute, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->out, cudaStreamNonBlocking);
+        for (int k = 0; k < kEvents && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&s->event[k], cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            destroy(s);
+            return e;
+        }
+        set_ = s;
+        return cudaSuccess;
+    }
+    cudaStream_t compute() const { return set_->compute; }
+    cudaStream_t out() const { return set_->out; }
+    cudaEvent_t up(int k) const { return set_->event[k]; }
+    cudaEvent_t done(int k) const { return set_->event[kMaxPanels + k]; }
+
+private:
+    static constexpr int kPipesKept = 2;
+    struct Set {
+        int device = -1;
+        cudaStream_t compute = nullptr, out = nullptr;
+        cudaEvent_t event[kEvents] = {};
+    };
+    static void destroy(Set* s)
+    {
+        for (cudaEvent_t ev : s->event)
+            if (ev) cudaEventDestroy(ev);
+        if (s->compute) cudaStreamDestroy(s->compute);
+        if (s->out) cudaStreamDestroy(s->out);
+        delete s;
+    }
+    static std::mutex& mutex()
+    {
+        static std::mutex m;
+        return m;
+    }
+    static std::vector<Set*>& pool()
+    {
+        static std::vector<Set*>* kept = new std::vector<Set*>();  // not destroyed: CUDA may be gone by then
+        return *kept;
+    }
+    Set* set_ = nullptr;
+};
+
+// Rows of `width` bytes between host and device; one plain copy when both sides are packed (the copy engine takes
+// packed rows of 24 floats at a third of the link's rate when they are described as a pitched matrix).
+cudaError_t copy_matrix(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows, cudaMemcpyKind kind, cudaStream_t st)
+{
+    if (rows == 0 || width == 0) return cudaSuccess;
+    if (rows == 1 || (dpitch == width && spitch == width)) return cudaMemcpyAsync(dst, src, width * rows, kind, st);
+    return cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, kind, st);
+}
+
+// Panels to ask column_panel_layout for: 0 = its own rule (and the environment's say).  Below that rule's 256 MiB a
+// product whose time is B going up and C coming down still gains from panels of 64 columns and more (256-byte
+// segments; narrower ones copy too slowly in both directions at once): 262 144 rows, 128 columns 5.40 -> 4.72 ms in
+// two, 60 000 x 256 2.39 -> 1.88 in four, 15 000 x 512 1.27 -> 0.98, 6000 x 512 (25 MB) 0.62 -> 0.55.  Where A is
+// a fair share of the bytes, or one of B and C is small, row blocks overlap more.
+int host_panels(const csrspmm_b200_args* a, size_t a_bytes)
+{
+    const char* e = std::getenv("CSRSPMM_HOST_PANELS");
+    const double b = (double)a->Kd * a->Nd * 4, c = (double)a->M * a->Nd * 4;
+    const bool ruled = b >= 268435456.0 && a->Nd >= 256;
+    if ((e != nullptr && std::atoi(e) > 0) || ruled || a->Nd < 128 || b + c < 2.0e7 || (double)a_bytes > (b + c) / 4 || b > 4 * c || c > 4 * b)
+        return 0;
+    return a->Nd >= 256 ? 4 : a->Nd / 64;
+}
+
 struct HostBuffers {
     int32_t* rp;
     int32_t* ci;
@@ -292,48 +395,36 @@ struct HostBuffers {
     int32_t* status;
 };
 
-int spmm_host_panels(const csrspmm_b200_args* a, const HostBuffers& d, int panels, cudaStream_t st, int* word)
+int spmm_host_panels(const csrspmm_b200_args* a, const HostBuffers& d, int want_panels, cudaStream_t st, int* word)
 {
     int32_t first[kMaxPanels], width[kMaxPanels];
-    panels = column_panel_layout(a->Kd, a->Nd, panels, first, width);
+    const int panels = column_panel_layout(a->Kd, a->Nd, want_panels, first, width);
 
-    cudaStream_t compute = nullptr, out = nullptr;
-    cudaEvent_t up[kMaxPanels] = {}, done[kMaxPanels] = {};
-    int n_up = 0, n_done = 0;
-    auto cleanup = [&]() {
-        for (int k = 0; k < n_up; ++k) cudaEventDestroy(up[k]);
-        for (int k = 0; k < n_done; ++k) cudaEventDestroy(done[k]);
-        if (compute) cudaStreamDestroy(compute);
-        if (out) cudaStreamDestroy(out);
-    };
+    HostPipe pipe;
 #define CUDA_TRY_PANEL(expr)                                                                \
     do {                                                                                    \
         cudaError_t e__ = (expr);                                                           \
         if (e__ != cudaSuccess) {                                                           \
             set_last_error("%s failed: %s", #expr, cudaGetErrorString(e__));                \
             cudaDeviceSynchronize();                                                        \
-            cleanup();                                                                      \
             return CSRSPMM_B200_ERR_CUDA;                                                   \
         }                                                                                   \
     } while (0)
 
-    CUDA_TRY_PANEL(cudaStreamCreateWithFlags(&compute, cudaStreamNonBlocking));
-    CUDA_TRY_PANEL(cudaStreamCreateWithFlags(&out, cudaStreamNonBlocking));
-    for (; n_up < panels; ++n_up) CUDA_TRY_PANEL(cudaEventCreateWithFlags(&up[n_up], cudaEventDisableTiming));
-    for (; n_done < panels; ++n_done) CUDA_TRY_PANEL(cudaEventCreateWithFlags(&done[n_done], cudaEventDisableTiming));
+    CUDA_TRY_PANEL(pipe.init());
+    const cudaStream_t compute = pipe.compute(), out = pipe.out();
 
     for (int q = 0; q < panels; ++q) {
         const int c0 = first[q], w = width[q];
         float* dB = d.B + (size_t)a->Kd * (size_t)c0;
         float* dC = d.C + (size_t)a->M * (size_t)c0;
         if (a->beta != 0.0f)
-            CUDA_TRY_PANEL(cudaMemcpy2DAsync(dC, (size_t)w * 4, a->C + c0, (size_t)a->ldc * 4, (size_t)w * 4,
-                                             (size_t)a->M, cudaMemcpyHostToDevice, st));
+            CUDA_TRY_PANEL(copy_matrix(dC, (size_t)w * 4, a->C + c0, (size_t)a->ldc * 4, (size_t)w * 4, (size_t)a->M, cudaMemcpyHostToDevice, st));
         if (a->Kd > 0)
             CUDA_TRY_PANEL(cudaMemcpy2DAsync(dB, (size_t)w * 4, a->B + c0, (size_t)a->ldb * 4, (size_t)w * 4,
                                              (size_t)a->Kd, cudaMemcpyHostToDevice, st));
-        CUDA_TRY_PANEL(cudaEventRecord(up[q], st));
-        CUDA_TRY_PANEL(cudaStreamWaitEvent(compute, up[q], 0));
+        CUDA_TRY_PANEL(cudaEventRecord(pipe.up(q), st));
+        CUDA_TRY_PANEL(cudaStreamWaitEvent(compute, pipe.up(q), 0));
 
         csrspmm_b200_args pa = *a;
         pa.Nd = w;
@@ -350,11 +441,10 @@ int spmm_host_panels(const csrspmm_b200_args* a, const HostBuffers& d, int panel
         const int status = enqueue(&pa, compute);
         if (status != CSRSPMM_B200_OK) {
             cudaDeviceSynchronize();
-            cleanup();
             return status;
         }
-        CUDA_TRY_PANEL(cudaEventRecord(done[q], compute));
-        CUDA_TRY_PANEL(cudaStreamWaitEvent(out, done[q], 0));
+        CUDA_TRY_PANEL(cudaEventRecord(pipe.done(q), compute));
+        CUDA_TRY_PANEL(cudaStreamWaitEvent(out, pipe.done(q), 0));
         CUDA_TRY_PANEL(cudaMemcpy2DAsync(a->C + c0, (size_t)a->ldc * 4, dC, (size_t)w * 4, (size_t)w * 4, (size_t)a->M,
                                          cudaMemcpyDeviceToHost, out));
     }
@@ -362,7 +452,6 @@ int spmm_host_panels(const csrspmm_b200_args* a, const HostBuffers& d, int panel
     CUDA_TRY_PANEL(cudaStreamSynchronize(compute));
     CUDA_TRY_PANEL(cudaStreamSynchronize(out));
     CUDA_TRY_PANEL(cudaStreamSynchronize(st));
-    cleanup();
     return CSRSPMM_B200_OK;
 #undef CUDA_TRY_PANEL
 }
@@ -502,8 +591,9 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
     if (ci_dev) d_ci = const_cast<int32_t*>(a->col_idx);
     if (va_dev) d_va = const_cast<char*>(static_cast<const char*>(a->values));
 
-    const int panels = column_panel_layout(a->Kd, a->Nd, 0, nullptr, nullptr);
-    if (panels > 1) {
+    const size_t a_up = (rp_dev ? 0 : rp_bytes) + (ci_dev ? 0 : ci_bytes) + (va_dev ? 0 : vbytes);
+    const int want_panels = host_panels(a, a_up);
+    if (column_panel_layout(a->Kd, a->Nd, want_panels, nullptr, nullptr) > 1) {
         // A first, on the caller's stream; the panels of B follow it on the same stream
         int word = 0;
         cudaError_t e = cudaMemsetAsync(d_status, 0, 4, st);
@@ -515,7 +605,7 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
             status = CSRSPMM_B200_ERR_CUDA;
         } else {
             const HostBuffers hb = {d_rp, d_ci, d_va, d_B, d_C, d_ws, align256(ws_bytes), d_status};
-            status = spmm_host_panels(a, hb, panels, st, &word);
+            status = spmm_host_panels(a, hb, want_panels, st, &word);
         }
         if (owned) {
             cudaFreeAsync(arena, st);
@@ -533,10 +623,21 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
         return CSRSPMM_B200_OK;
     }
 
-    // C goes back in row blocks on a second stream while the next block is being computed, so
-    // the device->host copy of a large C hides the kernel time (and vice versa).
-    constexpr int kMaxBlocks = 8;
-    int blocks = (c_bytes >= ((size_t)64 << 20) && a->M >= 64) ? kMaxBlocks : 1;
+    // In row blocks, each direction of the link on a stream of its own: B goes up first, then A (and C_old) block by
+    // block, and each block of C comes down while the next block of A goes up and is multiplied.  A large C always
+    // goes in four blocks (kernels overlap its copy); a smaller product only when part of A comes from the host, in
+    // blocks of 8 MB and more.  More and smaller copies in both directions at once slow each other down: 151 202 rows, 64
+    // columns, 66 MB in all: 1.40 / 1.25 / 1.23 / 1.30 / 1.37 ms with 2 / 3 / 4 / 8 / 12 blocks, 1.35 for the copies alone one
+    // after the other.
+    constexpr int kMaxBlocks = 4;
+    static_assert(kMaxBlocks <= kMaxPanels, "one pair of events per block");
+    int blocks = 1;
+    if (c_bytes >= ((size_t)64 << 20) && a->M >= 64) {
+        blocks = kMaxBlocks;
+    } else if (!rp_dev && !(ci_dev && va_dev) && a->M >= 64) {
+        const size_t n = (c_bytes + ci_bytes + vbytes) >> 23;
+        blocks = n < 1 ? 1 : (n > kMaxBlocks ? kMaxBlocks : (int)n);
+    }
     int32_t bounds[kMaxBlocks + 1] = {0};
     bounds[1] = a->M;
     // the row blocks are cut on the host: a row_ptr that lives on the device is read back once (4 bytes per row)
@@ -551,23 +652,31 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
         h_rp = h_rp_copy;
     }
     if (blocks > 1 && csrspmm_b200_partition_rows(a->M, h_rp, blocks, 1.0, bounds) != CSRSPMM_B200_OK) blocks = 1;
-    if (blocks > 1 && e2m1)  // packed values can only be offset by whole bytes
-        for (int k = 1; k < blocks; ++k)
-            if (h_rp[bounds[k]] & 1) blocks = 1;
+    if (blocks > 1) {
+        if (e2m1)  // packed values can only be cut at whole bytes: move a cut down to a row that begins at one
+            for (int k = 1; k < blocks; ++k) {
+                if (bounds[k] < bounds[k - 1]) bounds[k] = bounds[k - 1];
+                while (bounds[k] < a->M && (h_rp[bounds[k]] & 1)) ++bounds[k];
+            }
+        bool sane = h_rp[bounds[0]] >= 0;  // offsets the copies below can rely on, else one block
+        for (int k = 1; k <= blocks && sane; ++k)
+            sane = bounds[k] >= bounds[k - 1] && h_rp[bounds[k]] >= h_rp[bounds[k - 1]] && h_rp[bounds[k]] <= a->nnz;
+        if (!sane) blocks = 1;
+    }
     if (blocks == 1) bounds[1] = a->M;
 
-    cudaStream_t copy_stream = nullptr;
-    cudaEvent_t done[kMaxBlocks] = {};
-    int events = 0;
+    HostPipe pipe;
+    PinnedSlot pinned;
     auto cleanup = [&]() {
         // also the way out of every failure below: nothing may still be copying into or out of the
         // arena, or into this frame's `word`, when they go away (errors of these waits are ignored)
         cudaStreamSynchronize(st);
-        if (copy_stream) cudaStreamSynchronize(copy_stream);
+        if (blocks > 1) {
+            cudaStreamSynchronize(pipe.compute());
+            cudaStreamSynchronize(pipe.out());
+        }
         std::free(h_rp_copy);
         h_rp_copy = nullptr;
-        for (int k = 0; k < events; ++k) cudaEventDestroy(done[k]);
-        if (copy_stream) cudaStreamDestroy(copy_stream);
         if (owned) cudaFreeAsync(arena, st);
     };
 #define CUDA_TRY_HOST(expr)                                                                 \
@@ -581,61 +690,69 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
     } while (0)
 
     if (blocks > 1) {
-        CUDA_TRY_HOST(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
-        for (; events < blocks; ++events) CUDA_TRY_HOST(cudaEventCreateWithFlags(&done[events], cudaEventDisableTiming));
+        const cudaError_t e = pipe.init();
+        if (e != cudaSuccess) {
+            blocks = 1;  // cleanup() must not touch the pipe
+            bounds[1] = a->M;
+            cudaGetLastError();
+        }
     }
+    const cudaStream_t compute = blocks > 1 ? pipe.compute() : st, out = blocks > 1 ? pipe.out() : st;
+    const size_t row_bytes = (size_t)a->Nd * 4;
     CUDA_TRY_HOST(cudaMemsetAsync(d_status, 0, 4, st));
     if (!rp_dev) CUDA_TRY_HOST(cudaMemcpyAsync(d_rp, a->row_ptr, rp_bytes, cudaMemcpyHostToDevice, st));
-    if (a->nnz > 0) {
-        if (!ci_dev) CUDA_TRY_HOST(cudaMemcpyAsync(d_ci, a->col_idx, ci_bytes, cudaMemcpyHostToDevice, st));
-        if (!va_dev) CUDA_TRY_HOST(cudaMemcpyAsync(d_va, a->values, vbytes, cudaMemcpyHostToDevice, st));
-    }
-    if (a->Kd > 0) {
-        // B rows are packed on the device (ldb = Nd) whatever the host stride is
-        CUDA_TRY_HOST(cudaMemcpy2DAsync(d_B, (size_t)a->Nd * 4, a->B, (size_t)a->ldb * 4,
-                                        (size_t)a->Nd * 4, (size_t)a->Kd, cudaMemcpyHostToDevice, st));
-    }
-    if (a->beta != 0.0f) {
-        CUDA_TRY_HOST(cudaMemcpy2DAsync(d_C, (size_t)a->Nd * 4, a->C, (size_t)a->ldc * 4,
-                                        (size_t)a->Nd * 4, (size_t)a->M, cudaMemcpyHostToDevice, st));
-    }
+    // B rows are packed on the device (ldb = Nd) whatever the host stride is
+    CUDA_TRY_HOST(copy_matrix(d_B, row_bytes, a->B, (size_t)a->ldb * 4, row_bytes, (size_t)a->Kd, cudaMemcpyHostToDevice, st));
     for (int k = 0; k < blocks; ++k) {
         const int32_t r0 = bounds[k], r1 = bounds[k + 1];
         if (r1 <= r0) continue;
         // (one block: the whole matrix, and row_ptr may be device memory that the host cannot read)
         const int32_t j0 = blocks > 1 ? h_rp[r0] : 0, j1 = blocks > 1 ? h_rp[r1] : (int32_t)a->nnz;
+        const size_t n = (size_t)(j1 - j0);
+        const size_t v0 = e2m1 ? (size_t)j0 / 2 : (size_t)j0 * 4;
+        if (n > 0 && !ci_dev) CUDA_TRY_HOST(cudaMemcpyAsync(d_ci + j0, a->col_idx + j0, n * 4, cudaMemcpyHostToDevice, st));
+        if (n > 0 && !va_dev)
+            CUDA_TRY_HOST(cudaMemcpyAsync(d_va + v0, static_cast<const char*>(a->values) + v0, e2m1 ? (n + 1) / 2 : n * 4,
+                                          cudaMemcpyHostToDevice, st));
+        float* const host_C = a->C + (size_t)r0 * (size_t)a->ldc;
+        float* const block_C = d_C + (size_t)r0 * (size_t)a->Nd;
+        if (a->beta != 0.0f)
+            CUDA_TRY_HOST(copy_matrix(block_C, row_bytes, host_C, (size_t)a->ldc * 4, row_bytes, (size_t)(r1 - r0), cudaMemcpyHostToDevice, st));
+        if (blocks > 1) {
+            CUDA_TRY_HOST(cudaEventRecord(pipe.up(k), st));
+            CUDA_TRY_HOST(cudaStreamWaitEvent(compute, pipe.up(k), 0));
+        }
         csrspmm_b200_args d = *a;
         d.M = r1 - r0;
-        d.nnz = (int64_t)j1 - j0;
+        d.nnz = (int64_t)n;
         d.row_ptr = d_rp + r0;
         d.row_ptr_base = j0;
         d.col_idx = d_ci + j0;
-        d.values = e2m1 ? static_cast<const void*>(d_va + j0 / 2) : static_cast<const void*>(d_va + (size_t)j0 * 4);
+        d.values = d_va + v0;
         d.B = d_B;
         d.ldb = a->Nd;
-        d.C = d_C + (size_t)r0 * (size_t)a->Nd;
+        d.C = block_C;
         d.ldc = a->Nd;
         d.workspace = d_ws;
         d.workspace_bytes = align256(ws_bytes);
         d.status_word = d_status;
-        status = enqueue(&d, st);
+        status = enqueue(&d, compute);
         if (status != CSRSPMM_B200_OK) {
             cleanup();
             return status;
         }
-        cudaStream_t out_stream = st;
         if (blocks > 1) {
-            CUDA_TRY_HOST(cudaEventRecord(done[k], st));
-            CUDA_TRY_HOST(cudaStreamWaitEvent(copy_stream, done[k], 0));
-            out_stream = copy_stream;
+            CUDA_TRY_HOST(cudaEventRecord(pipe.done(k), compute));
+            CUDA_TRY_HOST(cudaStreamWaitEvent(out, pipe.done(k), 0));
         }
-        CUDA_TRY_HOST(cudaMemcpy2DAsync(a->C + (size_t)r0 * (size_t)a->ldc, (size_t)a->ldc * 4, d.C, (size_t)a->Nd * 4,
-                                        (size_t)a->Nd * 4, (size_t)(r1 - r0), cudaMemcpyDeviceToHost, out_stream));
+        CUDA_TRY_HOST(copy_matrix(host_C, (size_t)a->ldc * 4, block_C, row_bytes, row_bytes, (size_t)(r1 - r0), cudaMemcpyDeviceToHost, out));
     }
     int word = 0;
-    CUDA_TRY_HOST(cudaMemcpyAsync(&word, d_status, 4, cudaMemcpyDeviceToHost, st));
+    int* const word_at = pinned.words() != nullptr ? reinterpret_cast<int*>(const_cast<long long*>(pinned.words())) : &word;
+    CUDA_TRY_HOST(cudaMemcpyAsync(word_at, d_status, 4, cudaMemcpyDeviceToHost, out));
+    CUDA_TRY_HOST(cudaStreamSynchronize(out));
     CUDA_TRY_HOST(cudaStreamSynchronize(st));
-    if (copy_stream) CUDA_TRY_HOST(cudaStreamSynchronize(copy_stream));
+    word = *static_cast<volatile int*>(word_at);
     cleanup();
     if (owned) CUDA_TRY(cudaStreamSynchronize(st));
     if (word & kStatusWaitTimeout) {
@@ -664,9 +781,8 @@ int csrspmm_b200_copy_rows(void* dst, size_t dst_pitch_bytes, const void* src, s
         set_last_error("copy_rows: null pointer or pitch smaller than the row width");
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
-    CUDA_TRY(cudaMemcpy2DAsync(dst, dst_pitch_bytes, src, src_pitch_bytes, width_bytes, rows,
-                               to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
-                               reinterpret_cast<cudaStream_t>(stream)));
+    CUDA_TRY(copy_matrix(dst, dst_pitch_bytes, src, src_pitch_bytes, width_bytes, rows,
+                         to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, reinterpret_cast<cudaStream_t>(stream)));
     return CSRSPMM_B200_OK;
 }
 

@@ -336,6 +336,11 @@ def spmm_host(row_ptr, col_idx, values, B, C_host, alpha=1.0, beta=0.0, *, entry
                        kernel=_lib.KERNEL_IDS[kernel], max_row_nnz=max_row_nnz)
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
+        if arena is None and M > 0 and Nd > 0:
+            # from torch's allocator, which has the pages mapped: the stream-ordered allocator gives them back at every
+            # call's wait and maps 170 MB anew for 2.5 ms (negative sizes and the like: 0 bytes, refused below)
+            need = int(_lib.lib().csrspmm_b200_host_arena_bytes(C.byref(a)))
+            arena = torch.empty(need, dtype=torch.uint8, device=dev) if need > 0 else None
         stream = torch.cuda.current_stream(dev).cuda_stream
         st = _lib.lib().csrspmm_b200_spmm_host(C.byref(a), arena.data_ptr() if arena is not None else None,
                                                arena.numel() if arena is not None else 0, C.c_void_p(stream))
