@@ -38,6 +38,7 @@ void fill_params(const csrspmm_b200_args* a, const Plan& plan, SpmmParams* out)
     p.ncolv = plan.ncolv;
     p.num_items = plan.num_items;
     p.release_early = plan.fills_chip;
+    p.tg = plan.tg;
     p.row_ptr = a->row_ptr;
     p.rp_base = a->row_ptr_base;
     p.col_idx = a->col_idx;

@@ -88,7 +88,9 @@ extern "C" int csrspmm_b200_spmm_noalloc(const csrspmm_b200_args* args, csrspmm_
     a.workspace_bytes = 0;
     a.schedule = nullptr;  // a schedule's scratch would not fit the fixed array's contract
     Plan plan;
-    status = make_plan(&a, &plan);
+    status = make_plan(&a, &plan);  // the same tiles as csrspmm_b200_spmm, unless they leave too many carry rows
+    if (status == CSRSPMM_B200_OK && plan.workspace_bytes > (size_t)CSRSPMM_B200_NOALLOC_SCRATCH_BYTES)
+        status = make_plan(&a, &plan, true, /*coarse=*/true);
     if (status != CSRSPMM_B200_OK) return status;
     if (plan.workspace_bytes > (size_t)CSRSPMM_B200_NOALLOC_SCRATCH_BYTES) {
         set_last_error("csrspmm_b200_spmm_noalloc: this problem (M + nnz = %lld, Nd = %d) needs %zu bytes of "

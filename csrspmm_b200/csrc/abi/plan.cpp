@@ -115,21 +115,12 @@ static int forced_kernel_from_env()
     return CSRSPMM_B200_KERNEL_AUTO;
 }
 
-int merge_tile_for(int shape, long long num_items, bool* small)
+static void fill_split_geometry(const csrspmm_b200_args* a, Plan* plan, int groups, int tg)
 {
-    const int groups = CSRSPMM_TUNE_MERGE_THREADS / kShapes[shape].G;
-    const int big = groups * kShapes[shape].TG;
-    const bool use_small = CSRSPMM_TUNE_MERGE_TG_SMALL < kShapes[shape].TG &&
-                           num_items < (long long)big * 148 * CSRSPMM_TUNE_MERGE_SMALL_BELOW_CTAS_PER_SM;
-    if (small != nullptr) *small = use_small;
-    return use_small ? groups * CSRSPMM_TUNE_MERGE_TG_SMALL : big;
-}
-
-static void fill_split_geometry(const csrspmm_b200_args* a, Plan* plan, int tile)
-{
-    plan->tile = tile;
+    plan->tg = tg;
+    plan->tile = groups * tg;
     plan->num_items = (long long)a->M + a->nnz;
-    plan->num_tiles = (plan->num_items + tile - 1) / tile;
+    plan->num_tiles = (plan->num_items + plan->tile - 1) / plan->tile;
     plan->grid = plan->num_tiles;
     plan->carry_ld = ((long long)a->Nd + 3) / 4 * 4;
     plan->carry_row_bytes = align_up((size_t)plan->num_tiles * sizeof(int32_t), 256);
@@ -137,7 +128,22 @@ static void fill_split_geometry(const csrspmm_b200_args* a, Plan* plan, int tile
         plan->carry_row_bytes + (size_t)plan->num_tiles * (size_t)plan->carry_ld * sizeof(float);
 }
 
-int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow)
+// Items per lane group of the merge kernel: up to three waves of CTAs get tiles of one size that fill the waves;
+// longer grids take the largest tile (most).  A tile of fixed size left 1.1 M items with 363 CTAs for 592 slots, and
+// problems of a few ten thousand items with 64-item walks on a few CTAs: 65 536 rows of 16, 64 columns 32.0 -> 27.9 us,
+// 16 384 rows of 16, 256 columns 31.7 -> 23.3, 16 384 rows of 4, 64 columns 13.6 -> 10.4, 1024 rows 11.7 -> 7.7.  Beyond
+// three waves equal tiles gain nothing and their CTAs march in step (1 M rows of 16: 618 us against 600).  Not below
+// `least`: a CTA's search and staging cost as much as a walk of some 16 items.
+static int merge_items_per_group(long long num_items, int groups, int ctas_per_sm, int most, int least)
+{
+    const long long wave = 148LL * ctas_per_sm * groups;
+    const long long waves = (num_items + wave * most - 1) / (wave * most);
+    if (waves > 3) return most;
+    const long long tg = waves > 0 ? (num_items + wave * waves - 1) / (wave * waves) : 1;
+    return (int)(tg < least ? least : (tg > most ? most : tg));
+}
+
+int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow, bool coarse)
 {
     int st = check_args(a, false);
     if (st != CSRSPMM_B200_OK) return st;
@@ -155,20 +161,23 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow)
         if (kernel == CSRSPMM_B200_KERNEL_TMA && !tma_can_run(a)) kernel = CSRSPMM_B200_KERNEL_AUTO;
     }
     if (kernel == CSRSPMM_B200_KERNEL_AUTO) {
-        // Measured on B200: the bulk-copy path completes about one row copy per 80
-        // cycles per SM, so it only keeps HBM busy when a row of B is 2 KB (384 < Nd <= 512),
-        // where it is 3-4 % ahead of the merge kernel -- provided B is far larger than L2, since
-        // an L2-resident B is served faster through the load/store units.  Whole-row mapping
-        // wins when the longest row is known and close to the mean; everything else (unknown
-        // or skewed row lengths) takes the merge-path kernel.  The entry point asked for does
-        // not change the choice.
+        // Measured on B200.  The bulk-copy path completes about one row copy per 80 cycles per SM, so it
+        // only keeps HBM busy when a row of B is 2 KB (384 < Nd <= 512), where it is 3-4 % ahead of the merge
+        // kernel -- provided B is far larger than L2, since an L2-resident B is served faster through the
+        // load/store units.  Whole-row mapping wins when the longest row is known and close to the mean and B
+        // comes from L2.  Beyond about 48 MB of B the time is the wait for HBM, and a lane group that stops at every
+        // row end (bounds, columns, rows of B, store, each a round trip) asks for too little of it at once: the
+        // merge kernel walks on across row ends (1 M rows of 16, 64 columns: 600 us against 812; 262 144 rows of 8:
+        // 73 against 94; of 4: 51 against 74), unless rows are long and wide enough to keep it busy by themselves
+        // (64 entries of 128 columns: 773 against 745; 32 of 256: 1012 either way).  Everything else (unknown or skewed row lengths) takes
+        // the merge kernel.  The entry point asked for does not change the choice.
         const double avg = a->M > 0 ? (double)a->nnz / (double)a->M : 0.0;
         const double row_limit = avg * 4.0 > 64.0 ? avg * 4.0 : 64.0;
         const double b_bytes = (double)a->Kd * (double)a->Nd * 4.0;
         const bool rows_even = a->max_row_nnz > 0 && (double)a->max_row_nnz <= row_limit;
         if (tma_can_run(a) && a->Nd > 384 && b_bytes >= 1073741824.0 && !rows_even)
             kernel = CSRSPMM_B200_KERNEL_TMA;
-        else if (rows_even)
+        else if (rows_even && (b_bytes < 48e6 || (avg * a->Nd >= 8192.0 && a->Nd > 64)))
             kernel = CSRSPMM_B200_KERNEL_ROW;
         else
             kernel = CSRSPMM_B200_KERNEL_MERGE;
@@ -185,7 +194,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow)
         plan->G = 32;
         plan->NV = plan->ncolv <= 32 ? 1 : (plan->ncolv <= 64 ? 2 : 4);
         plan->shape = plan->NV == 1 ? 2 : (plan->NV == 2 ? 3 : 4);
-        fill_split_geometry(a, plan, (CSRSPMM_TUNE_MERGE_THREADS / 32) * CSRSPMM_TUNE_TMA_TG);
+        fill_split_geometry(a, plan, CSRSPMM_TUNE_MERGE_THREADS / 32, CSRSPMM_TUNE_TMA_TG);
         const size_t slot = align_up((size_t)a->Nd * 4, 128);
         size_t ring = (size_t)CSRSPMM_TUNE_TMA_SLOTS * slot;          // per warp
         if (ring < (size_t)512 * plan->NV) ring = (size_t)512 * plan->NV;  // must also hold the partial sums
@@ -203,9 +212,14 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow)
             plan->G = ns.G;
             plan->NV = ns.NV;
             plan->full = plan->VW == 4 && plan->G * plan->NV == plan->ncolv;
-            fill_split_geometry(a, plan, (CSRSPMM_TUNE_MERGE_THREADS / ns.G) * ns.TG);
+            const int groups = CSRSPMM_TUNE_MERGE_THREADS / ns.G;
+            fill_split_geometry(a, plan, groups, merge_items_per_group(plan->num_items, groups, merge_min_blocks(1), ns.TG, coarse ? ns.TG : ns.G));
         } else if (kernel == CSRSPMM_B200_KERNEL_MERGE) {
-            fill_split_geometry(a, plan, merge_tile_for(plan->shape, plan->num_items, &plan->small_tile));
+            const int groups = CSRSPMM_TUNE_MERGE_THREADS / plan->G, most = kShapes[plan->shape].TG;
+            const int least = coarse ? CSRSPMM_TUNE_MERGE_TG_SMALL : CSRSPMM_TUNE_MERGE_TG_LEAST;
+            const int tg = merge_items_per_group(plan->num_items, groups, merge_min_blocks(plan->NV), most, least);
+            plan->small_tile = tg <= CSRSPMM_TUNE_MERGE_TG_SMALL;
+            fill_split_geometry(a, plan, groups, tg);
         } else {
             const int groups = CSRSPMM_TUNE_ROW_THREADS / plan->G;
             plan->grid = ((long long)a->M + groups - 1) / groups;
@@ -235,18 +249,22 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow)
 size_t worst_case_workspace(const csrspmm_b200_args* a, bool any_row_block)
 {
     if (check_args(a, false) != CSRSPMM_B200_OK) return 0;
-    // sized for the smallest tile any split kernel uses (most CTAs, most carry rows).  A row block of
-    // a large matrix may fall under the small-problem threshold although the whole matrix does not,
-    // so a caller that multiplies row blocks out of one scratch buffer asks for the small tile
-    // whatever the size (any_row_block).
-    int tile = (CSRSPMM_TUNE_MERGE_THREADS / 32) * CSRSPMM_TUNE_TMA_TG;  // TMA kernel
-    for (int k = 0; k < kNumShapes; ++k) {
-        const int t = merge_tile_for(k, any_row_block ? 0 : (long long)a->M + a->nnz, nullptr);
-        if (t < tile) tile = t;
-    }
+    // Most CTAs any split kernel takes: the bulk-copy kernel's fixed tile, or the merge kernel's waves of equal
+    // tiles -- no more than the largest tile gives plus one wave, whatever the size, so the same bound holds for
+    // every row block of the matrix.
+    (void)any_row_block;
+    const long long items = (long long)a->M + a->nnz;
     Plan p;
-    fill_split_geometry(a, &p, tile);
-    return p.workspace_bytes;
+    fill_split_geometry(a, &p, CSRSPMM_TUNE_MERGE_THREADS / 32, CSRSPMM_TUNE_TMA_TG);
+    long long tiles = p.num_tiles;
+    auto consider = [&](int groups, int most, int ctas_per_sm) {
+        const long long t = items / ((long long)groups * most) + 1 + 148LL * ctas_per_sm;
+        if (t > tiles) tiles = t;
+    };
+    for (const ShapeDesc& k : kShapes) consider(CSRSPMM_TUNE_MERGE_THREADS / k.G, k.TG, merge_min_blocks(k.NV));
+    for (const ShapeDesc& k : kNarrowShapes) consider(CSRSPMM_TUNE_MERGE_THREADS / k.G, k.TG, merge_min_blocks(1));
+    if (items < tiles) tiles = items;  // no CTA without an item
+    return align_up((size_t)tiles * sizeof(int32_t), 256) + (size_t)tiles * (size_t)p.carry_ld * sizeof(float);
 }
 
 }  // namespace csrspmm_b200

@@ -18,12 +18,13 @@ struct Plan {
     int shape = 0;                         // index into kShapes (tuning.h)
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
-    bool small_tile = false;               // merge kernel: the small-problem tile (fewer items per lane group)
+    bool small_tile = false;               // merge kernel: the build with shared memory for small tiles
     int narrow = 0;                        // merge kernel: 1 + index into kNarrowShapes when the dense operand has at
                                            // most four column vectors (lane groups of 1, 2 or 4 lanes), else 0
     bool fills_chip = false;               // the grid takes every CTA slot of the chip at least once
     int G = 8, NV = 1, VW = 4;             // lanes per group, vectors per lane, vector width
     int ncolv = 0;                         // ceil(Nd / VW)
+    int tg = 0;                            // merge-path items per lane group (split kernels)
     int tile = 0;                          // merge-path items per CTA (split kernels)
     long long num_items = 0;               // M + nnz
     long long num_tiles = 0;               // CTAs of the split kernels
@@ -43,11 +44,8 @@ bool vector_layout_ok(const csrspmm_b200_args* a);
 
 // Resolves AUTO (and the CSRSPMM_FORCE_KERNEL override) and fills the launch geometry.
 // Returns CSRSPMM_B200_OK or an error status.
-int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow = true);
-
-// Merge-path items per CTA of the merge kernel for lane-group shape `shape` on a problem of
-// `num_items` = M + nnz items (*small says whether the small-problem tile was chosen).
-int merge_tile_for(int shape, long long num_items, bool* small);
+// coarse: no tiles smaller than 64 items per lane group (fewer carry rows), for callers with a fixed scratch.
+int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow = true, bool coarse = false);
 
 // Workspace of the split kernels for a given plan-independent worst case: what
 // csrspmm_b200_workspace_bytes reports (the larger of the MERGE and TMA needs).  any_row_block:

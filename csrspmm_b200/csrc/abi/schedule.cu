@@ -188,14 +188,6 @@ int scheduled_plan(const csrspmm_b200_args* a, Plan* plan)
     m.schedule = nullptr;
     int status = make_plan(&m, plan, /*allow_narrow=*/false);  // the SKIP build exists for the regular shapes only
     if (status != CSRSPMM_B200_OK) return status;
-    if (plan->small_tile) {  // few items but a large B: keep the one instantiated tile
-        plan->small_tile = false;
-        const int tile = (CSRSPMM_TUNE_MERGE_THREADS / kShapes[plan->shape].G) * kShapes[plan->shape].TG;
-        plan->tile = tile;
-        plan->num_tiles = (plan->num_items + tile - 1) / tile;
-        plan->grid = plan->num_tiles;
-        plan->workspace_bytes = 0;  // recomputed below
-    }
     plan->carry_row_bytes = align256((size_t)plan->num_tiles * sizeof(int32_t));
     plan->workspace_bytes = plan->carry_row_bytes + align256((size_t)plan->num_tiles * (size_t)plan->carry_ld * sizeof(float));
     return CSRSPMM_B200_OK;

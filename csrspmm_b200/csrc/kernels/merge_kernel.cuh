@@ -7,7 +7,7 @@
 // The list of row ends (row_ptr[1..M]) is merged with the list of non-zero positions
 // (0..nnz-1); consuming a row end means "row finished, write it", consuming a position means
 // "one multiply-add per output column".  Diagonal d of that merge is found by binary search,
-// so CTA t owns items [t*TILE, (t+1)*TILE) and lane group g of the CTA owns TG of them, whatever
+// so CTA t owns items [t*T, (t+1)*T) and lane group g of the CTA owns p.tg of those T items, whatever
 // the row lengths are.
 //
 //   1. two warps search the CTA's two diagonals in row_ptr (32 probes per step);
@@ -73,6 +73,7 @@ __device__ __forceinline__ int merge_search_local(int d, const int* s_rowend, in
     return lo;
 }
 
+// TG: items per lane group it has room for (the launch says how many it takes, p.tg).
 template <int G, int NV, int VW, int TG>
 struct MergeSmem {
     static constexpr int GROUPS = kMergeThreads / G;
@@ -101,18 +102,18 @@ struct TileRange {
 // is inconsistent, or (SKIP) the tile lies inside one scheduled row.
 // SKIP: rows of p.skip_len entries or more belong to the scheduled pieces; they are marked in
 // s.longbits and 32-entry runs that lie wholly inside such a row are not fetched.
-template <class Smem, int G, int TG, int FMT, bool SKIP = false>
+template <class Smem, int G, int FMT, bool SKIP = false>
 __device__ __forceinline__ bool merge_tile_setup(const SpmmParams& p, Smem& s, TileRange& r)
 {
-    constexpr int TILE = Smem::TILE;
+    const int tile_items = Smem::GROUPS * p.tg;  // at most Smem::TILE
     constexpr int SB = CSRSPMM_TUNE_MERGE_STAGE_BATCH;
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int* __restrict__ row_end = p.row_ptr + 1;
 
     // ---- 1. the CTA's two diagonals --------------------------------------------------------
-    const long long d0 = (long long)blockIdx.x * TILE;
-    const long long d1 = min(d0 + (long long)TILE, p.num_items);
+    const long long d0 = (long long)blockIdx.x * tile_items;
+    const long long d1 = min(d0 + (long long)tile_items, p.num_items);
     if (warp < 2) {
         const long long d = warp == 0 ? d0 : d1;
         const int i = merge_search_warp(d, row_end, p.rp_base, p.M, p.nnz, tid & 31);
@@ -126,7 +127,7 @@ __device__ __forceinline__ bool merge_tile_setup(const SpmmParams& p, Smem& s, T
     r.j0 = s.coord[1];
     r.nrows = s.coord[2] - r.i0;
     r.nnzt = s.coord[3] - r.j0;
-    if (r.nrows < 0 || r.nnzt < 0 || r.nrows + r.nnzt > TILE) {  // malformed row_ptr: touch nothing
+    if (r.nrows < 0 || r.nnzt < 0 || r.nrows + r.nnzt > tile_items) {  // malformed row_ptr: touch nothing
         if (tid == 0) {
             report_status(p, kStatusBadTile);
             p.carry_row[blockIdx.x] = -1;
@@ -136,7 +137,7 @@ __device__ __forceinline__ bool merge_tile_setup(const SpmmParams& p, Smem& s, T
 
     // ---- 2. stage the slice ----------------------------------------------------------------
     // SB global loads in flight per thread and list, then the stores to shared memory: a load-store
-    // pair per iteration would make the staging a chain of TILE / kMergeThreads round trips to memory.
+    // pair per iteration would make the staging a chain of tile_items / kMergeThreads round trips to memory.
     auto clamp_col = [&](int c) {
         if ((unsigned)c >= (unsigned)p.Kd) {  // never fault on a bad index
             c = min(max(c, 0), p.Kd - 1);
@@ -232,8 +233,8 @@ __device__ __forceinline__ bool merge_tile_setup(const SpmmParams& p, Smem& s, T
     // ---- 3. the group's own range ----------------------------------------------------------
     const int g = tid / G;
     const int total = r.nrows + r.nnzt;
-    const int dl0 = min(g * TG, total);
-    const int dl1 = min(dl0 + TG, total);
+    const int dl0 = min(g * p.tg, total);
+    const int dl1 = min(dl0 + p.tg, total);
     r.il0 = merge_search_local(dl0, s.rowend, r.nrows, r.nnzt);
     r.jl0 = dl0 - r.il0;
     r.il1 = merge_search_local(dl1, s.rowend, r.nrows, r.nnzt);
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
     __shared__ Smem s;
 
     TileRange r;
-    if (!merge_tile_setup<Smem, G, TG, FMT, SKIP>(p, s, r)) return;
+    if (!merge_tile_setup<Smem, G, FMT, SKIP>(p, s, r)) return;
     const int g = threadIdx.x / G;
     const int lane = threadIdx.x % G;
     const char* const b_lane = reinterpret_cast<const char*>(p.B) + (size_t)lane * (VW * 4);

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kMergeThreads, CSRSPMM_TUNE_TMA_MINB) spmm_tma
     // the __syncthreads inside merge_tile_setup make the initialised barriers visible
 
     TileRange r;
-    if (!merge_tile_setup<Smem, G, TG, FMT>(p, s, r)) return;
+    if (!merge_tile_setup<Smem, G, FMT>(p, s, r)) return;
 
     const unsigned row_bytes = (unsigned)p.Nd * 4u;
     const unsigned ring_base = smem_u32(my_ring);

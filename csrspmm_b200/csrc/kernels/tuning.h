@@ -238,13 +238,13 @@
 
 namespace csrspmm_b200 {
 
-// merge kernel on small problems: when the regular tiles would give fewer than this many CTAs
-// per SM, lane groups take CSRSPMM_TUNE_MERGE_TG_SMALL items instead, so that the chip still fills
+// merge kernel: lane groups take no fewer items than this, and tiles of up to TG_SMALL items per group run the
+// build that has shared memory for just those (more of it left to L1)
+#ifndef CSRSPMM_TUNE_MERGE_TG_LEAST
+#define CSRSPMM_TUNE_MERGE_TG_LEAST 16
+#endif
 #ifndef CSRSPMM_TUNE_MERGE_TG_SMALL
 #define CSRSPMM_TUNE_MERGE_TG_SMALL 64
-#endif
-#ifndef CSRSPMM_TUNE_MERGE_SMALL_BELOW_CTAS_PER_SM
-#define CSRSPMM_TUNE_MERGE_SMALL_BELOW_CTAS_PER_SM 2
 #endif
 
 struct ShapeDesc {
