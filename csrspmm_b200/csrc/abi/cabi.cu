@@ -81,20 +81,25 @@ namespace {
         }                                                                                   \
     } while (0)
 
+template <int S, int VW, int FMT, bool FULL>
+cudaError_t launch_row_full(const SpmmParams& p, const Plan& plan, cudaStream_t st)
+{
+    constexpr int G = kShapes[S].G, NV = kShapes[S].NV;
+    constexpr int USHORT = row_unroll(VW, G, NV, FULL, true), ULONG = row_unroll(VW, G, NV, FULL, false);
+    constexpr int ULOW = row_unroll_low(NV);
+    constexpr int MINB = row_min_blocks(NV);
+    const unsigned grid = (unsigned)plan.grid;
+    if constexpr (VW == 4 && ULOW != ULONG)
+        if (plan.low_occupancy) return launch_overlapped(spmm_row_kernel<G, NV, VW, ULOW, FMT, FULL, 2>, grid, kRowThreads, 0, st, p);
+    if (plan.short_rows) return launch_overlapped(spmm_row_kernel<G, NV, VW, USHORT, FMT, FULL, MINB>, grid, kRowThreads, 0, st, p);
+    return launch_overlapped(spmm_row_kernel<G, NV, VW, ULONG, FMT, FULL, MINB>, grid, kRowThreads, 0, st, p);
+}
+
 template <int S, int VW, int FMT>
 cudaError_t launch_row(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
-    constexpr int G = kShapes[S].G, NV = kShapes[S].NV;
-    constexpr int U = VW == 1 ? 8 : row_unroll(NV);
-    constexpr int ULOW = VW == 1 ? 8 : row_unroll_low(NV);
-    constexpr int MINB = row_min_blocks(NV);
-    const unsigned grid = (unsigned)plan.grid;
-    const bool low = plan.low_occupancy && ULOW != U;
-    if (VW == 4 && plan.full)
-        return low ? launch_overlapped(spmm_row_kernel<G, NV, VW, ULOW, FMT, (VW == 4), 2>, grid, kRowThreads, 0, st, p)
-                   : launch_overlapped(spmm_row_kernel<G, NV, VW, U, FMT, (VW == 4), MINB>, grid, kRowThreads, 0, st, p);
-    return low ? launch_overlapped(spmm_row_kernel<G, NV, VW, ULOW, FMT, false, 2>, grid, kRowThreads, 0, st, p)
-               : launch_overlapped(spmm_row_kernel<G, NV, VW, U, FMT, false, MINB>, grid, kRowThreads, 0, st, p);
+    if (VW == 4 && plan.full) return launch_row_full<S, VW, FMT, (VW == 4)>(p, plan, st);
+    return launch_row_full<S, VW, FMT, false>(p, plan, st);
 }
 
 template <int NV, int FMT>
@@ -464,6 +469,7 @@ namespace csrspmm_b200 {
 cudaError_t launch_row_kernel(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st)
 {
     if (plan.VW == 4) return e2m1 ? dispatch_row<4, kValuesE2M1>(p, plan, st) : dispatch_row<4, kValuesF32>(p, plan, st);
+    if (plan.VW == 2) return e2m1 ? dispatch_row<2, kValuesE2M1>(p, plan, st) : dispatch_row<2, kValuesF32>(p, plan, st);
     return e2m1 ? dispatch_row<1, kValuesE2M1>(p, plan, st) : dispatch_row<1, kValuesF32>(p, plan, st);
 }
 

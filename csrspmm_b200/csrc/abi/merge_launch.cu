@@ -18,7 +18,7 @@ cudaError_t launch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
     constexpr int G = kShapes[S].G, NV = kShapes[S].NV, TG = kShapes[S].TG;
     constexpr int TGS = CSRSPMM_TUNE_MERGE_TG_SMALL < TG ? CSRSPMM_TUNE_MERGE_TG_SMALL : TG;
-    constexpr int U = VW == 1 ? 8 : merge_unroll(NV);
+    constexpr int U = merge_unroll(VW, NV);
     const unsigned grid = (unsigned)plan.grid;
     if (plan.small_tile) {  // few items: smaller tiles, more CTAs
         if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TGS, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
@@ -33,7 +33,7 @@ template <int K, int VW, int FMT>
 cudaError_t launch_merge_narrow(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
     constexpr int G = kNarrowShapes[K].G, NV = kNarrowShapes[K].NV, TG = kNarrowShapes[K].TG;
-    constexpr int U = VW == 1 ? 8 : merge_unroll(NV);
+    constexpr int U = merge_unroll(VW, NV);
     const unsigned grid = (unsigned)plan.grid;
     if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
     return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, grid, kMergeThreads, 0, st, p);
@@ -62,6 +62,7 @@ cudaError_t dispatch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t s
 cudaError_t launch_merge_kernel(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st)
 {
     if (plan.VW == 4) return e2m1 ? dispatch_merge<4, kValuesE2M1>(p, plan, st) : dispatch_merge<4, kValuesF32>(p, plan, st);
+    if (plan.VW == 2) return e2m1 ? dispatch_merge<2, kValuesE2M1>(p, plan, st) : dispatch_merge<2, kValuesF32>(p, plan, st);
     return e2m1 ? dispatch_merge<1, kValuesE2M1>(p, plan, st) : dispatch_merge<1, kValuesF32>(p, plan, st);
 }
 
@@ -69,7 +70,7 @@ cudaError_t launch_fixup_kernel(const SpmmParams& p, const Plan& plan, cudaStrea
 {
     const int warps = 256 / 32;
     const unsigned grid = (unsigned)((plan.num_tiles + warps - 1) / warps);
-    return launch_overlapped(plan.VW == 4 ? spmm_fixup_kernel<4> : spmm_fixup_kernel<1>, grid, 256, 0, st, p, (int)plan.num_tiles);
+    return launch_overlapped(plan.VW == 4 ? spmm_fixup_kernel<4> : plan.VW == 2 ? spmm_fixup_kernel<2> : spmm_fixup_kernel<1>, grid, 256, 0, st, p, (int)plan.num_tiles);
 }
 
 }  // namespace csrspmm_b200

@@ -90,7 +90,7 @@ extern "C" int csrspmm_b200_spmm_noalloc(const csrspmm_b200_args* args, csrspmm_
     Plan plan;
     status = make_plan(&a, &plan);  // the same tiles as csrspmm_b200_spmm, unless they leave too many carry rows
     if (status == CSRSPMM_B200_OK && plan.workspace_bytes > (size_t)CSRSPMM_B200_NOALLOC_SCRATCH_BYTES)
-        status = make_plan(&a, &plan, true, /*coarse=*/true);
+        status = make_plan(&a, &plan, kPlanCoarse);
     if (status != CSRSPMM_B200_OK) return status;
     if (plan.workspace_bytes > (size_t)CSRSPMM_B200_NOALLOC_SCRATCH_BYTES) {
         set_last_error("csrspmm_b200_spmm_noalloc: this problem (M + nnz = %lld, Nd = %d) needs %zu bytes of "

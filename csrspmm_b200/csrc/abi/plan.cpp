@@ -91,6 +91,12 @@ bool vector_layout_ok(const csrspmm_b200_args* a)
            (reinterpret_cast<uintptr_t>(a->C) & 15u) == 0;
 }
 
+static bool pair_layout_ok(const csrspmm_b200_args* a)
+{
+    return a->Nd % 2 == 0 && a->ldb % 2 == 0 && a->ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(a->B) & 7u) == 0 &&
+           (reinterpret_cast<uintptr_t>(a->C) & 7u) == 0;
+}
+
 static int shape_for(int ncolv)
 {
     if (ncolv <= 8) return 0;
@@ -143,14 +149,17 @@ static int merge_items_per_group(long long num_items, int groups, int ctas_per_s
     return (int)(tg < least ? least : (tg > most ? most : tg));
 }
 
-int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow, bool coarse)
+int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
 {
+    const bool coarse = (flags & kPlanCoarse) != 0;
     int st = check_args(a, false);
     if (st != CSRSPMM_B200_OK) return st;
     *plan = Plan();
     const bool vec = vector_layout_ok(a);
-    plan->VW = vec ? 4 : 1;
-    plan->ncolv = vec ? a->Nd / 4 : a->Nd;
+    // rows that do not start on 16 bytes but on 8 (50 columns, say) go two floats at a time
+    const bool pairs = !vec && (flags & kPlanNoPairs) == 0 && pair_layout_ok(a);
+    plan->VW = vec ? 4 : (pairs ? 2 : 1);
+    plan->ncolv = a->Nd / plan->VW;
     plan->num_items = (long long)a->M + a->nnz;
 
     int kernel = a->kernel;
@@ -168,8 +177,8 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow, bool co
         // comes from L2.  Beyond about 48 MB of B the time is the wait for HBM, and a lane group that stops at every
         // row end (bounds, columns, rows of B, store, each a round trip) asks for too little of it at once: the
         // merge kernel walks on across row ends (1 M rows of 16, 64 columns: 600 us against 812; 262 144 rows of 8:
-        // 73 against 94; of 4: 51 against 74), unless rows are long and wide enough to keep it busy by themselves
-        // (64 entries of 128 columns: 773 against 745; 32 of 256: 1012 either way).  Everything else (unknown or skewed row lengths) takes
+        // 73 against 94; of 4: 51 against 74), unless rows are long enough to keep it busy by themselves (64 entries
+        // of 128 columns: 773 against 745; 32 of 256: 1012 either way; 143 of 56: 703 against 601).  Everything else (unknown or skewed row lengths) takes
         // the merge kernel.  The entry point asked for does not change the choice.
         const double avg = a->M > 0 ? (double)a->nnz / (double)a->M : 0.0;
         const double row_limit = avg * 4.0 > 64.0 ? avg * 4.0 : 64.0;
@@ -177,7 +186,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow, bool co
         const bool rows_even = a->max_row_nnz > 0 && (double)a->max_row_nnz <= row_limit;
         if (tma_can_run(a) && a->Nd > 384 && b_bytes >= 1073741824.0 && !rows_even)
             kernel = CSRSPMM_B200_KERNEL_TMA;
-        else if (rows_even && (b_bytes < 48e6 || (avg * a->Nd >= 8192.0 && a->Nd > 64)))
+        else if (rows_even && (b_bytes < 48e6 || avg > 64.0 || (avg * a->Nd >= 8192.0 && a->Nd > 64)))
             kernel = CSRSPMM_B200_KERNEL_ROW;
         else
             kernel = CSRSPMM_B200_KERNEL_MERGE;
@@ -205,7 +214,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow, bool co
         plan->G = kShapes[plan->shape].G;
         plan->NV = kShapes[plan->shape].NV;
         plan->full = plan->VW == 4 && plan->G * plan->NV == plan->ncolv;
-        if (CSRSPMM_TUNE_MERGE_NARROW && kernel == CSRSPMM_B200_KERNEL_MERGE && allow_narrow && plan->ncolv >= 1 && plan->ncolv <= 4) {
+        if (CSRSPMM_TUNE_MERGE_NARROW && kernel == CSRSPMM_B200_KERNEL_MERGE && (flags & kPlanNoNarrow) == 0 && plan->ncolv >= 1 && plan->ncolv <= 4) {
             // one, two or four column vectors: lane groups of that many lanes (kNarrowShapes)
             plan->narrow = plan->ncolv == 1 ? 1 : (plan->ncolv == 2 ? 2 : 3);
             const ShapeDesc& ns = kNarrowShapes[plan->narrow - 1];
@@ -223,6 +232,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow, bool co
         } else {
             const int groups = CSRSPMM_TUNE_ROW_THREADS / plan->G;
             plan->grid = ((long long)a->M + groups - 1) / groups;
+            plan->short_rows = a->nnz <= (long long)CSRSPMM_TUNE_ROW_SHORT_MEAN * (long long)a->M;
             plan->low_occupancy = (long long)a->M * plan->G / 32 < 148LL * 8;
 #if CSRSPMM_TUNE_ROW_PERSISTENT > 0
             // many short rows: a CTA that lives for four 16-entry rows costs more to start than to

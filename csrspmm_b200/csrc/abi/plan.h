@@ -17,6 +17,7 @@ struct Plan {
     int kernel = CSRSPMM_B200_KERNEL_ROW;  // resolved, never AUTO
     int shape = 0;                         // index into kShapes (tuning.h)
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
+    bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
     bool small_tile = false;               // merge kernel: the build with shared memory for small tiles
     int narrow = 0;                        // merge kernel: 1 + index into kNarrowShapes when the dense operand has at
@@ -44,8 +45,10 @@ bool vector_layout_ok(const csrspmm_b200_args* a);
 
 // Resolves AUTO (and the CSRSPMM_FORCE_KERNEL override) and fills the launch geometry.
 // Returns CSRSPMM_B200_OK or an error status.
-// coarse: no tiles smaller than 64 items per lane group (fewer carry rows), for callers with a fixed scratch.
-int make_plan(const csrspmm_b200_args* a, Plan* plan, bool allow_narrow = true, bool coarse = false);
+constexpr unsigned kPlanNoNarrow = 1;  // no lane groups of fewer than eight lanes
+constexpr unsigned kPlanCoarse = 2;    // no tiles smaller than 64 items per lane group: fewer carry rows
+constexpr unsigned kPlanNoPairs = 4;   // vector widths 4 and 1 only
+int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags = 0);
 
 // Workspace of the split kernels for a given plan-independent worst case: what
 // csrspmm_b200_workspace_bytes reports (the larger of the MERGE and TMA needs).  any_row_block:

@@ -186,7 +186,7 @@ int scheduled_plan(const csrspmm_b200_args* a, Plan* plan)
     csrspmm_b200_args m = *a;
     m.kernel = CSRSPMM_B200_KERNEL_MERGE;
     m.schedule = nullptr;
-    int status = make_plan(&m, plan, /*allow_narrow=*/false);  // the SKIP build exists for the regular shapes only
+    int status = make_plan(&m, plan, kPlanNoNarrow | kPlanNoPairs);  // what the SKIP build exists for
     if (status != CSRSPMM_B200_OK) return status;
     plan->carry_row_bytes = align256((size_t)plan->num_tiles * sizeof(int32_t));
     plan->workspace_bytes = plan->carry_row_bytes + align256((size_t)plan->num_tiles * (size_t)plan->carry_ld * sizeof(float));

@@ -98,7 +98,7 @@ int csrspmm_b200_spmm_tiled(const csrspmm_b200_args* args, int32_t panel_rows, c
     csrspmm_b200_args a = *args;
     a.kernel = CSRSPMM_B200_KERNEL_ROW;
     Plan plan;
-    status = make_plan(&a, &plan);
+    status = make_plan(&a, &plan, kPlanNoPairs);
     if (status != CSRSPMM_B200_OK) return status;
 
     const size_t need = passes > 1 ? csrspmm_b200_tiled_workspace_bytes(args) : 0;

@@ -133,7 +133,7 @@ __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_g
 template <int N>
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// ---- column vectors (VW = 4: float4, 16-byte aligned; VW = 1: one float) --------------------------
+// ---- column vectors (VW = 4: float4, 16-byte aligned; VW = 2: float2, 8-byte aligned; VW = 1: one float) --------------------------
 
 template <int VW>
 struct Vec;
@@ -214,6 +214,74 @@ struct Vec<4> {
         r.v.y = __fadd_rn(old.v.y, __fmul_rn(alpha, v.y));
         r.v.z = __fadd_rn(old.v.z, __fmul_rn(alpha, v.z));
         r.v.w = __fadd_rn(old.v.w, __fmul_rn(alpha, v.w));
+        return r;
+    }
+};
+
+template <>
+struct Vec<2> {
+    float2 v;
+    __device__ __forceinline__ void zero() { v = make_float2(0.f, 0.f); }
+    __device__ __forceinline__ void load_nc(const float* p) { v = __ldg(reinterpret_cast<const float2*>(p)); }
+    __device__ __forceinline__ void load_b(const float* p, unsigned long long pol)
+    {
+#if CSRSPMM_TUNE_B_EVICT_LAST_PCT > 0
+        asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+            : "=f"(v.x), "=f"(v.y)
+            : "l"(p), "l"(pol));
+#else
+        (void)pol;
+        load_nc(p);
+#endif
+    }
+    // read-only load carrying an L2 eviction policy made by createpolicy
+    __device__ __forceinline__ void load_hint(const float* p, unsigned long long pol)
+    {
+        asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+            : "=f"(v.x), "=f"(v.y)
+            : "l"(p), "l"(pol));
+    }
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float2*>(p); }
+    __device__ __forceinline__ void store(float* p) const { *reinterpret_cast<float2*>(p) = v; }
+    __device__ __forceinline__ void store_streaming(float* p) const { __stcs(reinterpret_cast<float2*>(p), v); }
+    __device__ __forceinline__ Vec shuffle(int src_lane) const  // this value as held by src_lane of the warp
+    {
+        Vec r;
+        r.v.x = __shfl_sync(0xffffffffu, v.x, src_lane);
+        r.v.y = __shfl_sync(0xffffffffu, v.y, src_lane);
+        return r;
+    }
+    __device__ __forceinline__ void fma(float a, const Vec& b)
+    {
+        v.x = __fmaf_rn(a, b.v.x, v.x);
+        v.y = __fmaf_rn(a, b.v.y, v.y);
+    }
+    __device__ __forceinline__ void add(const Vec& b)
+    {
+        v.x = __fadd_rn(v.x, b.v.x);
+        v.y = __fadd_rn(v.y, b.v.y);
+    }
+    // alpha*this + beta*old, nothing fused
+    __device__ __forceinline__ Vec epilogue(float alpha, float beta, const Vec& old) const
+    {
+        Vec r;
+        r.v.x = __fadd_rn(__fmul_rn(alpha, v.x), __fmul_rn(beta, old.v.x));
+        r.v.y = __fadd_rn(__fmul_rn(alpha, v.y), __fmul_rn(beta, old.v.y));
+        return r;
+    }
+    __device__ __forceinline__ Vec epilogue0(float alpha) const
+    {
+        Vec r;
+        r.v.x = __fadd_rn(__fmul_rn(alpha, v.x), 0.0f);
+        r.v.y = __fadd_rn(__fmul_rn(alpha, v.y), 0.0f);
+        return r;
+    }
+    // old + alpha*this (fix-up of a finished row)
+    __device__ __forceinline__ Vec add_scaled_to(float alpha, const Vec& old) const
+    {
+        Vec r;
+        r.v.x = __fadd_rn(old.v.x, __fmul_rn(alpha, v.x));
+        r.v.y = __fadd_rn(old.v.y, __fmul_rn(alpha, v.y));
         return r;
     }
 };

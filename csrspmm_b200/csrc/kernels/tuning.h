@@ -13,7 +13,7 @@
 #ifndef CSRSPMM_TUNE_MERGE_U_NV4
 #define CSRSPMM_TUNE_MERGE_U_NV4 3
 #endif
-// ... and row kernel
+// ... and row kernel (row_unroll below)
 #ifndef CSRSPMM_TUNE_ROW_U_NV1
 #define CSRSPMM_TUNE_ROW_U_NV1 4
 #endif
@@ -21,7 +21,14 @@
 #define CSRSPMM_TUNE_ROW_U_NV2 2
 #endif
 #ifndef CSRSPMM_TUNE_ROW_U_NV4
-#define CSRSPMM_TUNE_ROW_U_NV4 4
+#define CSRSPMM_TUNE_ROW_U_NV4 3
+#endif
+#ifndef CSRSPMM_TUNE_ROW_U_SHORT
+#define CSRSPMM_TUNE_ROW_U_SHORT 6
+#endif
+// mean row length up to which rows count as short
+#ifndef CSRSPMM_TUNE_ROW_SHORT_MEAN
+#define CSRSPMM_TUNE_ROW_SHORT_MEAN 48
 #endif
 
 // scheduled pieces (sliced_kernel.cuh): consecutive pieces per lane group
@@ -277,6 +284,29 @@ constexpr ShapeDesc kShapes[kNumShapes] = {
 constexpr int merge_unroll(int nv) { return nv == 1 ? CSRSPMM_TUNE_MERGE_U_NV1 : (nv == 2 ? CSRSPMM_TUNE_MERGE_U_NV2 : CSRSPMM_TUNE_MERGE_U_NV4); }
 constexpr int row_unroll(int nv) { return nv == 1 ? CSRSPMM_TUNE_ROW_U_NV1 : (nv == 2 ? CSRSPMM_TUNE_ROW_U_NV2 : CSRSPMM_TUNE_ROW_U_NV4); }
 constexpr int row_unroll_low(int nv) { return nv == 1 ? CSRSPMM_TUNE_ROW_ULOW_NV1 : (nv == 2 ? CSRSPMM_TUNE_ROW_ULOW_NV2 : CSRSPMM_TUNE_ROW_ULOW_NV4); }
+// vector width 2 (rows on 8-byte boundaries): as many loads in flight as the same registers hold; width 1: eight
+#ifndef CSRSPMM_TUNE_PAIR_U_NV1
+#define CSRSPMM_TUNE_PAIR_U_NV1 6
+#endif
+#ifndef CSRSPMM_TUNE_PAIR_U_WIDE
+#define CSRSPMM_TUNE_PAIR_U_WIDE 4
+#endif
+constexpr int merge_unroll(int vw, int nv)
+{
+    return vw == 4 ? merge_unroll(nv) : vw == 1 ? 8 : nv == 1 ? CSRSPMM_TUNE_PAIR_U_NV1 : CSRSPMM_TUNE_PAIR_U_WIDE;
+}
+// Row kernel: six loads in flight for short rows of one vector per lane where the registers last (64 columns, rows of 16:
+// 65 536 of them 30.6 -> 24.4 us, 16 384 10.3 -> 8.6; 32 columns, rows of 8 15.2 -> 12.5), four where they do not (a column
+// guard; 128 columns: 12.0 us with four, 12.6 with six) and for long rows, whose chunks of G entries are then whole batches
+// (30 columns, rows of 100: 25.9 us with four, 31.6 with six).  Three with four vectors per lane (8192 rows, 4096
+// columns: 239 us with four, 212 with three, 234 with two).
+constexpr int row_unroll(int vw, int g, int nv, bool full, bool short_rows)
+{
+    if (vw == 1) return 8;
+    if (nv > 1) return vw == 4 ? row_unroll(nv) : CSRSPMM_TUNE_PAIR_U_WIDE;
+    return short_rows && (vw == 2 || (full && g <= 16)) ? CSRSPMM_TUNE_ROW_U_SHORT : CSRSPMM_TUNE_ROW_U_NV1;
+}
+
 constexpr int row_min_blocks(int nv) { return nv == 1 ? CSRSPMM_TUNE_ROW_MINB_NV1 : (nv == 2 ? CSRSPMM_TUNE_ROW_MINB_NV2 : CSRSPMM_TUNE_ROW_MINB_NV4); }
 constexpr int merge_min_blocks(int nv) { return nv == 1 ? CSRSPMM_TUNE_MERGE_MINB_NV1 : (nv == 2 ? CSRSPMM_TUNE_MERGE_MINB_NV2 : CSRSPMM_TUNE_MERGE_MINB_NV4); }
 
