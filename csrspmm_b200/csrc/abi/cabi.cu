@@ -15,6 +15,7 @@
 
 #include "../kernels/aux_kernels.cuh"
 #include "../kernels/merge_kernel.cuh"
+#include "../kernels/resident_kernel.cuh"
 #include "../kernels/row_kernel.cuh"
 #include "../kernels/tma_kernel.cuh"
 #include "csrspmm_b200.h"
@@ -123,6 +124,25 @@ cudaError_t launch_tma(const SpmmParams& p, const Plan& plan, cudaStream_t st)
     }
     return launch_overlapped(kern, (unsigned)plan.grid, kMergeThreads, plan.dynamic_smem, st, p, (unsigned)plan.tma_slot_bytes,
                              (unsigned)(plan.dynamic_smem / (CSRSPMM_TUNE_MERGE_THREADS / 32)));
+}
+
+// One CTA per SM; the opt-in to its shared memory is made once per device and build, as for the bulk-copy kernel.
+template <int G, int FMT>
+cudaError_t launch_resident(const SpmmParams& p, cudaStream_t st)
+{
+    auto kern = spmm_resident_kernel<G, FMT>;
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_smem_bytes<G>(kResidentPanelBytes / (G * 16)));
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    const long long total = (long long)((p.ncolv + G - 1) / G) * p.M;
+    const unsigned grid = (unsigned)(total < 148 ? total : 148);
+    return launch_overlapped(kern, grid, kResidentThreads, (size_t)resident_smem_bytes<G>(p.Kd), st, p, total);
 }
 
 template <int VW, int FMT>
@@ -468,6 +488,8 @@ namespace csrspmm_b200 {
 
 cudaError_t launch_row_kernel(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st)
 {
+    if (plan.resident == 32) return e2m1 ? launch_resident<32, kValuesE2M1>(p, st) : launch_resident<32, kValuesF32>(p, st);
+    if (plan.resident == 16) return e2m1 ? launch_resident<16, kValuesE2M1>(p, st) : launch_resident<16, kValuesF32>(p, st);
     if (plan.VW == 4) return e2m1 ? dispatch_row<4, kValuesE2M1>(p, plan, st) : dispatch_row<4, kValuesF32>(p, plan, st);
     if (plan.VW == 2) return e2m1 ? dispatch_row<2, kValuesE2M1>(p, plan, st) : dispatch_row<2, kValuesF32>(p, plan, st);
     return e2m1 ? dispatch_row<1, kValuesE2M1>(p, plan, st) : dispatch_row<1, kValuesF32>(p, plan, st);

@@ -149,6 +149,21 @@ static int merge_items_per_group(long long num_items, int groups, int ctas_per_s
     return (int)(tg < least ? least : (tg > most ? most : tg));
 }
 
+// Lanes per group of the resident kernel for this product, 0 when the row kernel is the better one.  A panel of B has to
+// fit shared memory (4 floats per lane and row of B) and to be used often enough to pay for being loaded; rows have to
+// be long enough to hide the next row's bounds and entries (4096 x 128 times 4096 columns, rows of 1.3: 23.8 us against
+// 21.1; of 6.4: 32.1 against 38.8).  Widths that the row kernel covers exactly in one pass it does well itself, helped by L1
+// (6000 x 800 times 512 columns, rows of 100: 52 us against 66; 60 000 x 400 times 128, rows of 20: 35 against 30).
+static int resident_lanes(const csrspmm_b200_args* a, const Plan& plan)
+{
+    if (plan.VW != 4 || a->Kd <= 0 || a->max_row_nnz <= 0 || a->nnz < 4LL * a->M) return 0;
+    const int lanes = a->Kd * 512LL <= 200 * 1024 && plan.ncolv > 16 ? 32 : (a->Kd * 256LL <= 200 * 1024 ? 16 : 0);
+    if (lanes == 0 || plan.ncolv < lanes || (plan.full && lanes == 16)) return 0;
+    const long long panels = (plan.ncolv + lanes - 1) / lanes;
+    const long long reuse = plan.full ? 16 : CSRSPMM_TUNE_RESIDENT_REUSE;  // entries per CTA and row of B
+    return a->nnz * panels >= reuse * 148LL * a->Kd ? lanes : 0;
+}
+
 int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
 {
     const bool coarse = (flags & kPlanCoarse) != 0;
@@ -232,6 +247,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         } else {
             const int groups = CSRSPMM_TUNE_ROW_THREADS / plan->G;
             plan->grid = ((long long)a->M + groups - 1) / groups;
+            plan->resident = (flags & kPlanNoPairs) == 0 ? resident_lanes(a, *plan) : 0;
             plan->short_rows = a->nnz <= (long long)CSRSPMM_TUNE_ROW_SHORT_MEAN * (long long)a->M;
             plan->low_occupancy = (long long)a->M * plan->G / 32 < 148LL * 8;
 #if CSRSPMM_TUNE_ROW_PERSISTENT > 0

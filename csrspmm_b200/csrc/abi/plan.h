@@ -17,6 +17,7 @@ struct Plan {
     int kernel = CSRSPMM_B200_KERNEL_ROW;  // resolved, never AUTO
     int shape = 0;                         // index into kShapes (tuning.h)
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
+    int resident = 0;                      // whole-row mapping by the resident kernel: lanes per group (16, 32), else 0
     bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
     bool small_tile = false;               // merge kernel: the build with shared memory for small tiles

@@ -26,6 +26,10 @@
 #ifndef CSRSPMM_TUNE_ROW_U_SHORT
 #define CSRSPMM_TUNE_ROW_U_SHORT 6
 #endif
+// resident kernel: entries per CTA and row of B from which it is taken
+#ifndef CSRSPMM_TUNE_RESIDENT_REUSE
+#define CSRSPMM_TUNE_RESIDENT_REUSE 2
+#endif
 // mean row length up to which rows count as short
 #ifndef CSRSPMM_TUNE_ROW_SHORT_MEAN
 #define CSRSPMM_TUNE_ROW_SHORT_MEAN 48

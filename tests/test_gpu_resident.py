@@ -1,0 +1,32 @@
+"""The resident kernel (a panel of B in shared memory) at the edges of its range, bit for bit against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from csrspmm_b200 import generators as G, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,Kd,Nd,mean", [(3, 1, 128, 1), (700, 64, 132, 6), (150, 97, 1024, 33), (1000, 400, 388, 40), (900, 401, 200, 40),
+                                          (517, 800, 68, 90), (200, 256, 4096, 64), (40, 30, 2496, 29)])
+@pytest.mark.parametrize("beta,packed", [(0.0, False), (0.5, False), (0.0, True)])
+def test_resident_panels(cuda_lib, M, Kd, Nd, mean, beta, packed):
+    rng = np.random.default_rng(M + Kd)
+    lens = np.minimum(rng.poisson(mean, M), Kd)
+    lens[:: max(M // 7, 1)] = 0  # empty rows among them, the first one too
+    lens[M // 2] = min(Kd, 4 * mean)
+    p = G.random_csr(M, Kd, Nd, 0.0, seed=5, lengths=lens)
+    t = [torch.from_numpy(x).cuda() for x in (p.row_ptr, p.col_idx, p.values, p.B)]
+    C0 = rng.standard_normal((M, Nd), dtype=np.float32)
+    C = torch.from_numpy(C0).cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    kw = dict(max_row_nnz=max(int(lens.max()), 1), kernel="row", status_word=status, sync=True)
+    values = p.values
+    if packed:
+        t[2], scale = ops.e2m1_quantize(t[2])
+        values = oracle.e2m1_decode(t[2].cpu().numpy(), p.nnz, scale)
+        kw.update(e2m1_scale=scale, nnz=p.nnz)
+    got = ops.spmm(*t, C, 1.25, beta, **kw)
+    assert np.array_equal(got.cpu().numpy(), oracle.spmm(p.row_ptr, p.col_idx, values, p.B, C0, 1.25, beta)) and int(status) == 0
