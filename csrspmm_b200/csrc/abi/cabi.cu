@@ -40,6 +40,7 @@ void fill_params(const csrspmm_b200_args* a, const Plan& plan, SpmmParams* out)
     p.num_items = plan.num_items;
     p.release_early = plan.fills_chip;
     p.tg = plan.tg;
+    p.row_aligned = plan.row_aligned;
     p.row_ptr = a->row_ptr;
     p.rp_base = a->row_ptr_base;
     p.col_idx = a->col_idx;
@@ -227,7 +228,7 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
     } else {
         err = e2m1 ? dispatch_tma<kValuesE2M1>(p, plan, st) : dispatch_tma<kValuesF32>(p, plan, st);
     }
-    if (err == cudaSuccess && split) err = launch_fixup_kernel(p, plan, st);
+    if (err == cudaSuccess && split && !plan.row_aligned) err = launch_fixup_kernel(p, plan, st);
     if (ws_owned) {
         cudaError_t ferr = cudaFreeAsync(ws, st);
         if (err == cudaSuccess) err = ferr;

@@ -109,7 +109,7 @@ extern "C" int csrspmm_b200_spmm_noalloc(const csrspmm_b200_args* args, csrspmm_
 
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t err = launch_merge_kernel(p, plan, a.value_format == CSRSPMM_B200_VALUES_E2M1, st);
-    if (err == cudaSuccess) err = launch_fixup_kernel(p, plan, st);
+    if (err == cudaSuccess && !plan.row_aligned) err = launch_fixup_kernel(p, plan, st);
     if (err != cudaSuccess) {
         set_last_error("csrspmm_b200_spmm_noalloc: kernel launch failed: %s", cudaGetErrorString(err));
         return CSRSPMM_B200_ERR_CUDA;

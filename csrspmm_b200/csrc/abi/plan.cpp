@@ -149,6 +149,13 @@ static int merge_items_per_group(long long num_items, int groups, int ctas_per_s
     return (int)(tg < least ? least : (tg > most ? most : tg));
 }
 
+// Whether the merge kernel can cut its tiles at row starts: a tile and the longest row behind it have to fit the
+// shared memory of the largest tile, and the grid to be short enough for the fix-up kernel to be worth saving.
+static bool rows_fit_tiles(const csrspmm_b200_args* a, const Plan& plan, int groups, int most)
+{
+    return a->max_row_nnz > 0 && plan.tg < most && (long long)plan.tile + a->max_row_nnz + 1 <= (long long)groups * most;
+}
+
 // Lanes per group of the resident kernel for this product, 0 when the row kernel is the better one.  A panel of B has to
 // fit shared memory (4 floats per lane and row of B) and to be used often enough to pay for being loaded; rows have to
 // be long enough to hide the next row's bounds and entries (4096 x 128 times 4096 columns, rows of 1.3: 23.8 us against
@@ -238,12 +245,15 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
             plan->full = plan->VW == 4 && plan->G * plan->NV == plan->ncolv;
             const int groups = CSRSPMM_TUNE_MERGE_THREADS / ns.G;
             fill_split_geometry(a, plan, groups, merge_items_per_group(plan->num_items, groups, merge_min_blocks(1), ns.TG, coarse ? ns.TG : ns.G));
+            plan->row_aligned = rows_fit_tiles(a, *plan, groups, ns.TG);
         } else if (kernel == CSRSPMM_B200_KERNEL_MERGE) {
             const int groups = CSRSPMM_TUNE_MERGE_THREADS / plan->G, most = kShapes[plan->shape].TG;
             const int least = coarse ? CSRSPMM_TUNE_MERGE_TG_SMALL : CSRSPMM_TUNE_MERGE_TG_LEAST;
             const int tg = merge_items_per_group(plan->num_items, groups, merge_min_blocks(plan->NV), most, least);
             plan->small_tile = tg <= CSRSPMM_TUNE_MERGE_TG_SMALL;
             fill_split_geometry(a, plan, groups, tg);
+            plan->row_aligned = rows_fit_tiles(a, *plan, groups, most);
+            if (plan->row_aligned && plan->small_tile) plan->small_tile = plan->tile + a->max_row_nnz + 1 <= groups * CSRSPMM_TUNE_MERGE_TG_SMALL;
         } else {
             const int groups = CSRSPMM_TUNE_ROW_THREADS / plan->G;
             plan->grid = ((long long)a->M + groups - 1) / groups;

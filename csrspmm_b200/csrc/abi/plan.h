@@ -20,6 +20,7 @@ struct Plan {
     int resident = 0;                      // whole-row mapping by the resident kernel: lanes per group (16, 32), else 0
     bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
+    bool row_aligned = false;              // merge kernel: tiles cut at row starts, no carries and no fix-up
     bool small_tile = false;               // merge kernel: the build with shared memory for small tiles
     int narrow = 0;                        // merge kernel: 1 + index into kNarrowShapes when the dense operand has at
                                            // most four column vectors (lane groups of 1, 2 or 4 lanes), else 0

@@ -188,6 +188,7 @@ int scheduled_plan(const csrspmm_b200_args* a, Plan* plan)
     m.schedule = nullptr;
     int status = make_plan(&m, plan, kPlanNoNarrow | kPlanNoPairs);  // what the SKIP build exists for
     if (status != CSRSPMM_B200_OK) return status;
+    plan->row_aligned = false;  // tiles step over the scheduled rows, whose length is what row_aligned is about
     plan->carry_row_bytes = align256((size_t)plan->num_tiles * sizeof(int32_t));
     plan->workspace_bytes = plan->carry_row_bytes + align256((size_t)plan->num_tiles * (size_t)plan->carry_ld * sizeof(float));
     return CSRSPMM_B200_OK;

@@ -45,6 +45,7 @@ struct SpmmParams {
     float alpha;
     float beta;
     int tg;              // split kernels: merge-path items per lane group (Plan::tg)
+    int row_aligned;     // merge kernel: tiles are cut at row starts and leave no carries (Plan::row_aligned)
     int* carry_row;      // one per tile: row the tile leaves unfinished, or -1
     float* carry_val;    // one row of carry_ld floats per tile
     long long carry_ld;  // multiple of 4

@@ -5,7 +5,7 @@
 
 // B-row loads kept in flight per lane, by number of column vectors per lane (NV) -- merge kernel
 #ifndef CSRSPMM_TUNE_MERGE_U_NV1
-#define CSRSPMM_TUNE_MERGE_U_NV1 6
+#define CSRSPMM_TUNE_MERGE_U_NV1 5
 #endif
 #ifndef CSRSPMM_TUNE_MERGE_U_NV2
 #define CSRSPMM_TUNE_MERGE_U_NV2 4
