@@ -8,6 +8,7 @@
 #include "../kernels/codec_kernels.cuh"
 #include "../kernels/convert_kernels.cuh"
 #include "csrspmm_b200.h"
+#include "pdl.h"
 #include "plan.h"
 #include "scan.h"
 #include "scratch.h"
@@ -70,9 +71,8 @@ int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64
     CUDA_TRY(results.init());
     const int wpr = convert_warps_per_row(W);
     const unsigned grid = convert_grid(H, wpr);
-    if (rows_on_16_bytes(dense, ld)) dense_count_kernel<true><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, counts);
-    else dense_count_kernel<false><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, counts);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_overlapped(rows_on_16_bytes(dense, ld) ? dense_count_kernel<true> : dense_count_kernel<false>, grid, kConvertThreads, 0, st,
+                               H, W, dense, ld, tol, wpr, counts));
     CUDA_TRY(exclusive_scan(counts, H, row_ptr, scratch.as<void>(), results.ptr(), st));
     long long out[2] = {0, 0};
     CUDA_TRY(results.wait(out, 2));
@@ -100,11 +100,8 @@ int csrspmm_b200_dense2csr_fill(int32_t H, int32_t W, const float* dense, int64_
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int wpr = convert_warps_per_row(W);
     const unsigned grid = convert_grid(H, wpr);
-    if (rows_on_16_bytes(dense, ld))
-        dense_fill_kernel<true><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, row_ptr, col_idx, values);
-    else
-        dense_fill_kernel<false><<<grid, kConvertThreads, 0, st>>>(H, W, dense, ld, tol, wpr, row_ptr, col_idx, values);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_overlapped(rows_on_16_bytes(dense, ld) ? dense_fill_kernel<true> : dense_fill_kernel<false>, grid, kConvertThreads, 0, st,
+                               H, W, dense, ld, tol, wpr, row_ptr, col_idx, values));
     return CSRSPMM_B200_OK;
 }
 
@@ -137,8 +134,7 @@ int csrspmm_b200_e2m1_scale_device(int64_t n, const float* values, float* scale_
     Scratch partial(st);
     CUDA_TRY(partial.alloc(sizeof(float) * kCodecMaxCtas));
     const unsigned grid = codec_grid(n);
-    e2m1_absmax_kernel<<<grid, kCodecThreads, 0, st>>>(n, values, partial.as<float>());
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_overlapped(e2m1_absmax_kernel, grid, kCodecThreads, 0, st, n, values, partial.as<float>()));
     float h[kCodecMaxCtas];
     CUDA_TRY(cudaMemcpyAsync(h, partial.as<float>(), sizeof(float) * grid, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -156,8 +152,8 @@ int csrspmm_b200_e2m1_encode_device(int64_t n, const float* values, float scale,
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
     if (n == 0) return CSRSPMM_B200_OK;
-    e2m1_encode_kernel<<<codec_grid(n), kCodecThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, values, scale, nullptr, 0, packed, nullptr);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_overlapped(e2m1_encode_kernel, codec_grid(n), kCodecThreads, 0, reinterpret_cast<cudaStream_t>(stream), n, values, scale,
+                               nullptr, 0, packed, nullptr));
     return CSRSPMM_B200_OK;
 }
 
@@ -176,9 +172,9 @@ int csrspmm_b200_e2m1_quantize_device(int64_t n, const float* values, float* sca
     Results results(st);
     CUDA_TRY(results.init());
     const unsigned grid = codec_grid(n);
-    e2m1_absmax_kernel<<<grid, kCodecThreads, 0, st>>>(n, values, partial.as<float>());
-    e2m1_encode_kernel<<<grid, kCodecThreads, 0, st>>>(n, values, 1.0f, partial.as<float>(), (int)grid, packed, results.ptr());
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_overlapped(e2m1_absmax_kernel, grid, kCodecThreads, 0, st, n, values, partial.as<float>()));
+    CUDA_TRY(launch_overlapped(e2m1_encode_kernel, grid, kCodecThreads, 0, st, n, values, 1.0f, partial.as<float>(), (int)grid, packed,
+                               results.ptr()));
     long long bits = 0;
     CUDA_TRY(results.wait(&bits, 1));
     const unsigned word = (unsigned)bits;

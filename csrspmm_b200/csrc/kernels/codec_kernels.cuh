@@ -45,6 +45,8 @@ __device__ __forceinline__ float codec_block_max(float mx)
 __global__ void __launch_bounds__(kCodecThreads) e2m1_absmax_kernel(long long n, const float* __restrict__ values,
                                                                     float* __restrict__ cta_max)
 {
+    wait_for_previous_grid();
+    release_next_grid();
     float mx = 0.0f;
     const long long stride = (long long)gridDim.x * (kCodecThreads * kCodecPer);
     for (long long i = ((long long)blockIdx.x * kCodecThreads + threadIdx.x) * kCodecPer; i < n; i += stride) {
@@ -85,6 +87,8 @@ __global__ void __launch_bounds__(kCodecThreads) e2m1_encode_kernel(long long n,
                                                                     const float* __restrict__ cta_max, int num_max,
                                                                     unsigned char* __restrict__ packed, long long* scale_bits)
 {
+    wait_for_previous_grid();
+    release_next_grid();
     if (cta_max != nullptr) {
         float mx = 0.0f;
         for (int k = threadIdx.x; k < num_max; k += kCodecThreads) mx = fmaxf(mx, cta_max[k]);

@@ -15,6 +15,8 @@
 
 #include <cuda_runtime.h>
 
+#include "common.cuh"
+
 namespace csrspmm_b200 {
 
 constexpr int kConvertThreads = 256;
@@ -65,6 +67,8 @@ template <bool VEC>
 __global__ void __launch_bounds__(kConvertThreads) dense_count_kernel(int H, int W, const float* __restrict__ dense,
                                                                       long long ld, float tol, int wpr, int* __restrict__ counts)
 {
+    wait_for_previous_grid();
+    release_next_grid();
     __shared__ int s_count[kConvertThreads / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rows_per_cta = (kConvertThreads / 32) / wpr;
@@ -100,6 +104,8 @@ __global__ void __launch_bounds__(kConvertThreads) dense_fill_kernel(int H, int 
                                                                      float tol, int wpr, const int* __restrict__ row_ptr,
                                                                      int* __restrict__ col_idx, float* __restrict__ values)
 {
+    wait_for_previous_grid();
+    release_next_grid();
     __shared__ int s_count[2][kConvertThreads / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rows_per_cta = (kConvertThreads / 32) / wpr;

@@ -95,8 +95,8 @@ class CsrMatrix:
     def schedule(self, Nd: int):
         """The per-matrix schedule for a B of ``Nd`` columns, built on first use (a few milliseconds) and kept;
         None when the library finds nothing worth scheduling for this matrix and width."""
-        Nd = int(Nd)
         if Nd not in self._schedules:
+            Nd = int(Nd)
             sched = None
             if self.row_ptr.is_cuda and self.nnz > 0:
                 sched = ops.Schedule(self.row_ptr, self.col_idx, self.shape[1], Nd)
@@ -120,26 +120,17 @@ class CsrMatrix:
     def matmul(self, B: torch.Tensor, alpha: float = 1.0, *, out: torch.Tensor | None = None, beta: float = 0.0,
                kernel: str = "auto") -> torch.Tensor:
         """alpha * A @ B (+ beta * out).  Differentiable in B when ``out`` is None."""
+        sched = self.schedule(B.shape[1]) if kernel == "auto" else None
         if out is None and B.requires_grad:
-            return _CsrMatmul.apply(self, B, float(alpha), kernel)
+            return _lib.binding().matmul(self, self.row_ptr, self.col_idx, self.values, B, alpha, _lib.KERNEL_IDS[kernel],
+                                         self.max_row_nnz, sched.handle if sched is not None else 0)
         return ops.spmm(self.row_ptr, self.col_idx, self.values, B, out, alpha, beta, kernel=kernel,
-                        max_row_nnz=self.max_row_nnz, schedule=self.schedule(B.shape[1]) if kernel == "auto" else None)
+                        max_row_nnz=self.max_row_nnz, schedule=sched)
+
+    def _transpose_parts(self, Nd: int, kernel: int):
+        """What the backward product of ``matmul`` needs (called from the binding)."""
+        At = self.t()
+        sched = At.schedule(Nd) if kernel == _lib.KERNEL_AUTO else None
+        return At.row_ptr, At.col_idx, At.values, At.max_row_nnz, sched.handle if sched is not None else 0
 
     __matmul__ = matmul
-
-
-class _CsrMatmul(torch.autograd.Function):
-    """A @ B with the cached transpose for the backward product."""
-
-    @staticmethod
-    def forward(ctx, A: CsrMatrix, B: torch.Tensor, alpha: float, kernel: str):
-        ctx.A, ctx.alpha, ctx.kernel = A, alpha, kernel
-        return ops.spmm(A.row_ptr, A.col_idx, A.values, B.contiguous(), None, alpha, 0.0, kernel=kernel,
-                        max_row_nnz=A.max_row_nnz, schedule=A.schedule(B.shape[1]) if kernel == "auto" else None)
-
-    @staticmethod
-    def backward(ctx, grad_C):
-        At = ctx.A.t()
-        dB = ops.spmm(At.row_ptr, At.col_idx, At.values, grad_C.contiguous(), None, ctx.alpha, 0.0, kernel=ctx.kernel,
-                      max_row_nnz=At.max_row_nnz, schedule=At.schedule(grad_C.shape[1]) if ctx.kernel == "auto" else None)
-        return None, dB, None, None
