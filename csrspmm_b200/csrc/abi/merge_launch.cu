@@ -19,7 +19,14 @@ cudaError_t launch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t st)
     constexpr int G = kShapes[S].G, NV = kShapes[S].NV, TG = kShapes[S].TG;
     constexpr int TGS = CSRSPMM_TUNE_MERGE_TG_SMALL < TG ? CSRSPMM_TUNE_MERGE_TG_SMALL : TG;
     constexpr int U = merge_unroll(VW, NV);
+    // one more row in flight where the grid is many waves long, hence waiting for HBM (262 144 rows of 16, 128 columns:
+    // 218.5 us with six, 222 with five; shorter grids the other way round: 47.5 and 45.2)
+    constexpr int ULONG = VW == 4 && NV == 1 && G >= 16 ? CSRSPMM_TUNE_MERGE_U_LONG : U;
     const unsigned grid = (unsigned)plan.grid;
+    if (ULONG != U && plan.tg == TG) {
+        if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, ULONG, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
+        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, ULONG, FMT, false>, grid, kMergeThreads, 0, st, p);
+    }
     if (plan.small_tile) {  // few items: smaller tiles, more CTAs
         if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TGS, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
         return launch_overlapped(spmm_merge_kernel<G, NV, VW, TGS, U, FMT, false>, grid, kMergeThreads, 0, st, p);

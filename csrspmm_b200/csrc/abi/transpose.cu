@@ -1,6 +1,8 @@
 // extern "C" transposition of a device-resident CSR matrix (declared in include/csrspmm_b200.h).
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../kernels/transpose_kernels.cuh"
 #include "csrspmm_b200.h"
 #include "pdl.h"
@@ -77,20 +79,25 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
         const int2* in = first ? nullptr : pairs(p.pairs[(k - 1) & 1]);
         int* out_keys = last ? ints(p.keys) : ints(p.buffer[k & 1]);
         int2* out = last ? nullptr : pairs(p.pairs[k & 1]);
-        cudaError_t e = launch_overlapped(transpose_count_kernel<ITEMS>, (unsigned)p.tiles, kTransposeThreads, 0, st, ps, keys, Kd, ints(p.counts));
-        if (e == cudaSuccess) e = exclusive_scan(ints(p.counts), p.counters, ints(p.offsets), ws + p.scan, results, st);
+        const bool self = p.tiles <= kSelfTiles;
+        cudaError_t e = launch_overlapped(self ? transpose_count_kernel<ITEMS, true> : transpose_count_kernel<ITEMS, false>, (unsigned)p.tiles,
+                                          kTransposeThreads, 0, st, ps, keys, Kd, ints(p.counts));
+        if (e == cudaSuccess && !self) e = exclusive_scan(ints(p.counts), p.counters, ints(p.offsets), ws + p.scan, results, st);
         if (e != cudaSuccess) return e;
         auto scatter = [&](auto kernel) {
             // (racing first calls repeat the same setting)
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
             return launch_overlapped(kernel, (unsigned)p.tiles, kTransposeThreads, (size_t)smem, st, ps, keys, in, row_ptr, M, Kd, values,
-                                     ints(p.offsets), out_keys, out, t_col_idx, t_values);
+                                     ints(self ? p.counts : p.offsets), out_keys, out, t_col_idx, t_values);
         };
-        e = first && last ? scatter(transpose_scatter_kernel<ITEMS, true, true>)
-            : first       ? scatter(transpose_scatter_kernel<ITEMS, true, false>)
-            : last        ? scatter(transpose_scatter_kernel<ITEMS, false, true>)
-                          : scatter(transpose_scatter_kernel<ITEMS, false, false>);
+        auto pick = [&](auto first_c, auto last_c) {
+            constexpr bool F = decltype(first_c)::value, L = decltype(last_c)::value;
+            return self ? scatter(transpose_scatter_kernel<ITEMS, F, L, true>) : scatter(transpose_scatter_kernel<ITEMS, F, L, false>);
+        };
+        using T = std::true_type;
+        using F = std::false_type;
+        e = first && last ? pick(T(), T()) : first ? pick(T(), F()) : last ? pick(F(), T()) : pick(F(), F());
         if (e != cudaSuccess) return e;
     }
     if (nnz >= Kd)

@@ -7,6 +7,9 @@
 #ifndef CSRSPMM_TUNE_MERGE_U_NV1
 #define CSRSPMM_TUNE_MERGE_U_NV1 5
 #endif
+#ifndef CSRSPMM_TUNE_MERGE_U_LONG
+#define CSRSPMM_TUNE_MERGE_U_LONG 6
+#endif
 #ifndef CSRSPMM_TUNE_MERGE_U_NV2
 #define CSRSPMM_TUNE_MERGE_U_NV2 4
 #endif

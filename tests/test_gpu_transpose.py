@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,Kd,nnz,hub", [(1, 1, 1, False), (5, 1, 1023, False), (300, 2, 1024, False), (300, 1024, 1025, False),
-                                          (70, 1025, 5000, True), (4000, 70001, 30000, False), (17, (1 << 20) + 1, 2000, False),
+                                          (70, 1025, 5000, True), (4000, 70001, 30000, False), (900, 3000, 131072, False), (900, 3000, 131073, True), (17, (1 << 20) + 1, 2000, False),
                                           (50000, 2048, 1300000, True), (60000, (1 << 22) + 3, 1250000, False)])
 def test_transpose(cuda_lib, M, Kd, nnz, hub):
     rng = np.random.default_rng(nnz)
