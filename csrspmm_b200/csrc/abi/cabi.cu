@@ -213,7 +213,7 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
             }
             ws = a->workspace;
         } else {
-            CUDA_TRY(cudaMallocAsync(&ws, plan.workspace_bytes, st));
+            CUDA_TRY(product_scratch_alloc(&ws, plan.workspace_bytes, st));
             ws_owned = true;
         }
         set_carry_scratch(plan, ws, &p);

@@ -23,6 +23,7 @@
 #include "csrspmm_b200.h"
 #include "launch.h"
 #include "plan.h"
+#include "scratch.h"
 
 using namespace csrspmm_b200;
 
@@ -261,7 +262,7 @@ int enqueue_scheduled(const csrspmm_b200_args* a, cudaStream_t st)
         }
         ws = a->workspace;
     } else {
-        CUDA_TRY(cudaMallocAsync(&ws, need, st));
+        CUDA_TRY(product_scratch_alloc(&ws, need, st));
         ws_owned = true;
     }
 
@@ -411,14 +412,18 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
     int* d_rows = nullptr;
     int* d_bounds = nullptr;
     unsigned* d_slab = nullptr;
+    int4* d_long_rows = nullptr;
+    // temporaries come from the scratch pool: mapping and unmapping them by cudaMalloc and cudaFree made a build of
+    // 3 ms take 600 at times
+    auto release_temporaries = [&]() {
+        for (void* ptr : {static_cast<void*>(d_counters), static_cast<void*>(d_rows), static_cast<void*>(d_bounds),
+                          static_cast<void*>(d_slab), static_cast<void*>(d_long_rows)})
+            if (ptr != nullptr) scratch_free(ptr, st);
+    };
     auto fail = [&](int code) {
+        release_temporaries();
         cudaStreamSynchronize(st);
-        cudaFree(d_counters);
-        cudaFree(d_rows);
-        cudaFree(d_bounds);
-        cudaFree(d_slab);
         cudaFree(s->pieces);
-        cudaFree(s->long_rows);
         delete s;
         return code;
     };
@@ -433,12 +438,12 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
 
     SCHED_TRY(cudaGetDevice(&s->device));
     if (!pointless && !pointless_auto && a->M > 0 && a->nnz > 0) {
-        SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&d_counters), kSchedCounters * sizeof(unsigned)));
+        SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_counters), kSchedCounters * sizeof(unsigned), st));
         SCHED_TRY(cudaMemsetAsync(d_counters, 0, kSchedCounters * sizeof(unsigned), st));
         // a row of `threshold` entries or more: at most nnz / threshold of them
         const long long cap_ll = a->nnz / threshold + 1;
         const int capacity = (int)(cap_ll < (long long)a->M ? cap_ll : (long long)a->M);
-        SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&d_rows), (size_t)capacity * sizeof(int)));
+        SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_rows), (size_t)capacity * sizeof(int), st));
         long long blocks = ((long long)a->M + 255) / 256;
         if (blocks > 148 * 16) blocks = 148 * 16;
         sched_list_long_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>(a->M, a->row_ptr, threshold, d_rows, capacity, d_counters);
@@ -454,15 +459,15 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
 
         if (num_long > 0) {
             const size_t bounds_bytes = (size_t)num_long * (size_t)(num_slabs + 1) * sizeof(int);
-            SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&d_bounds), bounds_bytes));
+            SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_bounds), bounds_bytes, st));
             SCHED_TRY(cudaMemsetAsync(d_bounds, 0, bounds_bytes, st));
-            SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&d_slab), (size_t)num_slabs * 2 * sizeof(unsigned)));
+            SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_slab), (size_t)num_slabs * 2 * sizeof(unsigned), st));
             SCHED_TRY(cudaMemsetAsync(d_slab, 0, (size_t)num_slabs * 2 * sizeof(unsigned), st));
-            SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&s->long_rows), (size_t)num_long * sizeof(int4)));
+            SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_long_rows), (size_t)num_long * sizeof(int4), st));
             const int warps = 8;
             sched_cut_rows_kernel<<<(unsigned)((num_long + warps - 1) / warps), warps * 32, 0, st>>>(
                 (int)num_long, d_rows, a->row_ptr, a->col_idx, (int)a->nnz, slab_rows, num_slabs, piece, d_bounds, d_slab,
-                s->long_rows, d_counters);
+                d_long_rows, d_counters);
             SCHED_TRY(cudaGetLastError());
             std::vector<unsigned> slab_count((size_t)num_slabs);
             SCHED_TRY(cudaMemcpyAsync(h_counters, d_counters, sizeof(h_counters), cudaMemcpyDeviceToHost, st));
@@ -478,7 +483,10 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
             if (!sorted) {
                 s->columns_sorted = 0;  // an empty schedule: the plain kernels run
             } else if (total > 0 && total <= 0x7fffffffLL && total == (long long)h_counters[5]) {
-                SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&s->pieces), (size_t)total * sizeof(int4)));
+                // what stays is one allocation: pieces, then rows
+                SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&s->pieces), ((size_t)total + (size_t)num_long) * sizeof(int4)));
+                s->long_rows = s->pieces + total;
+                SCHED_TRY(cudaMemcpyAsync(s->long_rows, d_long_rows, (size_t)num_long * sizeof(int4), cudaMemcpyDeviceToDevice, st));
                 unsigned* d_fill = d_slab + num_slabs;
                 SCHED_TRY(cudaMemcpyAsync(d_fill, slab_first.data(), (size_t)num_slabs * sizeof(unsigned), cudaMemcpyHostToDevice, st));
                 sched_emit_pieces_kernel<<<(unsigned)((num_long + 127) / 128), 128, 0, st>>>(
@@ -491,20 +499,8 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
                 s->device_bytes = (size_t)total * sizeof(int4) + (size_t)num_long * sizeof(int4);
             }
         }
-        cudaFree(d_counters);
-        cudaFree(d_rows);
-        cudaFree(d_bounds);
-        cudaFree(d_slab);
-        d_counters = nullptr;
-        d_rows = nullptr;
-        d_bounds = nullptr;
-        d_slab = nullptr;
-        if (s->num_long == 0) {  // nothing scheduled: keep no device memory
-            cudaFree(s->pieces);
-            cudaFree(s->long_rows);
-            s->pieces = nullptr;
-            s->long_rows = nullptr;
-        }
+        release_temporaries();
+        SCHED_TRY(cudaStreamSynchronize(st));
     }
 #undef SCHED_TRY
     s->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -521,8 +517,7 @@ int csrspmm_b200_schedule_destroy(csrspmm_b200_schedule* s)
     }
     int current = -1;
     const bool switched = cudaGetDevice(&current) == cudaSuccess && current != s->device && cudaSetDevice(s->device) == cudaSuccess;
-    cudaFree(s->pieces);
-    cudaFree(s->long_rows);
+    cudaFree(s->pieces);  // and the rows behind them
     if (switched) cudaSetDevice(current);
     s->magic = 0;
     delete s;

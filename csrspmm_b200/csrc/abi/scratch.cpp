@@ -51,6 +51,14 @@ cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t st)
     return pool != nullptr ? cudaMallocFromPoolAsync(ptr, bytes, pool, st) : cudaMallocAsync(ptr, bytes, st);
 }
 
+cudaError_t product_scratch_alloc(void** ptr, size_t bytes, cudaStream_t st)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(st, &capture);
+    if (e != cudaSuccess) return e;
+    return capture == cudaStreamCaptureStatusNone ? scratch_alloc(ptr, bytes, st) : cudaMallocAsync(ptr, bytes, st);
+}
+
 PinnedSlot::PinnedSlot()
 {
     std::lock_guard<std::mutex> lock(g_mutex);

@@ -28,8 +28,6 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_row_kernel(const SpmmP
 {
     wait_for_previous_grid();
     if (p.release_early) release_next_grid();
-    wait_for_previous_grid();
-    if (p.release_early) release_next_grid();
     constexpr int GROUPS = kRowThreads / G;
     const cg::thread_block_tile<G> tile = cg::tiled_partition<G>(cg::this_thread_block());
     const int lane = tile.thread_rank();
