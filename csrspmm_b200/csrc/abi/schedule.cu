@@ -422,8 +422,8 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
     };
     auto fail = [&](int code) {
         release_temporaries();
+        if (s->pieces != nullptr) scratch_free(s->pieces, st);
         cudaStreamSynchronize(st);
-        cudaFree(s->pieces);
         delete s;
         return code;
     };
@@ -483,8 +483,9 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
             if (!sorted) {
                 s->columns_sorted = 0;  // an empty schedule: the plain kernels run
             } else if (total > 0 && total <= 0x7fffffffLL && total == (long long)h_counters[5]) {
-                // what stays is one allocation: pieces, then rows
-                SCHED_TRY(cudaMalloc(reinterpret_cast<void**>(&s->pieces), ((size_t)total + (size_t)num_long) * sizeof(int4)));
+                // what stays is one allocation: pieces, then rows -- from the pool too, where the next schedule finds the
+                // memory of a destroyed one mapped (cudaMalloc of 21 MB: up to 50 ms now and then)
+                SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&s->pieces), ((size_t)total + (size_t)num_long) * sizeof(int4), st));
                 s->long_rows = s->pieces + total;
                 SCHED_TRY(cudaMemcpyAsync(s->long_rows, d_long_rows, (size_t)num_long * sizeof(int4), cudaMemcpyDeviceToDevice, st));
                 unsigned* d_fill = d_slab + num_slabs;
@@ -517,7 +518,10 @@ int csrspmm_b200_schedule_destroy(csrspmm_b200_schedule* s)
     }
     int current = -1;
     const bool switched = cudaGetDevice(&current) == cudaSuccess && current != s->device && cudaSetDevice(s->device) == cudaSuccess;
-    cudaFree(s->pieces);  // and the rows behind them
+    if (s->pieces != nullptr) {
+        cudaDeviceSynchronize();  // products that use it, on whatever stream
+        scratch_free(s->pieces, nullptr);  // and the rows behind them
+    }
     if (switched) cudaSetDevice(current);
     s->magic = 0;
     delete s;
