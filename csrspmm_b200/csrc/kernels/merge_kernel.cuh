@@ -432,8 +432,6 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
 {
     wait_for_previous_grid();
     if (p.release_early) release_next_grid();
-    wait_for_previous_grid();
-    if (p.release_early) release_next_grid();
     using Smem = MergeSmem<G, NV, VW, TG>;
     __shared__ Smem s;
 
@@ -608,8 +606,6 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
 template <int VW>
 __global__ void __launch_bounds__(256) spmm_fixup_kernel(const SpmmParams p, int num_tiles)
 {
-    wait_for_previous_grid();
-    if (p.release_early) release_next_grid();
     wait_for_previous_grid();
     if (p.release_early) release_next_grid();
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
