@@ -41,6 +41,7 @@ void fill_params(const csrspmm_b200_args* a, const Plan& plan, SpmmParams* out)
     p.release_early = plan.fills_chip;
     p.tg = plan.tg;
     p.row_aligned = plan.row_aligned;
+    p.c_ragged = plan.c_ragged;
     p.row_ptr = a->row_ptr;
     p.rp_base = a->row_ptr_base;
     p.col_idx = a->col_idx;
@@ -179,6 +180,8 @@ bool validation_requested()
     return on;
 }
 
+size_t align256(size_t v) { return (v + 255) / 256 * 256; }
+
 int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
 {
     int status = check_args(a, true);
@@ -194,11 +197,28 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
     if (schedule_applies(a)) return enqueue_scheduled(a, st);
 
     Plan plan;
-    status = make_plan(a, &plan);
+    float* padded = nullptr;  // a copy of B, when it pays and the caller's scratch has room for it
+    if (a->workspace != nullptr && (reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0) {
+        const size_t pad = padded_b_bytes(a);
+        if (pad > 0 && make_plan(a, &plan, kPlanPadded) == CSRSPMM_B200_OK) {
+            const size_t at = align256(plan.workspace_bytes);
+            if (at + pad <= a->workspace_bytes) padded = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + at);
+        }
+    }
+    if (padded == nullptr) status = make_plan(a, &plan);
     if (status != CSRSPMM_B200_OK) return status;
 
     SpmmParams p;
     fill_params(a, plan, &p);
+    if (padded != nullptr) {
+        const long long vectors = (long long)a->Kd * plan.ncolv;
+        const long long ctas = (vectors + 255) / 256;
+        CUDA_TRY(launch_overlapped(pad_rows_kernel, (unsigned)(ctas < 148 * 16 ? ctas : 148 * 16), 256, 0, st, vectors, plan.ncolv, a->Nd, a->B,
+                                   (long long)a->ldb, reinterpret_cast<float4*>(padded)));
+        p.B = padded;
+        p.ldb = 4LL * plan.ncolv;
+        p.ldb_bytes = (unsigned)(p.ldb * 4);
+    }
 
     const bool split = plan.kernel != CSRSPMM_B200_KERNEL_ROW;
     void* ws = nullptr;
@@ -239,8 +259,6 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
     }
     return CSRSPMM_B200_OK;
 }
-
-size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 // True when `ptr` is device memory of the current context (an operand the caller kept on the GPU).
 bool on_device(const void* ptr)
@@ -549,7 +567,7 @@ size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args)
 {
     if (args != nullptr && args->struct_size == sizeof(csrspmm_b200_args) && schedule_applies(args))
         return scheduled_workspace_bytes(args);
-    return worst_case_workspace(args);
+    return check_args(args, false) == CSRSPMM_B200_OK ? align256(worst_case_workspace(args)) + padded_b_bytes(args) : 0;
 }
 
 int csrspmm_b200_select_kernel(const csrspmm_b200_args* args)
@@ -559,6 +577,12 @@ int csrspmm_b200_select_kernel(const csrspmm_b200_args* args)
     if (status != CSRSPMM_B200_OK) return -status;
     if (schedule_applies(args)) return CSRSPMM_B200_KERNEL_SCHEDULED;
     return plan.kernel;
+}
+
+int csrspmm_b200_uses_workspace(const csrspmm_b200_args* args)
+{
+    const int kernel = csrspmm_b200_select_kernel(args);
+    return kernel < 0 ? kernel : (kernel != CSRSPMM_B200_KERNEL_ROW || padded_b_bytes(args) > 0 ? 1 : 0);
 }
 
 size_t csrspmm_b200_host_arena_bytes(const csrspmm_b200_args* a)

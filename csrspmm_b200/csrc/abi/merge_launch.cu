@@ -77,6 +77,11 @@ cudaError_t launch_fixup_kernel(const SpmmParams& p, const Plan& plan, cudaStrea
 {
     const int warps = 256 / 32;
     const unsigned grid = (unsigned)((plan.num_tiles + warps - 1) / warps);
+    if (plan.c_ragged) {  // carries lie column by column: added float by float where C is not aligned
+        SpmmParams q = p;
+        q.ncolv = p.Nd;
+        return launch_overlapped(spmm_fixup_kernel<1>, grid, 256, 0, st, q, (int)plan.num_tiles);
+    }
     return launch_overlapped(plan.VW == 4 ? spmm_fixup_kernel<4> : plan.VW == 2 ? spmm_fixup_kernel<2> : spmm_fixup_kernel<1>, grid, 256, 0, st, p, (int)plan.num_tiles);
 }
 

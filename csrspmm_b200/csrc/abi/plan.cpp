@@ -179,9 +179,11 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
     *plan = Plan();
     const bool vec = vector_layout_ok(a);
     // rows that do not start on 16 bytes but on 8 (50 columns, say) go two floats at a time
-    const bool pairs = !vec && (flags & kPlanNoPairs) == 0 && pair_layout_ok(a);
-    plan->VW = vec ? 4 : (pairs ? 2 : 1);
-    plan->ncolv = a->Nd / plan->VW;
+    const bool padded = (flags & kPlanPadded) != 0;  // B is a copy with whole vectors, C stays as it is
+    const bool pairs = !vec && !padded && (flags & kPlanNoPairs) == 0 && pair_layout_ok(a);
+    plan->VW = vec || padded ? 4 : (pairs ? 2 : 1);
+    plan->ncolv = (a->Nd + plan->VW - 1) / plan->VW;
+    plan->c_ragged = padded;
     plan->num_items = (long long)a->M + a->nnz;
 
     int kernel = a->kernel;
@@ -235,14 +237,14 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         plan->shape = shape_for(plan->ncolv);
         plan->G = kShapes[plan->shape].G;
         plan->NV = kShapes[plan->shape].NV;
-        plan->full = plan->VW == 4 && plan->G * plan->NV == plan->ncolv;
+        plan->full = plan->VW == 4 && !padded && plan->G * plan->NV == plan->ncolv;
         if (CSRSPMM_TUNE_MERGE_NARROW && kernel == CSRSPMM_B200_KERNEL_MERGE && (flags & kPlanNoNarrow) == 0 && plan->ncolv >= 1 && plan->ncolv <= 4) {
             // one, two or four column vectors: lane groups of that many lanes (kNarrowShapes)
             plan->narrow = plan->ncolv == 1 ? 1 : (plan->ncolv == 2 ? 2 : 3);
             const ShapeDesc& ns = kNarrowShapes[plan->narrow - 1];
             plan->G = ns.G;
             plan->NV = ns.NV;
-            plan->full = plan->VW == 4 && plan->G * plan->NV == plan->ncolv;
+            plan->full = plan->VW == 4 && !padded && plan->G * plan->NV == plan->ncolv;
             const int groups = CSRSPMM_TUNE_MERGE_THREADS / ns.G;
             fill_split_geometry(a, plan, groups, merge_items_per_group(plan->num_items, groups, merge_min_blocks(1), ns.TG, coarse ? ns.TG : ns.G));
             plan->row_aligned = rows_fit_tiles(a, *plan, groups, ns.TG);
@@ -257,7 +259,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         } else {
             const int groups = CSRSPMM_TUNE_ROW_THREADS / plan->G;
             plan->grid = ((long long)a->M + groups - 1) / groups;
-            plan->resident = (flags & kPlanNoPairs) == 0 ? resident_lanes(a, *plan) : 0;
+            plan->resident = (flags & kPlanNoPairs) == 0 && !padded ? resident_lanes(a, *plan) : 0;
             plan->short_rows = a->nnz <= (long long)CSRSPMM_TUNE_ROW_SHORT_MEAN * (long long)a->M;
             plan->low_occupancy = (long long)a->M * plan->G / 32 < 148LL * 8;
 #if CSRSPMM_TUNE_ROW_PERSISTENT > 0
@@ -280,6 +282,16 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         return CSRSPMM_B200_ERR_UNSUPPORTED;
     }
     return CSRSPMM_B200_OK;
+}
+
+size_t padded_b_bytes(const csrspmm_b200_args* a)
+{
+    if (a->Nd % 4 == 0 || a->Nd < 17 || a->M <= 0 || a->Kd <= 0 || a->kernel == CSRSPMM_B200_KERNEL_TMA) return 0;
+    const double mean = (double)a->nnz / a->M, uses = (double)a->nnz / a->Kd;
+    const double gather = (double)a->nnz * a->Nd * 4.0;
+    const bool pays = a->Nd % 2 ? uses >= (a->Nd <= 256 ? 8.0 : 24.0) && gather >= 64e6 && (a->Nd >= 32 || mean <= 64.0)
+                                : uses >= 64.0 && a->Nd >= 96 && gather >= 256e6;
+    return pays ? align_up((size_t)a->Kd * (size_t)((a->Nd + 3) / 4) * 16, 256) : 0;
 }
 
 size_t worst_case_workspace(const csrspmm_b200_args* a, bool any_row_block)

@@ -18,6 +18,7 @@ struct Plan {
     int shape = 0;                         // index into kShapes (tuning.h)
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
     int resident = 0;                      // whole-row mapping by the resident kernel: lanes per group (16, 32), else 0
+    bool c_ragged = false;                 // kPlanPadded: the last vector of a row of C is partly beyond it
     bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
     bool row_aligned = false;              // merge kernel: tiles cut at row starts, no carries and no fix-up
@@ -49,6 +50,7 @@ bool vector_layout_ok(const csrspmm_b200_args* a);
 // Returns CSRSPMM_B200_OK or an error status.
 constexpr unsigned kPlanNoNarrow = 1;  // no lane groups of fewer than eight lanes
 constexpr unsigned kPlanCoarse = 2;    // no tiles smaller than 64 items per lane group: fewer carry rows
+constexpr unsigned kPlanPadded = 8;    // for a copy of B padded to whole vectors (padded_b_bytes)
 constexpr unsigned kPlanNoPairs = 4;   // vector widths 4 and 1 only
 int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags = 0);
 
@@ -56,6 +58,15 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags = 0);
 // csrspmm_b200_workspace_bytes reports (the larger of the MERGE and TMA needs).  any_row_block:
 // also enough for any contiguous block of the matrix's rows multiplied on its own.
 size_t worst_case_workspace(const csrspmm_b200_args* a, bool any_row_block = false);
+
+// Scratch for a copy of B with rows padded to whole 16-byte vectors, or 0 where the product does without.  Rows of
+// 57 or 150 columns start on any 4 or 8 bytes, and gathered one or two floats per lane they come at half the rate; a copy
+// costs B read and written once, which eight uses of each row repay for odd widths (200 000 rows of 8, 19 columns 68 -> 37
+// us, 57 columns 81 -> 71; 20 000 rows of 24, 201 columns 61 -> 35; wider than 256 from 24 on: 200 000 of 8, 323 columns
+// 430 and 445) and 64 for even ones (100 000 rows of 16 over 5000, 150 columns 113 -> 90; 20 000 of 100, 510 columns 260 ->
+// 240).  Below 64 MB of gather (256 for even widths) the launch costs more than it gives, and long rows of few columns
+// leave too few lane groups when they are cut to vectors (20 000 of 100, 19 columns 30 -> 35).
+size_t padded_b_bytes(const csrspmm_b200_args* a);
 
 void set_last_error(const char* fmt, ...);
 const char* get_last_error();

@@ -37,6 +37,24 @@ __global__ void validate_csr_kernel(int M, int Kd, long long nnz, const int* __r
     if (bad) atomicOr(problems, bad);
 }
 
+// A copy of B whose rows are whole vectors of four, zeros behind the last column.
+__global__ void __launch_bounds__(256) pad_rows_kernel(long long vectors, int vectors_per_row, int Nd, const float* __restrict__ B, long long ldb,
+                                                       float4* __restrict__ out)
+{
+    wait_for_previous_grid();
+    release_next_grid();
+    for (long long k = (long long)blockIdx.x * 256 + threadIdx.x; k < vectors; k += (long long)gridDim.x * 256) {
+        const long long row = k / vectors_per_row;
+        const int c = (int)(k - row * vectors_per_row) * 4;
+        const float* src = B + row * ldb + c;
+        float4 v = make_float4(__ldg(src), 0.f, 0.f, 0.f);
+        if (c + 1 < Nd) v.y = __ldg(src + 1);
+        if (c + 2 < Nd) v.z = __ldg(src + 2);
+        if (c + 3 < Nd) v.w = __ldg(src + 3);
+        out[k] = v;
+    }
+}
+
 // Four numbers over all threads of a CTA: v[0] maximum, v[1..3] sums; valid in thread 0.
 constexpr int kStatsThreads = 256;
 constexpr int kStatsMaxCtas = 148 * 4;

@@ -45,6 +45,7 @@ struct SpmmParams {
     float alpha;
     float beta;
     int tg;              // split kernels: merge-path items per lane group (Plan::tg)
+    int c_ragged;        // B is a padded copy: vectors of four columns, the last of a row of C partly beyond Nd, C unaligned
     int row_aligned;     // merge kernel: tiles are cut at row starts and leave no carries (Plan::row_aligned)
     int* carry_row;      // one per tile: row the tile leaves unfinished, or -1
     float* carry_val;    // one row of carry_ld floats per tile
@@ -336,8 +337,9 @@ struct Vec<1> {
     }
 };
 
-// Write one finished row segment: C[row, cv] = alpha*acc + beta*C_old for this lane's NV vectors.
-template <int G, int NV, int VW>
+// Write one finished row segment: C[row, cv] = alpha*acc + beta*C_old for this lane's NV vectors.  RAGGED: the build
+// also serves p.c_ragged, whose rows of C are written float by float.
+template <int G, int NV, int VW, bool RAGGED = false>
 __device__ __forceinline__ void store_row(const SpmmParams& p, int row, int cb, int lane,
                                           const Vec<VW> (&acc)[NV])
 {
@@ -347,6 +349,26 @@ __device__ __forceinline__ void store_row(const SpmmParams& p, int row, int cb, 
         const int cv = cb + lane + v * G;
         if (cv < p.ncolv) {
             float* cp = crow + (long long)cv * VW;
+            if constexpr (RAGGED && VW == 4) {
+                if (p.c_ragged) {
+                    const float sum[4] = {acc[v].v.x, acc[v].v.y, acc[v].v.z, acc[v].v.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (cv * 4 + e < p.Nd) {
+                            Vec<1> one;
+                            one.v = sum[e];
+                            if (p.beta != 0.0f) {
+                                Vec<1> old;
+                                old.load(cp + e);
+                                one.epilogue(p.alpha, p.beta, old).store(cp + e);
+                            } else {
+                                one.epilogue0(p.alpha).store(cp + e);
+                            }
+                        }
+                    }
+                    continue;
+                }
+            }
 #if CSRSPMM_TUNE_C_STREAMING
             if (p.beta != 0.0f) {
                 Vec<VW> old;

@@ -319,7 +319,7 @@ __device__ __forceinline__ void merge_carry_by_warp(const SpmmParams& p, Smem& s
 // Steps 4-5 for one column pass.  acc = the group's unfinished partial sum (valid when dirty),
 // head = its held-back first finished row (valid when il1 > il0).  Contains one __syncthreads.
 // head_skip: the group's first finished row belongs to the scheduled pieces and is not written.
-template <class Smem, int G, int NV, int VW>
+template <class Smem, int G, int NV, int VW, bool RAGGED = false>
 __device__ __forceinline__ void merge_tile_finish(const SpmmParams& p, Smem& s, const TileRange& r,
                                                   int cb, int g, int lane, const Vec<VW> (&acc)[NV],
                                                   Vec<VW> (&head)[NV], bool dirty, bool head_skip = false)
@@ -355,7 +355,7 @@ __device__ __forceinline__ void merge_tile_finish(const SpmmParams& p, Smem& s, 
                 head[v] = sum[v];
             }
         }
-        store_row<G, NV, VW>(p, r.i0 + r.il0, cb, lane, head);
+        store_row<G, NV, VW, RAGGED>(p, r.i0 + r.il0, cb, lane, head);
     }
 
     // ---- 5. the row this CTA leaves unfinished ------------------------------------------------
@@ -417,7 +417,7 @@ __device__ __noinline__ void merge_rows_directly(const SpmmParams& p, const int 
                     }
                 }
             }
-            store_row<G, NV, VW>(p, row, cb, lane, acc);
+            store_row<G, NV, VW, true>(p, row, cb, lane, acc);
         }
     }
 }
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
 #pragma unroll
                 for (int v = 0; v < NV; ++v) head[v] = acc[v];
             } else {
-                store_row<G, NV, VW>(p, r.i0 + i, cb, lane, acc);
+                store_row<G, NV, VW, !FULL && !SKIP>(p, r.i0 + i, cb, lane, acc);
             }
 #pragma unroll
             for (int v = 0; v < NV; ++v) acc[v].zero();
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
         }  // !SKIP
         while (i < r.il1) finish_row();
 
-        merge_tile_finish<Smem, G, NV, VW>(p, s, r, cb, g, lane, acc, head, dirty, head_skip);
+        merge_tile_finish<Smem, G, NV, VW, !FULL && !SKIP>(p, s, r, cb, g, lane, acc, head, dirty, head_skip);
         if (cb + G * NV < p.ncolv) __syncthreads();  // tails are rewritten by the next pass
     }
 }

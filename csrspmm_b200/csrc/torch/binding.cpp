@@ -34,7 +34,7 @@ namespace {
 struct Library {
     int (*spmm)(const csrspmm_b200_args*, csrspmm_b200_stream_t);
     int (*spmm_sync)(const csrspmm_b200_args*, csrspmm_b200_stream_t);
-    int (*select_kernel)(const csrspmm_b200_args*);
+    int (*uses_workspace)(const csrspmm_b200_args*);
     size_t (*workspace_bytes)(const csrspmm_b200_args*);
     int (*row_stats)(int32_t, const int32_t*, int64_t*, csrspmm_b200_stream_t);
     int (*dense2csr_count)(int32_t, int32_t, const float*, int64_t, float, int32_t*, int64_t*, int32_t*, csrspmm_b200_stream_t);
@@ -191,9 +191,9 @@ at::Tensor run_product(Product& q)
     const auto stream = c10::cuda::getCurrentCUDAStream(q.B.device().index());
     Scratch scratch;
     if (M > 0 && Nd > 0) {
-        const int chosen = g_lib.select_kernel(&a);
-        if (chosen < 0) throw LibraryError{-chosen, "csrspmm_b200_select_kernel"};
-        if (chosen != CSRSPMM_B200_KERNEL_ROW) {
+        const int uses = g_lib.uses_workspace(&a);
+        if (uses < 0) throw LibraryError{-uses, "csrspmm_b200_select_kernel"};
+        if (uses > 0) {
             const size_t need = g_lib.workspace_bytes(&a);
             if (q.workspace.defined() && q.workspace.nbytes() >= need) {
                 a.workspace = q.workspace.data_ptr();
@@ -299,7 +299,7 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     };
     fill(g_lib.spmm, "spmm");
     fill(g_lib.spmm_sync, "spmm_sync");
-    fill(g_lib.select_kernel, "select_kernel");
+    fill(g_lib.uses_workspace, "uses_workspace");
     fill(g_lib.workspace_bytes, "workspace_bytes");
     fill(g_lib.row_stats, "row_stats_device");
     fill(g_lib.dense2csr_count, "dense2csr_count");

@@ -203,7 +203,7 @@ class SpmmCall:
             self.kernel = _lib.KERNEL_NAMES[k]
             # scheduled: pieces, slot sums, merge-path over the other rows, fix-up
             self.launches = 1 if k == _lib.KERNEL_ROW else (4 if k == _lib.KERNEL_SCHEDULED else 2)
-            if k != _lib.KERNEL_ROW:
+            if self.L.csrspmm_b200_uses_workspace(C.byref(self.args)) > 0:
                 need = int(self.L.csrspmm_b200_workspace_bytes(C.byref(self.args)))
                 if workspace is None or workspace.numel() * workspace.element_size() < need:
                     workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=B.device)

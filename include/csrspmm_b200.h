@@ -194,9 +194,14 @@ int32_t csrspmm_b200_tiled_panel_rows(const csrspmm_b200_args* args);
 size_t csrspmm_b200_tiled_workspace_bytes(const csrspmm_b200_args* args);
 int csrspmm_b200_spmm_tiled(const csrspmm_b200_args* args, int32_t panel_rows, csrspmm_b200_stream_t stream);
 
-/* Scratch the split kernels need for this problem (0 for the row kernel).  Depends only on
- * sizes, never on matrix contents. */
+/* Scratch for this problem: the split kernels' carries and, for dense widths that are no multiple of four and rows of
+ * B used often enough, a padded copy of B (without room for it the product runs on B as it is).  Depends only
+ * on sizes, never on matrix contents. */
 size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args);
+
+/* 1 when a product with these arguments makes use of args.workspace, 0 when it does not, or a negative
+ * csrspmm_b200_status.  Host-only logic. */
+int csrspmm_b200_uses_workspace(const csrspmm_b200_args* args);
 
 /* The kernel AUTO resolves to for these arguments (host-only logic, no CUDA call);
  * returns a csrspmm_b200_kernel, or a negative csrspmm_b200_status on bad arguments.

@@ -1,0 +1,35 @@
+"""Products on a padded copy of B (widths that are no multiple of four), and the same without room for the copy."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from csrspmm_b200 import generators as G, ops
+
+pytestmark = pytest.mark.gpu  # the last test needs no GPU, but the library
+
+
+@pytest.mark.parametrize("Nd", [19, 33, 57, 99, 130, 201, 255, 257, 510])
+@pytest.mark.parametrize("kernel,skew,beta", [("row", False, 0.0), ("merge", False, 0.5), ("merge", True, -0.5)])
+def test_padded_copy(cuda_lib, Nd, kernel, skew, beta):
+    rng = np.random.default_rng(Nd)
+    M, Kd = 9001, 2500
+    lens = rng.integers(0, 2 * max(20, 9_000_000 // Nd // (M // 8)), M) % 1200
+    if Nd % 2 == 0:
+        lens = rng.integers(20, 120, M)
+    if skew:
+        lens[77] = Kd
+    p = G.random_csr(M, Kd, Nd, 0.0, seed=3, lengths=lens)
+    t = [torch.from_numpy(x).cuda() for x in (p.row_ptr, p.col_idx, p.values)]
+    wide = torch.randn((Kd, Nd + 2), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    B = wide[:, 1:1 + Nd]  # rows that start anywhere, and do not follow each other
+    C0 = rng.standard_normal((M, Nd), dtype=np.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ops.spmm(*t, B, torch.from_numpy(C0).cuda(), 1.5, beta, kernel=kernel, max_row_nnz=0 if skew else int(lens.max()),
+                   status_word=status, sync=True).cpu().numpy()
+    f64, mag = oracle.spmm_f64(p.row_ptr, p.col_idx, p.values, np.ascontiguousarray(B.cpu().numpy()), C0, 1.5, beta, threads=4)
+    assert int(status) == 0 and (np.abs(got - f64) <= 1e-5 * mag + 1e-6).all()
+
+
+def test_the_copy_is_counted_as_scratch():
+    assert ops.workspace_bytes(200000, 200000, 57, 1_600_000) >= ops.workspace_bytes(200000, 200000, 60, 1_600_000) + 200000 * 240 - 256
