@@ -171,6 +171,18 @@ static int resident_lanes(const csrspmm_b200_args* a, const Plan& plan)
     return a->nnz * panels >= reuse * 148LL * a->Kd ? lanes : 0;
 }
 
+// Whether a whole-row product would be a chain of its longest rows' entries on a chip that is mostly idle: few rows, long
+// ones, and lane groups that share a warp, where the merge kernel cuts rows among all SMs.  512 rows of 200: 16 columns
+// 25.3 us whole and 9.1 cut, 64 12.4 and 7.3, 512 22.6 and 16.1; 8192 rows of 200: 32 columns 34.7 and 22.5, 64 31.4 and 27.8;
+// 18 000 of 100, 32 columns 23.4 and 24.5.  Widths that are no multiple of four lose earlier: their gather costs the
+// merge kernel more (50 columns, rows of 200: 16.7 and 7.6 with 512 rows, 36.0 and 40.4 with 8192).
+static bool rows_are_chains(long long M, double mean, const Plan& plan)
+{
+    const ShapeDesc& s = kShapes[shape_for(plan.ncolv)];
+    if (plan.VW == 4) return s.G == 32 ? M < 592 && mean >= 200.0 : M <= 12000 && mean >= (s.G == 8 ? 64.0 : 150.0);
+    return s.G == 32 ? M < 592 && mean >= (s.NV == 1 ? 80.0 : 200.0) : M <= 2400 && mean >= 80.0;
+}
+
 int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
 {
     const bool coarse = (flags & kPlanCoarse) != 0;
@@ -208,9 +220,10 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         const double row_limit = avg * 4.0 > 64.0 ? avg * 4.0 : 64.0;
         const double b_bytes = (double)a->Kd * (double)a->Nd * 4.0;
         const bool rows_even = a->max_row_nnz > 0 && (double)a->max_row_nnz <= row_limit;
+        plan->rows_even = rows_even;
         if (tma_can_run(a) && a->Nd > 384 && b_bytes >= 1073741824.0 && !rows_even)
             kernel = CSRSPMM_B200_KERNEL_TMA;
-        else if (rows_even && (b_bytes < 48e6 || avg > 64.0 || (avg * a->Nd >= 8192.0 && a->Nd > 64)))
+        else if (rows_even && !rows_are_chains(a->M, avg, *plan) && (b_bytes < 48e6 || avg > 64.0 || (avg * a->Nd >= 8192.0 && a->Nd > 64)))
             kernel = CSRSPMM_B200_KERNEL_ROW;
         else
             kernel = CSRSPMM_B200_KERNEL_MERGE;

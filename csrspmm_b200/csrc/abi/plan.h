@@ -19,6 +19,7 @@ struct Plan {
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
     int resident = 0;                      // whole-row mapping by the resident kernel: lanes per group (16, 32), else 0
     bool c_ragged = false;                 // kPlanPadded: the last vector of a row of C is partly beyond it
+    bool rows_even = false;                // AUTO: the longest row is known to be close to the mean
     bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
     bool row_aligned = false;              // merge kernel: tiles cut at row starts, no carries and no fix-up

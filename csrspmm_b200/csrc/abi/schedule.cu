@@ -205,11 +205,11 @@ bool schedule_applies(const csrspmm_b200_args* a)
         env_forces_other_kernel())
         return false;
     if (a->kernel == CSRSPMM_B200_KERNEL_AUTO) {
-        // rows known to be even: the whole-row kernel is what AUTO would run, and it is the better choice
+        // rows known to be even: a schedule for long rows among short ones has nothing to offer
         csrspmm_b200_args plain = *a;
         plain.schedule = nullptr;
         Plan plan;
-        if (make_plan(&plain, &plan) == CSRSPMM_B200_OK && plan.kernel == CSRSPMM_B200_KERNEL_ROW) return false;
+        if (make_plan(&plain, &plan) == CSRSPMM_B200_OK && plan.rows_even) return false;
     }
     return true;
 }
