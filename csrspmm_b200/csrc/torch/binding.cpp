@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/VariableTypeUtils.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -667,6 +668,19 @@ TORCH_LIBRARY_IMPL(csrspmm_b200, CUDA, m)
 }
 
 TORCH_LIBRARY_IMPL(csrspmm_b200, Autograd, m) { m.impl("spmm", autograd_spmm); }
+
+// The dispatcher does not raise the version counter of a tensor that a schema names as written, and the kernel writes
+// through an address: without this a C that a backward saved and spmm_ overwrote would give a wrong gradient.
+void spmm_inplace_marking(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, const at::Tensor& C,
+                          double alpha, double beta, c10::string_view kernel)
+{
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("csrspmm_b200::spmm_", "").typed<decltype(op_spmm_inplace)>();
+    if (!C.is_inference()) torch::autograd::increment_version(C);
+    at::AutoDispatchBelowADInplaceOrView below;
+    op.call(rp, ci, va, B, C, alpha, beta, kernel);
+}
+
+TORCH_LIBRARY_IMPL(csrspmm_b200, ADInplaceOrView, m) { m.impl("spmm_", spmm_inplace_marking); }
 
 #define FASTCALL(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL
 PyMethodDef g_methods[] = {

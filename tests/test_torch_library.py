@@ -34,6 +34,22 @@ def test_fake_implementation_traces_without_a_gpu():
         assert out.shape == (13, 4) and out.dtype == torch.float32
 
 
+def test_the_inplace_operator_marks_c_as_modified():
+    lib = torch.library.Library("csrspmm_b200", "IMPL")  # a stand-in for the product: what is looked at is above it
+    lib.impl("spmm_", lambda rp, ci, va, B, C, alpha, beta, kernel: None, "CPU")
+    a = [torch.zeros(2, dtype=torch.int32), torch.zeros(0, dtype=torch.int32), torch.zeros(0), torch.zeros(1, 4)]
+    x, C = torch.ones(1, 4, requires_grad=True), torch.ones(1, 4)
+    y = (x * C).sum()
+    torch.ops.csrspmm_b200.spmm_(*a, C, 1.0, 0.0, "auto")
+    assert C._version == 1
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
+    with torch.inference_mode():
+        D = torch.ones(1, 4)  # has no counter
+        torch.ops.csrspmm_b200.spmm_(*a, D, 1.0, 0.0, "auto")
+    lib._destroy()
+
+
 @pytest.mark.gpu
 def test_registered_ops_and_inplace_semantics(cuda_lib):
     p = G.random_csr(200, 150, 64, 0.05, seed=4)
