@@ -498,8 +498,8 @@ def main(argv=None):
     footprint = my_nnz * 8 + my_rows * 4 + (Kd + my_rows) * Nd * 4
     flush = footprint < 2 * L2_BYTES
     flush_buf = torch.empty(2 * L2_BYTES, dtype=torch.uint8, device=dev) if flush else None
-    chosen = ops.selected_kernel(my_rows, Kd, Nd, my_nnz, kernel=ns.kernel, max_row_nnz=0)
-    launches_per_step = 1 if chosen == "row" else 2
+    plan = ops.plan_info(my_rows, Kd, Nd, my_nnz, kernel=ns.kernel, max_row_nnz=0)
+    chosen, launches_per_step = plan["kernel"], plan["launches"]
     # per-matrix schedule (built once per matrix, outside the timed region, like cuSPARSE's preprocess): the
     # library decides by itself whether this matrix and this width of B are worth one
     schedule, sched_info = None, None

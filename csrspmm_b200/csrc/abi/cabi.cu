@@ -197,20 +197,13 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
     if (schedule_applies(a)) return enqueue_scheduled(a, st);
 
     Plan plan;
-    float* padded = nullptr;  // a copy of B, when it pays and the caller's scratch has room for it
-    if (a->workspace != nullptr && (reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0) {
-        const size_t pad = padded_b_bytes(a);
-        if (pad > 0 && make_plan(a, &plan, kPlanPadded) == CSRSPMM_B200_OK) {
-            const size_t at = align256(plan.workspace_bytes);
-            if (at + pad <= a->workspace_bytes) padded = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + at);
-        }
-    }
-    if (padded == nullptr) status = make_plan(a, &plan);
+    status = product_plan(a, &plan);
     if (status != CSRSPMM_B200_OK) return status;
 
     SpmmParams p;
     fill_params(a, plan, &p);
-    if (padded != nullptr) {
+    if (plan.c_ragged) {
+        float* const padded = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + padded_b_offset(plan));
         const long long vectors = (long long)a->Kd * plan.ncolv;
         const long long ctas = (vectors + 255) / 256;
         CUDA_TRY(launch_overlapped(pad_rows_kernel, (unsigned)(ctas < 148 * 16 ? ctas : 148 * 16), 256, 0, st, vectors, plan.ncolv, a->Nd, a->B,
@@ -573,10 +566,30 @@ size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args)
 int csrspmm_b200_select_kernel(const csrspmm_b200_args* args)
 {
     Plan plan;
-    int status = make_plan(args, &plan);
+    int status = product_plan(args, &plan);
     if (status != CSRSPMM_B200_OK) return -status;
     if (schedule_applies(args)) return CSRSPMM_B200_KERNEL_SCHEDULED;
     return plan.kernel;
+}
+
+int csrspmm_b200_plan_info_get(const csrspmm_b200_args* args, csrspmm_b200_plan_info* info)
+{
+    if (info == nullptr || info->struct_size != sizeof(csrspmm_b200_plan_info)) {
+        set_last_error("plan_info_get: info is null or info.struct_size wrong");
+        return CSRSPMM_B200_ERR_BAD_ARG;
+    }
+    Plan plan;
+    const int status = product_plan(args, &plan);
+    if (status != CSRSPMM_B200_OK) return status;
+    const bool scheduled = schedule_applies(args);
+    info->kernel = scheduled ? CSRSPMM_B200_KERNEL_SCHEDULED : plan.kernel;
+    info->padded_copy = !scheduled && plan.c_ragged;
+    info->resident_lanes = info->kernel == CSRSPMM_B200_KERNEL_ROW ? plan.resident : 0;
+    info->row_aligned = info->kernel == CSRSPMM_B200_KERNEL_MERGE && plan.row_aligned;
+    // scheduled: pieces, slot sums, merge-path over the other rows, fix-up; split: the kernel and its fix-up
+    info->launches = scheduled ? 4 : (plan.kernel == CSRSPMM_B200_KERNEL_ROW || plan.row_aligned ? 1 : 2) + info->padded_copy;
+    if (args->M == 0 || args->Nd == 0) info->launches = 0;
+    return CSRSPMM_B200_OK;
 }
 
 int csrspmm_b200_uses_workspace(const csrspmm_b200_args* args)

@@ -307,6 +307,17 @@ size_t padded_b_bytes(const csrspmm_b200_args* a)
     return pays ? align_up((size_t)a->Kd * (size_t)((a->Nd + 3) / 4) * 16, 256) : 0;
 }
 
+int product_plan(const csrspmm_b200_args* a, Plan* plan)
+{
+    if (a != nullptr && a->struct_size == sizeof(csrspmm_b200_args) && a->workspace != nullptr &&
+        (reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0) {
+        const size_t pad = padded_b_bytes(a);
+        if (pad > 0 && make_plan(a, plan, kPlanPadded) == CSRSPMM_B200_OK && padded_b_offset(*plan) + pad <= a->workspace_bytes)
+            return CSRSPMM_B200_OK;
+    }
+    return make_plan(a, plan);
+}
+
 size_t worst_case_workspace(const csrspmm_b200_args* a, bool any_row_block)
 {
     if (check_args(a, false) != CSRSPMM_B200_OK) return 0;

@@ -55,6 +55,11 @@ constexpr unsigned kPlanPadded = 8;    // for a copy of B padded to whole vector
 constexpr unsigned kPlanNoPairs = 4;   // vector widths 4 and 1 only
 int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags = 0);
 
+// What csrspmm_b200_spmm runs without a schedule: the plan for a padded copy of B (plan->c_ragged) when that pays and
+// args.workspace has room for it behind the carries, at padded_b_offset(); else the plan for B as it is.
+int product_plan(const csrspmm_b200_args* a, Plan* plan);
+inline size_t padded_b_offset(const Plan& plan) { return (plan.workspace_bytes + 255) / 256 * 256; }
+
 // Workspace of the split kernels for a given plan-independent worst case: what
 // csrspmm_b200_workspace_bytes reports (the larger of the MERGE and TMA needs).  any_row_block:
 // also enough for any contiguous block of the matrix's rows multiplied on its own.

@@ -197,19 +197,19 @@ class SpmmCall:
         self.kernel = "row"
         self.launches = 0
         if M > 0 and Nd > 0:
-            k = self.L.csrspmm_b200_select_kernel(C.byref(self.args))
-            if k < 0:
-                raise _lib.SpmmError(-k, "csrspmm_b200_select_kernel")
-            self.kernel = _lib.KERNEL_NAMES[k]
-            # scheduled: pieces, slot sums, merge-path over the other rows, fix-up
-            self.launches = 1 if k == _lib.KERNEL_ROW else (4 if k == _lib.KERNEL_SCHEDULED else 2)
-            if self.L.csrspmm_b200_uses_workspace(C.byref(self.args)) > 0:
+            uses = self.L.csrspmm_b200_uses_workspace(C.byref(self.args))
+            if uses < 0:
+                raise _lib.SpmmError(-uses, "csrspmm_b200_select_kernel")
+            if uses > 0:
                 need = int(self.L.csrspmm_b200_workspace_bytes(C.byref(self.args)))
                 if workspace is None or workspace.numel() * workspace.element_size() < need:
                     workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=B.device)
                 self.args.workspace = workspace.data_ptr()
                 self.args.workspace_bytes = workspace.numel() * workspace.element_size()
-        self.workspace = workspace  # scratch of the split kernels (None for the row kernel); may be shared
+            plan = _plan_info(self.args)
+            self.kernel, self.launches = plan["kernel"], plan["launches"]
+        # scratch of the split kernels and of a padded copy of B (None where neither runs); may be shared by calls on one stream
+        self.workspace = workspace
         self._keep = (row_ptr, col_idx, values, B, C_out, workspace, status_word, schedule)
         self._enqueue = _lib.binding().enqueue
         self._where = (C.addressof(self.args), B.device.index)
@@ -221,14 +221,28 @@ class SpmmCall:
         return self.out
 
 
-def selected_kernel(M, Kd, Nd, nnz, *, entry="naive", max_row_nnz=0, kernel="auto", aligned=True) -> str:
-    """Name of the kernel AUTO picks for these sizes (host-only, needs no GPU)."""
+def _plan_info(a) -> dict:
+    info = _lib.PlanInfo()
+    info.struct_size = C.sizeof(_lib.PlanInfo)
+    _lib.check(_lib.lib().csrspmm_b200_plan_info_get(C.byref(a), C.byref(info)), "csrspmm_b200_plan_info_get")
+    return dict(kernel=_lib.KERNEL_NAMES[info.kernel], launches=info.launches, padded_copy=bool(info.padded_copy),
+                resident_lanes=info.resident_lanes, row_aligned=bool(info.row_aligned))
+
+
+def plan_info(M, Kd, Nd, nnz, *, entry="naive", max_row_nnz=0, kernel="auto", aligned=True, workspace=True) -> dict:
+    """What ``spmm`` runs for these sizes (host-only, needs no GPU): the kernel, how many kernels are launched, and
+    whether B is copied first, whole rows run on a panel of B in shared memory, or tiles are cut at row starts.
+    ``workspace=False``: what the C ABI runs when it is given no workspace."""
     a = _lib.make_args(M, Kd, Nd, nnz, B=256 if aligned else 4, Cptr=256 if aligned else 4,
                        entry=_ENTRY[entry], kernel=_lib.KERNEL_IDS[kernel], max_row_nnz=max_row_nnz)
-    k = _lib.lib().csrspmm_b200_select_kernel(C.byref(a))
-    if k < 0:
-        raise _lib.SpmmError(-k, "csrspmm_b200_select_kernel")
-    return _lib.KERNEL_NAMES[k]
+    if workspace:
+        a.workspace, a.workspace_bytes = 256, _lib.lib().csrspmm_b200_workspace_bytes(C.byref(a))
+    return _plan_info(a)
+
+
+def selected_kernel(M, Kd, Nd, nnz, **kw) -> str:
+    """Name of the kernel ``spmm`` runs for these sizes (``plan_info``)."""
+    return plan_info(M, Kd, Nd, nnz, **kw)["kernel"]
 
 
 # ---- the reference's five ops (torch_csrspmm/__init__.py:10-23): new C = alpha * A @ B ---------------

@@ -203,10 +203,23 @@ size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args);
  * csrspmm_b200_status.  Host-only logic. */
 int csrspmm_b200_uses_workspace(const csrspmm_b200_args* args);
 
-/* The kernel AUTO resolves to for these arguments (host-only logic, no CUDA call);
- * returns a csrspmm_b200_kernel, or a negative csrspmm_b200_status on bad arguments.
+/* The kernel csrspmm_b200_spmm runs for these arguments (host-only logic, no CUDA call);
+ * returns a csrspmm_b200_kernel, or a negative csrspmm_b200_status on bad arguments.  The workspace given is part
+ * of the question: with room for a padded copy of B the choice can be another one than without.
  * The environment variable CSRSPMM_FORCE_KERNEL=row|merge|tma overrides AUTO. */
 int csrspmm_b200_select_kernel(const csrspmm_b200_args* args);
+
+/* The same decision in full. */
+typedef struct csrspmm_b200_plan_info {
+    uint32_t struct_size;   /* set to sizeof(csrspmm_b200_plan_info) by the caller */
+    int32_t kernel;         /* as csrspmm_b200_select_kernel */
+    int32_t launches;       /* kernels the product launches */
+    int32_t padded_copy;    /* 1: first a copy of B with rows of whole 16-byte vectors, in the workspace */
+    int32_t resident_lanes; /* kernel ROW: lanes per row of the build that keeps a panel of B in shared memory, 0: the
+                             * ordinary one (both sum each output in stored order) */
+    int32_t row_aligned;    /* kernel MERGE: 1 when tiles are cut at row starts, so that no row is split and no fix-up runs */
+} csrspmm_b200_plan_info;
+int csrspmm_b200_plan_info_get(const csrspmm_b200_args* args, csrspmm_b200_plan_info* info);
 
 /* ---- per-matrix schedule ---------------------------------------------------------------------
  * Stands where the reference's spmm() has a stub that inspects nothing (src/csrspmm.cpp:34-40).

@@ -12,3 +12,18 @@ from csrspmm_b200 import ops
     (1 << 20, 1 << 20, 64, 16, "merge"), (1 << 20, 1 << 20, 64, 65, "row"), (180000, 180000, 64, 16, "row")])  # B beyond 48 MB
 def test_even_rows(M, Kd, Nd, mean, want):
     assert ops.selected_kernel(M, Kd, Nd, M * mean, max_row_nnz=max(60, mean + mean // 2)) == want
+
+
+@pytest.mark.parametrize("sizes,longest,with_room,without", [
+    ((5000, 5000, 57, 1_500_000), 350, dict(kernel="merge", launches=2, padded_copy=True, row_aligned=True), dict(kernel="row")),
+    ((200_000, 200_000, 57, 1_600_000), 40, dict(kernel="row", launches=2, padded_copy=True), dict(kernel="row")),
+    ((20_000, 20_000, 201, 480_000), 0, dict(kernel="merge", launches=3, padded_copy=True), dict(kernel="merge", launches=2)),
+    ((16_384, 16_384, 64, 262_144), 40, dict(kernel="row"), dict(kernel="row")),
+    ((8192, 256, 4096, 209_715), 60, dict(kernel="row", resident_lanes=32), dict(kernel="row", resident_lanes=32)),
+    ((512, 4096, 64, 102_400), 300, dict(kernel="merge", row_aligned=True), dict(kernel="merge", row_aligned=True))])
+def test_plan_info_says_what_runs(sizes, longest, with_room, without):
+    for room, want in ((True, with_room), (False, without)):
+        got = ops.plan_info(*sizes, max_row_nnz=longest, workspace=room)
+        assert got == dict(dict(launches=1, padded_copy=False, resident_lanes=0, row_aligned=False), **want)
+    assert ops.selected_kernel(*sizes, max_row_nnz=longest) == with_room["kernel"]
+    assert ops.plan_info(0, 5, 64, 0)["launches"] == 0

@@ -1,4 +1,6 @@
 """Products on a padded copy of B (widths that are no multiple of four), and the same without room for the copy."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -6,7 +8,7 @@ import torch
 import oracle
 from csrspmm_b200 import generators as G, ops
 
-pytestmark = pytest.mark.gpu  # the last test needs no GPU, but the library
+pytestmark = pytest.mark.gpu  # the test of the scratch size needs no GPU, but the library
 
 
 @pytest.mark.parametrize("Nd", [19, 33, 57, 99, 130, 201, 255, 257, 510])
@@ -33,3 +35,20 @@ def test_padded_copy(cuda_lib, Nd, kernel, skew, beta):
 
 def test_the_copy_is_counted_as_scratch():
     assert ops.workspace_bytes(200000, 200000, 57, 1_600_000) >= ops.workspace_bytes(200000, 200000, 60, 1_600_000) + 200000 * 240 - 256
+
+
+@pytest.mark.parametrize("M,Kd,Nd,mean,longest", [(5000, 5000, 57, 300, 350), (60_000, 20_000, 57, 16, 40), (20_000, 20_000, 201, 24, 0), (9000, 9000, 64, 8, 20),
+                                                  (9000, 256, 2048, 25, 60)])
+def test_call_says_what_it_launches(cuda_lib, M, Kd, Nd, mean, longest):
+    lens = np.random.default_rng(M).integers(mean - mean // 8, mean + mean // 8 + 1, M)
+    p = G.random_csr(M, Kd, Nd, 0.0, seed=3, lengths=lens)
+    t = [torch.from_numpy(x).cuda() for x in (p.row_ptr, p.col_idx, p.values, p.B)]
+    call = ops.SpmmCall(*t, torch.empty((M, Nd), device="cuda"), max_row_nnz=longest)
+    assert call.kernel == ops.selected_kernel(M, Kd, Nd, p.nnz, max_row_nnz=longest)
+    call()  # the first call makes the settings that a capture may not
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        call()
+    count = ctypes.c_size_t(0)  # every node of the captured call is a kernel
+    assert ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(g.raw_cuda_graph()), None, ctypes.byref(count)) == 0
+    assert count.value == call.launches
