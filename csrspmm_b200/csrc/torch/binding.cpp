@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <optional>
 
 #include "csrspmm_b200.h"
 
@@ -143,7 +144,7 @@ struct Product {
     int max_row_nnz = 0;
     bool packed = false;
     double scale = 1.0;
-    int64_t nnz = -1;  // -1: col_idx's length
+    std::optional<int64_t> nnz;  // not given: col_idx's length
     int32_t* status_word = nullptr;
     const csrspmm_b200_schedule* schedule = nullptr;
     bool sync = false;
@@ -153,7 +154,7 @@ at::Tensor run_product(Product& q)
 {
     check_csr(q.rp, q.ci, q.va, q.B, q.packed);
     const int64_t M = q.rp.size(0) - 1, Kd = q.B.size(0), Nd = q.B.size(1);
-    const int64_t n = q.nnz < 0 ? q.ci.size(0) : q.nnz;
+    const int64_t n = q.nnz.value_or(q.ci.size(0));
     if (q.packed) want(q.va.size(0) >= (n + 1) / 2, "packed values too short");
     else want(q.va.size(0) == n, "values and col_idx differ in length");
     const c10::cuda::CUDAGuard guard(q.B.device());
@@ -283,6 +284,15 @@ long long as_integer(PyObject* o)
     return v;
 }
 
+// int(o): a whole number in any numeric type
+long long as_int_of(PyObject* o)
+{
+    if (PyLong_Check(o)) return as_integer(o);
+    const auto number = pybind11::reinterpret_steal<pybind11::object>(PyNumber_Long(o));
+    if (!number) throw python_error();
+    return as_integer(number.ptr());
+}
+
 void expect_args(Py_ssize_t got, Py_ssize_t wanted)
 {
     if (got != wanted) throw std::runtime_error("csrspmm_b200 binding: wrong number of arguments");
@@ -328,12 +338,12 @@ PyObject* py_spmm(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     if (args[4] != Py_None) q.C = tensor_of(args[4], "C_out");
     q.alpha = as_double(args[5]);
     q.beta = as_double(args[6]);
-    q.entry = static_cast<int>(as_integer(args[7]));
-    q.kernel = static_cast<int>(as_integer(args[8]));
-    q.max_row_nnz = static_cast<int>(as_integer(args[9]));
+    q.entry = static_cast<int>(as_int_of(args[7]));
+    q.kernel = static_cast<int>(as_int_of(args[8]));
+    q.max_row_nnz = static_cast<int>(as_int_of(args[9]));
     q.packed = args[10] != Py_None;
     if (q.packed) q.scale = as_double(args[10]);
-    if (args[11] != Py_None) q.nnz = as_integer(args[11]);
+    if (args[11] != Py_None) q.nnz = as_int_of(args[11]);
     if (args[12] != Py_None) q.workspace = tensor_of(args[12], "workspace");
     if (args[13] != Py_None) q.status_word = address<int32_t>(tensor_of(args[13], "status_word"));
     q.sync = PyObject_IsTrue(args[14]) == 1;
