@@ -641,6 +641,8 @@ PyObject* py_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     BEGIN_BINDING
     expect_args(nargs, 9);
     const at::Tensor B = tensor_of(args[4], "B");
+    // the product runs on an address and the node has no jvp: a tangent of B would be dropped without a word
+    TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(B), "CsrMatrix @ B has no forward-mode derivative");
     Product q;
     q.rp = tensor_of(args[1], "A_row_ptr");
     q.ci = tensor_of(args[2], "A_col_idx");

@@ -50,6 +50,15 @@ def test_the_inplace_operator_marks_c_as_modified():
     lib._destroy()
 
 
+def test_a_tangent_of_b_is_refused_not_dropped():
+    import torch.autograd.forward_ad as fwAD
+    p = G.random_csr(7, 5, 4, 0.4, seed=2)
+    rp, ci, va, B = _t(p)
+    A = TL.CsrMatrix(rp, ci, va, (p.M, p.Kd))
+    with fwAD.dual_level(), pytest.raises(NotImplementedError, match="forward-mode"):
+        A @ fwAD.make_dual(B.requires_grad_(True), torch.ones_like(B))
+
+
 @pytest.mark.gpu
 def test_registered_ops_and_inplace_semantics(cuda_lib):
     p = G.random_csr(200, 150, 64, 0.05, seed=4)
