@@ -128,13 +128,32 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
+def build_fake_runtime() -> Path:
+    """tests/cpp/_bin/libfake_cuda_library.so: the library's objects linked with a stand-in for the CUDA runtime
+    (tests/cpp/fake_cudart.cpp), for tests of its host code without a GPU."""
+    lib = build()
+    src = ROOT / "tests" / "cpp" / "fake_cudart.cpp"
+    out = src.parent / "_bin" / "libfake_cuda_library.so"
+    if out.exists() and out.stat().st_mtime >= max(src.stat().st_mtime, lib.stat().st_mtime):
+        return out
+    out.parent.mkdir(exist_ok=True)
+    cuda = Path(nvcc()).resolve().parent.parent
+    objs = [str(OBJ / (s.relative_to(CSRC).as_posix().replace("/", "__") + ".o")) for s in sources()]
+    cmd = [shutil.which("g++") or "g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic,--no-undefined", f"-I{cuda / 'include'}",
+           "-o", str(out), str(src), *objs]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src}:\n{res.stdout}\n{res.stderr}")
+    return out
+
+
 def build_cpp_tests(verbose: bool = False) -> list[Path]:
     """Compile tests/cpp/*.cu against include/ and the library into tests/cpp/_bin/."""
     lib = build(verbose=verbose)
     src_dir = ROOT / "tests" / "cpp"
     out_dir = src_dir / "_bin"
     out_dir.mkdir(exist_ok=True)
-    outs = []
+    outs = [build_fake_runtime()]
     for src in sorted(src_dir.glob("*.cu")):
         exe = out_dir / src.stem
         outs.append(exe)

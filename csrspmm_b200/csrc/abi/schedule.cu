@@ -408,20 +408,7 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
     s->piece_nnz = piece;
     s->columns_sorted = 1;
 
-    unsigned* d_counters = nullptr;
-    int* d_rows = nullptr;
-    int* d_bounds = nullptr;
-    unsigned* d_slab = nullptr;
-    int4* d_long_rows = nullptr;
-    // temporaries come from the scratch pool: mapping and unmapping them by cudaMalloc and cudaFree made a build of
-    // 3 ms take 600 at times
-    auto release_temporaries = [&]() {
-        for (void* ptr : {static_cast<void*>(d_counters), static_cast<void*>(d_rows), static_cast<void*>(d_bounds),
-                          static_cast<void*>(d_slab), static_cast<void*>(d_long_rows)})
-            if (ptr != nullptr) scratch_free(ptr, st);
-    };
     auto fail = [&](int code) {
-        release_temporaries();
         if (s->pieces != nullptr) scratch_free(s->pieces, st);
         cudaStreamSynchronize(st);
         delete s;
@@ -437,13 +424,18 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
     } while (0)
 
     SCHED_TRY(cudaGetDevice(&s->device));
+    // temporaries come from the scratch pool: mapping and unmapping them by cudaMalloc and cudaFree made a build of
+    // 3 ms take 600 at times
+    Scratch counters(st), rows(st), bounds(st), slabs(st), long_rows(st);
     if (!pointless && !pointless_auto && a->M > 0 && a->nnz > 0) {
-        SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_counters), kSchedCounters * sizeof(unsigned), st));
+        SCHED_TRY(counters.alloc(kSchedCounters * sizeof(unsigned)));
+        unsigned* const d_counters = counters.as<unsigned>();
         SCHED_TRY(cudaMemsetAsync(d_counters, 0, kSchedCounters * sizeof(unsigned), st));
         // a row of `threshold` entries or more: at most nnz / threshold of them
         const long long cap_ll = a->nnz / threshold + 1;
         const int capacity = (int)(cap_ll < (long long)a->M ? cap_ll : (long long)a->M);
-        SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_rows), (size_t)capacity * sizeof(int), st));
+        SCHED_TRY(rows.alloc((size_t)capacity * sizeof(int)));
+        int* const d_rows = rows.as<int>();
         long long blocks = ((long long)a->M + 255) / 256;
         if (blocks > 148 * 16) blocks = 148 * 16;
         sched_list_long_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>(a->M, a->row_ptr, threshold, d_rows, capacity, d_counters);
@@ -459,11 +451,14 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
 
         if (num_long > 0) {
             const size_t bounds_bytes = (size_t)num_long * (size_t)(num_slabs + 1) * sizeof(int);
-            SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_bounds), bounds_bytes, st));
+            SCHED_TRY(bounds.alloc(bounds_bytes));
+            int* const d_bounds = bounds.as<int>();
             SCHED_TRY(cudaMemsetAsync(d_bounds, 0, bounds_bytes, st));
-            SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_slab), (size_t)num_slabs * 2 * sizeof(unsigned), st));
+            SCHED_TRY(slabs.alloc((size_t)num_slabs * 2 * sizeof(unsigned)));
+            unsigned* const d_slab = slabs.as<unsigned>();
             SCHED_TRY(cudaMemsetAsync(d_slab, 0, (size_t)num_slabs * 2 * sizeof(unsigned), st));
-            SCHED_TRY(scratch_alloc(reinterpret_cast<void**>(&d_long_rows), (size_t)num_long * sizeof(int4), st));
+            SCHED_TRY(long_rows.alloc((size_t)num_long * sizeof(int4)));
+            int4* const d_long_rows = long_rows.as<int4>();
             const int warps = 8;
             sched_cut_rows_kernel<<<(unsigned)((num_long + warps - 1) / warps), warps * 32, 0, st>>>(
                 (int)num_long, d_rows, a->row_ptr, a->col_idx, (int)a->nnz, slab_rows, num_slabs, piece, d_bounds, d_slab,
@@ -500,7 +495,6 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
                 s->device_bytes = (size_t)total * sizeof(int4) + (size_t)num_long * sizeof(int4);
             }
         }
-        release_temporaries();
         SCHED_TRY(cudaStreamSynchronize(st));
     }
 #undef SCHED_TRY
