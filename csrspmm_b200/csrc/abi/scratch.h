@@ -58,12 +58,20 @@ private:
     int index_ = -1;
 };
 
-// Up to kPinnedWords results of a call: kernels write ptr()[k], wait() waits for the stream and reads them.
+// Up to kPinnedWords results of a call: kernels write ptr()[k], wait() waits for the stream and reads them.  A call that
+// fails in between waits here all the same: a kernel that it did launch must not write to the slot of the next call.
 class Results {
 public:
     explicit Results(cudaStream_t st) : st_(st), dev_(st) {}
+    Results(const Results&) = delete;
+    Results& operator=(const Results&) = delete;
+    ~Results()
+    {
+        if (lent_) cudaStreamSynchronize(st_);
+    }
     cudaError_t init()
     {
+        lent_ = slot_.words() != nullptr;
         if (slot_.words() != nullptr) return cudaSuccess;
         return dev_.alloc(kPinnedWords * sizeof(long long));  // every slot taken: plain scratch, copied back
     }
@@ -75,6 +83,7 @@ public:
             return e != cudaSuccess ? e : cudaStreamSynchronize(st_);
         }
         const cudaError_t e = cudaStreamSynchronize(st_);
+        lent_ = e != cudaSuccess;
         for (int k = 0; k < count; ++k) out[k] = slot_.words()[k];
         return e;
     }
@@ -83,6 +92,7 @@ private:
     cudaStream_t st_;
     PinnedSlot slot_;
     Scratch dev_;
+    bool lent_ = false;  // kernels may be writing to the slot
 };
 
 }  // namespace csrspmm_b200

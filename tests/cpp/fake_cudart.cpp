@@ -14,6 +14,8 @@ namespace {
 std::mutex g_mutex;
 std::set<void*> g_live;           // allocations not freed yet
 std::map<void*, bool> g_busy;     // streams with work that nobody has waited for
+std::map<void*, void*> g_event;   // the stream an event was recorded on
+std::map<void*, std::set<void*>> g_after;  // the streams whose work a stream's work comes after
 long g_calls = 0, g_fail_at = 0;  // the call that fails, counted from 1; 0: none
 long g_bad_frees = 0;
 cudaError_t g_last = cudaSuccess;
@@ -83,6 +85,7 @@ void fake_reset(long fail_at)
     g_bad_frees = 0;
     g_last = cudaSuccess;
     g_busy.clear();
+    g_after.clear();
 }
 long fake_calls() { return g_calls; }
 long fake_live() { return (long)g_live.size(); }
@@ -174,6 +177,7 @@ cudaError_t cudaStreamSynchronize(cudaStream_t st)
     std::lock_guard<std::mutex> lock(g_mutex);
     if (const cudaError_t e = call()) return e;
     g_busy[st] = false;
+    for (void* before : g_after[st]) g_busy[before] = false;
     return cudaSuccess;
 }
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s)
@@ -195,8 +199,22 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
     return cudaSuccess;
 }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return simple(); }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return simple(); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t st)
+{
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (const cudaError_t f = call()) return f;
+    g_event[e] = st;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t e, unsigned)
+{
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (const cudaError_t f = call()) return f;
+    const std::set<void*> before = g_after[g_event[e]];
+    g_after[st].insert(before.begin(), before.end());
+    g_after[st].insert(g_event[e]);
+    return cudaSuccess;
+}
 
 // ---- kernels ---------------------------------------------------------------------------------------
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return simple(); }
