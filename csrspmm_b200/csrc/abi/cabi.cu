@@ -500,6 +500,7 @@ namespace csrspmm_b200 {
 
 cudaError_t launch_row_kernel(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st)
 {
+    if (plan.any_count) return launch_whole_rows(p, plan, e2m1, st);
     if (plan.resident == 32) return e2m1 ? launch_resident<32, kValuesE2M1>(p, st) : launch_resident<32, kValuesF32>(p, st);
     if (plan.resident == 16) return e2m1 ? launch_resident<16, kValuesE2M1>(p, st) : launch_resident<16, kValuesF32>(p, st);
     if (plan.VW == 4) return e2m1 ? dispatch_row<4, kValuesE2M1>(p, plan, st) : dispatch_row<4, kValuesF32>(p, plan, st);

@@ -25,6 +25,8 @@ cudaError_t launch_merge_kernel(const SpmmParams& p, const Plan& plan, bool e2m1
 cudaError_t launch_fixup_kernel(const SpmmParams& p, const Plan& plan, cudaStream_t st);
 // The whole-row kernel for a plan whose kernel is ROW.
 cudaError_t launch_row_kernel(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st);
+// The panel kernel in one pass over all columns (Plan::any_count): the same result.
+cudaError_t launch_whole_rows(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st);
 
 // A product under a schedule (args.schedule != NULL): schedule.cu.
 int enqueue_scheduled(const csrspmm_b200_args* a, cudaStream_t st);

@@ -192,7 +192,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
     const bool vec = vector_layout_ok(a);
     // rows that do not start on 16 bytes but on 8 (50 columns, say) go two floats at a time
     const bool padded = (flags & kPlanPadded) != 0;  // B is a copy with whole vectors, C stays as it is
-    const bool pairs = !vec && !padded && (flags & kPlanNoPairs) == 0 && pair_layout_ok(a);
+    const bool pairs = !vec && !padded && (flags & kPlanNoPairs) == 0 && a->nnz <= kWholeRowEntries && pair_layout_ok(a);
     plan->VW = vec || padded ? 4 : (pairs ? 2 : 1);
     plan->ncolv = (a->Nd + plan->VW - 1) / plan->VW;
     plan->c_ragged = padded;
@@ -272,7 +272,8 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         } else {
             const int groups = CSRSPMM_TUNE_ROW_THREADS / plan->G;
             plan->grid = ((long long)a->M + groups - 1) / groups;
-            plan->resident = (flags & kPlanNoPairs) == 0 && !padded ? resident_lanes(a, *plan) : 0;
+            plan->any_count = a->nnz > kWholeRowEntries;
+            plan->resident = (flags & kPlanNoPairs) == 0 && !padded && !plan->any_count ? resident_lanes(a, *plan) : 0;
             plan->short_rows = a->nnz <= (long long)CSRSPMM_TUNE_ROW_SHORT_MEAN * (long long)a->M;
             plan->low_occupancy = (long long)a->M * plan->G / 32 < 148LL * 8;
 #if CSRSPMM_TUNE_ROW_PERSISTENT > 0
@@ -299,7 +300,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
 
 size_t padded_b_bytes(const csrspmm_b200_args* a)
 {
-    if (a->Nd % 4 == 0 || a->Nd < 17 || a->M <= 0 || a->Kd <= 0 || a->kernel == CSRSPMM_B200_KERNEL_TMA) return 0;
+    if (a->Nd % 4 == 0 || a->Nd < 17 || a->M <= 0 || a->Kd <= 0 || a->kernel == CSRSPMM_B200_KERNEL_TMA || a->nnz > kWholeRowEntries) return 0;
     const double mean = (double)a->nnz / a->M, uses = (double)a->nnz / a->Kd;
     const double gather = (double)a->nnz * a->Nd * 4.0;
     const bool pays = a->Nd % 2 ? uses >= (a->Nd <= 256 ? 8.0 : 24.0) && gather >= 64e6 && (a->Nd >= 32 || mean <= 64.0)

@@ -17,6 +17,7 @@ struct Plan {
     int kernel = CSRSPMM_B200_KERNEL_ROW;  // resolved, never AUTO
     int shape = 0;                         // index into kShapes (tuning.h)
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
+    bool any_count = false;                // whole-row mapping of more than kWholeRowEntries entries: the panel kernel, one pass
     int resident = 0;                      // whole-row mapping by the resident kernel: lanes per group (16, 32), else 0
     bool c_ragged = false;                 // kPlanPadded: the last vector of a row of C is partly beyond it
     bool rows_even = false;                // AUTO: the longest row is known to be close to the mean
@@ -40,6 +41,10 @@ struct Plan {
     size_t dynamic_smem = 0;               // TMA kernel only: 8 warps x ring_stride
     size_t tma_slot_bytes = 0;             // TMA kernel only: one row of B rounded up to 128 bytes
 };
+
+// Entries up to which the row and resident kernels' int positions, which run up to 63 beyond the last one, do not wrap.  The
+// panel kernel counts in unsigned and gives the same result, so it takes the few sizes above.
+constexpr int64_t kWholeRowEntries = 0x7fffffffLL - 64;
 
 // Checks the argument block (sizes, enums, pointers) without touching memory.
 int check_args(const csrspmm_b200_args* a, bool need_pointers);

@@ -18,6 +18,7 @@
 
 #include "../kernels/panel_kernel.cuh"
 #include "csrspmm_b200.h"
+#include "launch.h"
 #include "plan.h"
 
 using namespace csrspmm_b200;
@@ -63,7 +64,32 @@ void dispatch_panel(const SpmmParams& p, const PanelPass& pp, const Plan& plan, 
     }
 }
 
+cudaError_t launch_pass(const SpmmParams& p, const PanelPass& pp, const Plan& plan, bool e2m1, cudaStream_t st)
+{
+    if (plan.VW == 4) {
+        if (e2m1) dispatch_panel<4, kValuesE2M1>(p, pp, plan, st);
+        else dispatch_panel<4, kValuesF32>(p, pp, plan, st);
+    } else {
+        if (e2m1) dispatch_panel<1, kValuesE2M1>(p, pp, plan, st);
+        else dispatch_panel<1, kValuesF32>(p, pp, plan, st);
+    }
+    return cudaGetLastError();
+}
+
 }  // namespace
+
+namespace csrspmm_b200 {
+
+cudaError_t launch_whole_rows(const SpmmParams& p, const Plan& plan, bool e2m1, cudaStream_t st)
+{
+    PanelPass pp;
+    std::memset(&pp, 0, sizeof(pp));
+    pp.first = pp.last = 1;
+    pp.col_limit = INT_MAX;
+    return launch_pass(p, pp, plan, e2m1, st);
+}
+
+}  // namespace csrspmm_b200
 
 extern "C" {
 
@@ -158,14 +184,7 @@ int csrspmm_b200_spmm_tiled(const csrspmm_b200_args* args, int32_t panel_rows, c
         pp.first = t == 0;
         pp.last = t == passes - 1;
         pp.col_limit = pp.last ? INT_MAX : (int)((t + 1) * panel_rows);
-        if (plan.VW == 4) {
-            if (e2m1) dispatch_panel<4, kValuesE2M1>(p, pp, plan, st);
-            else dispatch_panel<4, kValuesF32>(p, pp, plan, st);
-        } else {
-            if (e2m1) dispatch_panel<1, kValuesE2M1>(p, pp, plan, st);
-            else dispatch_panel<1, kValuesF32>(p, pp, plan, st);
-        }
-        err = cudaGetLastError();
+        err = launch_pass(p, pp, plan, e2m1, st);
     }
     if (owned) {
         cudaError_t ferr = cudaFreeAsync(ws, st);

@@ -86,7 +86,7 @@ __device__ __forceinline__ float decode_e2m1(unsigned code, float scale)
 }
 
 template <int FMT>
-__device__ __forceinline__ float load_value(const void* values, int j, float scale)
+__device__ __forceinline__ float load_value(const void* values, unsigned j, float scale)
 {
     if constexpr (FMT == kValuesF32) {
         return __ldcs(reinterpret_cast<const float*>(values) + j);

@@ -31,14 +31,14 @@ inline int convert_warps_per_row(int W)
 
 // This lane's 16 entries of the chunk that starts at column c0: quad k, element e is column
 //   c0 + 128k + 4*lane + e (VEC: rows start on 16 bytes)   or   c0 + 128k + 32e + lane (any alignment).
-// Columns at or beyond W read as 0 and are reported not kept.
+// Columns at or beyond W read as 0 and are reported not kept.  (Unsigned: a chunk can end beyond 2^31 - 1.)
 template <bool VEC>
-__device__ __forceinline__ void load_chunk(const float* __restrict__ src, int c0, int W, int lane, float (&v)[kChunkQuads][4])
+__device__ __forceinline__ void load_chunk(const float* __restrict__ src, unsigned c0, unsigned W, int lane, float (&v)[kChunkQuads][4])
 {
 #pragma unroll
     for (int k = 0; k < kChunkQuads; ++k) {
         if constexpr (VEC) {
-            const int c = c0 + 128 * k + 4 * lane;
+            const unsigned c = c0 + 128 * k + 4 * lane;
             if (c + 3 < W) {
                 const float4 q = __ldg(reinterpret_cast<const float4*>(src + c));
                 v[k][0] = q.x, v[k][1] = q.y, v[k][2] = q.z, v[k][3] = q.w;
@@ -49,7 +49,7 @@ __device__ __forceinline__ void load_chunk(const float* __restrict__ src, int c0
         } else {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int c = c0 + 128 * k + 32 * e + lane;
+                const unsigned c = c0 + 128 * k + 32 * e + lane;
                 v[k][e] = c < W ? __ldg(src + c) : 0.0f;
             }
         }
@@ -57,7 +57,7 @@ __device__ __forceinline__ void load_chunk(const float* __restrict__ src, int c0
 }
 
 template <bool VEC>
-__device__ __forceinline__ int chunk_column(int c0, int k, int e, int lane)
+__device__ __forceinline__ unsigned chunk_column(unsigned c0, int k, int e, int lane)
 {
     return VEC ? c0 + 128 * k + 4 * lane + e : c0 + 128 * k + 32 * e + lane;
 }
@@ -76,14 +76,14 @@ __global__ void __launch_bounds__(kConvertThreads) dense_count_kernel(int H, int
     int count = 0;
     if (row < H) {
         const float* src = dense + row * ld;
-        for (int c0 = (warp % wpr) * kChunkCols; c0 < W; c0 += wpr * kChunkCols) {
+        for (unsigned c0 = (warp % wpr) * kChunkCols; c0 < (unsigned)W; c0 += wpr * kChunkCols) {
             float v[kChunkQuads][4];
             load_chunk<VEC>(src, c0, W, lane, v);
 #pragma unroll
             for (int k = 0; k < kChunkQuads; ++k)
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    if (fabsf(v[k][e]) > tol && chunk_column<VEC>(c0, k, e, lane) < W) ++count;
+                    if (fabsf(v[k][e]) > tol && chunk_column<VEC>(c0, k, e, lane) < (unsigned)W) ++count;
         }
     }
     count = __reduce_add_sync(0xffffffffu, count);
@@ -115,18 +115,18 @@ __global__ void __launch_bounds__(kConvertThreads) dense_fill_kernel(int H, int 
     const float* src = dense + (live ? row : 0) * ld;
     int base = live ? row_ptr[row] : 0;  // where the current round of chunks starts in the output
     int round = 0;
-    for (int r0 = 0; r0 < W; r0 += wpr * kChunkCols, round ^= 1) {
-        const int c0 = r0 + (warp % wpr) * kChunkCols;
+    for (unsigned r0 = 0; r0 < (unsigned)W; r0 += wpr * kChunkCols, round ^= 1) {
+        const unsigned c0 = r0 + (warp % wpr) * kChunkCols;
         float v[kChunkQuads][4];
         unsigned kept[kChunkQuads][4];
         int count = 0;
-        if (live && c0 < W) {
+        if (live && c0 < (unsigned)W) {
             load_chunk<VEC>(src, c0, W, lane, v);
 #pragma unroll
             for (int k = 0; k < kChunkQuads; ++k)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    kept[k][e] = __ballot_sync(0xffffffffu, fabsf(v[k][e]) > tol && chunk_column<VEC>(c0, k, e, lane) < W);
+                    kept[k][e] = __ballot_sync(0xffffffffu, fabsf(v[k][e]) > tol && chunk_column<VEC>(c0, k, e, lane) < (unsigned)W);
                     count += __popc(kept[k][e]);
                 }
         }
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kConvertThreads) dense_fill_kernel(int H, int 
         } else {
             base += count;
         }
-        if (live && c0 < W) {
+        if (live && c0 < (unsigned)W) {
             const unsigned below = (1u << lane) - 1u;
 #pragma unroll
             for (int k = 0; k < kChunkQuads; ++k) {
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kConvertThreads) dense_fill_kernel(int H, int 
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         if ((kept[k][e] >> lane) & 1u) {
-                            col_idx[mine] = chunk_column<VEC>(c0, k, e, lane);
+                            col_idx[mine] = (int)chunk_column<VEC>(c0, k, e, lane);
                             values[mine] = v[k][e];
                             ++mine;
                         }
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kConvertThreads) dense_fill_kernel(int H, int 
                     for (int e = 0; e < 4; ++e) {
                         if ((kept[k][e] >> lane) & 1u) {
                             const int mine = at + __popc(kept[k][e] & below);
-                            col_idx[mine] = chunk_column<VEC>(c0, k, e, lane);
+                            col_idx[mine] = (int)chunk_column<VEC>(c0, k, e, lane);
                             values[mine] = v[k][e];
                         }
                         at += __popc(kept[k][e]);
@@ -184,9 +184,9 @@ __global__ void csr_scatter_kernel(int H, int W, const int* __restrict__ row_ptr
     if (row >= H) return;
     float* dst = dense + row * ld;
     // a repeated column index keeps the last stored value, like the sequential host loop
-    const int rs = row_ptr[row], re = row_ptr[row + 1];
-    for (int j0 = rs; j0 < re; j0 += 32) {
-        const int j = j0 + lane;
+    const unsigned rs = (unsigned)max(row_ptr[row], 0), re = (unsigned)max(row_ptr[row + 1], 0);
+    for (unsigned j0 = rs; j0 < re; j0 += 32) {
+        const unsigned j = j0 + lane;
         const int c = j < re ? col_idx[j] : -1;
         const float v = j < re ? values[j] : 0.0f;
         // later lanes win over earlier ones with the same column

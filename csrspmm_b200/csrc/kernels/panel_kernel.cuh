@@ -52,13 +52,13 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_panel_kernel(const Spm
     const long long group_stride = (long long)gridDim.x * GROUPS;
     for (long long row_ll = (long long)blockIdx.x * GROUPS + (threadIdx.x / G); row_ll < p.M; row_ll += group_stride) {
         const int row = (int)row_ll;
-        // clamped so that a malformed row_ptr or cursor cannot index outside col_idx/values
-        const int row_lo = max(__ldg(p.row_ptr + row) - p.rp_base, 0);
-        const int re = min(__ldg(p.row_ptr + row + 1) - p.rp_base, p.nnz);
-        int rs = row_lo;
-        if (!pp.first) rs = max(pp.cursor[row], row_lo);
+        // clamped so that a malformed row_ptr or cursor cannot index outside col_idx/values; unsigned, so that a position a
+        // chunk beyond the last entry is representable whatever their number
+        unsigned rs = max(__ldg(p.row_ptr + row) - p.rp_base, 0);
+        const unsigned re = min((unsigned)max(__ldg(p.row_ptr + row + 1) - p.rp_base, 0), (unsigned)p.nnz);
+        if (!pp.first) rs = max((unsigned)pp.cursor[row], rs);
 
-        auto load_pair = [&](int jj, int& c, float& a) {
+        auto load_pair = [&](unsigned jj, int& c, float& a) {
             c = 0;
             a = 0.f;
             if (jj < re) {
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_panel_kernel(const Spm
             }
         };
         // how many entries at the head of the chunk that starts at `base` belong to this pass
-        auto leading = [&](int base, int c) -> int {
+        auto leading = [&](unsigned base, int c) -> int {
             const bool mine = (base + lane < re) && (c < pp.col_limit);
             const unsigned stop = ~tile.ballot(mine) & kGroupMask;
             return stop ? (__ffs(stop) - 1) : G;
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_panel_kernel(const Spm
         const int n_first = leading(rs, c_first);
         if (n_first == 0 && !pp.first && !pp.last) continue;  // nothing of this row in the panel
 
-        int end = rs;
+        unsigned end = rs;
         for (int cb = 0; cb < p.ncolv; cb += G * NV) {
             const char* const b_pass = b_lane + (size_t)cb * (VW * 4);
             bool col_ok[NV];
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_panel_kernel(const Spm
                 }
             };
 
-            int base = rs;
+            unsigned base = rs;
             int c_cur = c_first;
             float a_cur = a_first;
             int n = n_first;  // a further column pass walks the same entries again
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_panel_kernel(const Spm
                         acc[v].store(pp.partial + (long long)row * pp.ldp + (long long)(cb + lane + v * G) * VW);
             }
         }
-        if (!pp.last && lane == 0) pp.cursor[row] = end;
+        if (!pp.last && lane == 0) pp.cursor[row] = (int)end;
     }
 }
 

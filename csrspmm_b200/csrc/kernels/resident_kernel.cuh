@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) spmm_resident_kernel(cons
 
         // ---- the group's rows: row0 + g, + GROUPS, ... ------------------------------------------
         int row = row0 + g;
-        auto bounds = [&](int r, int& first, int& last) {  // clamped so that a malformed row_ptr stays inside the arrays
+        // clamped so that a malformed row_ptr stays inside the arrays; at most kWholeRowEntries, as in the row kernel
+        auto bounds = [&](int r, int& first, int& last) {
             first = last = 0;
             if (r < row1) {
                 first = max(__ldg(p.row_ptr + r) - p.rp_base, 0);

@@ -37,7 +37,9 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_row_kernel(const SpmmP
     for (long long row_ll = (long long)blockIdx.x * GROUPS + (threadIdx.x / G); row_ll < p.M; row_ll += group_stride) {
     const int row = (int)row_ll;
 
-    // clamped so that a malformed row_ptr cannot index outside col_idx/values
+    // clamped so that a malformed row_ptr cannot index outside col_idx/values; at most kWholeRowEntries, so that a position
+    // a chunk beyond the last entry fits an int (the same loop in unsigned arithmetic: 12.0 -> 12.15 us for 16 384 rows of 16,
+    // 128 columns)
     const int rs = max(__ldg(p.row_ptr + row) - p.rp_base, 0);
     const int re = min(__ldg(p.row_ptr + row + 1) - p.rp_base, p.nnz);
     const char* const b_lane = reinterpret_cast<const char*>(p.B) + (size_t)lane * (VW * 4);

@@ -119,18 +119,18 @@ __global__ void __launch_bounds__(kSlicedThreads, MINB) spmm_sliced_kernel(const
         for (int k = 0; k < ppg; ++k) {
             if (it0 + k >= run_last) break;
             const int4 d = __ldg(q.pieces + it0 + k);
-            const int rs = min(max(d.x, 0), p.nnz);
-            const int re = min(max(d.y, rs), min(p.nnz, rs + q.piece_cap));
+            const unsigned rs = (unsigned)min(max(d.x, 0), p.nnz);
+            const unsigned re = min(max((unsigned)max(d.y, 0), rs), min((unsigned)p.nnz, rs + q.piece_cap));
             if (lane == 0) {
                 off[k] = total;
                 slot_of[k] = d.z;
             }
-            for (int j0 = rs + lane; j0 < re; j0 += G * SB) {  // SB loads in flight per lane, then the stores
+            for (unsigned j0 = rs + lane; j0 < re; j0 += G * SB) {  // SB loads in flight per lane, then the stores
                 int c[SB];
                 float a[SB];
 #pragma unroll
                 for (int b = 0; b < SB; ++b) {
-                    const int j = j0 + b * G;
+                    const unsigned j = j0 + b * G;
                     if (j < re) {
                         c[b] = __ldcs(p.col_idx + j);
                         a[b] = load_value<FMT>(p.values, j, p.value_scale);
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kSlicedThreads, MINB) spmm_sliced_kernel(const
                 }
 #pragma unroll
                 for (int b = 0; b < SB; ++b) {
-                    const int j = j0 + b * G;
+                    const unsigned j = j0 + b * G;
                     if (j < re) {
                         if ((unsigned)c[b] >= (unsigned)p.Kd) {  // never fault on a bad index
                             c[b] = min(max(c[b], 0), p.Kd - 1);
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kSlicedThreads, MINB) spmm_sliced_kernel(const
                     }
                 }
             }
-            total += re - rs;
+            total += (int)(re - rs);
             ++np;
         }
         if (lane == 0) off[np] = total;
@@ -341,12 +341,12 @@ __global__ void sched_cut_rows_kernel(int num_long, const int* __restrict__ long
     const int lane = threadIdx.x & 31;
     if (h >= num_long) return;
     const int row = __ldg(long_rows + h);
-    const int rs = min(max(__ldg(row_ptr + row), 0), nnz);
-    const int re = min(max(__ldg(row_ptr + row + 1), rs), nnz);
+    const unsigned rs = (unsigned)min(max(__ldg(row_ptr + row), 0), nnz);
+    const unsigned re = max((unsigned)min(max(__ldg(row_ptr + row + 1), 0), nnz), rs);
     int* b = bounds + (long long)h * (num_slabs + 1);
     bool unsorted = false;
     // entry j starts every slab in (slab(j-1), slab(j)]; the first entry also starts slabs 0..slab(rs)
-    for (int j = rs + lane; j < re; j += 32) {
+    for (unsigned j = rs + lane; j < re; j += 32) {
         const int c = __ldg(col_idx + j);
         const int sj = min(max(c, 0) / slab_rows, num_slabs - 1);
         int sp = -1;
@@ -355,12 +355,12 @@ __global__ void sched_cut_rows_kernel(int num_long, const int* __restrict__ long
             if (cp >= c) unsorted = true;
             sp = min(max(cp, 0) / slab_rows, num_slabs - 1);
         }
-        for (int s = sp + 1; s <= sj; ++s) b[s] = j;
+        for (int s = sp + 1; s <= sj; ++s) b[s] = (int)j;
     }
     // slabs after the last entry's are empty
     int s_last = -1;
     if (re > rs) s_last = min(max(__ldg(col_idx + re - 1), 0) / slab_rows, num_slabs - 1);
-    for (int s = s_last + 1 + lane; s <= num_slabs; s += 32) b[s] = re;
+    for (int s = s_last + 1 + lane; s <= num_slabs; s += 32) b[s] = (int)re;
     if (__any_sync(0xffffffffu, unsorted)) {
         if (lane == 0) atomicOr(counters + 4, 1u);
     }
@@ -371,7 +371,7 @@ __global__ void sched_cut_rows_kernel(int num_long, const int* __restrict__ long
     for (int s = lane; s < num_slabs; s += 32) {
         const int len = b[s + 1] - b[s];
         if (len > 0) {
-            const int cnt = (len + piece_nnz - 1) / piece_nnz;
+            const int cnt = (len - 1) / piece_nnz + 1;
             atomicAdd(slab_count + s, (unsigned)cnt);
             mine += cnt;
         }
@@ -396,12 +396,12 @@ __global__ void sched_emit_pieces_kernel(int num_long, int num_slabs, int piece_
     for (int s = 0; s < num_slabs; ++s) {
         const int lo = b[s], len = b[s + 1] - lo;
         if (len <= 0) continue;
-        const int cnt = (len + piece_nnz - 1) / piece_nnz;
-        const int each = (len + cnt - 1) / cnt;  // equal pieces rather than full ones and a stub
+        const int cnt = (len - 1) / piece_nnz + 1;
+        const int each = (len - 1) / cnt + 1;  // equal pieces rather than full ones and a stub
         const unsigned pos = atomicAdd(slab_fill + s, (unsigned)cnt);
         for (int k = 0; k < cnt; ++k) {
-            const int a = lo + k * each;
-            const int e = min(a + each, lo + len);
+            const int at = min(k * each, len), a = lo + at;
+            const int e = a + min(each, len - at);
             if (pos + k < (unsigned)num_pieces) pieces[pos + k] = make_int4(a, e, slot, s);
             ++slot;
         }
