@@ -38,7 +38,7 @@ EXPORTED_SYMBOLS = (
     "csrspmm_b200_abi_version", "csrspmm_b200_status_string", "csrspmm_b200_last_error",
     "csrspmm_b200_spmm", "csrspmm_b200_spmm_sync", "csrspmm_b200_spmm_host", "csrspmm_b200_spmm_noalloc",
     "csrspmm_b200_host_arena_bytes", "csrspmm_b200_workspace_bytes", "csrspmm_b200_uses_workspace", "csrspmm_b200_select_kernel",
-    "csrspmm_b200_plan_info_get",
+    "csrspmm_b200_plan_info_get", "csrspmm_b200_release_memory",
     "csrspmm_b200_validate_csr_host", "csrspmm_b200_validate_csr_device",
     "csrspmm_b200_row_stats_device", "csrspmm_b200_partition_rows", "csrspmm_b200_e2m1_scale",
     "csrspmm_b200_e2m1_encode", "csrspmm_b200_e2m1_decode", "csrspmm_b200_dense2csr_count",
@@ -161,6 +161,8 @@ def lib() -> C.CDLL:
     L.csrspmm_b200_uses_workspace.restype = C.c_int
     L.csrspmm_b200_select_kernel.argtypes = [C.POINTER(Args)]
     L.csrspmm_b200_select_kernel.restype = C.c_int
+    L.csrspmm_b200_release_memory.argtypes = [C.POINTER(C.c_size_t)]
+    L.csrspmm_b200_release_memory.restype = C.c_int
     L.csrspmm_b200_plan_info_get.argtypes = [C.POINTER(Args), C.POINTER(PlanInfo)]
     L.csrspmm_b200_plan_info_get.restype = C.c_int
     L.csrspmm_b200_validate_csr_host.argtypes = [C.c_int32, C.c_int32, C.c_int64, C.c_void_p, C.c_void_p,

@@ -11,7 +11,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
-#include <vector>
+#include <utility>
 
 #include "../kernels/aux_kernels.cuh"
 #include "../kernels/merge_kernel.cuh"
@@ -323,32 +323,34 @@ int column_panel_layout(int32_t Kd, int32_t Nd, int requested, int32_t* first, i
 }
 
 // Two streams and the events of one host round trip.  Making and destroying them took 60 to 100 us of every call; up to
-// kPipesKept sets per device wait for the next call instead (what is above is destroyed at once).
+// kPipesKept sets per device wait for the next call instead (what is above is destroyed at once), until
+// csrspmm_b200_release_memory.
 class HostPipe {
 public:
     static constexpr int kEvents = 2 * kMaxPanels;
     ~HostPipe()
     {
         if (set_ == nullptr) return;
-        std::lock_guard<std::mutex> lock(mutex());
-        auto& kept = pool();
-        int same = 0;
-        for (const Set* k : kept) same += k->device == set_->device;
-        if (same < kPipesKept) kept.push_back(set_);
-        else destroy(set_);
+        if (set_->device >= 0 && set_->device < kMaxDevices) {
+            std::lock_guard<std::mutex> lock(mutex_);
+            for (Set*& slot : kept_[set_->device])
+                if (slot == nullptr) {
+                    slot = set_;
+                    return;
+                }
+        }
+        destroy(set_);
     }
     cudaError_t init()
     {
         int device = -1;
         cudaError_t e = cudaGetDevice(&device);
         if (e != cudaSuccess) return e;
-        {
-            std::lock_guard<std::mutex> lock(mutex());
-            auto& kept = pool();
-            for (size_t k = 0; k < kept.size(); ++k)
-                if (kept[k]->device == device) {
-                    set_ = kept[k];
-                    kept.erase(kept.begin() + (long)k);
+        if (device >= 0 && device < kMaxDevices) {
+            std::lock_guard<std::mutex> lock(mutex_);
+            for (Set*& slot : kept_[device])
+                if (slot != nullptr) {
+                    std::swap(set_, slot);
                     return cudaSuccess;
                 }
         }
@@ -365,13 +367,20 @@ public:
         set_ = s;
         return cudaSuccess;
     }
+    static void release()
+    {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (auto& device : kept_)
+            for (Set*& slot : device)
+                if (slot != nullptr) destroy(std::exchange(slot, nullptr));
+    }
     cudaStream_t compute() const { return set_->compute; }
     cudaStream_t out() const { return set_->out; }
     cudaEvent_t up(int k) const { return set_->event[k]; }
     cudaEvent_t done(int k) const { return set_->event[kMaxPanels + k]; }
 
 private:
-    static constexpr int kPipesKept = 2;
+    static constexpr int kPipesKept = 2, kMaxDevices = 64;
     struct Set {
         int device = -1;
         cudaStream_t compute = nullptr, out = nullptr;
@@ -385,16 +394,8 @@ private:
         if (s->out) cudaStreamDestroy(s->out);
         delete s;
     }
-    static std::mutex& mutex()
-    {
-        static std::mutex m;
-        return m;
-    }
-    static std::vector<Set*>& pool()
-    {
-        static std::vector<Set*>* kept = new std::vector<Set*>();  // not destroyed: CUDA may be gone by then
-        return *kept;
-    }
+    static inline std::mutex mutex_;
+    static inline Set* kept_[kMaxDevices][kPipesKept] = {};  // not destroyed at exit: CUDA may be gone by then
     Set* set_ = nullptr;
 };
 
@@ -833,6 +834,17 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
     }
     return CSRSPMM_B200_OK;
 #undef CUDA_TRY_HOST
+}
+
+int csrspmm_b200_release_memory(size_t* bytes)
+{
+    HostPipe::release();
+    const cudaError_t e = scratch_release(bytes);
+    if (e != cudaSuccess) {
+        set_last_error("release_memory: %s", cudaGetErrorString(e));
+        return CSRSPMM_B200_ERR_CUDA;
+    }
+    return CSRSPMM_B200_OK;
 }
 
 int csrspmm_b200_column_panels(int32_t Kd, int32_t Nd, int requested, int32_t* first_col, int32_t* width)

@@ -59,6 +59,22 @@ cudaError_t product_scratch_alloc(void** ptr, size_t bytes, cudaStream_t st)
     return capture == cudaStreamCaptureStatusNone ? scratch_alloc(ptr, bytes, st) : cudaMallocAsync(ptr, bytes, st);
 }
 
+cudaError_t scratch_release(size_t* bytes)
+{
+    if (bytes) *bytes = 0;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    for (cudaMemPool_t pool : g_pool) {
+        if (pool == nullptr) continue;
+        unsigned long long before = 0, after = 0;
+        cudaError_t e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &before);
+        if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
+        if (e == cudaSuccess) e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &after);
+        if (e != cudaSuccess) return e;
+        if (bytes) *bytes += (size_t)(before - after);
+    }
+    return cudaSuccess;
+}
+
 PinnedSlot::PinnedSlot()
 {
     std::lock_guard<std::mutex> lock(g_mutex);

@@ -11,12 +11,14 @@ namespace csrspmm_b200 {
 // Stream-ordered device scratch out of the library's own pool on the current device.  The default pool hands
 // everything back to the driver at each synchronisation, and mapping memory anew made a call that
 // waits for its result (row statistics, dense -> CSR, quantisation) cost 0.3 to 2 ms; this pool keeps up to
-// kScratchKept bytes per device for the next call (and what is above goes back as it does there).
+// kScratchKept bytes per device for the next call (and what is above goes back as it does there), until scratch_release.
 constexpr size_t kScratchKept = (size_t)64 << 20;
 cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t st);
 // The same for scratch of a product, which may be under stream capture: there it comes from cudaMallocAsync (a
 // graph owns its allocations, and making a pool is no call for a capture).
 cudaError_t product_scratch_alloc(void** ptr, size_t bytes, cudaStream_t st);
+// Gives back what the pools keep and nobody uses, on all devices; *bytes (may be null): how much that was.
+cudaError_t scratch_release(size_t* bytes);
 inline cudaError_t scratch_free(void* ptr, cudaStream_t st) { return cudaFreeAsync(ptr, st); }
 
 // Scratch that goes back to the pool when the scope ends, in stream order.

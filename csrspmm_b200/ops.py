@@ -308,6 +308,14 @@ def e2m1_dequantize(packed, n, scale):
     return torch.from_numpy(out)
 
 
+def release_memory() -> int:
+    """Gives back the device memory (up to 64 MiB per device) and streams that the library keeps between calls, as
+    ``torch.cuda.empty_cache`` does for torch's; returns the bytes."""
+    n = C.c_size_t(0)
+    _lib.check(_lib.lib().csrspmm_b200_release_memory(C.byref(n)), "csrspmm_b200_release_memory")
+    return int(n.value)
+
+
 def validate_csr(row_ptr, col_idx, Kd: int) -> int:
     """Checks a CSR structure (host or CUDA int32 tensors); returns the problem bits and raises
     SpmmError(ERR_INVALID_CSR) when the matrix cannot be multiplied safely."""

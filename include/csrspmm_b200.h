@@ -143,6 +143,11 @@ int csrspmm_b200_spmm_sync(const csrspmm_b200_args* args, csrspmm_b200_stream_t 
  * C is the same sequential sum as in one unsplit product. */
 int csrspmm_b200_spmm_host(const csrspmm_b200_args* args, void* device_arena,
                            size_t device_arena_bytes, csrspmm_b200_stream_t stream);
+
+/* The library keeps up to 64 MiB of device memory per device between calls (scratch of conversions, statistics,
+ * schedules' builds, products without a workspace) and the streams of two host round trips.  This gives them back: what
+ * no call is using, on all devices; later calls take them anew.  *bytes (may be NULL): the device memory given back. */
+int csrspmm_b200_release_memory(size_t* bytes);
 size_t csrspmm_b200_host_arena_bytes(const csrspmm_b200_args* args);
 
 /* No counterpart in the reference.  The column panels csrspmm_b200_spmm_host cuts a product of

@@ -3,6 +3,7 @@
 // (csrspmm_b200/build.py), so that every way out of a failed call can be walked through on the CPU.
 #include <cuda_runtime_api.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -18,6 +19,7 @@ std::map<void*, void*> g_event;   // the stream an event was recorded on
 std::map<void*, std::set<void*>> g_after;  // the streams whose work a stream's work comes after
 long g_calls = 0, g_fail_at = 0;  // the call that fails, counted from 1; 0: none
 long g_bad_frees = 0;
+std::atomic<long> g_streams{0};  // made and not destroyed
 cudaError_t g_last = cudaSuccess;
 char g_handles[4096];
 size_t g_next_handle = 0;
@@ -89,6 +91,7 @@ void fake_reset(long fail_at)
 }
 long fake_calls() { return g_calls; }
 long fake_live() { return (long)g_live.size(); }
+long fake_streams() { return g_streams; }
 long fake_bad_frees() { return g_bad_frees; }
 long fake_busy()
 {
@@ -114,6 +117,12 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* pool, const cudaMemPoolProps*)
     return cudaSuccess;
 }
 cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return simple(); }
+cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v)
+{
+    *static_cast<unsigned long long*>(v) = 0;
+    return simple();
+}
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t st)
 {
@@ -189,9 +198,14 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* st, unsigned)
 {
     if (const cudaError_t e = simple()) return e;
     new_handle(st);
+    ++g_streams;
     return cudaSuccess;
 }
-cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t)
+{
+    --g_streams;
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
 {
     if (const cudaError_t f = simple()) return f;

@@ -11,7 +11,7 @@ from csrspmm_b200 import _lib, build
 @pytest.fixture(scope="module")
 def fake():
     L = C.CDLL(str(build.build_fake_runtime()))
-    for name in ("fake_calls", "fake_live", "fake_bad_frees", "fake_busy"):
+    for name in ("fake_calls", "fake_live", "fake_bad_frees", "fake_busy", "fake_streams"):
         getattr(L, name).restype = C.c_long
     L.fake_reset.argtypes = [C.c_long]
     return L
@@ -124,3 +124,22 @@ def test_one_failed_call(fake, name):
         assert fake.fake_bad_frees() == 0, f"call {k} of {calls} fails: something is freed twice"
         assert fake.fake_live() == live, f"call {k} of {calls} fails: something is not freed"
         assert name not in LENDING or fake.fake_busy() == 0, f"call {k} of {calls} fails: work is still running"
+
+
+def test_kept_streams_are_bounded_and_given_back(fake):
+    import threading
+    fake.fake_reset(0)
+    assert fake.csrspmm_b200_release_memory(None) == 0 and fake.fake_streams() == 0
+    start = threading.Barrier(6)
+
+    def work():
+        keep = {}
+        start.wait()
+        for _ in range(3):
+            assert _host_blocks(fake, keep) == 0
+
+    threads = [threading.Thread(target=work) for _ in range(6)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert 2 <= fake.fake_streams() <= 4  # two sets of two
+    assert fake.csrspmm_b200_release_memory(None) == 0 and fake.fake_streams() == 0

@@ -30,3 +30,13 @@ def test_quantize_equals_the_host_codec(cuda_lib, n, offset):
     packed, scale = ops.e2m1_quantize(torch.from_numpy(v).cuda()[offset:])
     want, want_scale = ops.e2m1_quantize(torch.from_numpy(v[offset:].copy()))
     assert scale == want_scale and torch.equal(packed.cpu(), want)
+
+
+def test_kept_memory_is_given_back(cuda_lib):
+    dense = torch.ones(3_000_000, 2, device="cuda")  # its row counts: some 12 MB of scratch
+    ops.dense2csr(dense)
+    torch.cuda.synchronize()
+    assert ops.release_memory() >= 12_000_000
+    assert ops.release_memory() == 0
+    rp, _, _, longest = ops.dense2csr(dense)  # and calls go on
+    assert int(rp[-1]) == 6_000_000 and longest == 2
