@@ -108,40 +108,22 @@ cudaError_t launch_row(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 template <int NV, int FMT>
 cudaError_t launch_tma(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
-    auto kern = spmm_tma_kernel<NV, CSRSPMM_TUNE_TMA_TG, CSRSPMM_TUNE_TMA_SLOTS, FMT>;
-    // The opt-in to more than 48 KB of dynamic shared memory is made once per device and
-    // instantiation, for the largest ring the kernel can ask for (rows of 2 KB), so that later
-    // calls -- inside a stream capture too -- are a plain launch.  Racing first calls repeat the
-    // same setting.
+    constexpr auto kern = spmm_tma_kernel<NV, CSRSPMM_TUNE_TMA_TG, CSRSPMM_TUNE_TMA_SLOTS, FMT>;
+    // asked for the largest ring a build takes (rows of 2 KB) at once
     constexpr int kMaxRing = (CSRSPMM_TUNE_MERGE_THREADS / 32) * (CSRSPMM_TUNE_TMA_SLOTS * 2048 > 512 * NV ? CSRSPMM_TUNE_TMA_SLOTS * 2048 : 512 * NV);
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = allow_dynamic_smem<kern>(plan.dynamic_smem > (size_t)kMaxRing ? plan.dynamic_smem : (size_t)kMaxRing);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !configured[dev] || (int)plan.dynamic_smem > kMaxRing) {
-        const int want = (int)plan.dynamic_smem > kMaxRing ? (int)plan.dynamic_smem : kMaxRing;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
     return launch_overlapped(kern, (unsigned)plan.grid, kMergeThreads, plan.dynamic_smem, st, p, (unsigned)plan.tma_slot_bytes,
                              (unsigned)(plan.dynamic_smem / (CSRSPMM_TUNE_MERGE_THREADS / 32)));
 }
 
-// One CTA per SM; the opt-in to its shared memory is made once per device and build, as for the bulk-copy kernel.
+// One CTA per SM.
 template <int G, int FMT>
 cudaError_t launch_resident(const SpmmParams& p, cudaStream_t st)
 {
-    auto kern = spmm_resident_kernel<G, FMT>;
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    constexpr auto kern = spmm_resident_kernel<G, FMT>;
+    const cudaError_t e = allow_dynamic_smem<kern>(resident_smem_bytes<G>(kResidentPanelBytes / (G * 16)));
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_smem_bytes<G>(kResidentPanelBytes / (G * 16)));
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
     const long long total = (long long)((p.ncolv + G - 1) / G) * p.M;
     const unsigned grid = (unsigned)(total < 148 ? total : 148);
     return launch_overlapped(kern, grid, kResidentThreads, (size_t)resident_smem_bytes<G>(p.Kd), st, p, total);

@@ -22,6 +22,7 @@
 #include "../kernels/sliced_kernel.cuh"
 #include "csrspmm_b200.h"
 #include "launch.h"
+#include "pdl.h"
 #include "plan.h"
 #include "scratch.h"
 
@@ -105,35 +106,14 @@ bool env_forces_other_kernel()
 
 // ---- kernel dispatch --------------------------------------------------------------------------------
 
-template <class K>
-cudaError_t allow_dynamic_smem(K kern, size_t bytes, bool (&configured)[64], size_t (&granted)[64])
-{
-    // the opt-in to more than 48 KB of dynamic shared memory is per device and instantiation;
-    // repeated with a larger size when a later call needs more
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !configured[dev] || granted[dev] < bytes) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) {
-            configured[dev] = true;
-            granted[dev] = bytes;
-        }
-    }
-    return cudaSuccess;
-}
-
 template <int S, int VW, int FMT, bool FULL>
 cudaError_t launch_sliced_one(const SpmmParams& p, const SlicedParams& q, unsigned grid, cudaStream_t st)
 {
     constexpr int G = kPieceShapes[S].G, NV = kPieceShapes[S].NV;
     constexpr int D = VW == 1 ? 16 : kPieceShapes[S].D;
-    auto kern = spmm_sliced_kernel<G, NV, VW, D, FMT, FULL, CSRSPMM_TUNE_SLICED_MINB>;
+    constexpr auto kern = spmm_sliced_kernel<G, NV, VW, D, FMT, FULL, CSRSPMM_TUNE_SLICED_MINB>;
     const size_t smem = sliced_smem_bytes(G, NV, VW, D, q.pieces_per_group, q.piece_cap);
-    static bool configured[64] = {};
-    static size_t granted[64] = {};
-    cudaError_t e = allow_dynamic_smem(kern, smem, configured, granted);
+    const cudaError_t e = allow_dynamic_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     kern<<<grid, kSlicedThreads, smem, st>>>(p, q);
     return cudaGetLastError();

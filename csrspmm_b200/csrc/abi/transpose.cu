@@ -71,7 +71,6 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
     auto ints = [&](size_t off) { return reinterpret_cast<int*>(ws + off); };
     auto pairs = [&](size_t off) { return reinterpret_cast<int2*>(ws + off); };
     long long* results = reinterpret_cast<long long*>(ws + p.results);
-    const int smem = (int)sizeof(ScatterSmem<ITEMS>);
     for (int k = 0; k < p.passes; ++k) {
         const DigitPass ps = {k * p.digit_bits, p.digit_bits, 1 << p.digit_bits, p.tiles, nnz};
         const bool first = k == 0, last = k == p.passes - 1;
@@ -84,19 +83,16 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
                                           kTransposeThreads, 0, st, ps, keys, Kd, ints(p.counts));
         if (e == cudaSuccess && !self) e = exclusive_scan(ints(p.counts), p.counters, ints(p.offsets), ws + p.scan, results, st);
         if (e != cudaSuccess) return e;
-        auto scatter = [&](auto kernel) {
-            // (racing first calls repeat the same setting)
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        auto scatter = [&](auto first_c, auto last_c, auto self_c) {
+            constexpr auto kernel = transpose_scatter_kernel<ITEMS, decltype(first_c)::value, decltype(last_c)::value, decltype(self_c)::value>;
+            const cudaError_t e = allow_dynamic_smem<kernel>(sizeof(ScatterSmem<ITEMS>));
             if (e != cudaSuccess) return e;
-            return launch_overlapped(kernel, (unsigned)p.tiles, kTransposeThreads, (size_t)smem, st, ps, keys, in, row_ptr, M, Kd, values,
-                                     ints(self ? p.counts : p.offsets), out_keys, out, t_col_idx, t_values);
-        };
-        auto pick = [&](auto first_c, auto last_c) {
-            constexpr bool F = decltype(first_c)::value, L = decltype(last_c)::value;
-            return self ? scatter(transpose_scatter_kernel<ITEMS, F, L, true>) : scatter(transpose_scatter_kernel<ITEMS, F, L, false>);
+            return launch_overlapped(kernel, (unsigned)p.tiles, kTransposeThreads, sizeof(ScatterSmem<ITEMS>), st, ps, keys, in, row_ptr, M, Kd,
+                                     values, ints(self ? p.counts : p.offsets), out_keys, out, t_col_idx, t_values);
         };
         using T = std::true_type;
         using F = std::false_type;
+        auto pick = [&](auto first_c, auto last_c) { return self ? scatter(first_c, last_c, T()) : scatter(first_c, last_c, F()); };
         e = first && last ? pick(T(), T()) : first ? pick(T(), F()) : last ? pick(F(), T()) : pick(F(), F());
         if (e != cudaSuccess) return e;
     }

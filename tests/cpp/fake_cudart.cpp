@@ -19,6 +19,9 @@ std::map<void*, void*> g_event;   // the stream an event was recorded on
 std::map<void*, std::set<void*>> g_after;  // the streams whose work a stream's work comes after
 long g_calls = 0, g_fail_at = 0;  // the call that fails, counted from 1; 0: none
 long g_bad_frees = 0;
+std::map<const void*, int> g_smem;  // the dynamic shared memory a kernel may take, where it was set
+long g_settings = 0;                // how often it was
+long g_refused = 0;                 // launches that asked for more
 std::atomic<long> g_streams{0};  // made and not destroyed
 cudaError_t g_last = cudaSuccess;
 char g_handles[4096];
@@ -91,6 +94,8 @@ void fake_reset(long fail_at)
 }
 long fake_calls() { return g_calls; }
 long fake_live() { return (long)g_live.size(); }
+long fake_settings() { return g_settings; }
+long fake_refused() { return g_refused; }
 long fake_streams() { return g_streams; }
 long fake_bad_frees() { return g_bad_frees; }
 long fake_busy()
@@ -231,15 +236,23 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t e, unsigned)
 }
 
 // ---- kernels ---------------------------------------------------------------------------------------
-cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return simple(); }
-cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t st)
+cudaError_t cudaFuncSetAttribute(const void* kernel, cudaFuncAttribute, int value)
 {
-    return work_on(st, [] {});
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (const cudaError_t e = call()) return e;
+    g_smem[kernel] = value;
+    ++g_settings;
+    return cudaSuccess;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void**)
+cudaError_t launch(const void* kernel, size_t smem, cudaStream_t st)
 {
-    return work_on(c->stream, [] {});
+    return work_on(st, [&] {
+        const auto allowed = g_smem.find(kernel);
+        if (smem > (size_t)(allowed != g_smem.end() ? allowed->second : 48 << 10)) ++g_refused;
+    });
 }
+cudaError_t cudaLaunchKernel(const void* kernel, dim3, dim3, void**, size_t smem, cudaStream_t st) { return launch(kernel, smem, st); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel, void**) { return launch(kernel, c->dynamicSmemBytes, c->stream); }
 cudaError_t cudaGetLastError()
 {
     std::lock_guard<std::mutex> lock(g_mutex);

@@ -11,7 +11,7 @@ from csrspmm_b200 import _lib, build
 @pytest.fixture(scope="module")
 def fake():
     L = C.CDLL(str(build.build_fake_runtime()))
-    for name in ("fake_calls", "fake_live", "fake_bad_frees", "fake_busy", "fake_streams"):
+    for name in ("fake_calls", "fake_live", "fake_bad_frees", "fake_busy", "fake_streams", "fake_settings", "fake_refused"):
         getattr(L, name).restype = C.c_long
     L.fake_reset.argtypes = [C.c_long]
     return L
@@ -124,6 +124,16 @@ def test_one_failed_call(fake, name):
         assert fake.fake_bad_frees() == 0, f"call {k} of {calls} fails: something is freed twice"
         assert fake.fake_live() == live, f"call {k} of {calls} fails: something is not freed"
         assert name not in LENDING or fake.fake_busy() == 0, f"call {k} of {calls} fails: work is still running"
+
+
+def test_shared_memory_is_asked_for_once(fake):
+    fake.fake_reset(0)
+    keep = {}
+    for _ in range(2):
+        assert _transpose(fake, keep) == 0
+    before = fake.fake_settings()
+    assert before > 0 and _transpose(fake, keep) == 0 and fake.fake_settings() == before
+    assert fake.fake_refused() == 0  # and no launch, in any test so far, took more than it had asked for
 
 
 def test_kept_streams_are_bounded_and_given_back(fake):
