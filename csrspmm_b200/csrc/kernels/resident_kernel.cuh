@@ -112,9 +112,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) spmm_resident_kernel(cons
         async_wait<0>();
         __syncthreads();
 
-        const bool col_ok = cv0 + lane < p.ncolv;
-        Vec<4> acc;
-        acc.zero();
+        Vec<4> acc[1];
+        acc[0].zero();
         while (row < row1) {
             tile.sync();  // the previous chunk has been consumed by every lane of the group
 #pragma unroll
@@ -127,7 +126,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) spmm_resident_kernel(cons
             auto step = [&](int off, int bits) {
                 Vec<4> b;
                 b.v = *reinterpret_cast<const float4*>(b_lane + off);
-                acc.fma(__int_as_float(bits), b);
+                acc[0].fma(__int_as_float(bits), b);
             };
             int e = 0;
             for (; e + 4 <= n; e += 4) {
@@ -139,17 +138,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) spmm_resident_kernel(cons
             }
             for (; e < n; ++e) step(cv[e].x, cv[e].y);
             if (ends) {
-                if (col_ok) {
-                    float* cp = p.C + (long long)row * p.ldc + 4LL * (cv0 + lane);
-                    if (p.beta != 0.0f) {
-                        Vec<4> old;
-                        old.load(cp);
-                        acc.epilogue(p.alpha, p.beta, old).store(cp);
-                    } else {
-                        acc.epilogue0(p.alpha).store(cp);
-                    }
-                }
-                acc.zero();
+                store_row<G, 1, 4>(p, row, cv0, lane, acc);
+                acc[0].zero();
                 row += GROUPS;
                 j = next_first;
                 last = next_last;
