@@ -125,7 +125,7 @@ cudaError_t launch_resident(const SpmmParams& p, cudaStream_t st)
     const cudaError_t e = allow_dynamic_smem<kern>(resident_smem_bytes<G>(kResidentPanelBytes / (G * 16)));
     if (e != cudaSuccess) return e;
     const long long total = (long long)((p.ncolv + G - 1) / G) * p.M;
-    const unsigned grid = (unsigned)(total < 148 ? total : 148);
+    const unsigned grid = (unsigned)(total < kSms ? total : kSms);
     return launch_overlapped(kern, grid, kResidentThreads, (size_t)resident_smem_bytes<G>(p.Kd), st, p, total);
 }
 
@@ -188,7 +188,7 @@ int enqueue(const csrspmm_b200_args* a, cudaStream_t st)
         float* const padded = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + padded_b_offset(plan));
         const long long vectors = (long long)a->Kd * plan.ncolv;
         const long long ctas = (vectors + 255) / 256;
-        CUDA_TRY(launch_overlapped(pad_rows_kernel, (unsigned)(ctas < 148 * 16 ? ctas : 148 * 16), 256, 0, st, vectors, plan.ncolv, a->Nd, a->B,
+        CUDA_TRY(launch_overlapped(pad_rows_kernel, (unsigned)(ctas < kSms * 16 ? ctas : kSms * 16), 256, 0, st, vectors, plan.ncolv, a->Nd, a->B,
                                    (long long)a->ldb, reinterpret_cast<float4*>(padded)));
         p.B = padded;
         p.ldb = 4LL * plan.ncolv;
@@ -593,7 +593,7 @@ size_t csrspmm_b200_host_arena_bytes(const csrspmm_b200_args* a)
     total += align256(vbytes);
     total += align256((size_t)a->Kd * (size_t)a->Nd * 4);
     total += align256((size_t)a->M * (size_t)a->Nd * 4);
-    total += align256(worst_case_workspace(a, true));  // row blocks share it
+    total += align256(worst_case_workspace(a));  // row blocks share it
     total += 256;  // status word
     return total;
 }
@@ -625,7 +625,7 @@ int csrspmm_b200_spmm_host(const csrspmm_b200_args* a, void* device_arena, size_
     const size_t vbytes = e2m1 ? (size_t)(a->nnz + 1) / 2 : (size_t)a->nnz * 4;
     const size_t rp_bytes = ((size_t)a->M + 1) * 4, ci_bytes = (size_t)a->nnz * 4;
     const size_t c_bytes = (size_t)a->M * (size_t)a->Nd * 4;
-    const size_t ws_bytes = worst_case_workspace(a, true);  // enough for every row block below
+    const size_t ws_bytes = worst_case_workspace(a);  // enough for every row block below
     char* cur = arena;
     int32_t* d_rp = reinterpret_cast<int32_t*>(cur); cur += align256(rp_bytes);
     int32_t* d_ci = reinterpret_cast<int32_t*>(cur); cur += align256(ci_bytes);
@@ -865,7 +865,7 @@ int csrspmm_b200_validate_csr_device(int32_t M, int32_t Kd, int64_t nnz, const i
     const int threads = 256;
     long long blocks = ((long long)M + threads - 1) / threads;
     if (blocks < 1) blocks = 1;
-    if (blocks > 148 * 32) blocks = 148 * 32;
+    if (blocks > kSms * 32) blocks = kSms * 32;
     validate_csr_kernel<<<(unsigned)blocks, threads, 0, st>>>(M, Kd, nnz, row_ptr, col_idx, d_flags);
     CUDA_TRY(cudaGetLastError());
     unsigned flags = 0;

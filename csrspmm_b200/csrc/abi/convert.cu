@@ -195,7 +195,7 @@ int csrspmm_b200_e2m1_decode_device(int64_t n, const uint8_t* packed, float scal
     }
     if (n == 0) return CSRSPMM_B200_OK;
     const long long want = (n + 255) / 256;
-    const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
+    const unsigned grid = (unsigned)(want < kSms * 16 ? want : kSms * 16);
     e2m1_decode_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, packed, scale, values);
     CUDA_TRY(cudaGetLastError());
     return CSRSPMM_B200_OK;

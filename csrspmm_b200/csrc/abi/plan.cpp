@@ -142,7 +142,7 @@ static void fill_split_geometry(const csrspmm_b200_args* a, Plan* plan, int grou
 // `least`: a CTA's search and staging cost as much as a walk of some 16 items.
 static int merge_items_per_group(long long num_items, int groups, int ctas_per_sm, int most, int least)
 {
-    const long long wave = 148LL * ctas_per_sm * groups;
+    const long long wave = (long long)kSms * ctas_per_sm * groups;
     const long long waves = (num_items + wave * most - 1) / (wave * most);
     if (waves > 3) return most;
     const long long tg = waves > 0 ? (num_items + wave * waves - 1) / (wave * waves) : 1;
@@ -168,7 +168,7 @@ static int resident_lanes(const csrspmm_b200_args* a, const Plan& plan)
     if (lanes == 0 || plan.ncolv < lanes || (plan.full && lanes == 16)) return 0;
     const long long panels = (plan.ncolv + lanes - 1) / lanes;
     const long long reuse = plan.full ? 16 : CSRSPMM_TUNE_RESIDENT_REUSE;  // entries per CTA and row of B
-    return a->nnz * panels >= reuse * 148LL * a->Kd ? lanes : 0;
+    return a->nnz * panels >= reuse * (long long)kSms * a->Kd ? lanes : 0;
 }
 
 // Whether a whole-row product would be a chain of its longest rows' entries on a chip that is mostly idle: few rows, long
@@ -275,22 +275,23 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
             plan->any_count = a->nnz > kWholeRowEntries;
             plan->resident = (flags & kPlanNoPairs) == 0 && !padded && !plan->any_count ? resident_lanes(a, *plan) : 0;
             plan->short_rows = a->nnz <= (long long)CSRSPMM_TUNE_ROW_SHORT_MEAN * (long long)a->M;
-            plan->low_occupancy = (long long)a->M * plan->G / 32 < 148LL * 8;
+            plan->low_occupancy = (long long)a->M * plan->G / 32 < (long long)kSms * 8;
 #if CSRSPMM_TUNE_ROW_PERSISTENT > 0
             // many short rows: a CTA that lives for four 16-entry rows costs more to start than to
             // run (cfg2: 20.5 -> 18.6 us; 65536 rows of 13: 53 -> 45 us; long rows prefer the
             // finer dynamic balance of one CTA per few rows)
-            if (a->nnz <= (long long)CSRSPMM_TUNE_ROW_PERSISTENT_MAX_MEAN * (long long)a->M && plan->grid > 148LL * CSRSPMM_TUNE_ROW_PERSISTENT)
-                plan->grid = 148LL * CSRSPMM_TUNE_ROW_PERSISTENT;
+            if (a->nnz <= (long long)CSRSPMM_TUNE_ROW_PERSISTENT_MAX_MEAN * (long long)a->M && plan->grid > (long long)kSms * CSRSPMM_TUNE_ROW_PERSISTENT)
+                plan->grid = (long long)kSms * CSRSPMM_TUNE_ROW_PERSISTENT;
 #endif
         }
     }
     // A next grid placed early goes where slots are free.  Behind a grid that fills the chip those are the slots
     // its CTAs leave, one by one and evenly; behind a smaller one they crowd on the SMs that had room, and the
     // crowded SMs finish late (4096 rows of 410 entries, 128 columns: 46.2 us per product against 43.4).
-    plan->fills_chip = plan->grid >= 148LL * (kernel == CSRSPMM_B200_KERNEL_ROW     ? (plan->low_occupancy ? 2 : row_min_blocks(plan->NV))
-                                              : kernel == CSRSPMM_B200_KERNEL_MERGE ? merge_min_blocks(plan->NV)
-                                                                                    : CSRSPMM_TUNE_TMA_MINB);
+    const int resident_ctas = kernel == CSRSPMM_B200_KERNEL_ROW     ? (plan->low_occupancy ? 2 : row_min_blocks(plan->NV))
+                              : kernel == CSRSPMM_B200_KERNEL_MERGE ? merge_min_blocks(plan->NV)
+                                                                    : CSRSPMM_TUNE_TMA_MINB;
+    plan->fills_chip = plan->grid >= (long long)kSms * resident_ctas;
     if (plan->grid > 0x7fffffffLL) {
         set_last_error("grid of %lld CTAs exceeds the launch limit", plan->grid);
         return CSRSPMM_B200_ERR_UNSUPPORTED;
@@ -319,19 +320,18 @@ int product_plan(const csrspmm_b200_args* a, Plan* plan)
     return make_plan(a, plan);
 }
 
-size_t worst_case_workspace(const csrspmm_b200_args* a, bool any_row_block)
+size_t worst_case_workspace(const csrspmm_b200_args* a)
 {
     if (check_args(a, false) != CSRSPMM_B200_OK) return 0;
     // Most CTAs any split kernel takes: the bulk-copy kernel's fixed tile, or the merge kernel's waves of equal
     // tiles -- no more than the largest tile gives plus one wave, whatever the size, so the same bound holds for
     // every row block of the matrix.
-    (void)any_row_block;
     const long long items = (long long)a->M + a->nnz;
     Plan p;
     fill_split_geometry(a, &p, CSRSPMM_TUNE_MERGE_THREADS / 32, CSRSPMM_TUNE_TMA_TG);
     long long tiles = p.num_tiles;
     auto consider = [&](int groups, int most, int ctas_per_sm) {
-        const long long t = items / ((long long)groups * most) + 1 + 148LL * ctas_per_sm;
+        const long long t = items / ((long long)groups * most) + 1 + (long long)kSms * ctas_per_sm;
         if (t > tiles) tiles = t;
     };
     for (const ShapeDesc& k : kShapes) consider(CSRSPMM_TUNE_MERGE_THREADS / k.G, k.TG, merge_min_blocks(k.NV));

@@ -65,10 +65,9 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags = 0);
 int product_plan(const csrspmm_b200_args* a, Plan* plan);
 inline size_t padded_b_offset(const Plan& plan) { return (plan.workspace_bytes + 255) / 256 * 256; }
 
-// Workspace of the split kernels for a given plan-independent worst case: what
-// csrspmm_b200_workspace_bytes reports (the larger of the MERGE and TMA needs).  any_row_block:
-// also enough for any contiguous block of the matrix's rows multiplied on its own.
-size_t worst_case_workspace(const csrspmm_b200_args* a, bool any_row_block = false);
+// Workspace of the split kernels whatever the plan: what csrspmm_b200_workspace_bytes reports (the larger of the MERGE
+// and TMA needs), and enough for any contiguous block of the matrix's rows multiplied on its own.
+size_t worst_case_workspace(const csrspmm_b200_args* a);
 
 // Scratch for a copy of B with rows padded to whole 16-byte vectors, or 0 where the product does without.  Rows of
 // 57 or 150 columns start on any 4 or 8 bytes, and gathered one or two floats per lane they come at half the rate; a copy

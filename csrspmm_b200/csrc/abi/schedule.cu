@@ -268,7 +268,7 @@ int enqueue_scheduled(const csrspmm_b200_args* a, cudaStream_t st)
     // a persistent grid: every warp draws runs of pieces until the list is used up
     const long long per_cta = (long long)(kSlicedThreads / kPieceShapes[plan.shape].G) * q.pieces_per_group;
     const long long ctas_of_work = (s->num_pieces + per_cta - 1) / per_cta + 1;
-    int sms = 148;
+    int sms = kSms;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const unsigned grid_pieces = (unsigned)std::min<long long>(ctas_of_work, (long long)sms * kSlicedCtasPerSm);
     cudaError_t err = cudaMemsetAsync(q.tickets, 0, kTicketBytes, st);
@@ -417,7 +417,7 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
         SCHED_TRY(rows.alloc((size_t)capacity * sizeof(int)));
         int* const d_rows = rows.as<int>();
         long long blocks = ((long long)a->M + 255) / 256;
-        if (blocks > 148 * 16) blocks = 148 * 16;
+        if (blocks > kSms * 16) blocks = kSms * 16;
         sched_list_long_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>(a->M, a->row_ptr, threshold, d_rows, capacity, d_counters);
         SCHED_TRY(cudaGetLastError());
         unsigned h_counters[kSchedCounters] = {};

@@ -39,7 +39,7 @@ TransposePlan plan_transpose(int32_t Kd, int64_t nnz)
     int bits = 1;
     while (bits < 31 && ((int64_t)1 << bits) < Kd) ++bits;
     // eight entries per thread (runs of 8 with 256 digits) while sixteen would leave fewer than three CTAs per SM
-    p.items = nnz < 148LL * 3 * kTransposeThreads * 16 ? 8 : 16;
+    p.items = nnz < (long long)kSms * 3 * kTransposeThreads * 16 ? 8 : 16;
     p.passes = (bits + kMaxDigitBits - 1) / kMaxDigitBits;
     p.digit_bits = (bits + p.passes - 1) / p.passes;
     const int64_t tile = (int64_t)kTransposeThreads * p.items;

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(long long vectors, int ve
 
 // Four numbers over all threads of a CTA: v[0] maximum, v[1..3] sums; valid in thread 0.
 constexpr int kStatsThreads = 256;
-constexpr int kStatsMaxCtas = 148 * 4;
+constexpr int kStatsMaxCtas = kSms * 4;
 
 __device__ __forceinline__ void stats_of_cta(long long (&v)[4])
 {

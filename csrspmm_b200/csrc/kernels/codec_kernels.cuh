@@ -12,7 +12,7 @@ namespace csrspmm_b200 {
 // flight (arrays that do not start on 16 bytes: plain loads).
 constexpr int kCodecThreads = 256;
 constexpr int kCodecPer = 16;
-constexpr int kCodecMaxCtas = 148 * 4;
+constexpr int kCodecMaxCtas = kSms * 4;
 
 // 16 values from position i0 on (0 beyond n)
 __device__ __forceinline__ void load_codec(long long n, const float* __restrict__ values, long long i0, float (&v)[kCodecPer])

@@ -3,6 +3,11 @@
 // the defaults are the measured best on B200.
 #pragma once
 
+// SMs of the one GPU this library is for: what grids and thresholds are counted in
+#ifndef CSRSPMM_TUNE_SMS
+#define CSRSPMM_TUNE_SMS 148
+#endif
+
 // B-row loads kept in flight per lane, by number of column vectors per lane (NV) -- merge kernel
 #ifndef CSRSPMM_TUNE_MERGE_U_NV1
 #define CSRSPMM_TUNE_MERGE_U_NV1 5
@@ -251,6 +256,8 @@
 #endif
 
 namespace csrspmm_b200 {
+
+constexpr int kSms = CSRSPMM_TUNE_SMS;
 
 // merge kernel: lane groups take no fewer items than this, and tiles of up to TG_SMALL items per group run the
 // build that has shared memory for just those (more of it left to L1)
