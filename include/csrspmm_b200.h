@@ -326,6 +326,7 @@ int csrspmm_b200_csr2dense(int32_t H, int32_t W, const int32_t* row_ptr, const i
 
 /* CSR of A^T (Kd x M) from the CSR of A (M x Kd), device arrays, on `stream`, asynchronous: entries of a column keep
  * their stored order, so rows ascend in each column.  t_row_ptr has Kd + 1 entries, t_col_idx and t_values nnz.
+ * A column outside [0, Kd) counts as the nearest one inside, as in a product: the transpose of what was multiplied.
  * workspace: csrspmm_b200_transpose_workspace_bytes(Kd, nnz) bytes, 256-byte aligned.  No counterpart in the
  * reference. */
 size_t csrspmm_b200_transpose_workspace_bytes(int32_t Kd, int64_t nnz);

@@ -30,6 +30,14 @@ def test_transpose_of_nothing(cuda_lib):
     assert t_rp.tolist() == [0] * 10 and t_ci.numel() == t_va.numel() == 0
 
 
+@pytest.mark.parametrize("rp,ci", [([0, 2], [0, 9]), ([0, 2], [-1, 3]), ([0, 1], [0, 3])])
+def test_a_matrix_that_is_none_is_refused(cuda_lib, rp, ci):
+    t = torch.tensor(rp, dtype=torch.int32), torch.tensor(ci, dtype=torch.int32), torch.ones(2)
+    for arrays in (t, [x.cuda() for x in t]):
+        with pytest.raises((RuntimeError, IndexError)):
+            TL.transpose_csr(*arrays, 9)
+
+
 def test_operator_errors_keep_their_type(cuda_lib):
     rp, ci, va = torch.tensor([0, 1], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), torch.ones(1).cuda()
     with pytest.raises(_lib.SpmmError):  # the bulk-copy kernel needs whole vectors
