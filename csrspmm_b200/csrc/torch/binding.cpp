@@ -74,6 +74,9 @@ const at::Tensor& tensor_of(PyObject* o, const char* name)
     return THPVariable_Unpack(o);
 }
 
+// The kernels take a leading dimension of at least the row's length.
+bool rows_apart(const at::Tensor& t) { return t.size(0) <= 1 || t.stride(0) >= t.size(1); }
+
 // The checks of the reference's wrappers, with its wording (torch_csrspmm/torch_csrspmm_naive.cpp:19-26).
 void check_csr(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va, const at::Tensor& B, bool packed)
 {
@@ -90,6 +93,7 @@ void check_csr(const at::Tensor& rp, const at::Tensor& ci, const at::Tensor& va,
          "expected 1-D row_ptr/col_idx/values and 2-D B");
     want(rp.is_contiguous() && ci.is_contiguous() && va.is_contiguous(), "row_ptr, col_idx and values must be contiguous");
     want(B.stride(1) == 1 || B.size(1) <= 1, "B must be row-major (unit stride along its columns)");
+    want(rows_apart(B), "B must be row-major (rows that do not overlap)");  // an expanded row: its storage ends after one
     const auto dev = B.device();
     want(rp.device() == dev && ci.device() == dev && va.device() == dev, "all tensors must be on the same device");
 }
@@ -157,6 +161,7 @@ at::Tensor run_product(Product& q)
     const int64_t n = q.nnz.value_or(q.ci.size(0));
     if (q.packed) want(q.va.size(0) >= (n + 1) / 2, "packed values too short");
     else want(q.va.size(0) == n, "values and col_idx differ in length");
+    want(q.ci.size(0) >= n, "col_idx too short");
     const c10::cuda::CUDAGuard guard(q.B.device());
     if (!q.C.defined()) {
         want(q.beta == 0.0, "beta != 0 needs C_out");
@@ -165,7 +170,7 @@ at::Tensor run_product(Product& q)
         want(q.C.is_cuda() && q.C.scalar_type() == at::kFloat && q.C.dim() == 2 && q.C.size(0) == M && q.C.size(1) == Nd &&
                  q.C.device() == q.B.device(),
              "C_out must be a float32 CUDA tensor of shape (M, Nd) on B's device");
-        want(q.C.stride(1) == 1 || Nd <= 1, "C_out must be row-major");
+        want((q.C.stride(1) == 1 || Nd <= 1) && rows_apart(q.C), "C_out must be row-major");
     }
     csrspmm_b200_args a = {};
     a.struct_size = sizeof(a);
@@ -410,7 +415,7 @@ PyObject* py_dense2csr(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     expect_args(nargs, 2);
     const at::Tensor dense = tensor_of(args[0], "dense");
     const float tol = static_cast<float>(as_double(args[1]));
-    want(dense.is_cuda() && dense.scalar_type() == at::kFloat && dense.dim() == 2 && (dense.stride(1) == 1 || dense.size(1) <= 1),
+    want(dense.is_cuda() && dense.scalar_type() == at::kFloat && dense.dim() == 2 && (dense.stride(1) == 1 || dense.size(1) <= 1) && rows_apart(dense),
          "dense must be a row-major float32 CUDA matrix");
     const int64_t H = dense.size(0), W = dense.size(1);
     const int64_t ld = std::max(H > 1 ? dense.stride(0) : W, W);

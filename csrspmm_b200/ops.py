@@ -54,9 +54,27 @@ def _check_csr(row_ptr, col_idx, values, B, packed: bool):
         raise RuntimeError("row_ptr, col_idx and values must be contiguous")
     if B.stride(1) != 1 and B.size(1) > 1:
         raise RuntimeError("B must be row-major (unit stride along its columns)")
+    if B.size(0) > 1 and B.stride(0) < B.size(1):
+        raise RuntimeError("B must be row-major (rows that do not overlap)")
     dev = B.device
     if not (row_ptr.device == dev and col_idx.device == dev and values.device == dev):
         raise RuntimeError("all tensors must be on the same device")
+
+
+def _check_sizes(col_idx, values, n: int, packed: bool):
+    if not packed and values.numel() != n:
+        raise RuntimeError("values and col_idx differ in length")
+    if packed and values.numel() < (n + 1) // 2:
+        raise RuntimeError("packed values too short")
+    if col_idx.numel() < n:
+        raise RuntimeError("col_idx too short")
+
+
+def _check_out(C_out, M: int, Nd: int, B):
+    if not C_out.is_cuda or C_out.dtype != torch.float32 or C_out.shape != (M, Nd) or C_out.device != B.device:
+        raise RuntimeError("C_out must be a float32 CUDA tensor of shape (M, Nd) on B's device")
+    if (Nd > 1 and C_out.stride(1) != 1) or (M > 1 and C_out.stride(0) < Nd):
+        raise RuntimeError("C_out must be row-major")
 
 
 def workspace_bytes(M: int, Kd: int, Nd: int, nnz: int) -> int:
@@ -139,12 +157,13 @@ def spmm_tiled(row_ptr, col_idx, values, B, C_out=None, alpha=1.0, beta=0.0, *, 
     _check_csr(row_ptr, col_idx, values, B, packed)
     M, Kd, Nd = row_ptr.numel() - 1, B.size(0), B.size(1)
     n = int(col_idx.numel() if nnz is None else nnz)
+    _check_sizes(col_idx, values, n, packed)
     if C_out is None:
         if beta != 0.0:
             raise RuntimeError("beta != 0 needs C_out")
         C_out = torch.empty((M, Nd), dtype=torch.float32, device=B.device)
-    elif not C_out.is_cuda or C_out.dtype != torch.float32 or C_out.shape != (M, Nd) or C_out.device != B.device:
-        raise RuntimeError("C_out must be a float32 CUDA tensor of shape (M, Nd) on B's device")
+    else:
+        _check_out(C_out, M, Nd, B)
     L = _lib.lib()
     a = _lib.make_args(M, Kd, Nd, n, row_ptr.data_ptr(), col_idx.data_ptr(), values.data_ptr(), B.data_ptr(),
                        C_out.data_ptr(), ldb=max(B.stride(0) if Kd > 1 else Nd, Nd),
@@ -182,8 +201,8 @@ class SpmmCall:
         _check_csr(row_ptr, col_idx, values, B, packed)
         M, Kd, Nd = row_ptr.numel() - 1, B.size(0), B.size(1)
         n = int(col_idx.numel() if nnz is None else nnz)
-        if C_out.shape != (M, Nd) or C_out.dtype != torch.float32 or C_out.device != B.device:
-            raise RuntimeError("C_out must be a float32 CUDA tensor of shape (M, Nd) on B's device")
+        _check_sizes(col_idx, values, n, packed)
+        _check_out(C_out, M, Nd, B)
         self.device = B.device
         self.L = _lib.lib()
         self.args = _lib.make_args(
@@ -294,6 +313,8 @@ def e2m1_quantize(values_f32):
 def e2m1_dequantize(packed, n, scale):
     """Packed codes -> fp32 values (on the device for a CUDA tensor, else on the host)."""
     import numpy as np
+    if (packed.numel() if isinstance(packed, torch.Tensor) else len(packed)) < (int(n) + 1) // 2:
+        raise RuntimeError("packed values too short")
     if isinstance(packed, torch.Tensor) and packed.is_cuda:
         out = torch.empty(int(n), dtype=torch.float32, device=packed.device)
         with torch.cuda.device(packed.device):
