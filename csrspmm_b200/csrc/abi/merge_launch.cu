@@ -19,8 +19,10 @@ cudaError_t launch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t st)
     constexpr int G = kShapes[S].G, NV = kShapes[S].NV, TG = kShapes[S].TG;
     constexpr int TGS = CSRSPMM_TUNE_MERGE_TG_SMALL < TG ? CSRSPMM_TUNE_MERGE_TG_SMALL : TG;
     constexpr int U = merge_unroll(VW, NV);
-    // one more row in flight where the grid is many waves long, hence waiting for HBM (262 144 rows of 16, 128 columns:
-    // 218.5 us with six, 222 with five; shorter grids the other way round: 47.5 and 45.2)
+    // one more row in flight where the grid is many waves long, hence waiting for HBM.  Six against five, 128 columns: 262 144
+    // rows of 16 221.8 and 225.7 us, Zipf rows 221.2 and 229.5 (packed values 232.2 and 240.1), 200 000 Zipf rows 160.7 and
+    // 165.2; 100 columns, 500 000 Zipf rows of 20 571 and 591; 64 columns, 1 M Zipf rows 605 and 610, 300 000 even ones 126.1
+    // both; 48 columns 314.9 and 312.4.  Shorter grids the other way round: 47.5 and 45.2.
     constexpr int ULONG = VW == 4 && NV == 1 && G >= 16 ? CSRSPMM_TUNE_MERGE_U_LONG : U;
     const unsigned grid = (unsigned)plan.grid;
     if (ULONG != U && plan.tg == TG) {
