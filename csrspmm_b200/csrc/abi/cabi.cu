@@ -879,6 +879,31 @@ int csrspmm_b200_validate_csr_device(int32_t M, int32_t Kd, int64_t nnz, const i
     return CSRSPMM_B200_OK;
 }
 
+int csrspmm_b200_check_bounds_device(int32_t M, int32_t Kd, int64_t nnz, const int32_t* row_ptr, const int32_t* col_idx, uint32_t* problems,
+                                     csrspmm_b200_stream_t stream)
+{
+    if (M < 0 || Kd < 0 || nnz < 0 || row_ptr == nullptr || (nnz > 0 && col_idx == nullptr) || problems == nullptr) {
+        set_last_error("check_bounds_device: bad argument");
+        return CSRSPMM_B200_ERR_BAD_ARG;
+    }
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    Results results(st);
+    CUDA_TRY(results.init());
+    CUDA_TRY(results.clear());
+    const long long want = (nnz + kBoundsThreads * 8 - 1) / (kBoundsThreads * 8);
+    const unsigned grid = (unsigned)(want < 1 ? 1 : (want < kSms * 8 ? want : kSms * 8));
+    CUDA_TRY(launch_overlapped(check_bounds_kernel, grid, kBoundsThreads, 0, st, M, Kd, (long long)nnz, row_ptr, col_idx,
+                               static_cast<volatile long long*>(results.ptr())));
+    long long bits = 0;
+    CUDA_TRY(results.wait(&bits, 1));
+    *problems = (uint32_t)bits;
+    if (bits != 0) {
+        set_last_error("row_ptr or col_idx out of bounds, problem bits 0x%x", (unsigned)bits);
+        return CSRSPMM_B200_ERR_INVALID_CSR;
+    }
+    return CSRSPMM_B200_OK;
+}
+
 int csrspmm_b200_row_stats_device(int32_t M, const int32_t* row_ptr, int64_t stats[4],
                                   csrspmm_b200_stream_t stream)
 {

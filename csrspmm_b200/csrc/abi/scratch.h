@@ -77,6 +77,13 @@ public:
         if (slot_.words() != nullptr) return cudaSuccess;
         return dev_.alloc(kPinnedWords * sizeof(long long));  // every slot taken: plain scratch, copied back
     }
+    // word 0 = 0, for kernels that only write what they find
+    cudaError_t clear()
+    {
+        if (slot_.words() == nullptr) return cudaMemsetAsync(dev_.as<long long>(), 0, sizeof(long long), st_);
+        slot_.words()[0] = 0;
+        return cudaSuccess;
+    }
     long long* ptr() const { return slot_.words() != nullptr ? const_cast<long long*>(slot_.words()) : dev_.as<long long>(); }
     cudaError_t wait(long long* out, int count)
     {

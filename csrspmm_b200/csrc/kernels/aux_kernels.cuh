@@ -37,6 +37,27 @@ __global__ void validate_csr_kernel(int M, int Kd, long long nnz, const int* __r
     if (bad) atomicOr(problems, bad);
 }
 
+// Of the above what keeps a product from placing an entry: bits 2 (row_ptr's end) and 8 (a column out of range), without a
+// look at the rows.  *problems is zero before; whoever sees something writes all it saw.
+constexpr int kBoundsThreads = 256;
+
+__global__ void __launch_bounds__(kBoundsThreads) check_bounds_kernel(int M, int Kd, long long nnz, const int* __restrict__ row_ptr,
+                                                                      const int* __restrict__ col_idx, volatile long long* problems)
+{
+    wait_for_previous_grid();
+    release_next_grid();
+    constexpr int PER = 8;
+    unsigned bad = __ldg(row_ptr + M) != nnz ? 2u : 0u;
+    for (long long j = (long long)blockIdx.x * (kBoundsThreads * PER) + threadIdx.x; j < nnz; j += (long long)gridDim.x * (kBoundsThreads * PER)) {
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (j + k * kBoundsThreads < nnz && (unsigned)__ldg(col_idx + j + k * kBoundsThreads) >= (unsigned)Kd) bad |= 8u;
+    }
+    if (__syncthreads_or(bad & 2u)) bad |= 2u;
+    if (__syncthreads_or(bad & 8u)) bad |= 8u;
+    if (threadIdx.x == 0 && bad) *problems = bad;
+}
+
 // A copy of B whose rows are whole vectors of four, zeros behind the last column.
 __global__ void __launch_bounds__(256) pad_rows_kernel(long long vectors, int vectors_per_row, int Nd, const float* __restrict__ B, long long ldb,
                                                        float4* __restrict__ out)

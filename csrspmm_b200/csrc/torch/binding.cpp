@@ -44,6 +44,7 @@ struct Library {
     size_t (*transpose_workspace_bytes)(int32_t, int64_t);
     int (*transpose)(int32_t, int32_t, int64_t, const int32_t*, const int32_t*, const float*, int32_t*, int32_t*, float*, void*, size_t,
                      csrspmm_b200_stream_t);
+    int (*check_bounds)(int32_t, int32_t, int64_t, const int32_t*, const int32_t*, uint32_t*, csrspmm_b200_stream_t);
     int (*quantize)(int64_t, const float*, float*, uint8_t*, csrspmm_b200_stream_t);
 };
 Library g_lib = {};
@@ -323,6 +324,7 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     fill(g_lib.quantize, "e2m1_quantize_device");
     fill(g_lib.transpose_workspace_bytes, "transpose_workspace_bytes");
     fill(g_lib.transpose, "transpose");
+    fill(g_lib.check_bounds, "check_bounds_device");
     Py_INCREF(args[0]);
     Py_XSETREF(g_error, args[0]);
     Py_RETURN_NONE;
@@ -471,6 +473,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> transpose(const at::Tensor& rp, c
     want(rp.dim() == 1 && ci.dim() == 1 && va.dim() == 1 && rp.size(0) >= 1 && ci.size(0) == va.size(0) && rp.is_contiguous() &&
              ci.is_contiguous() && va.is_contiguous(),
          "expected contiguous 1-D row_ptr, col_idx and values");
+    want(Kd >= 0 && Kd < INT32_MAX && rp.size(0) <= INT32_MAX, "a matrix has fewer than 2^31 - 1 rows and columns");
     const auto device = rp.device();
     const c10::cuda::CUDAGuard guard(device);
     const int64_t nnz = ci.size(0);
@@ -490,12 +493,23 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> transpose(const at::Tensor& rp, c
     return {t_rp, t_ci, t_va};
 }
 
-// transpose(row_ptr, col_idx, values, Kd) -> (row_ptr, col_idx, values) of A^T
+// transpose(row_ptr, col_idx, values, Kd) -> (row_ptr, col_idx, values) of A^T, waiting: the kernels clamp columns out of
+// range, which transpose_csr's code for the host cannot place and refuses
 PyObject* py_transpose(PyObject*, PyObject* const* args, Py_ssize_t nargs)
 {
     BEGIN_BINDING
     expect_args(nargs, 4);
-    const auto t = transpose(tensor_of(args[0], "row_ptr"), tensor_of(args[1], "col_idx"), tensor_of(args[2], "values"), as_integer(args[3]));
+    const at::Tensor rp = tensor_of(args[0], "row_ptr"), ci = tensor_of(args[1], "col_idx");
+    const int64_t Kd = as_integer(args[3]), nnz = ci.numel();
+    const auto t = transpose(rp, ci, tensor_of(args[2], "values"), Kd);
+    {
+        const WithoutGil nogil;
+        const c10::cuda::CUDAGuard guard(rp.device());
+        uint32_t problems = 0;
+        check(g_lib.check_bounds((int32_t)(rp.size(0) - 1), (int32_t)Kd, nnz, address<int32_t>(rp), address<int32_t>(ci), &problems,
+                                 current_stream(rp.device())),
+              "csrspmm_b200_transpose");
+    }
     return Py_BuildValue("(NNN)", THPVariable_Wrap(std::get<0>(t)), THPVariable_Wrap(std::get<1>(t)), THPVariable_Wrap(std::get<2>(t)));
     END_BINDING
 }

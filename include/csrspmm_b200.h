@@ -301,6 +301,10 @@ int csrspmm_b200_validate_csr_host(int32_t M, int32_t Kd, int64_t nnz, const int
 int csrspmm_b200_validate_csr_device(int32_t M, int32_t Kd, int64_t nnz, const int32_t* row_ptr,
                                      const int32_t* col_idx, uint32_t* problems,
                                      csrspmm_b200_stream_t stream);
+/* Only BAD_ROWPTR_END and COL_RANGE, in one quick pass over col_idx (one of the two is set when both apply).  Waits for the
+ * stream. */
+int csrspmm_b200_check_bounds_device(int32_t M, int32_t Kd, int64_t nnz, const int32_t* row_ptr, const int32_t* col_idx,
+                                     uint32_t* problems, csrspmm_b200_stream_t stream);
 
 /* Device row_ptr -> stats[0] = longest row, stats[1] = empty rows, stats[2] = rows longer than
  * 32 * (mean + 1), stats[3] = nnz held by those rows.  Waits for the stream. */
