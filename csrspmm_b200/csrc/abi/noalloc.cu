@@ -1,7 +1,7 @@
 // csrspmm_b200_spmm_noalloc: the merge-path SpMM with its scratch inside the library image.
 //
 // Who this is for.  csrspmm_b200_spmm needs a few bytes of device scratch per CTA for the split
-// kernels; it takes them from the caller's workspace or, failing that, from cudaMallocAsync.  Some
+// kernels; it takes them from the caller's workspace or, failing that, from a pool of its own.  Some
 // hosts of this library can do neither: a process whose own memory manager claimed the whole
 // device at start-up (a later cudaMalloc or pool allocation fails, or comes back after a
 // device-wide synchronisation it cannot afford), a plug-in called from inside somebody else's

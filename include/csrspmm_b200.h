@@ -108,7 +108,7 @@ typedef struct csrspmm_b200_args {
                              row_ptr + r0, col_idx + row_ptr[r0], values + row_ptr[r0] (F32 values),
                              M = r1 - r0, nnz = row_ptr[r1] - row_ptr[r0], row_ptr_base = row_ptr[r0] */
     void* workspace;        /* device scratch for the split kernels, or NULL: the library then
-                               takes it from the stream-ordered allocator for this call */
+                               takes it from its pool, on the stream, for this call */
     size_t workspace_bytes; /* size of workspace when it is not NULL */
     int32_t* status_word;   /* optional device int32 the kernels OR error bits into */
     const struct csrspmm_b200_schedule* schedule; /* optional: a schedule built for this matrix by
