@@ -16,7 +16,8 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
-#include <vector>
+#include <memory>
+#include <new>
 
 #include "../kernels/merge_kernel.cuh"
 #include "../kernels/sliced_kernel.cuh"
@@ -444,16 +445,20 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
                 (int)num_long, d_rows, a->row_ptr, a->col_idx, (int)a->nnz, slab_rows, num_slabs, piece, d_bounds, d_slab,
                 d_long_rows, d_counters);
             SCHED_TRY(cudaGetLastError());
-            std::vector<unsigned> slab_count((size_t)num_slabs);
+            const std::unique_ptr<unsigned[]> slab(new (std::nothrow) unsigned[(size_t)num_slabs]);  // pieces per slab, then first of them
+            if (slab == nullptr) {
+                set_last_error("schedule_create: out of host memory");
+                return fail(CSRSPMM_B200_ERR_BAD_ARG);
+            }
             SCHED_TRY(cudaMemcpyAsync(h_counters, d_counters, sizeof(h_counters), cudaMemcpyDeviceToHost, st));
-            SCHED_TRY(cudaMemcpyAsync(slab_count.data(), d_slab, (size_t)num_slabs * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+            SCHED_TRY(cudaMemcpyAsync(slab.get(), d_slab, (size_t)num_slabs * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
             SCHED_TRY(cudaStreamSynchronize(st));
             const bool sorted = h_counters[4] == 0;
             long long total = 0;
-            std::vector<unsigned> slab_first((size_t)num_slabs);
             for (int k = 0; k < num_slabs; ++k) {
-                slab_first[(size_t)k] = (unsigned)total;
-                total += slab_count[(size_t)k];
+                const unsigned count = slab[k];
+                slab[k] = (unsigned)total;
+                total += count;
             }
             if (!sorted) {
                 s->columns_sorted = 0;  // an empty schedule: the plain kernels run
@@ -464,7 +469,7 @@ int csrspmm_b200_schedule_create(const csrspmm_b200_args* a, const csrspmm_b200_
                 s->long_rows = s->pieces + total;
                 SCHED_TRY(cudaMemcpyAsync(s->long_rows, d_long_rows, (size_t)num_long * sizeof(int4), cudaMemcpyDeviceToDevice, st));
                 unsigned* d_fill = d_slab + num_slabs;
-                SCHED_TRY(cudaMemcpyAsync(d_fill, slab_first.data(), (size_t)num_slabs * sizeof(unsigned), cudaMemcpyHostToDevice, st));
+                SCHED_TRY(cudaMemcpyAsync(d_fill, slab.get(), (size_t)num_slabs * sizeof(unsigned), cudaMemcpyHostToDevice, st));
                 sched_emit_pieces_kernel<<<(unsigned)((num_long + 127) / 128), 128, 0, st>>>(
                     (int)num_long, num_slabs, piece, d_bounds, d_fill, s->long_rows, s->pieces, (int)total);
                 SCHED_TRY(cudaGetLastError());
