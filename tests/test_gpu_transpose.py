@@ -24,6 +24,22 @@ def test_transpose(cuda_lib, M, Kd, nnz, hub):
     assert all(torch.equal(g.cpu(), w) for g, w in zip(got, want))
 
 
+# one tile and two, tiles of one and two entries per thread, one wave and two; columns per bucket 1 to 512 and the first width
+# beyond; buckets of one chunk and of many, all entries in one column, chunks of 8192
+@pytest.mark.parametrize("M,Kd,nnz,share", [(300, 512, 8192, 0.0), (300, 513, 8193, 0.4), (7, 3, 4097, 1.0), (2, 1, 4096, 1.0), (400, 64, 100000, 0.0),
+                                            (5000, 1 << 19, 151552, 0.3), (5000, (1 << 19) + 1, 151553, 0.3), (3000, 40000, 151553, 0.9),
+                                            (20000, 65536, 1212416, 1.0), (20000, 65535, 1212417, 0.05), (60000, 1 << 18, 2200000, 0.2)])
+def test_transpose_through_buckets(cuda_lib, M, Kd, nnz, share):
+    rng = np.random.default_rng(Kd)
+    rp = np.concatenate([[0], np.sort(rng.integers(0, nnz + 1, M - 1)), [nnz]]).astype(np.int32)
+    ci = rng.integers(0, Kd, nnz).astype(np.int32)
+    ci[rng.random(nnz) < share] = Kd // 3
+    t = [torch.from_numpy(x) for x in (rp, ci, rng.standard_normal(nnz, dtype=np.float32))]
+    want = TL.transpose_csr(*t, Kd)
+    got = TL.transpose_csr(*(x.cuda() for x in t), Kd)
+    assert all(torch.equal(g.cpu(), w) for g, w in zip(got, want))
+
+
 def test_transpose_of_nothing(cuda_lib):
     rp, ci, va = torch.zeros(4, dtype=torch.int32).cuda(), torch.zeros(0, dtype=torch.int32).cuda(), torch.zeros(0).cuda()
     t_rp, t_ci, t_va = TL.transpose_csr(rp, ci, va, 9)
