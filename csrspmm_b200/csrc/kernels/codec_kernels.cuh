@@ -81,6 +81,20 @@ __device__ __forceinline__ unsigned e2m1_encode_one(float v, float scale)
     return s | code;
 }
 
+// Largest magnitude whose code is k or less, k = 0 .. 6: the same answer as a division per value, which is monotone, for a dozen
+// instructions less (16 M values with the search for the scale: 71 -> 51 us).  The magnitude between codes k and k + 1 times the scale is a unit in the last
+// place or two away from it.  Scales that the product would leave the range with (kCodecScaleMin .. Max): division.
+constexpr float kCodecScaleMin = 1.17549435e-38f, kCodecScaleMax = 4.0e37f;
+
+__device__ __forceinline__ float e2m1_last_of_code(int k, float scale)
+{
+    const float middle = k < 2 ? 0.25f + 0.5f * k : k < 4 ? 1.25f + 0.5f * (k - 2) : k < 6 ? 2.5f + (k - 4) : 5.0f;
+    int bits = __float_as_int(__fmul_rn(middle, scale));
+    while (bits > 0 && e2m1_encode_one(__int_as_float(bits), scale) > (unsigned)k) --bits;
+    while (e2m1_encode_one(__int_as_float(bits + 1), scale) <= (unsigned)k) ++bits;
+    return __int_as_float(bits);
+}
+
 // The codes of 16 elements per thread and step, 8 bytes at a time.  The scale is the argument, or
 // (cta_max given) follows from the maxima a previous kernel left, in which case CTA 0 reports its bits.
 __global__ void __launch_bounds__(kCodecThreads) e2m1_encode_kernel(long long n, const float* __restrict__ values, float scale,
@@ -96,6 +110,20 @@ __global__ void __launch_bounds__(kCodecThreads) e2m1_encode_kernel(long long n,
         scale = mx > 0.0f ? __fdiv_rn(mx, 6.0f) : 1.0f;
         if (blockIdx.x == 0 && threadIdx.x == 0) *scale_bits = (long long)__float_as_uint(scale);
     }
+    __shared__ float last_of_code[7];
+    const bool by_limits = scale >= kCodecScaleMin && scale <= kCodecScaleMax;
+    if (by_limits && threadIdx.x < 7) last_of_code[threadIdx.x] = e2m1_last_of_code(threadIdx.x, scale);
+    __syncthreads();
+    float last[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) last[k] = last_of_code[k];
+    auto code_of = [&](float v) {
+        if (!by_limits) return e2m1_encode_one(v, scale);
+        unsigned code = (__float_as_uint(v) >> 28) & 8u;
+#pragma unroll
+        for (int k = 0; k < 7; ++k) code += fabsf(v) > last[k];
+        return v == v ? code : 0u;
+    };
     const long long stride = (long long)gridDim.x * (kCodecThreads * kCodecPer);
     const bool wide = (reinterpret_cast<uintptr_t>(packed) & 7u) == 0;
     for (long long i = ((long long)blockIdx.x * kCodecThreads + threadIdx.x) * kCodecPer; i < n; i += stride) {
@@ -103,7 +131,7 @@ __global__ void __launch_bounds__(kCodecThreads) e2m1_encode_kernel(long long n,
         load_codec(n, values, i, v);
         unsigned word[2] = {0u, 0u};  // elements beyond n are 0: code 0
 #pragma unroll
-        for (int q = 0; q < kCodecPer; ++q) word[q >> 3] |= (i + q < n ? e2m1_encode_one(v[q], scale) : 0u) << (4 * (q & 7));
+        for (int q = 0; q < kCodecPer; ++q) word[q >> 3] |= (i + q < n ? code_of(v[q]) : 0u) << (4 * (q & 7));
         if (wide && i + kCodecPer <= n) {
             *reinterpret_cast<uint2*>(packed + (i >> 1)) = make_uint2(word[0], word[1]);
         } else {
