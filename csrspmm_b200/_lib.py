@@ -42,7 +42,8 @@ EXPORTED_SYMBOLS = (
     "csrspmm_b200_validate_csr_host", "csrspmm_b200_validate_csr_device",
     "csrspmm_b200_row_stats_device", "csrspmm_b200_partition_rows", "csrspmm_b200_e2m1_scale",
     "csrspmm_b200_e2m1_encode", "csrspmm_b200_e2m1_decode", "csrspmm_b200_dense2csr_count",
-    "csrspmm_b200_dense2csr_fill", "csrspmm_b200_csr2dense", "csrspmm_b200_copy_rows", "csrspmm_b200_column_panels",
+    "csrspmm_b200_dense2csr_fill", "csrspmm_b200_dense2csr_mask_bytes", "csrspmm_b200_dense2csr_count_mask",
+    "csrspmm_b200_dense2csr_fill_mask", "csrspmm_b200_csr2dense", "csrspmm_b200_copy_rows", "csrspmm_b200_column_panels",
     "csrspmm_b200_e2m1_scale_device", "csrspmm_b200_e2m1_encode_device", "csrspmm_b200_e2m1_decode_device",
     "csrspmm_b200_e2m1_quantize_device", "csrspmm_b200_transpose", "csrspmm_b200_transpose_workspace_bytes",
     "csrspmm_b200_spmm_tiled", "csrspmm_b200_tiled_workspace_bytes", "csrspmm_b200_tiled_panel_rows",

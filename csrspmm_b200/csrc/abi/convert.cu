@@ -48,8 +48,16 @@ float scale_from(float absmax) { return absmax > 0.0f ? absmax / 6.0f : 1.0f; }
 
 extern "C" {
 
+size_t csrspmm_b200_dense2csr_mask_bytes(int32_t H, int32_t W) { return H > 0 && W > 0 ? (size_t)H * (size_t)words_per_row(W) * 4 : 0; }
+
 int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, int32_t* row_ptr,
                                  int64_t* nnz_out, int32_t* max_row_nnz_out, csrspmm_b200_stream_t stream)
+{
+    return csrspmm_b200_dense2csr_count_mask(H, W, dense, ld, tol, row_ptr, nullptr, nnz_out, max_row_nnz_out, stream);
+}
+
+int csrspmm_b200_dense2csr_count_mask(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, int32_t* row_ptr, uint32_t* mask,
+                                      int64_t* nnz_out, int32_t* max_row_nnz_out, csrspmm_b200_stream_t stream)
 {
     if (H < 0 || W < 0 || ld < W || row_ptr == nullptr || nnz_out == nullptr || (H > 0 && W > 0 && dense == nullptr)) {
         set_last_error("dense2csr_count: bad argument");
@@ -69,10 +77,10 @@ int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64
     int* counts = reinterpret_cast<int*>(scratch.as<char>() + scan_bytes);
     Results results(st);
     CUDA_TRY(results.init());
-    const int wpr = convert_warps_per_row(W);
+    const int wpr = convert_warps_per_row(W, kChunkCols);
     const unsigned grid = convert_grid(H, wpr);
     CUDA_TRY(launch_overlapped(rows_on_16_bytes(dense, ld) ? dense_count_kernel<true> : dense_count_kernel<false>, grid, kConvertThreads, 0, st,
-                               H, W, dense, ld, tol, wpr, counts));
+                               H, W, dense, ld, tol, wpr, counts, mask));
     CUDA_TRY(exclusive_scan(counts, H, row_ptr, scratch.as<void>(), results.ptr(), st));
     long long out[2] = {0, 0};
     CUDA_TRY(results.wait(out, 2));
@@ -88,6 +96,12 @@ int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64
 int csrspmm_b200_dense2csr_fill(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, const int32_t* row_ptr,
                                 int32_t* col_idx, float* values, csrspmm_b200_stream_t stream)
 {
+    return csrspmm_b200_dense2csr_fill_mask(H, W, dense, ld, tol, nullptr, row_ptr, col_idx, values, stream);
+}
+
+int csrspmm_b200_dense2csr_fill_mask(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, const uint32_t* mask, const int32_t* row_ptr,
+                                     int32_t* col_idx, float* values, csrspmm_b200_stream_t stream)
+{
     if (H < 0 || W < 0 || ld < W || row_ptr == nullptr) {
         set_last_error("dense2csr_fill: bad argument");
         return CSRSPMM_B200_ERR_BAD_ARG;
@@ -97,13 +111,12 @@ int csrspmm_b200_dense2csr_fill(int32_t H, int32_t W, const float* dense, int64_
         set_last_error("dense2csr_fill: null pointer");
         return CSRSPMM_B200_ERR_BAD_ARG;
     }
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const int wpr = convert_warps_per_row(W);
-    const unsigned grid = convert_grid(H, wpr);
-    CUDA_TRY(launch_overlapped(rows_on_16_bytes(dense, ld) ? dense_fill_kernel<true> : dense_fill_kernel<false>, grid, kConvertThreads, 0, st,
-                               H, W, dense, ld, tol, wpr, row_ptr, col_idx, values));
+    const int wpr = convert_warps_per_row(W, kSpanCols);
+    CUDA_TRY(launch_overlapped(rows_on_16_bytes(dense, ld) ? dense_fill_kernel<true> : dense_fill_kernel<false>, convert_grid(H, wpr), kConvertThreads,
+                               0, reinterpret_cast<cudaStream_t>(stream), H, W, dense, ld, tol, wpr, mask, row_ptr, col_idx, values));
     return CSRSPMM_B200_OK;
 }
+
 
 int csrspmm_b200_csr2dense(int32_t H, int32_t W, const int32_t* row_ptr, const int32_t* col_idx, const float* values,
                            float* dense, int64_t ld, csrspmm_b200_stream_t stream)

@@ -39,8 +39,10 @@ struct Library {
     int (*uses_workspace)(const csrspmm_b200_args*);
     size_t (*workspace_bytes)(const csrspmm_b200_args*);
     int (*row_stats)(int32_t, const int32_t*, int64_t*, csrspmm_b200_stream_t);
-    int (*dense2csr_count)(int32_t, int32_t, const float*, int64_t, float, int32_t*, int64_t*, int32_t*, csrspmm_b200_stream_t);
-    int (*dense2csr_fill)(int32_t, int32_t, const float*, int64_t, float, const int32_t*, int32_t*, float*, csrspmm_b200_stream_t);
+    size_t (*dense2csr_mask_bytes)(int32_t, int32_t);
+    int (*dense2csr_count)(int32_t, int32_t, const float*, int64_t, float, int32_t*, uint32_t*, int64_t*, int32_t*, csrspmm_b200_stream_t);
+    int (*dense2csr_fill)(int32_t, int32_t, const float*, int64_t, float, const uint32_t*, const int32_t*, int32_t*, float*,
+                          csrspmm_b200_stream_t);
     size_t (*transpose_workspace_bytes)(int32_t, int64_t);
     int (*transpose)(int32_t, int32_t, int64_t, const int32_t*, const int32_t*, const float*, int32_t*, int32_t*, float*, void*, size_t,
                      csrspmm_b200_stream_t);
@@ -319,8 +321,9 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     fill(g_lib.uses_workspace, "uses_workspace");
     fill(g_lib.workspace_bytes, "workspace_bytes");
     fill(g_lib.row_stats, "row_stats_device");
-    fill(g_lib.dense2csr_count, "dense2csr_count");
-    fill(g_lib.dense2csr_fill, "dense2csr_fill");
+    fill(g_lib.dense2csr_mask_bytes, "dense2csr_mask_bytes");
+    fill(g_lib.dense2csr_count, "dense2csr_count_mask");
+    fill(g_lib.dense2csr_fill, "dense2csr_fill_mask");
     fill(g_lib.quantize, "e2m1_quantize_device");
     fill(g_lib.transpose_workspace_bytes, "transpose_workspace_bytes");
     fill(g_lib.transpose, "transpose");
@@ -430,12 +433,19 @@ PyObject* py_dense2csr(PyObject*, PyObject* const* args, Py_ssize_t nargs)
         const WithoutGil nogil;
         const auto stream = current_stream(device);
         const float* data = address<float>(dense);
-        check(g_lib.dense2csr_count((int32_t)H, (int32_t)W, data, ld, tol, address<int32_t>(rp), &nnz, &longest, stream),
+        Scratch scratch;
+        uint32_t* mask = nullptr;
+        try {
+            mask = static_cast<uint32_t*>(
+                scratch.get(g_lib.dense2csr_mask_bytes((int32_t)H, (int32_t)W), c10::cuda::getCurrentCUDAStream(device.index())));
+        } catch (const c10::OutOfMemoryError&) {  // a bit per element more than the matrix: do without
+        }
+        check(g_lib.dense2csr_count((int32_t)H, (int32_t)W, data, ld, tol, address<int32_t>(rp), mask, &nnz, &longest, stream),
               "csrspmm_b200_dense2csr_count");
         ci = new_array(nnz, at::kInt, device);
         va = new_array(nnz, at::kFloat, device);
         if (nnz > 0)
-            check(g_lib.dense2csr_fill((int32_t)H, (int32_t)W, data, ld, tol, address<int32_t>(rp), address<int32_t>(ci),
+            check(g_lib.dense2csr_fill((int32_t)H, (int32_t)W, data, ld, tol, mask, address<int32_t>(rp), address<int32_t>(ci),
                                        address<float>(va), stream),
                   "csrspmm_b200_dense2csr_fill");
     }

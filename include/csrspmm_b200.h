@@ -325,6 +325,14 @@ int csrspmm_b200_dense2csr_count(int32_t H, int32_t W, const float* dense, int64
 int csrspmm_b200_dense2csr_fill(int32_t H, int32_t W, const float* dense, int64_t ld, float tol,
                                 const int32_t* row_ptr, int32_t* col_idx, float* values,
                                 csrspmm_b200_stream_t stream);
+/* The same in one reading of the matrix and a part of a second: _count_mask leaves one bit per element (mask:
+ * csrspmm_b200_dense2csr_mask_bytes(H, W) bytes of device memory), _fill_mask takes the entries from them.  Without
+ * room for them mask may be NULL in both: the fill reads the whole matrix again and tests against tol. */
+size_t csrspmm_b200_dense2csr_mask_bytes(int32_t H, int32_t W);
+int csrspmm_b200_dense2csr_count_mask(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, int32_t* row_ptr, uint32_t* mask,
+                                      int64_t* nnz_out, int32_t* max_row_nnz_out, csrspmm_b200_stream_t stream);
+int csrspmm_b200_dense2csr_fill_mask(int32_t H, int32_t W, const float* dense, int64_t ld, float tol, const uint32_t* mask, const int32_t* row_ptr,
+                                     int32_t* col_idx, float* values, csrspmm_b200_stream_t stream);
 int csrspmm_b200_csr2dense(int32_t H, int32_t W, const int32_t* row_ptr, const int32_t* col_idx,
                            const float* values, float* dense, int64_t ld, csrspmm_b200_stream_t stream);
 
