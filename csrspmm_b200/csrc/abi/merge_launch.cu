@@ -13,6 +13,15 @@ namespace csrspmm_b200 {
 
 namespace {
 
+// A build with a column guard, with stores for a padded B's rows of C where that is what runs.
+template <int G, int NV, int VW, int TG, int U, int FMT>
+cudaError_t launch_guarded(const SpmmParams& p, const Plan& plan, cudaStream_t st)
+{
+    if (VW == 4 && plan.c_ragged)
+        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, (VW == 4)>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
+    return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
+}
+
 template <int S, int VW, int FMT>
 cudaError_t launch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
@@ -27,14 +36,14 @@ cudaError_t launch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t st)
     const unsigned grid = (unsigned)plan.grid;
     if (ULONG != U && plan.tg == TG) {
         if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, ULONG, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
-        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, ULONG, FMT, false>, grid, kMergeThreads, 0, st, p);
+        return launch_guarded<G, NV, VW, TG, ULONG, FMT>(p, plan, st);
     }
     if (plan.small_tile) {  // few items: smaller tiles, more CTAs
         if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TGS, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
-        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TGS, U, FMT, false>, grid, kMergeThreads, 0, st, p);
+        return launch_guarded<G, NV, VW, TGS, U, FMT>(p, plan, st);
     }
     if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
-    return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, grid, kMergeThreads, 0, st, p);
+    return launch_guarded<G, NV, VW, TG, U, FMT>(p, plan, st);
 }
 
 // very narrow dense operands: lane groups of 1, 2 or 4 lanes (kNarrowShapes)
@@ -45,7 +54,7 @@ cudaError_t launch_merge_narrow(const SpmmParams& p, const Plan& plan, cudaStrea
     constexpr int U = merge_unroll(VW, NV);
     const unsigned grid = (unsigned)plan.grid;
     if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
-    return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, grid, kMergeThreads, 0, st, p);
+    return launch_guarded<G, NV, VW, TG, U, FMT>(p, plan, st);
 }
 
 template <int VW, int FMT>

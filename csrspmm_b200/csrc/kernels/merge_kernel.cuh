@@ -72,17 +72,42 @@ __device__ __forceinline__ int merge_search_warp(long long d, const int* __restr
     return lo;
 }
 
-// Same search inside the CTA's shared-memory slice (local coordinates).
-__device__ __forceinline__ int merge_search_local(int d, const int* s_rowend, int nrows, int nnzt)
+// Same search inside the CTA's shared-memory slice (local coordinates), for the two ends of a lane group's share at once: each step
+// every lane of the group probes one row for either end, and the votes say how many of the G equal parts lie before it.  One
+// lane after the other halving the range was two chains of eleven steps: 2600 cycles of a CTA's 53 000 with 16 lanes (65 536
+// rows of 16, 64 columns: 28.4 us), 1400 this way (27.1).
+template <int G>
+__device__ __forceinline__ void merge_search_local(int d0, int d1, const int* s_rowend, int nrows, int nnzt, int* i0, int* i1)
 {
-    int lo = max(0, d - nnzt);
-    int hi = min(d, nrows);
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (s_rowend[mid] <= d - mid - 1) lo = mid + 1;
-        else hi = mid;
+    const int lane = threadIdx.x % G;
+    int lo0 = max(0, d0 - nnzt), hi0 = min(d0, nrows), lo1 = max(0, d1 - nnzt), hi1 = min(d1, nrows);
+    if constexpr (G == 1) {
+        auto halve = [&](int d, int& lo, int hi) {
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (s_rowend[mid] <= d - mid - 1) lo = mid + 1;
+                else hi = mid;
+            }
+        };
+        halve(d0, lo0, hi0);
+        halve(d1, lo1, hi1);
+    } else {
+        // rows before the answer are those whose end lies on or before the diagonal: lane k probes the last row of part k
+        const unsigned group = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u)) << (threadIdx.x & 31 & ~(G - 1));
+        while (__any_sync(0xffffffffu, lo0 < hi0 || lo1 < hi1)) {
+            const int step0 = (hi0 - lo0 + G - 1) / G, step1 = (hi1 - lo1 + G - 1) / G;
+            const int at0 = lo0 + (lane + 1) * step0 - 1, at1 = lo1 + (lane + 1) * step1 - 1;
+            const bool below0 = at0 < hi0 && lo0 < hi0 && s_rowend[at0] <= d0 - at0 - 1;
+            const bool below1 = at1 < hi1 && lo1 < hi1 && s_rowend[at1] <= d1 - at1 - 1;
+            const unsigned votes0 = __ballot_sync(0xffffffffu, below0) & group, votes1 = __ballot_sync(0xffffffffu, below1) & group;
+            lo0 += __popc(votes0) * step0;
+            hi0 = min(hi0, lo0 + max(step0 - 1, 0));
+            lo1 += __popc(votes1) * step1;
+            hi1 = min(hi1, lo1 + max(step1 - 1, 0));
+        }
     }
-    return lo;
+    *i0 = lo0;
+    *i1 = lo1;
 }
 
 // TG: items per lane group it has room for (the launch says how many it takes, p.tg).
@@ -97,7 +122,13 @@ struct MergeSmem {
     int tail_row[GROUPS];
     unsigned longbits[TILE / 32 + 1];  // SKIP only: bit k = local row k is left to the scheduled pieces
     alignas(16) float tail[GROUPS][ROWW];
+    // the first row each group finishes, until the others have published their partial sums.  In registers it cost the walk its last
+    // ones: 128 columns, 262 144 Zipf rows 217 -> 214 us, 64 columns 103 -> 101, 24 columns 107 -> 103, 256 columns 167 -> 159;
+    // four vectors per lane have no room for it here, and eight or four bytes per lane no need
+    static constexpr bool HEADS = VW == 4 && NV <= 2;
+    alignas(16) float head[HEADS ? GROUPS : 1][HEADS ? ROWW : 4];
     __device__ __forceinline__ float* tail_of(int g) { return tail[g]; }
+    __device__ __forceinline__ float* head_of(int g) { return head[g]; }
     __device__ __forceinline__ bool is_long(int k) const { return (longbits[k >> 5] >> (k & 31)) & 1u; }
 };
 
@@ -258,9 +289,8 @@ __device__ __forceinline__ bool merge_tile_setup(const SpmmParams& p, Smem& s, T
     const int share = p.row_aligned ? (total + Smem::GROUPS - 1) / Smem::GROUPS : p.tg;
     const int dl0 = min(g * share, total);
     const int dl1 = min(dl0 + share, total);
-    r.il0 = merge_search_local(dl0, s.rowend, r.nrows, r.nnzt);
+    merge_search_local<G>(dl0, dl1, s.rowend, r.nrows, r.nnzt, &r.il0, &r.il1);
     r.jl0 = dl0 - r.il0;
-    r.il1 = merge_search_local(dl1, s.rowend, r.nrows, r.nnzt);
     r.jl1 = dl1 - r.il1;
     return true;
 }
@@ -427,7 +457,9 @@ __device__ __noinline__ void merge_rows_directly(const SpmmParams& p, const int 
 // scheduled pieces (sliced_kernel.cuh) and this kernel neither reads their entries nor writes
 // their rows of C.  The tiles still count those rows' items, so a tile inside a hub row is a
 // search and an exit.
-template <int G, int NV, int VW, int TG, int U, int FMT, bool FULL, bool SKIP = false>
+// RAGGED: also serves p.c_ragged, with VW = 4 and neither FULL nor SKIP.  A build of its own because its stores are compiled into
+// every row end of the walk (36 columns, 259 641 Zipf rows of 16: 111.6 us with them, 96.4 without; 100 columns 265 and 247).
+template <int G, int NV, int VW, int TG, int U, int FMT, bool FULL, bool SKIP = false, bool RAGGED = false>
 __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merge_kernel(const __grid_constant__ SpmmParams p)
 {
     wait_for_previous_grid();
@@ -452,11 +484,11 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
         for (int v = 0; v < NV; ++v) col_ok[v] = FULL || (cb + lane + v * G < p.ncolv);
 
         Vec<VW> acc[NV];
-        Vec<VW> head[NV];  // the first row this group finishes is held back until step 4
+        Vec<VW> head[NV];  // the first row this group finishes is held back until step 4 (HEADS: in s.head)
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             acc[v].zero();
-            head[v].zero();
+            if constexpr (!Smem::HEADS) head[v].zero();
         }
         int i = r.il0;
         int next_end = s.rowend[i];  // local position where row i ends (INT_MAX past the tile's rows)
@@ -470,9 +502,12 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
                 if (i == r.il0) head_skip = true;
             } else if (i == r.il0) {
 #pragma unroll
-                for (int v = 0; v < NV; ++v) head[v] = acc[v];
+                for (int v = 0; v < NV; ++v) {
+                    if constexpr (Smem::HEADS) acc[v].store(s.head_of(g) + (lane + v * G) * VW);
+                    else head[v] = acc[v];
+                }
             } else {
-                store_row<G, NV, VW, !FULL && !SKIP>(p, r.i0 + i, cb, lane, acc);
+                store_row<G, NV, VW, RAGGED>(p, r.i0 + i, cb, lane, acc);
             }
 #pragma unroll
             for (int v = 0; v < NV; ++v) acc[v].zero();
@@ -596,7 +631,11 @@ __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merg
         }  // !SKIP
         while (i < r.il1) finish_row();
 
-        merge_tile_finish<Smem, G, NV, VW, !FULL && !SKIP>(p, s, r, cb, g, lane, acc, head, dirty, head_skip);
+        if constexpr (Smem::HEADS) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) head[v].load(s.head_of(g) + (lane + v * G) * VW);  // this lane's own (nothing, if no row ended)
+        }
+        merge_tile_finish<Smem, G, NV, VW, RAGGED>(p, s, r, cb, g, lane, acc, head, dirty, head_skip);
         if (cb + G * NV < p.ncolv) __syncthreads();  // tails are rewritten by the next pass
     }
 }

@@ -207,8 +207,10 @@
 // lanes per group G, vectors per lane NV, merge-path items per group TG.  TG = 192 against 128:
 // fewer, longer-lived CTAs (one search, one staging round and one carry row each) -- config 3
 // 686 -> 654 us, the same matrix at Nd = 128 1361 -> 1285 us, config 5 at a quarter of its rows
-// 10.26 -> 10.04 ms; 224-256 gained nothing more and TG = 256 at G = 16 no longer fits the 48 KB
-// of static shared memory
+// 10.26 -> 10.04 ms; 224-384 gained nothing more at G = 32, whose walks wait for HBM, and TG = 256 at G = 16 no longer
+// fits the 48 KB of static shared memory.  G = 8: 96, the same 3072 items per CTA as G = 16 (64 before): 32 columns, 1 M
+// Zipf rows of 12 244 -> 226 us, 400 000 of 6 76 -> 72, 2 M of 4 268 -> 251, 500 000 even rows of 10 94.7 -> 90.7; 20 columns,
+// 300 000 of 30 140 -> 128
 #ifndef CSRSPMM_TUNE_S0_G
 #define CSRSPMM_TUNE_S0_G 8
 #endif
@@ -216,7 +218,7 @@
 #define CSRSPMM_TUNE_S0_NV 1
 #endif
 #ifndef CSRSPMM_TUNE_S0_TG
-#define CSRSPMM_TUNE_S0_TG 64
+#define CSRSPMM_TUNE_S0_TG 96
 #endif
 #ifndef CSRSPMM_TUNE_S1_G
 #define CSRSPMM_TUNE_S1_G 16
