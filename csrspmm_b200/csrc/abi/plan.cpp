@@ -283,12 +283,13 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
             if (a->nnz <= (long long)CSRSPMM_TUNE_ROW_PERSISTENT_MAX_MEAN * (long long)a->M && plan->grid > (long long)kSms * CSRSPMM_TUNE_ROW_PERSISTENT)
                 plan->grid = (long long)kSms * CSRSPMM_TUNE_ROW_PERSISTENT;
 #endif
+            if (plan->VW == 4 && !plan->low_occupancy && !plan->short_rows) plan->row_build = row_build_for(plan->G, plan->NV, plan->grid);
         }
     }
     // A next grid placed early goes where slots are free.  Behind a grid that fills the chip those are the slots
     // its CTAs leave, one by one and evenly; behind a smaller one they crowd on the SMs that had room, and the
     // crowded SMs finish late (4096 rows of 410 entries, 128 columns: 46.2 us per product against 43.4).
-    const int resident_ctas = kernel == CSRSPMM_B200_KERNEL_ROW     ? (plan->low_occupancy ? 2 : row_min_blocks(plan->NV))
+    const int resident_ctas = kernel == CSRSPMM_B200_KERNEL_ROW     ? (plan->low_occupancy ? 2 : plan->row_build ? row_build(plan->NV, plan->row_build).MINB : row_min_blocks(plan->NV))
                               : kernel == CSRSPMM_B200_KERNEL_MERGE ? merge_min_blocks(plan->NV)
                                                                     : CSRSPMM_TUNE_TMA_MINB;
     plan->fills_chip = plan->grid >= (long long)kSms * resident_ctas;

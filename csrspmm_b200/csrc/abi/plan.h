@@ -22,6 +22,7 @@ struct Plan {
     bool c_ragged = false;                 // kPlanPadded: the last vector of a row of C is partly beyond it
     bool rows_even = false;                // AUTO: the longest row is known to be close to the mean
     bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
+    int row_build = 0;                     // row kernel, long rows, vector width 4: row_build_for()
     bool full = false;                     // one pass covers the row exactly: G*NV == ncolv
     bool row_aligned = false;              // merge kernel: tiles cut at row starts, no carries and no fix-up
     bool small_tile = false;               // merge kernel: the build with shared memory for small tiles

@@ -323,6 +323,33 @@ constexpr int row_unroll(int vw, int g, int nv, bool full, bool short_rows)
     return short_rows && (vw == 2 || (full && g <= 16)) ? CSRSPMM_TUNE_ROW_U_SHORT : CSRSPMM_TUNE_ROW_U_NV1;
 }
 
+// Row kernel on long rows (a mean above CSRSPMM_TUNE_ROW_SHORT_MEAN), where the grid is a wave or two and a wave lasts as long as
+// a row: more rows of B in flight and fewer CTAs per SM where the grid does not fill them, or would leave a nearly empty wave behind.
+// Build k = 1 .. 3: U rows in flight at MINB CTAs per SM, for grids of (over, upto] CTAs; 0: as for long grids.  128 columns, rows
+// of 400: 2368 rows 30.9 -> 28.7 us, 1250 30.9 -> 24.7, 5200 75.5 -> 63.1, and with one row more (2420) 44.0 against 31.1.  256
+// columns: 2368 rows 50.8 -> 42.5, 5200 123 -> 107.  512 columns: 3000 rows 129 -> 103, 5200 184 -> 156 (2300 the other way
+// round: 72 and 100).  64 columns, rows of 60: 4600 12.4 -> 10.4, 10 400 20.7 -> 18.6; 32 columns: 9200 14.5 -> 12.4, 12 000
+// of 150 26.8 -> 22.7, 16 560 30.9 -> 26.8.  Rows of 60 gain less and lose nothing (128 columns: 1700 9.1 -> 8.4).
+struct RowBuild {
+    int U, MINB;
+};
+constexpr RowBuild row_build(int nv, int k)
+{
+    if (nv == 1) return k == 1 ? RowBuild{16, 4} : (k == 2 ? RowBuild{8, 6} : RowBuild{8, 7});
+    return nv == 2 ? RowBuild{6, 4} : RowBuild{4, 3};
+}
+constexpr int row_build_for(int g, int nv, long long grid)
+{
+    if (nv == 1) {
+        if (grid <= kSms * 4) return 1;
+        if (g <= 16 && grid <= kSms * 6) return 2;
+        if (g <= 16 && grid <= kSms * 7) return 3;
+        return grid > kSms * 8 && grid <= kSms * 12 ? 2 : 0;
+    }
+    if (nv == 2) return grid <= kSms * 4 || (grid > kSms * 8 && grid <= kSms * 10) ? 1 : 0;
+    return (grid > kSms * 4 && grid <= kSms * 6) || (grid > kSms * 8 && grid <= kSms * 9) ? 1 : 0;
+}
+
 constexpr int row_min_blocks(int nv) { return nv == 1 ? CSRSPMM_TUNE_ROW_MINB_NV1 : (nv == 2 ? CSRSPMM_TUNE_ROW_MINB_NV2 : CSRSPMM_TUNE_ROW_MINB_NV4); }
 constexpr int merge_min_blocks(int nv) { return nv == 1 ? CSRSPMM_TUNE_MERGE_MINB_NV1 : (nv == 2 ? CSRSPMM_TUNE_MERGE_MINB_NV2 : CSRSPMM_TUNE_MERGE_MINB_NV4); }
 
