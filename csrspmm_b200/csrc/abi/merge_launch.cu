@@ -17,8 +17,10 @@ namespace {
 template <int G, int NV, int VW, int TG, int U, int FMT>
 cudaError_t launch_guarded(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
-    if (VW == 4 && plan.c_ragged)
-        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, (VW == 4)>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
+    if (VW == 4 && plan.c_ragged == kRaggedPairs)
+        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, VW == 4 ? kRaggedPairs : 0>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
+    if (VW == 4 && plan.c_ragged == kRaggedFloats)
+        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, VW == 4 ? kRaggedFloats : 0>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
     return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
 }
 

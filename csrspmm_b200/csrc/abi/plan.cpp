@@ -195,7 +195,8 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
     const bool pairs = !vec && !padded && (flags & kPlanNoPairs) == 0 && a->nnz <= kWholeRowEntries && pair_layout_ok(a);
     plan->VW = vec || padded ? 4 : (pairs ? 2 : 1);
     plan->ncolv = (a->Nd + plan->VW - 1) / plan->VW;
-    plan->c_ragged = padded;
+    const bool c_pairs = a->Nd % 2 == 0 && a->ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(a->C) & 7u) == 0;
+    plan->c_ragged = padded ? (c_pairs ? 2 : 1) : 0;
     plan->num_items = (long long)a->M + a->nnz;
 
     int kernel = a->kernel;
@@ -305,8 +306,11 @@ size_t padded_b_bytes(const csrspmm_b200_args* a)
     if (a->Nd % 4 == 0 || a->Nd < 17 || a->M <= 0 || a->Kd <= 0 || a->kernel == CSRSPMM_B200_KERNEL_TMA || a->nnz > kWholeRowEntries) return 0;
     const double mean = (double)a->nnz / a->M, uses = (double)a->nnz / a->Kd;
     const double gather = (double)a->nnz * a->Nd * 4.0;
+    const int pairs = a->Nd / 2, slots = pairs <= 32 ? 32 : (pairs <= 64 ? 64 : 128);
+    const bool lanes_idle = a->Nd > 32 && a->Nd <= 256 && pairs * 100 <= slots * 85;
+    const double even_uses = a->Nd <= 32 ? (a->Nd == 30 ? 16.0 : 48.0) : (lanes_idle ? (slots == 64 ? 24.0 : 11.0) : 64.0);
     const bool pays = a->Nd % 2 ? uses >= (a->Nd <= 256 ? 8.0 : 24.0) && gather >= 64e6 && (a->Nd >= 32 || mean <= 64.0)
-                                : uses >= 64.0 && a->Nd >= 96 && gather >= 256e6;
+                                : uses >= even_uses && gather >= 250e6 && (a->Nd <= 32 || lanes_idle || a->Nd >= 96);
     return pays ? align_up((size_t)a->Kd * (size_t)((a->Nd + 3) / 4) * 16, 256) : 0;
 }
 

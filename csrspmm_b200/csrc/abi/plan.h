@@ -19,7 +19,7 @@ struct Plan {
     bool low_occupancy = false;            // row kernel: fewer than 8 warps of rows per SM
     bool any_count = false;                // whole-row mapping of more than kWholeRowEntries entries: the panel kernel, one pass
     int resident = 0;                      // whole-row mapping by the resident kernel: lanes per group (16, 32), else 0
-    bool c_ragged = false;                 // kPlanPadded: the last vector of a row of C is partly beyond it
+    int c_ragged = 0;                      // kPlanPadded: the last vector of a row of C is partly beyond it (SpmmParams::c_ragged)
     bool rows_even = false;                // AUTO: the longest row is known to be close to the mean
     bool short_rows = false;               // row kernel: mean of CSRSPMM_TUNE_ROW_SHORT_MEAN entries or fewer
     int row_build = 0;                     // row kernel, long rows, vector width 4: row_build_for()
@@ -74,9 +74,14 @@ size_t worst_case_workspace(const csrspmm_b200_args* a);
 // 57 or 150 columns start on any 4 or 8 bytes, and gathered one or two floats per lane they come at half the rate; a copy
 // costs B read and written once, which eight uses of each row repay for odd widths (200 000 rows of 8, 19 columns 68 -> 37
 // us, 57 columns 81 -> 71; 20 000 rows of 24, 201 columns 61 -> 35; wider than 256 from 24 on: 200 000 of 8, 323 columns
-// 430 and 445) and 64 for even ones (100 000 rows of 16 over 5000, 150 columns 113 -> 90; 20 000 of 100, 510 columns 260 ->
-// 240).  Below 64 MB of gather (256 for even widths) the launch costs more than it gives, and long rows of few columns
-// leave too few lane groups when they are cut to vectors (20 000 of 100, 19 columns 30 -> 35).
+// 430 and 445).  Even widths, whose rows of C are written in pairs, gain where their pairs leave lanes idle, from eleven uses on
+// (300 000 even rows of 10 over 200 000, 50 columns 120 -> 97; 300 000 Zipf rows of 12, 130 columns 430 -> 373; 100 000 of
+// 12, 150 columns 111 -> 100; with 59 of 64 lanes at work 33.9 and 35.5, with 31 of 32 87.6 and 87.3), of which 66 to 108
+// columns have two pairs per lane already and need 24 (90 columns, 30 uses 82 -> 78; 98, 12 uses 31.9 and 35.1); up to 32 columns
+// 30 from 16 on, eight whole vectors (500 000 of 14 142 -> 122), the others from 48 (22 columns, 150 uses 47 -> 41; 26, 30
+// uses 59 and 60); the rest from 64 uses on (20 000 of 100, 510 columns 260 -> 240).  Below 64 MB of gather (250 for even widths: 50 columns, 220 MB 45.6 and 45.9) the launch costs more
+// than it gives, and long rows of few columns leave too few lane groups when they are cut to vectors (20 000 of 100, 19
+// columns 30 -> 35).
 size_t padded_b_bytes(const csrspmm_b200_args* a);
 
 void set_last_error(const char* fmt, ...);

@@ -46,6 +46,7 @@ struct SpmmParams {
     float beta;
     int tg;              // split kernels: merge-path items per lane group (Plan::tg)
     int c_ragged;        // B is a padded copy: vectors of four columns, the last of a row of C partly beyond Nd, C unaligned
+                         // (kRaggedFloats) or on 8 bytes with an even Nd (kRaggedPairs)
     int row_aligned;     // merge kernel: tiles are cut at row starts and leave no carries (Plan::row_aligned)
     int* carry_row;      // one per tile: row the tile leaves unfinished, or -1
     float* carry_val;    // one row of carry_ld floats per tile
@@ -337,9 +338,25 @@ struct Vec<1> {
     }
 };
 
-// Write one finished row segment: C[row, cv] = alpha*acc + beta*C_old for this lane's NV vectors.  RAGGED: the build
-// also serves p.c_ragged, whose rows of C are written float by float.
-template <int G, int NV, int VW, bool RAGGED = false>
+// How rows of C are written that a padded copy of B gives (SpmmParams::c_ragged)
+constexpr int kRaggedFloats = 1, kRaggedPairs = 2;
+
+// `part` of a vector at its place in C
+template <int W>
+__device__ __forceinline__ void store_part(const SpmmParams& p, const Vec<W>& part, float* at)
+{
+    if (p.beta != 0.0f) {
+        Vec<W> old;
+        old.load(at);
+        part.epilogue(p.alpha, p.beta, old).store(at);
+    } else {
+        part.epilogue0(p.alpha).store(at);
+    }
+}
+
+// Write one finished row segment: C[row, cv] = alpha*acc + beta*C_old for this lane's NV vectors.  RAGGED: the values of
+// p.c_ragged that the build serves besides 0 (OR-ed); one alone is taken for granted.
+template <int G, int NV, int VW, int RAGGED = 0>
 __device__ __forceinline__ void store_row(const SpmmParams& p, int row, int cb, int lane,
                                           const Vec<VW> (&acc)[NV])
 {
@@ -349,22 +366,24 @@ __device__ __forceinline__ void store_row(const SpmmParams& p, int row, int cb, 
         const int cv = cb + lane + v * G;
         if (cv < p.ncolv) {
             float* cp = crow + (long long)cv * VW;
-            if constexpr (RAGGED && VW == 4) {
-                if (p.c_ragged) {
+            if constexpr ((RAGGED & kRaggedPairs) != 0 && VW == 4) {
+                if (RAGGED == kRaggedPairs || p.c_ragged == kRaggedPairs) {
+                    Vec<2> half;
+                    half.v = make_float2(acc[v].v.x, acc[v].v.y);
+                    store_part(p, half, cp);
+                    half.v = make_float2(acc[v].v.z, acc[v].v.w);
+                    if (cv * 4 + 2 < p.Nd) store_part(p, half, cp + 2);
+                    continue;
+                }
+            }
+            if constexpr ((RAGGED & kRaggedFloats) != 0 && VW == 4) {
+                if (RAGGED == kRaggedFloats || p.c_ragged == kRaggedFloats) {
                     const float sum[4] = {acc[v].v.x, acc[v].v.y, acc[v].v.z, acc[v].v.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        if (cv * 4 + e < p.Nd) {
-                            Vec<1> one;
-                            one.v = sum[e];
-                            if (p.beta != 0.0f) {
-                                Vec<1> old;
-                                old.load(cp + e);
-                                one.epilogue(p.alpha, p.beta, old).store(cp + e);
-                            } else {
-                                one.epilogue0(p.alpha).store(cp + e);
-                            }
-                        }
+                        Vec<1> one;
+                        one.v = sum[e];
+                        if (cv * 4 + e < p.Nd) store_part(p, one, cp + e);
                     }
                     continue;
                 }

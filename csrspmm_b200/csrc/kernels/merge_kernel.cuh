@@ -349,7 +349,7 @@ __device__ __forceinline__ void merge_carry_by_warp(const SpmmParams& p, Smem& s
 // Steps 4-5 for one column pass.  acc = the group's unfinished partial sum (valid when dirty),
 // head = its held-back first finished row (valid when il1 > il0).  Contains one __syncthreads.
 // head_skip: the group's first finished row belongs to the scheduled pieces and is not written.
-template <class Smem, int G, int NV, int VW, bool RAGGED = false>
+template <class Smem, int G, int NV, int VW, int RAGGED = 0>
 __device__ __forceinline__ void merge_tile_finish(const SpmmParams& p, Smem& s, const TileRange& r,
                                                   int cb, int g, int lane, const Vec<VW> (&acc)[NV],
                                                   Vec<VW> (&head)[NV], bool dirty, bool head_skip = false)
@@ -447,7 +447,7 @@ __device__ __noinline__ void merge_rows_directly(const SpmmParams& p, const int 
                     }
                 }
             }
-            store_row<G, NV, VW, true>(p, row, cb, lane, acc);
+            store_row<G, NV, VW, kRaggedFloats | kRaggedPairs>(p, row, cb, lane, acc);
         }
     }
 }
@@ -457,9 +457,9 @@ __device__ __noinline__ void merge_rows_directly(const SpmmParams& p, const int 
 // scheduled pieces (sliced_kernel.cuh) and this kernel neither reads their entries nor writes
 // their rows of C.  The tiles still count those rows' items, so a tile inside a hub row is a
 // search and an exit.
-// RAGGED: also serves p.c_ragged, with VW = 4 and neither FULL nor SKIP.  A build of its own because its stores are compiled into
+// RAGGED: for this value of p.c_ragged, with VW = 4 and neither FULL nor SKIP.  Builds of their own because its stores are compiled into
 // every row end of the walk (36 columns, 259 641 Zipf rows of 16: 111.6 us with them, 96.4 without; 100 columns 265 and 247).
-template <int G, int NV, int VW, int TG, int U, int FMT, bool FULL, bool SKIP = false, bool RAGGED = false>
+template <int G, int NV, int VW, int TG, int U, int FMT, bool FULL, bool SKIP = false, int RAGGED = 0>
 __global__ void __launch_bounds__(kMergeThreads, merge_min_blocks(NV)) spmm_merge_kernel(const __grid_constant__ SpmmParams p)
 {
     wait_for_previous_grid();

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) spmm_row_kernel(const SpmmP
 #undef ROW_COL
 #undef ROW_VAL
         }
-        store_row<G, NV, VW, !FULL>(p, row, cb, lane, acc);
+        store_row<G, NV, VW, FULL ? 0 : kRaggedFloats | kRaggedPairs>(p, row, cb, lane, acc);
     }
     }
 }

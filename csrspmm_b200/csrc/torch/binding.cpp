@@ -210,8 +210,14 @@ at::Tensor run_product(Product& q)
                 a.workspace_bytes = q.workspace.nbytes();
                 if (q.workspace.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(q.workspace.storage().data_ptr(), stream);
             } else {
-                a.workspace = scratch.get(need, stream);
-                a.workspace_bytes = std::max<size_t>(need, 256);
+                try {
+                    a.workspace = scratch.get(need, stream);
+                    a.workspace_bytes = std::max<size_t>(need, 256);
+                } catch (const c10::OutOfMemoryError&) {
+                    // no room for a padded copy of B: without a workspace the library does without the copy
+                    a.workspace = nullptr;
+                    a.workspace_bytes = 0;
+                }
             }
         }
     }

@@ -33,6 +33,31 @@ def test_padded_copy(cuda_lib, Nd, kernel, skew, beta):
     assert int(status) == 0 and (np.abs(got - f64) <= 1e-5 * mag + 1e-6).all()
 
 
+# even widths: C in pairs, or (an odd leading dimension, a start off 8 bytes) float by float
+@pytest.mark.parametrize("Nd", [18, 22, 30, 32 + 2, 66, 98, 130, 254])
+@pytest.mark.parametrize("kernel,beta", [("row", 0.5), ("merge", 0.0)])
+@pytest.mark.parametrize("ldc,start", [(0, 0), (2, 0), (1, 0), (0, 1)])
+def test_padded_copy_of_even_widths(cuda_lib, Nd, kernel, beta, ldc, start):
+    rng = np.random.default_rng(Nd)
+    M, Kd = 6001, 2500
+    mean = int(255e6 / 4 / Nd / M) + 2
+    lens = rng.integers(mean - mean // 8, mean + mean // 4, M)
+    lens[5] = 0
+    p = G.random_csr(M, Kd, Nd, 0.0, seed=3, lengths=np.minimum(lens, Kd))
+    # (254: 127 of 128 pairs at work, from 64 uses on)
+    assert ops.plan_info(M, Kd, Nd, p.nnz, kernel=kernel, max_row_nnz=int(lens.max()), workspace=True)["padded_copy"]
+    t = [torch.from_numpy(x).cuda() for x in (p.row_ptr, p.col_idx, p.values, p.B)]
+    C0 = rng.standard_normal((M, Nd + ldc), dtype=np.float32)
+    C = torch.full((M * (Nd + ldc) + start,), 7.0, device="cuda")[start:].view(M, Nd + ldc)
+    C.copy_(torch.from_numpy(C0))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.spmm(*t, C[:, :Nd], 1.5, beta, kernel=kernel, max_row_nnz=int(lens.max()), status_word=status, sync=True)
+    got = C.cpu().numpy()
+    f64, mag = oracle.spmm_f64(p.row_ptr, p.col_idx, p.values, p.B, C0[:, :Nd], 1.5, beta, threads=4)
+    assert int(status) == 0 and (np.abs(got[:, :Nd] - f64) <= 1e-5 * mag + 1e-6).all()
+    assert np.array_equal(got[:, Nd:], C0[:, Nd:])  # nothing beyond the rows
+
+
 def test_the_copy_is_counted_as_scratch():
     assert ops.workspace_bytes(200000, 200000, 57, 1_600_000) >= ops.workspace_bytes(200000, 200000, 60, 1_600_000) + 200000 * 240 - 256
 
