@@ -122,7 +122,7 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
     auto pairs = [&](size_t off) { return reinterpret_cast<int2*>(ws + off); };
     long long* results = reinterpret_cast<long long*>(ws + p.results);
     for (int k = 0; k < p.passes; ++k) {
-        const DigitPass ps = {k * p.digit_bits, p.digit_bits, 1 << p.digit_bits, p.tiles, nnz};
+        const DigitPass ps = {k * p.digit_bits, 1 << p.digit_bits, p.tiles, nnz};
         const bool first = k == 0, last = k == p.passes - 1;
         const int* keys = first ? col_idx : ints(p.buffer[(k - 1) & 1]);
         const int2* in = first ? nullptr : pairs(p.pairs[(k - 1) & 1]);

@@ -28,7 +28,6 @@ namespace csrspmm_b200 {
 constexpr int kConvertThreads = 256;
 constexpr int kChunkQuads = 4;                      // float4 per lane and chunk
 constexpr int kChunkCols = 32 * 4 * kChunkQuads;    // columns per warp and chunk
-
 constexpr int kSpanCols = 32 * 32;                  // columns per warp and round of the fill
 
 // Warps side by side on one row: as many as there are chunks (spans, for the fill) of `cols` columns, at most the CTA.

@@ -33,7 +33,7 @@ constexpr int kMaxDigitBits = 8;
 constexpr int kMaxDigits = 1 << kMaxDigitBits;
 
 struct DigitPass {
-    int shift, bits, digits;  // digit of key k = (k >> shift) & (digits - 1); digits = 1 << bits
+    int shift, digits;  // digit of key k = (k >> shift) & (digits - 1); digits a power of two
     int tiles;
     long long n;        // entries
 };
