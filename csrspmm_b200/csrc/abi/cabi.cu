@@ -100,11 +100,12 @@ cudaError_t launch_row_full(const SpmmParams& p, const Plan& plan, cudaStream_t 
             constexpr RowBuild b = row_build(NV, decltype(k)::value);
             return launch_overlapped(spmm_row_kernel<G, NV, VW, b.U, FMT, FULL, b.MINB>, grid, kRowThreads, 0, st, p);
         };
-        if (plan.row_build == 1) return build(std::integral_constant<int, 1>());
-        if constexpr (NV == 1) {
+        if constexpr (row_build_used(G, NV, FULL, 1))
+            if (plan.row_build == 1) return build(std::integral_constant<int, 1>());
+        if constexpr (row_build_used(G, NV, FULL, 2))
             if (plan.row_build == 2) return build(std::integral_constant<int, 2>());
+        if constexpr (row_build_used(G, NV, FULL, 3))
             if (plan.row_build == 3) return build(std::integral_constant<int, 3>());
-        }
     }
     if (plan.short_rows) return launch_overlapped(spmm_row_kernel<G, NV, VW, USHORT, FMT, FULL, MINB>, grid, kRowThreads, 0, st, p);
     return launch_overlapped(spmm_row_kernel<G, NV, VW, ULONG, FMT, FULL, MINB>, grid, kRowThreads, 0, st, p);

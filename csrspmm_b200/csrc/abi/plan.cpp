@@ -284,7 +284,7 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
             if (a->nnz <= (long long)CSRSPMM_TUNE_ROW_PERSISTENT_MAX_MEAN * (long long)a->M && plan->grid > (long long)kSms * CSRSPMM_TUNE_ROW_PERSISTENT)
                 plan->grid = (long long)kSms * CSRSPMM_TUNE_ROW_PERSISTENT;
 #endif
-            if (plan->VW == 4 && !plan->low_occupancy && !plan->short_rows) plan->row_build = row_build_for(plan->G, plan->NV, plan->grid);
+            if (plan->VW == 4 && !plan->low_occupancy && !plan->short_rows) plan->row_build = row_build_for(plan->G, plan->NV, plan->full, plan->grid);
         }
     }
     // A next grid placed early goes where slots are free.  Behind a grid that fills the chip those are the slots

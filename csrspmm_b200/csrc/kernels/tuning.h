@@ -325,11 +325,18 @@ constexpr int row_unroll(int vw, int g, int nv, bool full, bool short_rows)
 
 // Row kernel on long rows (a mean above CSRSPMM_TUNE_ROW_SHORT_MEAN), where the grid is a wave or two and a wave lasts as long as
 // a row: more rows of B in flight and fewer CTAs per SM where the grid does not fill them, or would leave a nearly empty wave behind.
-// Build k = 1 .. 3: U rows in flight at MINB CTAs per SM, for grids of (over, upto] CTAs; 0: as for long grids.  128 columns, rows
-// of 400: 2368 rows 30.9 -> 28.7 us, 1250 30.9 -> 24.7, 5200 75.5 -> 63.1, and with one row more (2420) 44.0 against 31.1.  256
-// columns: 2368 rows 50.8 -> 42.5, 5200 123 -> 107.  512 columns: 3000 rows 129 -> 103, 5200 184 -> 156 (2300 the other way
-// round: 72 and 100).  64 columns, rows of 60: 4600 12.4 -> 10.4, 10 400 20.7 -> 18.6; 32 columns: 9200 14.5 -> 12.4, 12 000
-// of 150 26.8 -> 22.7, 16 560 30.9 -> 26.8.  Rows of 60 gain less and lose nothing (128 columns: 1700 9.1 -> 8.4).
+// Grids in CTAs per SM.  Every line was measured on both sides: 870 products, rows of 49 to 900 entries, B of 0.1 to 240 MB, a quarter of
+// them packed (the long grids' time over this build's, mean and range).  "Full": every lane at work (32, 64, 128, 256 columns).
+//   1  one vector per lane, up to 4: 16 or 32 lanes 1.12, 0.99-1.25; eight, full 1.19, 1.05-1.31 (not full 1.00, 0.91-1.04)
+//      two, up to 4: 1.36, 1.19-1.63; 8 to 10: 1.06, 0.95-1.18
+//      four, 4 to 6: 1.16, 1.07-1.31; 8 to 9: 1.12, 0.98-1.21
+//   2  8 to 12: eight lanes 1.09, 1.00-1.37; sixteen, full 1.12, 1.01-1.21, not full 1.00, 0.94-1.13; 32, full 1.09, 0.93-1.23, not full 1.03,
+//      0.94-1.19
+//      up to 6: eight lanes 1.04, 0.97-1.20; sixteen, full 1.07, 0.97-1.12 (not full 0.96, 0.94-0.98: 48 columns, rows of 115 15.8 and
+//      16.5 us)
+//   3  6 to 7: eight or sixteen lanes, full 1.11, 1.08-1.14 (32 columns, rows of 595 94.2 and 82.3; not full 0.91, 0.85-0.96: 24 columns,
+//      rows of 323 55.9 and 62.1)
+// Elsewhere each of them loses (6 to 8, build 2: 0.69, 0.58-0.85).
 struct RowBuild {
     int U, MINB;
 };
@@ -338,16 +345,23 @@ constexpr RowBuild row_build(int nv, int k)
     if (nv == 1) return k == 1 ? RowBuild{16, 4} : (k == 2 ? RowBuild{8, 6} : RowBuild{8, 7});
     return nv == 2 ? RowBuild{6, 4} : RowBuild{4, 3};
 }
-constexpr int row_build_for(int g, int nv, long long grid)
+// 0: the long grids' build
+constexpr int row_build_for(int g, int nv, bool full, long long grid)
 {
     if (nv == 1) {
-        if (grid <= kSms * 4) return 1;
-        if (g <= 16 && grid <= kSms * 6) return 2;
-        if (g <= 16 && grid <= kSms * 7) return 3;
+        if (grid <= kSms * 4) return g >= 16 || full ? 1 : 2;
+        if (g <= 16 && grid <= kSms * 6) return full || g == 8 ? 2 : 0;
+        if (g <= 16 && grid <= kSms * 7) return full ? 3 : 0;
         return grid > kSms * 8 && grid <= kSms * 12 ? 2 : 0;
     }
     if (nv == 2) return grid <= kSms * 4 || (grid > kSms * 8 && grid <= kSms * 10) ? 1 : 0;
     return (grid > kSms * 4 && grid <= kSms * 6) || (grid > kSms * 8 && grid <= kSms * 9) ? 1 : 0;
+}
+// What row_build_for can answer.
+constexpr bool row_build_used(int g, int nv, bool full, int k)
+{
+    if (nv > 1) return k == 1;
+    return k == 1 ? g >= 16 || full : k == 2 || (g <= 16 && full);
 }
 
 constexpr int row_min_blocks(int nv) { return nv == 1 ? CSRSPMM_TUNE_ROW_MINB_NV1 : (nv == 2 ? CSRSPMM_TUNE_ROW_MINB_NV2 : CSRSPMM_TUNE_ROW_MINB_NV4); }

@@ -2,6 +2,7 @@
 // nothing, and one chosen call fails.  Linked with the library's objects in place of the real runtime
 // (csrspmm_b200/build.py), so that every way out of a failed call can be walked through on the CPU.
 #include <cuda_runtime_api.h>
+#include <cxxabi.h>
 
 #include <atomic>
 #include <cstdlib>
@@ -9,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <set>
+#include <string>
 
 namespace {
 
@@ -26,6 +28,25 @@ std::atomic<long> g_streams{0};  // made and not destroyed
 cudaError_t g_last = cudaSuccess;
 char g_handles[4096];
 size_t g_next_handle = 0;
+std::set<std::string> g_launched;  // names of the kernels launched since the last reset
+
+// The library's kernels by the address they are launched with.  Registered while its objects are loaded, which may be before this
+// file's own variables are.
+std::map<const void*, std::string>& kernels()
+{
+    static std::map<const void*, std::string> by_address;
+    return by_address;
+}
+
+// Copies the names, a line each, to `out` (null: only asks for the room they take).
+template <class Names>
+size_t list_names(const Names& names, char* out)
+{
+    std::string all;
+    for (const std::string& n : names) all += n + "\n";
+    if (out != nullptr) std::memcpy(out, all.c_str(), all.size() + 1);
+    return all.size() + 1;
+}
 
 // Counts a call that can fail.
 cudaError_t call(cudaError_t error = cudaErrorUnknown)
@@ -91,7 +112,15 @@ void fake_reset(long fail_at)
     g_last = cudaSuccess;
     g_busy.clear();
     g_after.clear();
+    g_launched.clear();
 }
+size_t fake_kernels(char* out)
+{
+    std::set<std::string> names;
+    for (const auto& k : kernels()) names.insert(k.second);
+    return list_names(names, out);
+}
+size_t fake_launched(char* out) { return list_names(g_launched, out); }
 long fake_calls() { return g_calls; }
 long fake_live() { return (long)g_live.size(); }
 long fake_settings() { return g_settings; }
@@ -247,6 +276,7 @@ cudaError_t cudaFuncSetAttribute(const void* kernel, cudaFuncAttribute, int valu
 cudaError_t launch(const void* kernel, size_t smem, cudaStream_t st)
 {
     return work_on(st, [&] {
+        g_launched.insert(kernels()[kernel]);
         const auto allowed = g_smem.find(kernel);
         if (smem > (size_t)(allowed != g_smem.end() ? allowed->second : 48 << 10)) ++g_refused;
     });
@@ -266,7 +296,12 @@ const char* cudaGetErrorString(cudaError_t) { return "injected"; }
 void** __cudaRegisterFatBinary(void*) { return reinterpret_cast<void**>(g_handles); }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+void __cudaRegisterFunction(void**, const char* address, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*)
+{
+    char* plain = abi::__cxa_demangle(name, nullptr, nullptr, nullptr);
+    kernels()[address] = plain != nullptr ? plain : name;
+    std::free(plain);
+}
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 static thread_local struct { dim3 grid, block; size_t smem; void* stream; } t_launch;
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, void* stream)
