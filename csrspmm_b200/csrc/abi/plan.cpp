@@ -301,16 +301,30 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
     return CSRSPMM_B200_OK;
 }
 
+// The rules' figures are beside padded_b_bytes's declaration.
+static bool odd_copy_pays(int Nd, double mean, double uses, double gather)
+{
+    return uses >= (Nd <= 256 ? 8.0 : 24.0) && gather >= 64e6 && (Nd >= 32 || mean <= 64.0);
+}
+
+static bool even_copy_pays(int M, int Nd, double mean, double uses, double gather)
+{
+    if (gather < 250e6) return false;
+    if (Nd <= 32) {
+        constexpr int wave = kSms * CSRSPMM_TUNE_ROW_MINB_NV1 * (CSRSPMM_TUNE_ROW_THREADS / CSRSPMM_TUNE_S0_G);  // rows of eight lanes each
+        return uses >= (Nd == 30 ? 16.0 : 48.0) && (mean <= 64.0 || M <= wave || M > wave + wave / 2);
+    }
+    const int pairs = Nd / 2, slots = pairs <= 32 ? 32 : (pairs <= 64 ? 64 : 128);
+    const bool lanes_idle = Nd <= 256 && pairs * 100 <= slots * 85;
+    return lanes_idle ? uses >= (slots == 128 ? 11.0 : 24.0) : uses >= 64.0 && Nd >= 96;
+}
+
 size_t padded_b_bytes(const csrspmm_b200_args* a)
 {
     if (a->Nd % 4 == 0 || a->Nd < 17 || a->M <= 0 || a->Kd <= 0 || a->kernel == CSRSPMM_B200_KERNEL_TMA || a->nnz > kWholeRowEntries) return 0;
     const double mean = (double)a->nnz / a->M, uses = (double)a->nnz / a->Kd;
     const double gather = (double)a->nnz * a->Nd * 4.0;
-    const int pairs = a->Nd / 2, slots = pairs <= 32 ? 32 : (pairs <= 64 ? 64 : 128);
-    const bool lanes_idle = a->Nd > 32 && a->Nd <= 256 && pairs * 100 <= slots * 85;
-    const double even_uses = a->Nd <= 32 ? (a->Nd == 30 ? 16.0 : 48.0) : (lanes_idle ? (slots == 64 ? 24.0 : 11.0) : 64.0);
-    const bool pays = a->Nd % 2 ? uses >= (a->Nd <= 256 ? 8.0 : 24.0) && gather >= 64e6 && (a->Nd >= 32 || mean <= 64.0)
-                                : uses >= even_uses && gather >= 250e6 && (a->Nd <= 32 || lanes_idle || a->Nd >= 96);
+    const bool pays = a->Nd % 2 ? odd_copy_pays(a->Nd, mean, uses, gather) : even_copy_pays(a->M, a->Nd, mean, uses, gather);
     return pays ? align_up((size_t)a->Kd * (size_t)((a->Nd + 3) / 4) * 16, 256) : 0;
 }
 

@@ -72,16 +72,18 @@ size_t worst_case_workspace(const csrspmm_b200_args* a);
 
 // Scratch for a copy of B with rows padded to whole 16-byte vectors, or 0 where the product does without.  Rows of
 // 57 or 150 columns start on any 4 or 8 bytes, and gathered one or two floats per lane they come at half the rate; a copy
-// costs B read and written once, which eight uses of each row repay for odd widths (200 000 rows of 8, 19 columns 68 -> 37
-// us, 57 columns 81 -> 71; 20 000 rows of 24, 201 columns 61 -> 35; wider than 256 from 24 on: 200 000 of 8, 323 columns
-// 430 and 445).  Even widths, whose rows of C are written in pairs, gain where their pairs leave lanes idle, from eleven uses on
-// (300 000 even rows of 10 over 200 000, 50 columns 120 -> 97; 300 000 Zipf rows of 12, 130 columns 430 -> 373; 100 000 of
-// 12, 150 columns 111 -> 100; with 59 of 64 lanes at work 33.9 and 35.5, with 31 of 32 87.6 and 87.3), of which 66 to 108
-// columns have two pairs per lane already and need 24 (90 columns, 30 uses 82 -> 78; 98, 12 uses 31.9 and 35.1); up to 32 columns
-// 30 from 16 on, eight whole vectors (500 000 of 14 142 -> 122), the others from 48 (22 columns, 150 uses 47 -> 41; 26, 30
-// uses 59 and 60); the rest from 64 uses on (20 000 of 100, 510 columns 260 -> 240).  Below 64 MB of gather (250 for even widths: 50 columns, 220 MB 45.6 and 45.9) the launch costs more
-// than it gives, and long rows of few columns leave too few lane groups when they are cut to vectors (20 000 of 100, 19
-// columns 30 -> 35).
+// costs B read and written once, and a launch.
+// Odd widths: from eight uses of each row of B on (200 000 rows of 8, 19 columns 68 -> 37 us, 57 columns 81 -> 71; 20 000 rows of 24, 201
+// columns 61 -> 35; wider than 256 from 24 on: 200 000 of 8, 323 columns 430 and 445) and 64 MB of gather; long rows of few columns leave
+// too few lane groups when they are cut to vectors (20 000 of 100, 19 columns 30 -> 35).  Over 360 products of both sides 1.33.
+// Even widths, whose rows of C are written in pairs.  Both sides measured on 1270 products, 18 to 510 columns, 6 to 250 uses, 0.2 to 5
+// GB of gather, even and Zipf rows (time without the copy over time with it; mean, range, and the share that loses 2 % and more):
+//   up to 32 columns, 48 uses (30 columns, eight whole vectors: 16): 1.11, 0.87-1.52, 6 %.  Not the rows of over 64 entries that fill one wave of
+//     eight-lane groups and leave half of the next one empty (19 010 of 370, 22 columns 81 and 102)
+//   pairs that leave lanes of a group idle: 34 to 54 columns, 24 uses 1.15, 0.87-1.51, 2 % (11 to 24 uses 1.04, 0.92-1.26, 28 %: 50 columns, 15 uses 761
+//     and 825); 66 to 108, 24 uses 1.11, 0.92-1.36, 6 %; 130 to 216, 11 uses 1.17, 0.90-1.54, 6 %
+//   other widths from 96 on, 64 uses: up to 256 1.07, 0.89-1.30, 15 %, beyond 1.16, 0.85-1.52, 5 %
+// Below 250 MB of gather the launch costs more than it gives (50 columns, 220 MB 45.6 and 45.9).
 size_t padded_b_bytes(const csrspmm_b200_args* a);
 
 void set_last_error(const char* fmt, ...);

@@ -27,3 +27,15 @@ def test_plan_info_says_what_runs(sizes, longest, with_room, without):
         assert got == dict(dict(launches=1, padded_copy=False, resident_lanes=0, row_aligned=False), **want)
     assert ops.selected_kernel(*sizes, max_row_nnz=longest) == with_room["kernel"]
     assert ops.plan_info(0, 5, 64, 0)["launches"] == 0
+
+
+# even widths: a padded copy of B only where it was measured to pay
+@pytest.mark.parametrize("M,Kd,Nd,mean,want", [
+    (80_910, 56_130, 30, 157, True), (308_165, 350_025, 30, 15, False), (100_000, 60_000, 26, 29, True), (100_000, 60_500, 26, 29, False),
+    (18_944, 10_000, 22, 370, True), (18_945, 58_783, 22, 370, False), (28_416, 58_783, 22, 370, False), (28_417, 58_783, 22, 370, True),  # waves
+    (60_000, 26_000, 22, 64, True), (150_000, 75_000, 50, 12, True), (253_847, 293_193, 54, 22, False),
+    (489_723, 1_227_653, 50, 37, False), (200_000, 100_000, 66, 12, True), (200_000, 101_000, 66, 12, False), (60_773, 4886, 138, 15, True),
+    (100_000, 100_000, 150, 12, True), (200_000, 200_000, 150, 10, False), (170_295, 18_568, 254, 20, True), (7911, 8319, 370, 130, True),
+    (100_000, 40_000, 62, 100, False), (100_000, 40_000, 118, 20, False)])
+def test_copies_of_even_widths(M, Kd, Nd, mean, want):
+    assert ops.plan_info(M, Kd, Nd, M * mean, max_row_nnz=0)["padded_copy"] == want
