@@ -14,11 +14,12 @@ namespace csrspmm_b200 {
 namespace {
 
 // A build with a column guard, with stores for a padded B's rows of C where that is what runs.
-template <int G, int NV, int VW, int TG, int U, int FMT>
+template <int G, int NV, int VW, int TG, int U, int FMT, bool PAIRS = VW == 4>
 cudaError_t launch_guarded(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
-    if (VW == 4 && plan.c_ragged == kRaggedPairs)
-        return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, VW == 4 ? kRaggedPairs : 0>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
+    if constexpr (PAIRS)
+        if (plan.c_ragged == kRaggedPairs)
+            return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, kRaggedPairs>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
     if (VW == 4 && plan.c_ragged == kRaggedFloats)
         return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false, false, VW == 4 ? kRaggedFloats : 0>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
     return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, (unsigned)plan.grid, kMergeThreads, 0, st, p);
@@ -40,23 +41,28 @@ cudaError_t launch_merge(const SpmmParams& p, const Plan& plan, cudaStream_t st)
         if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, ULONG, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
         return launch_guarded<G, NV, VW, TG, ULONG, FMT>(p, plan, st);
     }
-    if (plan.small_tile) {  // few items: smaller tiles, more CTAs
+    // Few items: smaller tiles, more CTAs.  A copy of B of even width is made for so many entries (padded_b_bytes) that only the
+    // first and the last shape can have small tiles on one.
+    constexpr bool kSmallPairs = VW == 4 && (S == 0 || S == 4);
+    if (plan.small_tile && (kSmallPairs || plan.c_ragged != kRaggedPairs)) {
         if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TGS, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
-        return launch_guarded<G, NV, VW, TGS, U, FMT>(p, plan, st);
+        return launch_guarded<G, NV, VW, TGS, U, FMT, kSmallPairs>(p, plan, st);
     }
     if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
     return launch_guarded<G, NV, VW, TG, U, FMT>(p, plan, st);
 }
 
-// very narrow dense operands: lane groups of 1, 2 or 4 lanes (kNarrowShapes)
+// Very narrow dense operands: lane groups of 1, 2 or 4 lanes (kNarrowShapes).  No padded copy is this narrow, and with 16-byte
+// vectors one or two lanes have a column each; only three vectors leave a lane idle.
 template <int K, int VW, int FMT>
 cudaError_t launch_merge_narrow(const SpmmParams& p, const Plan& plan, cudaStream_t st)
 {
     constexpr int G = kNarrowShapes[K].G, NV = kNarrowShapes[K].NV, TG = kNarrowShapes[K].TG;
     constexpr int U = merge_unroll(VW, NV);
     const unsigned grid = (unsigned)plan.grid;
-    if (VW == 4 && plan.full) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
-    return launch_guarded<G, NV, VW, TG, U, FMT>(p, plan, st);
+    if (VW == 4 && (G < 4 || plan.full)) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, (VW == 4)>, grid, kMergeThreads, 0, st, p);
+    if constexpr (VW != 4 || G == 4) return launch_overlapped(spmm_merge_kernel<G, NV, VW, TG, U, FMT, false>, grid, kMergeThreads, 0, st, p);
+    return cudaErrorInvalidValue;
 }
 
 template <int VW, int FMT>

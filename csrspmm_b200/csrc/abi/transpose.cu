@@ -121,6 +121,7 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
     auto ints = [&](size_t off) { return reinterpret_cast<int*>(ws + off); };
     auto pairs = [&](size_t off) { return reinterpret_cast<int2*>(ws + off); };
     long long* results = reinterpret_cast<long long*>(ws + p.results);
+    constexpr bool kCanSelf = ITEMS == 8;  // sixteen entries per thread are for more tiles than that (plan_transpose)
     for (int k = 0; k < p.passes; ++k) {
         const DigitPass ps = {k * p.digit_bits, 1 << p.digit_bits, p.tiles, nnz};
         const bool first = k == 0, last = k == p.passes - 1;
@@ -128,8 +129,8 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
         const int2* in = first ? nullptr : pairs(p.pairs[(k - 1) & 1]);
         int* out_keys = last ? ints(p.keys) : ints(p.buffer[k & 1]);
         int2* out = last ? nullptr : pairs(p.pairs[k & 1]);
-        const bool self = p.tiles <= kSelfTiles;
-        cudaError_t e = launch_overlapped(self ? transpose_count_kernel<ITEMS, true> : transpose_count_kernel<ITEMS, false>, (unsigned)p.tiles,
+        const bool self = kCanSelf && p.tiles <= kSelfTiles;
+        cudaError_t e = launch_overlapped(self ? transpose_count_kernel<ITEMS, kCanSelf> : transpose_count_kernel<ITEMS, false>, (unsigned)p.tiles,
                                           kTransposeThreads, 0, st, ps, keys, Kd, ints(p.counts));
         if (e == cudaSuccess && !self) e = exclusive_scan(ints(p.counts), p.counters, ints(p.offsets), ws + p.scan, results, st);
         if (e != cudaSuccess) return e;
@@ -142,7 +143,9 @@ cudaError_t run_transpose(const TransposePlan& p, int32_t M, int32_t Kd, int64_t
         };
         using T = std::true_type;
         using F = std::false_type;
-        auto pick = [&](auto first_c, auto last_c) { return self ? scatter(first_c, last_c, T()) : scatter(first_c, last_c, F()); };
+        auto pick = [&](auto first_c, auto last_c) {
+            return self ? scatter(first_c, last_c, std::bool_constant<kCanSelf>()) : scatter(first_c, last_c, F());
+        };
         e = first && last ? pick(T(), T()) : first ? pick(T(), F()) : last ? pick(F(), T()) : pick(F(), F());
         if (e != cudaSuccess) return e;
     }
