@@ -92,8 +92,8 @@ def _scale(L, keep):
     return L.csrspmm_b200_e2m1_scale_device(C.c_int64(5000), C.c_void_p(v.ctypes.data), C.byref(C.c_float()), None)
 
 
-def _transpose(L, keep):
-    M, Kd, n = 3000, 70_000, 300_000  # three passes, with the scan
+def _transpose(L, keep, Kd=70_000):  # through buckets
+    M, n = 3000, 300_000
     if not keep:
         keep["csr"] = _csr(M, Kd, 100)
         keep["out"] = np.zeros(Kd + 1, np.int32), np.zeros(n, np.int32), np.zeros(n, np.float32)
@@ -105,11 +105,15 @@ def _transpose(L, keep):
                                     C.c_size_t(keep["bytes"]), None)
 
 
+def _transpose_digits(L, keep):
+    return _transpose(L, keep, 600_000)  # three passes, with the scan
+
+
 # the entry points that lend host memory to the GPU (the caller's operands, page-locked words that the next call gets), and
 # the others, which read results back by copies to pageable memory, complete when the copy returns
 LENDING = {"schedule": _schedule, "host_blocks": _host_blocks, "host_panels": _host_panels, "row_stats": _row_stats, "dense2csr": _dense2csr,
            "quantize": _quantize, "bounds": _bounds}
-CALLS = dict(LENDING, spmm=_spmm, tiled=_tiled, transpose=_transpose, validate=_validate, scale=_scale)
+CALLS = dict(LENDING, spmm=_spmm, tiled=_tiled, transpose=_transpose, transpose_digits=_transpose_digits, validate=_validate, scale=_scale)
 
 
 @pytest.mark.parametrize("name", sorted(CALLS))
@@ -133,11 +137,11 @@ def test_one_failed_call(fake, name):
 
 def test_shared_memory_is_asked_for_once(fake):
     fake.fake_reset(0)
-    keep = {}
+    keep, digits = {}, {}
     for _ in range(2):
-        assert _transpose(fake, keep) == 0
+        assert _transpose(fake, keep) == 0 and _transpose_digits(fake, digits) == 0
     before = fake.fake_settings()
-    assert before > 0 and _transpose(fake, keep) == 0 and fake.fake_settings() == before
+    assert before > 0 and _transpose(fake, keep) == 0 and _transpose_digits(fake, digits) == 0 and fake.fake_settings() == before
     assert fake.fake_refused() == 0  # and no launch, in any test so far, took more than it had asked for
 
 

@@ -6,6 +6,8 @@ import re
 import pytest
 
 from csrspmm_b200 import _lib, build
+from test_failed_cuda_calls import CALLS
+from test_gpu_transpose import BUCKETS, DIGITS, SIZES
 
 
 @pytest.fixture(scope="module")
@@ -73,3 +75,27 @@ def test_nothing_is_compiled_that_no_call_launches(fake):
     for nnz, bits in itertools.product((1, 3000, 9000, 100_000, 1_000_000, 1_900_000, 6_000_000), range(1, 27)):
         assert _transpose(fake, 1000, 1 << bits, nnz) == 0
     assert sorted(every - _names(fake.fake_launched)) == []
+
+
+def test_gpu_tests_run_every_kernel_of_the_transposition(fake):
+    fake.fake_reset(0)
+    for M, Kd, nnz, _ in (*SIZES, *BUCKETS, *DIGITS):
+        assert _transpose(fake, M, Kd, nnz) == 0
+    assert sorted({k for k in _names(fake.fake_kernels) if "transpose_" in k} - _names(fake.fake_launched)) == []
+
+
+@pytest.mark.parametrize("size", DIGITS)
+def test_sizes_of_the_digit_passes_take_them(fake, size):
+    fake.fake_reset(0)
+    assert _transpose(fake, *size[:3]) == 0
+    launched = _names(fake.fake_launched)
+    assert any("transpose_scatter_kernel" in k for k in launched) and not any("bucket" in k for k in launched)
+
+
+def test_failed_calls_of_the_transposition_take_both_ways(fake):
+    for name, kernels in (("transpose", ("bucket_count", "bucket_offsets", "bucket_scatter", "chunk_count", "bucket_sort")),
+                          ("transpose_digits", ("transpose_count", "transpose_scatter", "scan_tiles", "scan_finish", "row_ptr"))):
+        fake.fake_reset(0)
+        assert CALLS[name](fake, {}) == 0
+        launched = _names(fake.fake_launched)
+        assert all(any(k in full for full in launched) for k in kernels), (name, launched)
