@@ -37,7 +37,7 @@ CSR_BAD_ROWPTR0, CSR_BAD_ROWPTR_END, CSR_NOT_MONOTONE, CSR_COL_RANGE, CSR_COL_UN
 EXPORTED_SYMBOLS = (
     "csrspmm_b200_abi_version", "csrspmm_b200_status_string", "csrspmm_b200_last_error",
     "csrspmm_b200_spmm", "csrspmm_b200_spmm_sync", "csrspmm_b200_spmm_host", "csrspmm_b200_spmm_noalloc",
-    "csrspmm_b200_host_arena_bytes", "csrspmm_b200_workspace_bytes", "csrspmm_b200_uses_workspace", "csrspmm_b200_select_kernel",
+    "csrspmm_b200_host_arena_bytes", "csrspmm_b200_workspace_bytes", "csrspmm_b200_least_workspace_bytes", "csrspmm_b200_uses_workspace", "csrspmm_b200_select_kernel",
     "csrspmm_b200_plan_info_get", "csrspmm_b200_release_memory", "csrspmm_b200_check_bounds_device",
     "csrspmm_b200_validate_csr_host", "csrspmm_b200_validate_csr_device",
     "csrspmm_b200_row_stats_device", "csrspmm_b200_partition_rows", "csrspmm_b200_e2m1_scale",
@@ -158,6 +158,8 @@ def lib() -> C.CDLL:
     L.csrspmm_b200_host_arena_bytes.restype = C.c_size_t
     L.csrspmm_b200_workspace_bytes.argtypes = [C.POINTER(Args)]
     L.csrspmm_b200_workspace_bytes.restype = C.c_size_t
+    L.csrspmm_b200_least_workspace_bytes.argtypes = [C.POINTER(Args)]
+    L.csrspmm_b200_least_workspace_bytes.restype = C.c_size_t
     L.csrspmm_b200_uses_workspace.argtypes = [C.POINTER(Args)]
     L.csrspmm_b200_uses_workspace.restype = C.c_int
     L.csrspmm_b200_select_kernel.argtypes = [C.POINTER(Args)]

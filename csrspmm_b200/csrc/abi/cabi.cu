@@ -560,6 +560,13 @@ size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args)
     return check_args(args, false) == CSRSPMM_B200_OK ? align256(worst_case_workspace(args)) + padded_b_bytes(args) : 0;
 }
 
+size_t csrspmm_b200_least_workspace_bytes(const csrspmm_b200_args* args)
+{
+    Plan plan;
+    if (make_plan(args, &plan) != CSRSPMM_B200_OK) return 0;
+    return schedule_applies(args) ? scheduled_workspace_bytes(args) : plan.workspace_bytes;
+}
+
 int csrspmm_b200_select_kernel(const csrspmm_b200_args* args)
 {
     Plan plan;

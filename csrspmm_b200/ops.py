@@ -222,9 +222,10 @@ class SpmmCall:
             if uses > 0:
                 need = int(self.L.csrspmm_b200_workspace_bytes(C.byref(self.args)))
                 if workspace is None or workspace.numel() * workspace.element_size() < need:
-                    workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=B.device)
-                self.args.workspace = workspace.data_ptr()
-                self.args.workspace_bytes = workspace.numel() * workspace.element_size()
+                    workspace = self._workspace(need, workspace)
+                if workspace is not None:
+                    self.args.workspace = workspace.data_ptr()
+                    self.args.workspace_bytes = workspace.numel() * workspace.element_size()
             plan = _plan_info(self.args)
             self.kernel, self.launches = plan["kernel"], plan["launches"]
         # scratch of the split kernels and of a padded copy of B (None where neither runs); may be shared by calls on one stream
@@ -233,6 +234,16 @@ class SpmmCall:
         self._enqueue = _lib.binding().enqueue
         self._where = (C.addressof(self.args), B.device.index)
         self.out = C_out
+
+    def _workspace(self, need: int, given):
+        """``need`` bytes, or, where memory has no room for a copy of B, what the product without one takes."""
+        try:
+            return torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
+        except torch.OutOfMemoryError:
+            least = int(self.L.csrspmm_b200_least_workspace_bytes(C.byref(self.args)))
+            if least == 0 or (given is not None and given.numel() * given.element_size() >= least):
+                return given
+            return torch.empty(max(least, 256), dtype=torch.uint8, device=self.device)
 
     def __call__(self):
         """Enqueue on the current stream of the operands' device (which must be the current device)."""

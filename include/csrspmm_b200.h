@@ -204,6 +204,10 @@ int csrspmm_b200_spmm_tiled(const csrspmm_b200_args* args, int32_t panel_rows, c
  * on sizes, never on matrix contents. */
 size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args);
 
+/* What of it the product cannot do without: the carries of the kernel that runs when there is no copy of B, 0 for a
+ * kernel without any.  A workspace of this size is what a caller falls back on where memory for the other is not to be had. */
+size_t csrspmm_b200_least_workspace_bytes(const csrspmm_b200_args* args);
+
 /* 1 when a product with these arguments makes use of args.workspace, 0 when it does not, or a negative
  * csrspmm_b200_status.  Host-only logic. */
 int csrspmm_b200_uses_workspace(const csrspmm_b200_args* args);

@@ -1,0 +1,47 @@
+"""Scratch that only makes a call faster (a padded copy of B, a bit per element of a matrix) where memory has no room for it: the
+call does without.  The limit is torch's own, on what this process takes."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from csrspmm_b200 import generators as G, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def limit_memory(cuda_lib):
+    """limit(n): n bytes more than what torch holds now."""
+    def limit(more):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + more) / torch.cuda.get_device_properties(0).total_memory)
+    yield limit
+    torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def _problem(skew):
+    M, Kd, Nd = 180_000, 150_000, 50  # a copy of B is 31 MB, more than what torch keeps free behind smaller tensors
+    lens = np.random.default_rng(3).integers(20, 29, M)
+    if skew:
+        lens[7] = 30_000
+    p = G.random_csr(M, Kd, Nd, 0.0, seed=3, lengths=lens)
+    t = [torch.from_numpy(x).cuda() for x in (p.row_ptr, p.col_idx, p.values, p.B)]
+    f64, mag = oracle.spmm_f64(p.row_ptr, p.col_idx, p.values, p.B, threads=4)
+    longest = 0 if skew else int(lens.max())
+    assert ops.plan_info(M, Kd, Nd, p.nnz, max_row_nnz=longest)["padded_copy"]
+    return p, t, longest, lambda C: bool((np.abs(C.cpu().numpy() - f64) <= 1e-5 * mag + 1e-6).all())
+
+
+@pytest.mark.parametrize("skew", [False, True])
+@pytest.mark.parametrize("given", [0, 256, 8 << 20])
+def test_prepared_call(limit_memory, skew, given):
+    p, t, longest, right = _problem(skew)
+    out = torch.empty((p.M, p.Nd), device="cuda")
+    workspace = torch.empty(given, dtype=torch.uint8, device="cuda") if given else None
+    limit_memory(6 << 20)
+    call = ops.SpmmCall(*t, out, max_row_nnz=longest, workspace=workspace)
+    want = ops.plan_info(p.M, p.Kd, p.Nd, p.nnz, max_row_nnz=longest, workspace=False)
+    assert (call.kernel, call.launches) == (want["kernel"], want["launches"]) and want["kernel"] == ("merge" if skew else "row")
+    assert right(call())

@@ -266,3 +266,19 @@ def test_copy_rows_rejects_bad_arguments_before_any_cuda_call():
     assert L.csrspmm_b200_copy_rows(None, 16, buf.ctypes.data, 16, 16, 4, 0, None) == _lib.ERR_BAD_ARG
     assert L.csrspmm_b200_copy_rows(buf.ctypes.data, 8, buf.ctypes.data, 16, 16, 4, 0, None) == _lib.ERR_BAD_ARG
     assert L.csrspmm_b200_copy_rows(None, 0, None, 0, 0, 4, 0, None) == _lib.OK  # nothing to copy
+
+
+def test_least_workspace_is_enough_without_a_copy():
+    L = _lib.lib()
+    for M, Kd, Nd, nnz, longest in [(60_000, 50_000, 50, 1_440_000, 0), (60_000, 50_000, 50, 1_440_000, 28), (20_000, 20_000, 201, 480_000, 0),
+                                    (4096, 4096, 128, 1_600_000, 0), (1000, 1000, 64, 5000, 8)]:
+        a = _lib.make_args(M, Kd, Nd, nnz, B=256, Cptr=256, max_row_nnz=longest)
+        least = L.csrspmm_b200_least_workspace_bytes(C.byref(a))
+        assert least <= L.csrspmm_b200_workspace_bytes(C.byref(a))
+        without = ops.plan_info(M, Kd, Nd, nnz, max_row_nnz=longest, workspace=False)
+        assert (least > 0) == (without["kernel"] != "row")
+        a.workspace, a.workspace_bytes = 256, least
+        info = _lib.PlanInfo()
+        info.struct_size = C.sizeof(info)
+        assert L.csrspmm_b200_plan_info_get(C.byref(a), C.byref(info)) == 0 and info.padded_copy == 0 and info.launches == without["launches"]
+    assert L.csrspmm_b200_least_workspace_bytes(None) == 0
