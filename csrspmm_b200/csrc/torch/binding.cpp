@@ -26,7 +26,9 @@
 #include <torch/library.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdint>
+#include <mutex>
 #include <optional>
 
 #include "csrspmm_b200.h"
@@ -38,6 +40,7 @@ struct Library {
     int (*spmm_sync)(const csrspmm_b200_args*, csrspmm_b200_stream_t);
     int (*uses_workspace)(const csrspmm_b200_args*);
     size_t (*workspace_bytes)(const csrspmm_b200_args*);
+    size_t (*least_workspace_bytes)(const csrspmm_b200_args*);
     int (*row_stats)(int32_t, const int32_t*, int64_t*, csrspmm_b200_stream_t);
     size_t (*dense2csr_mask_bytes)(int32_t, int32_t);
     int (*dense2csr_count)(int32_t, int32_t, const float*, int64_t, float, int32_t*, uint32_t*, int64_t*, int32_t*, csrspmm_b200_stream_t);
@@ -138,10 +141,76 @@ public:
         ptr_ = c10::cuda::CUDACachingAllocator::raw_alloc_with_stream(std::max<size_t>(bytes, 256), stream);
         return ptr_;
     }
+    // For scratch that only makes a call faster: null where memory has no room for it.
+    void* get_if_room(size_t bytes, c10::cuda::CUDAStream stream)
+    {
+        namespace Allocator = c10::cuda::CUDACachingAllocator;
+        const c10::DeviceIndex device = stream.device_index();
+        int64_t active = -1;
+        try {
+            const auto stats = Allocator::getDeviceStats(device);
+            active = stats.active_bytes[0].current;
+            const int64_t reserved = stats.reserved_bytes[0].current;
+            if (reserved - active < (int64_t)bytes) {  // not in torch's free blocks: what may it take, and what is there?
+                if (Full::known(device, bytes, active)) return nullptr;
+                constexpr int64_t kSegment = 2 << 20;  // what torch rounds larger allocations up to
+                const int64_t want = ((int64_t)bytes + kSegment - 1) / kSegment * kSegment;
+                size_t there = 0, total = 0;
+                C10_CUDA_CHECK(cudaMemGetInfo(&there, &total));
+                const int64_t allowed = (int64_t)(Allocator::getMemoryFraction(device) * (double)total) - reserved;
+                if (reserved - active + std::min((int64_t)there, allowed) < want) {
+                    Full::note(device, bytes, active);
+                    return nullptr;
+                }
+            }
+        } catch (const c10::Error&) {  // an allocator that does not tell
+        }
+        try {
+            return get(bytes, stream);
+        } catch (const c10::OutOfMemoryError&) {
+            if (active >= 0) Full::note(device, bytes, active);
+            return nullptr;
+        }
+    }
 
 private:
+    // Where there was no room for so many bytes a moment ago, with no more in use than now.  An allocation that fails makes torch
+    // give all its free blocks back to the driver first, and asking the driver takes 200 us a time (200 000 rows of 24, 50 columns,
+    // 101 us without the copy: 237 and 535 us a call), so a program that lives with full memory pays for one of them once a second.
+    class Full {
+    public:
+        static bool known(c10::DeviceIndex device, size_t bytes, int64_t active)
+        {
+            if (device < 0 || device >= kDevices) return false;
+            const std::lock_guard<std::mutex> lock(mutex_);
+            const Full& f = full_[device];
+            return bytes >= f.bytes_ && active >= f.active_ && Clock::now() < f.until_;
+        }
+        static void note(c10::DeviceIndex device, size_t bytes, int64_t active)
+        {
+            if (device < 0 || device >= kDevices) return;
+            const std::lock_guard<std::mutex> lock(mutex_);
+            Full& f = full_[device];
+            const auto now = Clock::now();
+            const bool fresh = now < f.until_;
+            f.bytes_ = fresh ? std::min(f.bytes_, bytes) : bytes;
+            f.active_ = fresh ? std::min(f.active_, active) : active;
+            f.until_ = now + std::chrono::seconds(1);
+        }
+
+    private:
+        using Clock = std::chrono::steady_clock;
+        static constexpr int kDevices = 64;
+        static inline std::mutex mutex_;
+        static Full full_[kDevices];
+        size_t bytes_ = 0;
+        int64_t active_ = 0;
+        Clock::time_point until_ = {};
+    };
+
     void* ptr_ = nullptr;
 };
+Scratch::Full Scratch::Full::full_[kDevices];
 
 struct Product {
     at::Tensor rp, ci, va, B, C;  // C undefined: allocate it
@@ -205,19 +274,30 @@ at::Tensor run_product(Product& q)
         if (uses < 0) throw LibraryError{-uses, "csrspmm_b200_select_kernel"};
         if (uses > 0) {
             const size_t need = g_lib.workspace_bytes(&a);
-            if (q.workspace.defined() && q.workspace.nbytes() >= need) {
+            const size_t given = q.workspace.defined() ? q.workspace.nbytes() : 0;
+            const auto use_given = [&] {
                 a.workspace = q.workspace.data_ptr();
-                a.workspace_bytes = q.workspace.nbytes();
+                a.workspace_bytes = given;
                 if (q.workspace.is_cuda()) c10::cuda::CUDACachingAllocator::recordStream(q.workspace.storage().data_ptr(), stream);
-            } else {
-                try {
-                    a.workspace = scratch.get(need, stream);
-                    a.workspace_bytes = std::max<size_t>(need, 256);
-                } catch (const c10::OutOfMemoryError&) {
-                    // no room for a padded copy of B: without a workspace the library does without the copy
-                    a.workspace = nullptr;
-                    a.workspace_bytes = 0;
+            };
+            const auto take = [&](void* memory, size_t bytes) {
+                a.workspace = memory;
+                a.workspace_bytes = std::max<size_t>(bytes, 256);
+                return memory != nullptr;
+            };
+            const bool with_copy = Nd % 4 != 0 && need > (size_t)Kd * (size_t)Nd * 4;  // of B, which the product can do without
+            try {
+                if (given >= need) {
+                    use_given();
+                } else if (!with_copy) {
+                    take(scratch.get(need, stream), need);
+                } else if (!take(scratch.get_if_room(need, stream), need)) {
+                    const size_t least = g_lib.least_workspace_bytes(&a);
+                    if (given >= least && given > 0) use_given();
+                    else if (least > 0) take(scratch.get(least, stream), least);
                 }
+            } catch (const c10::OutOfMemoryError&) {
+                a.workspace = nullptr;  // the library's own pool may have it
             }
         }
     }
@@ -326,6 +406,7 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     fill(g_lib.spmm_sync, "spmm_sync");
     fill(g_lib.uses_workspace, "uses_workspace");
     fill(g_lib.workspace_bytes, "workspace_bytes");
+    fill(g_lib.least_workspace_bytes, "least_workspace_bytes");
     fill(g_lib.row_stats, "row_stats_device");
     fill(g_lib.dense2csr_mask_bytes, "dense2csr_mask_bytes");
     fill(g_lib.dense2csr_count, "dense2csr_count_mask");
@@ -440,12 +521,8 @@ PyObject* py_dense2csr(PyObject*, PyObject* const* args, Py_ssize_t nargs)
         const auto stream = current_stream(device);
         const float* data = address<float>(dense);
         Scratch scratch;
-        uint32_t* mask = nullptr;
-        try {
-            mask = static_cast<uint32_t*>(
-                scratch.get(g_lib.dense2csr_mask_bytes((int32_t)H, (int32_t)W), c10::cuda::getCurrentCUDAStream(device.index())));
-        } catch (const c10::OutOfMemoryError&) {  // a bit per element more than the matrix: do without
-        }
+        const size_t mask_bytes = g_lib.dense2csr_mask_bytes((int32_t)H, (int32_t)W);  // a bit per element, or without
+        uint32_t* const mask = static_cast<uint32_t*>(scratch.get_if_room(mask_bytes, c10::cuda::getCurrentCUDAStream(device.index())));
         check(g_lib.dense2csr_count((int32_t)H, (int32_t)W, data, ld, tol, address<int32_t>(rp), mask, &nnz, &longest, stream),
               "csrspmm_b200_dense2csr_count");
         ci = new_array(nnz, at::kInt, device);

@@ -45,3 +45,44 @@ def test_prepared_call(limit_memory, skew, given):
     want = ops.plan_info(p.M, p.Kd, p.Nd, p.nnz, max_row_nnz=longest, workspace=False)
     assert (call.kernel, call.launches) == (want["kernel"], want["launches"]) and want["kernel"] == ("merge" if skew else "row")
     assert right(call())
+
+
+def _retries():
+    return torch.cuda.memory_stats()["num_alloc_retries"]
+
+
+@pytest.mark.parametrize("skew", [False, True])
+@pytest.mark.parametrize("given", [0, 8 << 20])
+def test_product_without_room(limit_memory, skew, given):
+    """... and does not make torch give its free blocks back to find that out, call after call."""
+    p, t, longest, right = _problem(skew)
+    out = torch.empty((p.M, p.Nd), device="cuda")
+    workspace = torch.empty(given, dtype=torch.uint8, device="cuda") if given else None
+    limit_memory(6 << 20)
+    before = _retries()
+    for _ in range(5):
+        out.zero_()
+        ops.spmm(*t, out, max_row_nnz=longest, workspace=workspace)
+        assert right(out)
+    assert _retries() == before
+
+
+def test_product_with_just_enough_room(limit_memory):
+    p, t, longest, right = _problem(False)
+    out = torch.empty((p.M, p.Nd), device="cuda")
+    limit_memory(64 << 20)
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    ops.spmm(*t, out, max_row_nnz=longest)
+    assert right(out) and torch.cuda.max_memory_allocated() >= held + p.Kd * 208  # the copy was made
+
+
+def test_conversion_without_room(limit_memory):
+    dense = torch.zeros((4096, 24_576), device="cuda")  # its bits: 12.6 MB
+    dense.view(-1)[::1009] = 1.5
+    want = ops.dense2csr(dense)
+    limit_memory(6 << 20)
+    before = _retries()
+    for _ in range(3):
+        got = ops.dense2csr(dense)
+    assert _retries() == before and got[3] == want[3] and all(torch.equal(a, b) for a, b in zip(got[:3], want[:3]))
