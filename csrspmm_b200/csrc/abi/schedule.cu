@@ -70,7 +70,8 @@ int env_int(const char* name)
 }
 
 // Slab of B that should stay in L2 while its pieces run.  The 126 MB of L2 are two partitions, one per die, and
-// a line that SMs of both dies read is held in both (tests/cpp/l2_partition_probe.cu measures it), so a slab
+// a line that SMs of both dies read is held in both (its atomics take 305 cycles from one die and 694 from the other, its
+// loads some 300 from either once it has been read there), so a slab
 // of 64 MiB that every SM gathers from fills the L2 about once over, next to the streams of A and the slots;
 // the pieces kernel then reads B from HBM about twice (once per die).  Smaller slabs are read once but cut
 // the rows into more pieces, each with a slot of its own; measured on config 5 (rows of B of 2 KB), persistent
