@@ -183,6 +183,12 @@ static bool rows_are_chains(long long M, double mean, const Plan& plan)
     return s.G == 32 ? M < 592 && mean >= (s.NV == 1 ? 80.0 : 200.0) : M <= 2400 && mean >= 80.0;
 }
 
+// Whether the longest row is known and close to the mean.
+static bool rows_known_even(const csrspmm_b200_args* a, double mean)
+{
+    return a->max_row_nnz > 0 && (double)a->max_row_nnz <= (mean * 4.0 > 64.0 ? mean * 4.0 : 64.0);
+}
+
 int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
 {
     const bool coarse = (flags & kPlanCoarse) != 0;
@@ -218,9 +224,8 @@ int make_plan(const csrspmm_b200_args* a, Plan* plan, unsigned flags)
         // of 128 columns: 773 against 745; 32 of 256: 1012 either way; 143 of 56: 703 against 601).  Everything else (unknown or skewed row lengths) takes
         // the merge kernel.  The entry point asked for does not change the choice.
         const double avg = a->M > 0 ? (double)a->nnz / (double)a->M : 0.0;
-        const double row_limit = avg * 4.0 > 64.0 ? avg * 4.0 : 64.0;
         const double b_bytes = (double)a->Kd * (double)a->Nd * 4.0;
-        const bool rows_even = a->max_row_nnz > 0 && (double)a->max_row_nnz <= row_limit;
+        const bool rows_even = rows_known_even(a, avg);
         plan->rows_even = rows_even;
         if (tma_can_run(a) && a->Nd > 384 && b_bytes >= 1073741824.0 && !rows_even)
             kernel = CSRSPMM_B200_KERNEL_TMA;
@@ -307,7 +312,7 @@ static bool odd_copy_pays(int Nd, double mean, double uses, double gather)
     return uses >= (Nd <= 256 ? 8.0 : 24.0) && gather >= 64e6 && (Nd >= 32 || mean <= 64.0);
 }
 
-static bool even_copy_pays(int M, int Nd, double mean, double uses, double gather)
+static bool even_copy_pays(int M, int Nd, double mean, double uses, double gather, bool rows_even)
 {
     if (gather < 250e6) return false;
     if (Nd <= 32) {
@@ -316,7 +321,7 @@ static bool even_copy_pays(int M, int Nd, double mean, double uses, double gathe
     }
     const int pairs = Nd / 2, slots = pairs <= 32 ? 32 : (pairs <= 64 ? 64 : 128);
     const bool lanes_idle = Nd <= 256 && pairs * 100 <= slots * 85;
-    return lanes_idle ? uses >= (slots == 128 ? 11.0 : 24.0) : uses >= 64.0 && Nd >= 96;
+    return lanes_idle ? uses >= (slots == 128 || (slots == 32 && rows_even) ? 11.0 : 24.0) : uses >= 64.0 && Nd >= 96;
 }
 
 size_t padded_b_bytes(const csrspmm_b200_args* a)
@@ -324,7 +329,7 @@ size_t padded_b_bytes(const csrspmm_b200_args* a)
     if (a->Nd % 4 == 0 || a->Nd < 17 || a->M <= 0 || a->Kd <= 0 || a->kernel == CSRSPMM_B200_KERNEL_TMA || a->nnz > kWholeRowEntries) return 0;
     const double mean = (double)a->nnz / a->M, uses = (double)a->nnz / a->Kd;
     const double gather = (double)a->nnz * a->Nd * 4.0;
-    const bool pays = a->Nd % 2 ? odd_copy_pays(a->Nd, mean, uses, gather) : even_copy_pays(a->M, a->Nd, mean, uses, gather);
+    const bool pays = a->Nd % 2 ? odd_copy_pays(a->Nd, mean, uses, gather) : even_copy_pays(a->M, a->Nd, mean, uses, gather, rows_known_even(a, mean));
     return pays ? align_up((size_t)a->Kd * (size_t)((a->Nd + 3) / 4) * 16, 256) : 0;
 }
 

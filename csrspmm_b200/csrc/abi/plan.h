@@ -80,8 +80,9 @@ size_t worst_case_workspace(const csrspmm_b200_args* a);
 // GB of gather, even and Zipf rows (time without the copy over time with it; mean, range, and the share that loses 2 % and more):
 //   up to 32 columns, 48 uses (30 columns, eight whole vectors: 16): 1.11, 0.87-1.52, 6 %.  Not the rows of over 64 entries that fill one wave of
 //     eight-lane groups and leave half of the next one empty (19 010 of 370, 22 columns 81 and 102)
-//   pairs that leave lanes of a group idle: 34 to 54 columns, 24 uses 1.15, 0.87-1.51, 2 % (11 to 24 uses 1.04, 0.92-1.26, 28 %: 50 columns, 15 uses 761
-//     and 825); 66 to 108, 24 uses 1.11, 0.92-1.36, 6 %; 130 to 216, 11 uses 1.17, 0.90-1.54, 6 %
+//   pairs that leave lanes of a group idle: 34 to 54 columns, 24 uses 1.15, 0.87-1.51, 2 %, and rows known to be even from 11 uses on (11 to
+//     24: even 1.11, 0.94-1.26, 2 of 12: 300 000 of 10 over 200 000, 50 columns 120 -> 97; uneven 0.99, 0.92-1.11, 7 of 20: 50 columns,
+//     15 uses 761 and 825); 66 to 108, 24 uses 1.11, 0.92-1.36, 6 %; 130 to 216, 11 uses 1.17, 0.90-1.54, 6 %
 //   other widths from 96 on, 64 uses: up to 256 1.07, 0.89-1.30, 15 %, beyond 1.16, 0.85-1.52, 5 %
 // Below 250 MB of gather the launch costs more than it gives (50 columns, 220 MB 45.6 and 45.9).
 size_t padded_b_bytes(const csrspmm_b200_args* a);

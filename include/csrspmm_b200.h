@@ -201,7 +201,7 @@ int csrspmm_b200_spmm_tiled(const csrspmm_b200_args* args, int32_t panel_rows, c
 
 /* Scratch for this problem: the split kernels' carries and, for dense widths that are no multiple of four and rows of
  * B used often enough, a padded copy of B (without room for it the product runs on B as it is).  Depends only
- * on sizes, never on matrix contents. */
+ * on sizes and on the longest row given, never on matrix contents. */
 size_t csrspmm_b200_workspace_bytes(const csrspmm_b200_args* args);
 
 /* What of it the product cannot do without: the carries of the kernel that runs when there is no copy of B, 0 for a

@@ -39,3 +39,9 @@ def test_plan_info_says_what_runs(sizes, longest, with_room, without):
     (100_000, 40_000, 62, 100, False), (100_000, 40_000, 118, 20, False)])
 def test_copies_of_even_widths(M, Kd, Nd, mean, want):
     assert ops.plan_info(M, Kd, Nd, M * mean, max_row_nnz=0)["padded_copy"] == want
+
+
+@pytest.mark.parametrize("Nd,mean,longest,want", [(50, 10, 60, True), (50, 10, 0, False), (50, 10, 65, False), (34, 10, 60, True), (50, 7, 60, False),
+                                                  (54, 15, 64, True), (58, 15, 64, False), (66, 15, 64, False)])
+def test_copies_for_even_rows(Nd, mean, longest, want):
+    assert ops.plan_info(300_000, 200_000, Nd, 300_000 * mean, max_row_nnz=longest)["padded_copy"] == want
