@@ -117,7 +117,6 @@ int csrspmm_b200_dense2csr_fill_mask(int32_t H, int32_t W, const float* dense, i
     return CSRSPMM_B200_OK;
 }
 
-
 int csrspmm_b200_csr2dense(int32_t H, int32_t W, const int32_t* row_ptr, const int32_t* col_idx, const float* values,
                            float* dense, int64_t ld, csrspmm_b200_stream_t stream)
 {

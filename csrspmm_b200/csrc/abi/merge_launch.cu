@@ -96,7 +96,7 @@ cudaError_t launch_fixup_kernel(const SpmmParams& p, const Plan& plan, cudaStrea
 {
     const int warps = 256 / 32;
     const unsigned grid = (unsigned)((plan.num_tiles + warps - 1) / warps);
-    if (plan.c_ragged) {  // carries lie column by column: added float by float where C is not aligned
+    if (plan.c_ragged) {  // carries lie column by column, and C is not aligned to their vectors: added float by float (also pairs)
         SpmmParams q = p;
         q.ncolv = p.Nd;
         return launch_overlapped(spmm_fixup_kernel<1>, grid, 256, 0, st, q, (int)plan.num_tiles);

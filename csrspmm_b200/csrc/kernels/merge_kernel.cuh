@@ -122,9 +122,11 @@ struct MergeSmem {
     int tail_row[GROUPS];
     unsigned longbits[TILE / 32 + 1];  // SKIP only: bit k = local row k is left to the scheduled pieces
     alignas(16) float tail[GROUPS][ROWW];
-    // the first row each group finishes, until the others have published their partial sums.  In registers it cost the walk its last
-    // ones: 128 columns, 262 144 Zipf rows 217 -> 214 us, 64 columns 103 -> 101, 24 columns 107 -> 103, 256 columns 167 -> 159;
-    // four vectors per lane have no room for it here, and eight or four bytes per lane no need
+    // The first row each group finishes, until the others have published their partial sums; in registers it cost the walk its last
+    // ones.  Measured with what came at the same time, a padded copy's stores in builds of their own, shares found by votes and 3072
+    // items per tile up to 32 columns: Zipf rows, 112 columns, 262 144 rows of 16 242 -> 227 us, 36 columns, 260 000 121 -> 106, 24 columns,
+    // 100 000 51 -> 33, 100 columns, 500 000 of 20 598 -> 584, 256 columns, 100 000 of 10 103 -> 101; 64 and 128 columns of 262 144 and
+    // more rows of 16 the same.  Four vectors per lane have no room for it here, and eight or four bytes per lane no need.
     static constexpr bool HEADS = VW == 4 && NV <= 2;
     alignas(16) float head[HEADS ? GROUPS : 1][HEADS ? ROWW : 4];
     __device__ __forceinline__ float* tail_of(int g) { return tail[g]; }

@@ -5,9 +5,10 @@
 // keys with a general sort, gathering and counting took 520 us for 1 M entries and 65 536 columns.
 //
 // An entry's key is its column; entries of one column keep their stored order, so the result has ascending
-// rows in each column and is the same on every run (no atomics decide a place).  Matrices of up to some four million
-// entries and 2^19 columns go through buckets (second half of this file); the others take one to four passes over
-// digits of up to eight bits, least significant first.  A pass is three steps:
+// rows in each column and is the same on every run (no atomics decide a place).  Matrices whose buckets are small enough
+// for a CTA each go through buckets (second half of this file): up to 2^19 columns, and up to 4096 entries for each of at most
+// 1024 runs of columns, so 4.2 million entries with 1024 columns and more, 262 144 with 64.  The others take one to four passes
+// over digits of up to eight bits, least significant first.  A pass is three steps:
 //   count    every CTA counts the digits of its tile of entries -> counts[digit][tile]
 //   scan     exclusive scan of the counts in that order (scan_kernels.cuh): where each tile's entries with
 //            each digit begin
@@ -366,7 +367,8 @@ __global__ void __launch_bounds__(256) transpose_row_ptr_search_kernel(int Kd, i
 //   scatter  the tile in bucket order, written out run by run
 //   sort     one CTA per bucket
 // A bucket of more entries than a CTA holds (a hub column) is cut into chunks, a CTA each, whose digits a kernel of
-// its own counts before the sort; without such a bucket that kernel has nothing to do (2.5 us).
+// its own counts before the sort; without such a bucket that kernel has nothing to do (2.5 us).  Up to one chunk of entries there is
+// none, so two launches; up to one tile three (nothing to count across tiles), else five.
 //
 // Measured against the passes (us): 1 M entries and 65 536 columns 68 -> 31, 5 % of them in one column 69 -> 38, all in one 68 -> 54,
 // columns by a power law 67 -> 49; 250 000 entries 50 -> 20; 600 000 and 200 000 columns 80 -> 27; 2 M and 262 144 columns 150 ->
