@@ -15,6 +15,7 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -155,6 +156,7 @@ public:
                 if (Full::known(device, bytes, active)) return nullptr;
                 constexpr int64_t kSegment = 2 << 20;  // what torch rounds larger allocations up to
                 const int64_t want = ((int64_t)bytes + kSegment - 1) / kSegment * kSegment;
+                const c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};  // as torch does where it allocates
                 size_t there = 0, total = 0;
                 C10_CUDA_CHECK(cudaMemGetInfo(&there, &total));
                 const int64_t allowed = (int64_t)(Allocator::getMemoryFraction(device) * (double)total) - reserved;

@@ -1,5 +1,7 @@
 """Scratch that only makes a call faster (a padded copy of B, a bit per element of a matrix) where memory has no room for it: the
 call does without.  The limit is torch's own, on what this process takes."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -75,6 +77,23 @@ def test_product_with_just_enough_room(limit_memory):
     held = torch.cuda.memory_allocated()
     ops.spmm(*t, out, max_row_nnz=longest)
     assert right(out) and torch.cuda.max_memory_allocated() >= held + p.Kd * 208  # the copy was made
+
+
+@pytest.mark.parametrize("more,copied", [(256 << 20, True), (48 << 20, False)])
+def test_captured_product(limit_memory, more, copied):
+    """Into a graph whose pool has nothing yet: with room for the copy of B, and with room for C alone."""
+    p, t, longest, right = _problem(False)
+    ops.spmm(*t, max_row_nnz=longest)  # settings that a capture may not make
+    limit_memory(more)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        out = ops.spmm(*t, max_row_nnz=longest)
+    count = ctypes.c_size_t(0)  # every node of the captured call is a kernel
+    assert ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(count)) == 0
+    assert count.value == ops.plan_info(p.M, p.Kd, p.Nd, p.nnz, max_row_nnz=longest, workspace=copied)["launches"] == 1 + copied
+    out.zero_()
+    graph.replay()
+    assert right(out)
 
 
 def test_conversion_without_room(limit_memory):
