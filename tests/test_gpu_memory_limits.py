@@ -1,6 +1,7 @@
 """Scratch that only makes a call faster (a padded copy of B, a bit per element of a matrix) where memory has no room for it: the
 call does without.  The limit is torch's own, on what this process takes."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -14,12 +15,24 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture
 def limit_memory(cuda_lib):
-    """limit(n): n bytes more than what torch holds now."""
+    """limit(n): n bytes more than what torch holds now, and none of that free."""
+    held = []
+
     def limit(more):
+        set_limit = lambda n: torch.cuda.set_per_process_memory_fraction(n / torch.cuda.get_device_properties(0).total_memory)
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
-        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + more) / torch.cuda.get_device_properties(0).total_memory)
+        set_limit(torch.cuda.memory_reserved())
+        for size in (16 << 20, 2 << 20):
+            try:
+                while True:
+                    held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                pass
+        set_limit(torch.cuda.memory_reserved() + more)
+        time.sleep(1.1)  # the binding remembers for a second that there was no room
     yield limit
+    held.clear()
     torch.cuda.set_per_process_memory_fraction(1.0)
 
 
