@@ -289,7 +289,7 @@ at::Tensor run_product(Product& q)
             };
             const bool with_copy = Nd % 4 != 0 && need > (size_t)Kd * (size_t)Nd * 4;  // of B, which the product can do without
             try {
-                if (given >= need) {
+                if (q.workspace.defined() && given >= need) {
                     use_given();
                 } else if (!with_copy) {
                     take(scratch.get(need, stream), need);
